@@ -12,11 +12,11 @@
 //      the 3x3 hat block and gathers the tile's blocks into the slots of A in a fixed order. Test tiles are coloured
 //      so that no two tiles of one launch share a row slot: the scatter needs no atomics and A is reproducible bit
 //      for bit;
-//   3. near, touching and contact tiers: one warp per test triangle (triangles coloured by shared slots, one launch
-//      per colour) walks its non-far sources in order, builds each pair's rule as the reference does (self, edge,
-//      vertex with wide-corner wedges, contact splits, recursive near subdivision), and evaluates the rule's points
-//      across its lanes: FP64 for the touching and contact tiers, FP32 or FP64 for the near tier, FP64 for the
-//      wake's tip filaments.
+//   3. near, touching and contact tiers: the near pairs one per lane in chunks of 32, the others (self, edge, vertex
+//      with wide-corner wedges, contact splits) one warp per pair with the reference's rules, all test triangles in one
+//      launch each. Every pair's block goes to the pair's own place in a workspace, and one kernel per colour of test
+//      triangles adds the blocks to A, column by column in a fixed order. FP64 for the touching and contact tiers, FP32
+//      or FP64 for the near tier, FP64 for the wake's tip filaments.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -215,11 +215,16 @@ __global__ void __launch_bounds__(FAR_NT) far_kernel_batch(const FarArgs* __rest
 }
 
 // ---- the near tier, one pair per lane ---------------------------------------------------------------------------
-// A warp takes up to 32 sources of its test triangle at once. Each lane decides its own pair's tier (FP64, exactly as
-// pair_rule / wake_pair_rule) and, for a pair in the near tier, walks near_pieces' quadtree to its leaves. The
-// warp then evaluates all leaves' points of the 32 pairs together, one point per lane (FP32, guarded; flagged points
-// are queued and evaluated 32 at a time in FP64), reduces them per pair in a fixed order and adds the blocks to A
-// pair by pair. Pairs of the other tiers are returned (a lane mask) for the warp-cooperative path.
+// A warp takes a chunk of up to 32 consecutive sources of its test triangle at once. Each lane decides its own pair's
+// tier (exactly as pair_rule / wake_pair_rule) and, for a pair in the near tier, walks near_pieces' quadtree to its
+// leaves. The warp then evaluates all leaves' points of the 32 pairs together, one point per lane (FP32, guarded;
+// flagged points are queued and evaluated 32 at a time in FP64), reduces them per pair in a fixed order and writes
+// each pair's block to the pair's place in blk. Pairs of the other tiers are appended to the rest list.
+//
+// Chunks are independent (nothing is added to A here), so a test triangle's chunks go to several warps and all test
+// triangles to one launch. When one warp took a whole test triangle, one launch per colour, and added its blocks to A
+// pair by pair, the kernel ran ~1 warp per SM on a 1,676-triangle wing (348 ms in FP64) and waited on a
+// read-modify-write of A per pair.
 struct NearChunkSh {
     NearPlanSh pl;         // the pairs' leaves and FP32 frames
     double acc[32][9];     // per pair: sum of W psi_a w (FP64 evaluations)
@@ -227,6 +232,8 @@ struct NearChunkSh {
     int off[33];           // points before each pair
     int qp[64], qk[64];    // queued FP64 points: pair, point within the pair
 };
+
+constexpr int BLK_B = 12, BLK_W = 9;  // doubles of a pair's block: body pairs carry their right hand side terms
 
 // the FP64 evaluation of point k of pair p (queued by the FP32 guard): contributions in v
 __device__ void near_point64(const NearArgs& a, const TriGeo& T, const TriGeo& S, const NearChunkSh& ns, int p, int k,
@@ -275,8 +282,9 @@ __device__ void near_point64(const NearArgs& a, const TriGeo& T, const TriGeo& S
     }
 }
 
-__device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* list, int cnt, bool wake, int col0,
-                               double* rbt, unsigned long long* P, unsigned long long* Q, unsigned long long& Q64) {
+// list: the chunk's sources, p0 the first one's place in nf_src / wf_src; returns the lanes of the rest pairs
+__device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* list, int cnt, bool wake, long long p0,
+                               unsigned long long* P, unsigned long long* Q, unsigned long long& Q64) {
     const NearArgs& a = *pc.a;
     const TriGeo& T = *pc.T;
     const int lane = pc.lane;
@@ -415,34 +423,23 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
         }
     }
     __syncwarp();
-    // 4. the pairs' blocks, added pair by pair in source order
-    double blk[9], rb[3] = {0, 0, 0};
+    // 4. the pairs' blocks
     if (near) {
-        double Pp[9];
+        double Pp[9], blk[BLK_B];
         for (int k = 0; k < 9; ++k) Pp[k] = ns.acc[lane][k] + double(ns.accf[lane][k]);
         v3<double> nT = ld3(T.n);
         for (int bb = 0; bb < 3; ++bb) {
             v3<double> mv = cross(nT, ld3(S.gam + 3 * bb));
             for (int ai = 0; ai < 3; ++ai) blk[3 * ai + bb] = Pp[3 * ai] * mv.x + Pp[3 * ai + 1] * mv.y + Pp[3 * ai + 2] * mv.z;
         }
-        for (int ai = 0; ai < 3; ++ai) rb[ai] = -S.sigma * (Pp[3 * ai] * nT.x + Pp[3 * ai + 1] * nT.y + Pp[3 * ai + 2] * nT.z);
-    }
-    for (int k = 0; k < cnt; ++k) {
-        if (!((nearmask >> k) & 1u)) continue;
-        double vk[9];
-        for (int z = 0; z < 9; ++z) vk[z] = __shfl_sync(FULL, blk[z], k);
+        const int nb = wake ? BLK_W : BLK_B;
         if (!wake)
-            for (int z = 0; z < 3; ++z) rbt[z] += __shfl_sync(FULL, rb[z], k);
-        if (lane < 9) {
-            int ai = lane / 3, bb = lane % 3;
-            const TriGeo& Sk = wake ? a.wtri[list[k]] : a.tri[list[k]];
-            double* dst = a.A + size_t(T.slot[ai]) * size_t(a.lda) + col0 + Sk.slot[bb];
-            double val = vk[0];
-            for (int z = 1; z < 9; ++z)
-                if (z == lane) val = vk[z];
-            *dst += val;
-        }
-        __syncwarp();
+            for (int ai = 0; ai < 3; ++ai)
+                blk[9 + ai] = S.sigma * (Pp[3 * ai] * nT.x + Pp[3 * ai + 1] * nT.y + Pp[3 * ai + 2] * nT.z);
+        double* dst = a.blk[wake ? 1 : 0] + size_t(p0 + lane - a.blk0[wake ? 1 : 0]) * nb;
+#pragma unroll
+        for (int k = 0; k < BLK_B; ++k)
+            if (k < nb) dst[k] = blk[k];
     }
     P[TIER_NEAR] += __popc(nearmask);
     Q[TIER_NEAR] += (unsigned long long)total;
@@ -450,8 +447,10 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
     return __ballot_sync(FULL, valid && !near);
 }
 
-// near tier, one pair per lane; the other pairs are listed for near_kernel_pairs. One warp, test triangle t.
-__device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, NearChunkSh& sh) {
+// near tier, one pair per lane; the other pairs are listed for near_kernel_pairs. Warp w of nw of test triangle t: every
+// nw-th chunk of its body and wake lists.
+__device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, const int w, const int nw,
+                                                NearChunkSh& sh) {
     const int lane = threadIdx.x & 31;
     const TriGeo& T = a.tri[t];
     PairCtx pc;
@@ -460,25 +459,17 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
     pc.sh = nullptr;
     pc.lane = lane;
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
-    double rbt[3] = {0, 0, 0};
-    for (int set = 0; set < 2; ++set) {
-        const bool wake = set == 1;
-        const long long e0 = wake ? a.wf_ptr[t] : a.nf_ptr[t], e1 = wake ? a.wf_ptr[t + 1] : a.nf_ptr[t + 1];
-        const int* src = wake ? a.wf_src : a.nf_src;
-        int* rest = wake ? a.wrest_src : a.rest_src;
-        const int col0 = wake ? a.nslot : 0;
-        int nrest = 0;
-        for (long long c0 = e0; c0 < e1; c0 += 32) {
-            const int cnt = int(e1 - c0 < 32 ? e1 - c0 : 32);
-            unsigned m = near_chunk(pc, sh, t, src + c0, cnt, wake, col0, rbt, P, Q, Q64);
-            if ((m >> lane) & 1u) rest[e0 + nrest + __popc(m & ((1u << lane) - 1u))] = src[c0 + lane];
-            nrest += __popc(m);
-            __syncwarp();
-        }
-        if (lane == 0) a.rest_cnt[2 * t + set] = nrest;
+    const long long b0 = a.nf_ptr[t], nb = a.nf_ptr[t + 1] - b0, w0 = a.wf_ptr[t], nwk = a.wf_ptr[t + 1] - w0;
+    const int cb = int((nb + 31) >> 5), cw = int((nwk + 31) >> 5);
+    for (int c = w; c < cb + cw; c += nw) {
+        const bool wake = c >= cb;
+        const long long e = 32LL * (wake ? c - cb : c), n = (wake ? nwk : nb) - e, p0 = (wake ? w0 : b0) + e;
+        const int cnt = int(n < 32 ? n : 32);
+        const unsigned m = near_chunk(pc, sh, t, (wake ? a.wf_src : a.nf_src) + p0, cnt, wake, p0, P, Q, Q64);
+        rest_append(a, 2 * t + (wake ? 1 : 0), p0, m, lane);
+        __syncwarp();
     }
     if (lane == 0) {
-        for (int k = 0; k < 3; ++k) a.b[T.slot[k]] += rbt[k];
         for (int k = 0; k < 6; ++k) {
             if (P[k]) atomicAdd(a.stats + k, P[k]);
             if (Q[k]) atomicAdd(a.stats + 6 + k, Q[k]);
@@ -487,23 +478,15 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
     }
 }
 
-__global__ void __launch_bounds__(32 * NEAR_WARPS) near_kernel_lanes(NearArgs a) {
+// the kernels of the non-far tiers take one system's arguments by value, or (BATCH) those of system work[i].x from sys
+template <bool BATCH>
+__global__ void __launch_bounds__(32 * NEAR_WARPS) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
+                                                                  const int2* __restrict__ work) {
     extern __shared__ __align__(16) unsigned char near_smem[];
     NearChunkSh* shm = reinterpret_cast<NearChunkSh*>(near_smem);
-    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
-    if (idx >= a.ntests) return;
-    near_lanes_body(a, a.tests[idx], shm[threadIdx.x >> 5]);
-}
-
-// a batch of systems: warp i takes test triangle work[i].y of system work[i].x
-__global__ void __launch_bounds__(32 * NEAR_WARPS) near_kernel_lanes_batch(const NearArgs* __restrict__ sys,
-                                                                        const int2* __restrict__ work, int nwork) {
-    extern __shared__ __align__(16) unsigned char near_smem[];
-    NearChunkSh* shm = reinterpret_cast<NearChunkSh*>(near_smem);
-    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
-    if (idx >= nwork) return;
-    const int2 wk = work[idx];
-    near_lanes_body(sys[wk.x], wk.y, shm[threadIdx.x >> 5]);
+    const int2 wk = work[blockIdx.x];
+    near_lanes_body(BATCH ? sys[wk.x] : a, wk.y, blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), gridDim.y * NEAR_WARPS,
+                    shm[threadIdx.x >> 5]);
 }
 
 // the block of one pair: the per-lane sums reduced and contracted with n_T x gamma_b (9 values, row-major), and the
@@ -522,27 +505,47 @@ __device__ void pair_block_out(PairCtx& pc, FwdAcc& acc, const TriGeo& S, double
         int ai = pc.lane / 3, bb = pc.lane % 3;
         v3<double> m = cross(nT, ld3(S.gam + 3 * bb));
         out[pc.lane] = P[3 * ai] * m.x + P[3 * ai + 1] * m.y + P[3 * ai + 2] * m.z;
-    } else if (pc.lane < 12) {
+    } else if (with_rhs && pc.lane < 12) {
         int ai = pc.lane - 9;
-        out[pc.lane] = with_rhs ? S.sigma * (P[3 * ai] * nT.x + P[3 * ai + 1] * nT.y + P[3 * ai + 2] * nT.z) : 0.0;
+        out[pc.lane] = S.sigma * (P[3 * ai] * nT.x + P[3 * ai + 1] * nT.y + P[3 * ai + 2] * nT.z);
     }
     __syncwarp();
 }
 
 // the self, touching and contact pairs, one warp per pair: a persistent grid whose warps take the next pair of the
 // list from a counter, so that test triangles with many contact pairs (thin panels at a sharp trailing edge) do not
-// hold a launch; the blocks go to pair_out and near_kernel_rest adds them in the list's order
-// rest pair idx of system a: its block to a.pair_out, its tier and points counted in P, Q, Q64
-__device__ __forceinline__ void near_pair_item(const NearArgs& a, PairCtx& pc, const long long idx,
-                                               unsigned long long* P, unsigned long long* Q,
-                                               unsigned long long& Q64) {
-        const int lane = pc.lane;
-        const int n = 2 * a.ntri;
-        const int g = rest_entry(a.rest_off, n, idx);
-        const int t = g >> 1;
+// hold a launch; each block goes to its pair's place in blk
+template <bool BATCH>
+__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs a1, const NearArgs* __restrict__ sys,
+                                                                     int nsys) {
+    __shared__ WarpSh shm[NEAR_WARPS];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = (long long)*a1.rest_n;
+    PairCtx pc;
+    pc.sh = &shm[w];
+    pc.lane = lane;
+    unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
+    auto flush = [&](const NearArgs& a) {  // the counts of system a so far
+        if (lane == 0) {
+            for (int k = 0; k < 6; ++k) {
+                if (P[k]) atomicAdd(a.stats + k, P[k]);
+                if (Q[k]) atomicAdd(a.stats + 6 + k, Q[k]);
+            }
+            if (Q64) atomicAdd(a.stats + 12, Q64);
+        }
+        for (int k = 0; k < 6; ++k) P[k] = Q[k] = 0;
+        Q64 = 0;
+    };
+    for (;;) {
+        const long long idx = next_rest_pair(a1.next, lane);
+        if (idx >= total) break;
+        const NearArgs& a = BATCH ? sys[a1.rest_sys[idx]] : a1;
+        pc.a = &a;
+        const unsigned long long item = a1.rest_item[idx];
+        const int g = int(item >> REST_SHIFT), t = g >> 1;
         const bool wake = (g & 1) != 0;
-        const long long e0 = wake ? a.wf_ptr[t] : a.nf_ptr[t];
-        const int s = (wake ? a.wrest_src : a.rest_src)[e0 + (idx - a.rest_off[g])];
+        const long long p = (long long)(item & ((1ull << REST_SHIFT) - 1));
+        const int s = (wake ? a.wf_src : a.nf_src)[p];
         pc.T = &a.tri[t];
         FwdAcc acc = {};
         pc.kind = 0;
@@ -551,68 +554,14 @@ __device__ __forceinline__ void near_pair_item(const NearArgs& a, PairCtx& pc, c
         pc.nleaf = 0;
         pc.nq64 = 0;
         const int tier = tri_pair(pc, acc, t, s, wake);
-        pair_block_out(pc, acc, wake ? a.wtri[s] : a.tri[s], a.pair_out + 12 * idx, !wake);
+        pair_block_out(pc, acc, wake ? a.wtri[s] : a.tri[s],
+                       a.blk[wake ? 1 : 0] + size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B), !wake);
         P[tier] += 1;
         Q[tier] += pc.npts;
         Q64 += pc.n64;
-        (void)lane;
-}
-
-__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs a) {
-    __shared__ WarpSh shm[NEAR_WARPS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long total = a.rest_off[2 * a.ntri];
-    PairCtx pc;
-    pc.a = &a;
-    pc.sh = &shm[w];
-    pc.lane = lane;
-    unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
-    for (;;) {
-        const long long idx = next_rest_pair(a.next, lane);
-        if (idx >= total) break;
-        near_pair_item(a, pc, idx, P, Q, Q64);
+        if (BATCH) flush(a);
     }
-    if (lane == 0) {
-        for (int k = 0; k < 6; ++k) {
-            if (P[k]) atomicAdd(a.stats + k, P[k]);
-            if (Q[k]) atomicAdd(a.stats + 6 + k, Q[k]);
-        }
-        if (Q64) atomicAdd(a.stats + 12, Q64);
-    }
-}
-
-// a batch of systems in one persistent launch: the systems' rest pairs in one index space (system k's pairs at
-// base[k] .. base[k + 1]), taken from one counter; each pair's counts go to its own system's statistics
-__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs_batch(const NearArgs* __restrict__ sys, int nsys,
-                                                                           const long long* __restrict__ base,
-                                                                           unsigned long long* next) {
-    __shared__ WarpSh shm[NEAR_WARPS];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long total = base[nsys];
-    PairCtx pc;
-    pc.sh = &shm[w];
-    pc.lane = lane;
-    for (;;) {
-        const long long idx = next_rest_pair(next, lane);
-        if (idx >= total) break;
-        int lo = 0, hi = nsys - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (base[mid] <= idx) lo = mid;
-            else hi = mid - 1;
-        }
-        const NearArgs& a = sys[lo];
-        pc.a = &a;
-        unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
-        near_pair_item(a, pc, idx - base[lo], P, Q, Q64);
-        if (lane == 0) {
-            for (int k = 0; k < 6; ++k) {
-                if (P[k]) atomicAdd(a.stats + k, P[k]);
-                if (Q[k]) atomicAdd(a.stats + 6 + k, Q[k]);
-            }
-            if (Q64) atomicAdd(a.stats + 12, Q64);
-        }
-    }
+    if (!BATCH) flush(a1);
 }
 
 // one far tip filament of test triangle T, summed by one lane: segment_block (assemble.jl:312-321) with the far rule
@@ -644,128 +593,100 @@ __device__ void far_filament_fwd(const NearArgs& a, const TriGeo& T, v3<double> 
     }
 }
 
-// the blocks of the self, touching and contact pairs (from near_kernel_pairs, added in the order of the test
-// triangle's list), the tip filaments and the freestream: one warp per test triangle, a launch per colour
-__device__ __forceinline__ void near_rest_body(const NearArgs& a, const int t, WarpSh& wsh) {
+// the tip filaments (assemble.jl:344-354): segment_rule (:299-306) and segment_block (:312-321), FP64. A warp takes 32
+// filaments of one test triangle: a far one (the far rule's few points) is summed by its own lane, the others by the
+// whole warp. Every (test triangle, filament) writes the columns of its two ends to fil_out; near_kernel_gather adds
+// them, so all test triangles share one launch.
+template <bool BATCH>
+__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_filaments(NearArgs a1, const NearArgs* __restrict__ sys,
+                                                                         const int2* __restrict__ work, int nwork) {
+    __shared__ WarpSh shm[NEAR_WARPS];
+    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
+    if (idx >= nwork) return;
+    const int2 wk = work[idx];
+    const NearArgs& a = BATCH ? sys[wk.x] : a1;
+    const int f0 = blockIdx.y * 32;
+    if (f0 >= a.nfil) return;
+    const int t = wk.y;
     const int lane = threadIdx.x & 31;
     const TriGeo& T = a.tri[t];
     PairCtx pc;
     pc.a = &a;
     pc.T = &T;
-    pc.sh = &wsh;
+    pc.sh = &shm[threadIdx.x >> 5];
     pc.lane = lane;
     pc.nleaf = 0;
     pc.nq64 = 0;
     pc.fp32 = 0;
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
-    double rbt[3] = {0, 0, 0};
     const double corners[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    for (int set = 0; set < 2; ++set) {
-        const bool wake = set == 1;
-        const long long e0 = wake ? a.wf_ptr[t] : a.nf_ptr[t];
-        const int n = a.rest_cnt[2 * t + set];
-        const int* rest = wake ? a.wrest_src : a.rest_src;
-        const int col0 = wake ? a.nslot : 0;
-        const double* blk = a.pair_out + 12 * a.rest_off[2 * t + set];
-        for (int e = 0; e < n; ++e) {
-            const TriGeo& S = wake ? a.wtri[rest[e0 + e]] : a.tri[rest[e0 + e]];
-            const double* pb = blk + 12 * e;
-            if (lane < 9) {
-                double* dst = a.A + size_t(T.slot[lane / 3]) * size_t(a.lda) + col0 + S.slot[lane % 3];
-                *dst += pb[lane];
-            }
-            if (!wake)
-                for (int ai = 0; ai < 3; ++ai) rbt[ai] -= pb[9 + ai];
-            __syncwarp();
-        }
-    }
-    // tip filaments (assemble.jl:344-354): segment_rule (:299-306) and segment_block (:312-321), FP64. A warp takes 32
-    // filaments at once: a far one (the far rule's few points) is summed by its own lane, the others by the whole
-    // warp; the columns are added in the filaments' order.
-    for (int f0 = 0; f0 < a.nfil; f0 += 32) {
-        const int cnt = a.nfil - f0 < 32 ? a.nfil - f0 : 32;
-        int mia = 0, mib = 0;
-        double mca[3] = {0, 0, 0}, mcb[3] = {0, 0, 0};
-        bool mfar = false;
-        if (lane < cnt) {
-            mia = a.fil[2 * (f0 + lane)];
-            mib = a.fil[2 * (f0 + lane) + 1];
-            const v3<double> fa = ld3(a.wx + 3 * mia), fb = ld3(a.wx + 3 * mib);
-            mfar = vnorm((fa + fb) / 2.0 - ld3(T.c)) > a.far_ratio * fmax(T.diam, vnorm(fb - fa));
-            if (mfar) far_filament_fwd(a, T, fa, fb, mca, mcb);
-        }
-        const unsigned farmask = __ballot_sync(0xffffffffu, mfar);
-        for (int q = 0; q < cnt; ++q) {
-            const int ia = __shfl_sync(0xffffffffu, mia, q), ib = __shfl_sync(0xffffffffu, mib, q);
-            if ((farmask >> q) & 1u) {
-                double ca[3], cb[3];
-                for (int k = 0; k < 3; ++k) {
-                    ca[k] = __shfl_sync(0xffffffffu, mca[k], q);
-                    cb[k] = __shfl_sync(0xffffffffu, mcb[k], q);
-                }
-                if (lane < 3) {
-                    double* row = a.A + size_t(T.slot[lane]) * size_t(a.lda) + a.nslot;
-                    row[ia] += lane == 0 ? ca[0] : (lane == 1 ? ca[1] : ca[2]);
-                    __syncwarp(0x7u);
-                    row[ib] += lane == 0 ? cb[0] : (lane == 1 ? cb[1] : cb[2]);
-                }
-                __syncwarp();
-                P[TIER_FAR] += 1;
-                Q[TIER_FAR] += a.nrule[R_FAR];
-                continue;
-            }
-            // near and vertex filaments (segment_rule, assemble.jl:299-306), the whole warp
-            const v3<double> fa = ld3(a.wx + 3 * ia), fb = ld3(a.wx + 3 * ib);
-            if (lane == 0) {
-                for (int k = 0; k < 3; ++k) {
-                    pc.sh->E[9 * k + 0] = T.x[3 * k + 0] - fa.x;
-                    pc.sh->E[9 * k + 1] = T.x[3 * k + 1] - fa.y;
-                    pc.sh->E[9 * k + 2] = T.x[3 * k + 2] - fa.z;
-                    pc.sh->E[9 * k + 3] = T.x[3 * k + 0] - fb.x;
-                    pc.sh->E[9 * k + 4] = T.x[3 * k + 1] - fb.y;
-                    pc.sh->E[9 * k + 5] = T.x[3 * k + 2] - fb.z;
-                }
-            }
-            __syncwarp();
-            FwdAcc acc = {};
-            pc.kind = 1;
-            pc.npts = 0;
-            pc.n64 = 0;
-            pc.side = 0;
-            pc.fp32 = 0;
-            int tier, kv = -1;
-            for (int k = 0; k < 3 && kv < 0; ++k)
-                if (fmin(vnorm(ld3(T.x + 3 * k) - fa), vnorm(ld3(T.x + 3 * k) - fb)) <= 1e-12 * T.diam) kv = k;
-            if (kv >= 0) {
-                tier = TIER_VERTEX;
-                vertex_rule(pc, acc, kv);
-            } else {
-                tier = TIER_NEAR;
-                SrcRef src{1, nullptr, fa, fb};
-                near_pieces(pc, acc, src, corners, 1.0, a.near_depth);
-                flush_leaves(pc, acc);
-            }
-            double ca[3], cb[3];
+    double* out = a.fil_out + 6 * (size_t(t - a.fil_t0) * a.nfil + f0);
+    const int cnt = a.nfil - f0 < 32 ? a.nfil - f0 : 32;
+    bool mfar = false;
+    if (lane < cnt) {
+        const v3<double> fa = ld3(a.wx + 3 * a.fil[2 * (f0 + lane)]), fb = ld3(a.wx + 3 * a.fil[2 * (f0 + lane) + 1]);
+        mfar = vnorm((fa + fb) / 2.0 - ld3(T.c)) > a.far_ratio * fmax(T.diam, vnorm(fb - fa));
+        if (mfar) {
+            double mca[3] = {0, 0, 0}, mcb[3] = {0, 0, 0};
+            far_filament_fwd(a, T, fa, fb, mca, mcb);
             for (int k = 0; k < 3; ++k) {
-                ca[k] = warp_sum(acc.ca[k]);
-                cb[k] = warp_sum(acc.cb[k]);
+                out[6 * lane + k] = mca[k];
+                out[6 * lane + 3 + k] = mcb[k];
             }
-            if (lane < 3) {
-                double* row = a.A + size_t(T.slot[lane]) * size_t(a.lda) + a.nslot;
-                row[ia] += ca[lane];
-                __syncwarp(0x7u);
-                row[ib] += cb[lane];
-            }
-            __syncwarp();
-            P[tier] += 1;
-            Q[tier] += pc.npts;
-            Q64 += pc.n64;
         }
     }
-    // freestream, exact (assemble.jl:422), and the rows of b
+    const unsigned farmask = __ballot_sync(0xffffffffu, mfar);
+    P[TIER_FAR] += __popc(farmask);
+    Q[TIER_FAR] += (unsigned long long)__popc(farmask) * a.nrule[R_FAR];
+    for (int q = 0; q < cnt; ++q) {
+        if ((farmask >> q) & 1u) continue;
+        // near and vertex filaments, the whole warp
+        const v3<double> fa = ld3(a.wx + 3 * a.fil[2 * (f0 + q)]), fb = ld3(a.wx + 3 * a.fil[2 * (f0 + q) + 1]);
+        if (lane == 0) {
+            for (int k = 0; k < 3; ++k) {
+                pc.sh->E[9 * k + 0] = T.x[3 * k + 0] - fa.x;
+                pc.sh->E[9 * k + 1] = T.x[3 * k + 1] - fa.y;
+                pc.sh->E[9 * k + 2] = T.x[3 * k + 2] - fa.z;
+                pc.sh->E[9 * k + 3] = T.x[3 * k + 0] - fb.x;
+                pc.sh->E[9 * k + 4] = T.x[3 * k + 1] - fb.y;
+                pc.sh->E[9 * k + 5] = T.x[3 * k + 2] - fb.z;
+            }
+        }
+        __syncwarp();
+        FwdAcc acc = {};
+        pc.kind = 1;
+        pc.npts = 0;
+        pc.n64 = 0;
+        pc.side = 0;
+        pc.fp32 = 0;
+        int tier, kv = -1;
+        for (int k = 0; k < 3 && kv < 0; ++k)
+            if (fmin(vnorm(ld3(T.x + 3 * k) - fa), vnorm(ld3(T.x + 3 * k) - fb)) <= 1e-12 * T.diam) kv = k;
+        if (kv >= 0) {
+            tier = TIER_VERTEX;
+            vertex_rule(pc, acc, kv);
+        } else {
+            tier = TIER_NEAR;
+            SrcRef src{1, nullptr, fa, fb};
+            near_pieces(pc, acc, src, corners, 1.0, a.near_depth);
+            flush_leaves(pc, acc);
+        }
+        double ca[3], cb[3];
+        for (int k = 0; k < 3; ++k) {
+            ca[k] = warp_sum(acc.ca[k]);
+            cb[k] = warp_sum(acc.cb[k]);
+        }
+        if (lane == 0)
+            for (int k = 0; k < 3; ++k) {
+                out[6 * q + k] = ca[k];
+                out[6 * q + 3 + k] = cb[k];
+            }
+        __syncwarp();
+        P[tier] += 1;
+        Q[tier] += pc.npts;
+        Q64 += pc.n64;
+    }
     if (lane == 0) {
-        double vn = (a.vinf[0] * T.n[0] + a.vinf[1] * T.n[1] + a.vinf[2] * T.n[2]) * T.area;
-        for (int k = 0; k < 3; ++k) a.b[T.slot[k]] += rbt[k] - vn * a.tint[k];
         for (int k = 0; k < 6; ++k) {
             if (P[k]) atomicAdd(a.stats + k, P[k]);
             if (Q[k]) atomicAdd(a.stats + 6 + k, Q[k]);
@@ -774,20 +695,95 @@ __device__ __forceinline__ void near_rest_body(const NearArgs& a, const int t, W
     }
 }
 
-__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_rest(NearArgs a) {
-    __shared__ WarpSh shm[NEAR_WARPS];
-    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
-    if (idx >= a.ntests) return;
-    near_rest_body(a, a.tests[idx], shm[threadIdx.x >> 5]);
+// the place of source s in the ascending list of n sources, or -1
+__device__ __forceinline__ int find_source(const int* list, int n, int s) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (list[mid] < s) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < n && list[lo] == s ? lo : -1;
 }
 
-__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_rest_batch(const NearArgs* __restrict__ sys,
-                                                                          const int2* __restrict__ work, int nwork) {
-    __shared__ WarpSh shm[NEAR_WARPS];
-    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
-    if (idx >= nwork) return;
-    const int2 wk = work[idx];
-    near_rest_body(sys[wk.x], wk.y, shm[threadIdx.x >> 5]);
+constexpr int GATHER_NT = 128;
+constexpr int GATHER_LIST = 2048;  // sources of a list staged in shared memory (8 KB); longer lists are searched in place
+
+// One CTA per test triangle, one launch per colour (no two test triangles of a launch share a row): the blocks of its
+// non-far pairs and its filaments' columns added to its three rows of A, its right hand side to b, in a fixed order.
+// A thread takes a (pair, source corner) and adds its column's whole sum if no earlier pair of the list has that
+// column: the pairs with the column are those of the column's triangles that binary search finds in the list. Every
+// entry of A is read and written once, by one thread, all columns in parallel; bound by reading the blocks.
+template <bool BATCH>
+__global__ void __launch_bounds__(GATHER_NT) near_kernel_gather(NearArgs a1, const NearArgs* __restrict__ sys,
+                                                              const int2* __restrict__ work) {
+    __shared__ int s_list[GATHER_LIST];
+    __shared__ double red[3][GATHER_NT];
+    const int2 wk = work[blockIdx.x];
+    const NearArgs& a = BATCH ? sys[wk.x] : a1;
+    const int t = wk.y, tid = threadIdx.x;
+    const TriGeo& T = a.tri[t];
+    double* row[3];
+    for (int k = 0; k < 3; ++k) row[k] = a.A + size_t(T.slot[k]) * size_t(a.lda);
+    double rb[3] = {0, 0, 0};
+    for (int set = 0; set < 2; ++set) {
+        const long long p0 = (set ? a.wf_ptr : a.nf_ptr)[t];
+        const int n = int((set ? a.wf_ptr : a.nf_ptr)[t + 1] - p0);
+        const int* src = (set ? a.wf_src : a.nf_src) + p0;
+        const int nb = set ? BLK_W : BLK_B;
+        const double* blk = a.blk[set] + size_t(p0 - a.blk0[set]) * nb;
+        const int col0 = set ? a.nslot : 0;
+        const int *slots = a.slots[set], *ptr = a.col_ptr[set], *ent = a.col_ent[set];
+        const bool staged = n <= GATHER_LIST;
+        __syncthreads();
+        if (staged)
+            for (int i = tid; i < n; i += GATHER_NT) s_list[i] = src[i];
+        __syncthreads();
+        const int* list = staged ? s_list : src;
+        for (int i = tid; i < 3 * n; i += GATHER_NT) {
+            const int p = i / 3, b = i - 3 * p, s = list[p], c = slots[3 * s + b];
+            double v[3] = {0, 0, 0};
+            bool own = false;
+            for (int u = ptr[c]; u < ptr[c + 1]; ++u) {
+                const int e = ent[u], se = e / 3, be = e - 3 * se;
+                const bool me = e == 3 * s + b;
+                const int q = me ? p : find_source(list, n, se);
+                if (q < 0) continue;
+                if (!me && !own) break;  // an earlier pair has this column
+                own = true;
+                const double* pb = blk + size_t(q) * nb + be;
+                v[0] += pb[0];
+                v[1] += pb[3];
+                v[2] += pb[6];
+            }
+            if (own)
+                for (int k = 0; k < 3; ++k) row[k][col0 + c] += v[k];
+        }
+        if (!set)
+            for (int p = tid; p < n; p += GATHER_NT)
+                for (int k = 0; k < 3; ++k) rb[k] -= blk[size_t(p) * nb + 9 + k];
+    }
+    if (a.nfil > 0) {
+        __syncthreads();  // the wake's columns are the filaments' too
+        const double* fo = a.fil_out + 6 * size_t(t - a.fil_t0) * a.nfil;
+        for (int i = tid; i < a.nfnode; i += GATHER_NT) {
+            double v[3] = {0, 0, 0};
+            for (int u = a.fnode_ptr[i]; u < a.fnode_ptr[i + 1]; ++u)
+                for (int k = 0; k < 3; ++k) v[k] += fo[3 * a.fnode_ent[u] + k];
+            for (int k = 0; k < 3; ++k) row[k][a.nslot + a.fnode[i]] += v[k];
+        }
+    }
+    // the right hand side: the pairs' terms, and the freestream, exact (assemble.jl:422)
+    for (int k = 0; k < 3; ++k) red[k][tid] = rb[k];
+    for (int o = GATHER_NT / 2; o > 0; o >>= 1) {
+        __syncthreads();
+        if (tid < o)
+            for (int k = 0; k < 3; ++k) red[k][tid] += red[k][tid + o];
+    }
+    if (tid == 0) {
+        const double vn = (a.vinf[0] * T.n[0] + a.vinf[1] * T.n[1] + a.vinf[2] * T.n[2]) * T.area;
+        for (int k = 0; k < 3; ++k) a.b[T.slot[k]] += red[k][0] - vn * a.tint[k];
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -839,7 +835,6 @@ struct AsmJob {
     std::vector<std::vector<int>> near_col;  // test triangles, per colour
     NearArgs na{};
     unsigned long long* d_stats = nullptr;
-    long long nrest = 0;
     std::chrono::steady_clock::time_point t0;
     ~AsmJob() {
         if (sys) vp_system_free(sys);
@@ -934,14 +929,44 @@ int job_prepare(vp_ctx* ctx, AsmJob& j) {
     j.na.A = sys->A;
     j.na.b = sys->b;
     j.na.stats = j.d_stats;
-    int *d_rest, *d_wrest, *d_rcnt;
-    if ((r = dl.alloc(ctx, &d_rest, size_t(std::max(ps.nfptr[ntri], 1LL)))) ||
-        (r = dl.alloc(ctx, &d_wrest, size_t(std::max(ps.wfptr[ntri], 1LL)))) ||
-        (r = dl.alloc(ctx, &d_rcnt, size_t(2) * ntri)))
-        return r;
-    j.na.rest_src = d_rest;
-    j.na.wrest_src = d_wrest;
-    j.na.rest_cnt = d_rcnt;
+    // the columns' triangles (and corners), the filaments' nodes
+    std::vector<int> wslots(3 * size_t(nwtri));
+    for (int t = 0; t < nwtri; ++t)
+        for (int k = 0; k < 3; ++k) wslots[3 * size_t(t) + k] = ps.wg[t].slot[k];
+    auto csr = [](const int* key, int n, int nkey, std::vector<int>& ptr, std::vector<int>& ent) {
+        ptr.assign(size_t(nkey) + 1, 0);
+        ent.assign(std::max(n, 1), 0);
+        for (int i = 0; i < n; ++i) ptr[key[i] + 1]++;
+        for (int c = 0; c < nkey; ++c) ptr[c + 1] += ptr[c];
+        std::vector<int> at(ptr.begin(), ptr.end() - 1);
+        for (int i = 0; i < n; ++i) ent[at[key[i]]++] = i;
+    };
+    const int* keys[2] = {in.corner_slot, wslots.data()};
+    const int nel[2] = {ntri, nwtri}, nkey[2] = {nslot, in.nwnode};
+    for (int set = 0; set < 2; ++set) {
+        std::vector<int> ptr, ent, sl(keys[set], keys[set] + 3 * size_t(nel[set]));
+        csr(keys[set], 3 * nel[set], nkey[set], ptr, ent);
+        int *d_sl, *d_ptr, *d_ent;
+        if ((r = dl.up(ctx, &d_sl, sl)) || (r = dl.up(ctx, &d_ptr, ptr)) || (r = dl.up(ctx, &d_ent, ent))) return r;
+        j.na.slots[set] = d_sl;
+        j.na.col_ptr[set] = d_ptr;
+        j.na.col_ent[set] = d_ent;
+    }
+    if (in.nfil > 0) {
+        std::vector<int> ptr, ent, node, nptr{0};
+        csr(in.fil, 2 * in.nfil, in.nwnode, ptr, ent);
+        for (int i = 0; i < in.nwnode; ++i)
+            if (ptr[i + 1] > ptr[i]) {
+                node.push_back(i);
+                nptr.push_back(ptr[i + 1]);
+            }
+        int *d_node, *d_ptr, *d_ent;
+        if ((r = dl.up(ctx, &d_node, node)) || (r = dl.up(ctx, &d_ptr, nptr)) || (r = dl.up(ctx, &d_ent, ent))) return r;
+        j.na.nfnode = int(node.size());
+        j.na.fnode = d_node;
+        j.na.fnode_ptr = d_ptr;
+        j.na.fnode_ent = d_ent;
+    }
     return VP_OK;
 }
 
@@ -1028,128 +1053,128 @@ int far_launch_batch(vp_ctx* ctx, std::vector<std::unique_ptr<AsmJob>>& jobs, De
     return VP_OK;
 }
 
-// one system: the near tier's lanes per colour, the rest pairs' list, the persistent pair kernel, the rest per colour
-int near_launch(vp_ctx* ctx, AsmJob& j) {
-    DevList& dl = j.ps.dl;
-    NearArgs& na = j.na;
-    std::vector<int> all;
-    std::vector<int> off{0};
-    for (auto& c : j.near_col) {
-        all.insert(all.end(), c.begin(), c.end());
-        off.push_back((int)all.size());
-    }
-    int* d_tests;
-    int r;
-    if ((r = dl.up(ctx, &d_tests, all))) return r;
-    vp_phase_begin(ctx, PH_NEAR);
-    const size_t near_smem = sizeof(NearChunkSh) * NEAR_WARPS;
-    VP_CUDA(ctx, cudaFuncSetAttribute(near_kernel_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(near_smem)));
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1) {
-            // the rest pairs as one list, evaluated pair-parallel into per-pair blocks
-            long long nrest = 0;
-            double* d_pairs;
-            if ((r = rest_list(ctx, dl, na, &nrest)) ||
-                (r = dl.alloc(ctx, &d_pairs, size_t(12) * size_t(std::max(nrest, 1LL)))))
-                return r;
-            na.pair_out = d_pairs;
-            if (nrest > 0) {
-                const int nb = persistent_blocks(ctx, near_kernel_pairs, 32 * NEAR_WARPS, 0);
-                vp_phase_end(ctx);
-                vp_phase_begin(ctx, PH_NEAR_PAIRS);
-                near_kernel_pairs<<<nb, 32 * NEAR_WARPS, 0, ctx->stream>>>(na);
-                vp_phase_end(ctx);
-                vp_phase_begin(ctx, PH_NEAR);
-                ctx->launches++;
-            }
-        }
-        for (size_t c = 0; c < j.near_col.size(); ++c) {
-            na.tests = d_tests + off[c];
-            na.ntests = off[c + 1] - off[c];
-            int nb = (na.ntests + NEAR_WARPS - 1) / NEAR_WARPS;
-            if (!nb) continue;
-            if (pass == 0)
-                near_kernel_lanes<<<nb, 32 * NEAR_WARPS, near_smem, ctx->stream>>>(na);
-            else
-                near_kernel_rest<<<nb, 32 * NEAR_WARPS, 0, ctx->stream>>>(na);
-            ctx->launches++;
-        }
-    }
-    vp_phase_end(ctx);
-    VP_CUDA(ctx, cudaGetLastError());
-    return VP_OK;
-}
+// the pair blocks' workspace of one pass over test triangles, at most (a pass holds at least one test triangle)
+constexpr size_t NEAR_PASS_BYTES = size_t(1) << 30;
 
-// a batch: the lanes kernel per colour over every system, every system's rest list, one persistent launch of the
-// pair kernel over all of them, the rest kernel per colour over every system
-int near_launch_batch(vp_ctx* ctx, std::vector<std::unique_ptr<AsmJob>>& jobs, DevList& dl) {
+// The non-far tiers of the jobs (one: BATCH false). The test triangles go in passes whose pair blocks fit the workspace;
+// a pass is: the lanes kernel over all its test triangles (blocks of the near pairs, the list of the rest), the
+// persistent pair kernel (blocks of the rest), the filaments, and per colour the kernel that adds the blocks to A.
+template <bool BATCH>
+int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
     int r;
     const int nsys = int(jobs.size());
-    size_t ncol = 0;
-    for (auto& j : jobs) ncol = std::max(ncol, j->near_col.size());
-    auto colour_work = [&](size_t c) {
-        std::vector<int2> work;
-        for (int k = 0; k < nsys; ++k)
-            if (c < jobs[k]->near_col.size())
-                for (int t : jobs[k]->near_col[c]) work.push_back(make_int2(k, t));
-        return work;
+    struct Range {
+        int sys, t0, t1;
     };
-    auto upload_args = [&](NearArgs** d) {
-        std::vector<NearArgs> args;
-        for (auto& j : jobs) args.push_back(j->na);
-        return dl.up(ctx, d, args);
+    std::vector<std::vector<Range>> passes;
+    size_t used = 0, most = 0, most_items = 0, items = 0, most_fil = 0, fil = 0;
+    long long max_pairs = 0;
+    auto close = [&]() {
+        most = std::max(most, used);
+        most_items = std::max(most_items, items);
+        most_fil = std::max(most_fil, fil);
+        used = items = fil = 0;
     };
-    NearArgs* d_args;
-    if ((r = upload_args(&d_args))) return r;
-    vp_phase_begin(ctx, PH_NEAR);
+    for (int k = 0; k < nsys; ++k) {
+        const AsmJob& j = *jobs[k];
+        const int nfil = j.in.nfil;
+        for (int t = 0; t < j.in.ntri; ++t) {
+            const size_t nb = size_t(j.ps.nfptr[t + 1] - j.ps.nfptr[t]), nw = size_t(j.ps.wfptr[t + 1] - j.ps.wfptr[t]);
+            const size_t need = 8 * (BLK_B * nb + BLK_W * nw + 6 * size_t(nfil)) + 8 * (nb + nw);
+            max_pairs = std::max(max_pairs, (long long)std::max(nb, nw));
+            if (passes.empty() || (used > 0 && used + need > NEAR_PASS_BYTES)) {
+                close();
+                passes.emplace_back();
+            }
+            auto& p = passes.back();
+            if (p.empty() || p.back().sys != k) p.push_back({k, t, t});
+            p.back().t1 = t + 1;
+            used += need;
+            items += nb + nw;
+            fil += 6 * size_t(nfil);
+        }
+    }
+    close();
+    double *d_blk, *d_fil;
+    unsigned long long *d_items, *d_cnt;
+    int* d_sysof = nullptr;
+    if ((r = dl.alloc(ctx, &d_blk, size_t(BLK_B) * most_items)) || (r = dl.alloc(ctx, &d_fil, most_fil)) ||
+        (r = dl.alloc(ctx, &d_items, most_items)) || (r = dl.alloc(ctx, &d_cnt, 2)) ||
+        (BATCH && (r = dl.alloc(ctx, &d_sysof, most_items))))
+        return r;
     const size_t near_smem = sizeof(NearChunkSh) * NEAR_WARPS;
-    VP_CUDA(ctx, cudaFuncSetAttribute(near_kernel_lanes_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(near_smem)));
-    for (size_t c = 0; c < ncol; ++c) {
-        std::vector<int2> work = colour_work(c);
-        if (work.empty()) continue;
+    VP_CUDA(ctx, cudaFuncSetAttribute(near_kernel_lanes<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(near_smem)));
+    const int npb = persistent_blocks(ctx, near_kernel_pairs<BATCH>, 32 * NEAR_WARPS, 0);
+    for (auto& pass : passes) {
+        // the systems' places in the workspace, the work lists: all test triangles, then by colour
+        std::vector<NearArgs> args(nsys);
+        std::vector<int2> work;
+        std::vector<size_t> off;
+        size_t at = 0, fat = 0, ncol = 0;
+        int nfil = 0;
+        for (const Range& g : pass) {
+            AsmJob& j = *jobs[g.sys];
+            NearArgs& na = j.na;
+            na.sys = g.sys;
+            na.rest_item = d_items;
+            na.rest_sys = d_sysof;
+            na.rest_n = d_cnt;
+            na.next = d_cnt + 1;
+            na.blk0[0] = j.ps.nfptr[g.t0];
+            na.blk0[1] = j.ps.wfptr[g.t0];
+            na.blk[0] = d_blk + at;
+            at += size_t(BLK_B) * size_t(j.ps.nfptr[g.t1] - j.ps.nfptr[g.t0]);
+            na.blk[1] = d_blk + at;
+            at += size_t(BLK_W) * size_t(j.ps.wfptr[g.t1] - j.ps.wfptr[g.t0]);
+            na.fil_out = d_fil + fat;
+            na.fil_t0 = g.t0;
+            fat += 6 * size_t(na.nfil) * size_t(g.t1 - g.t0);
+            nfil = std::max(nfil, na.nfil);
+            args[g.sys] = na;
+            ncol = std::max(ncol, j.near_col.size());
+            for (int t = g.t0; t < g.t1; ++t) work.push_back(make_int2(g.sys, t));
+        }
+        const int ntests = int(work.size());
+        for (size_t c = 0; c < ncol; ++c) {
+            off.push_back(work.size());
+            for (const Range& g : pass) {
+                const auto& col = jobs[g.sys]->near_col;
+                if (c >= col.size()) continue;
+                auto lo = std::lower_bound(col[c].begin(), col[c].end(), g.t0);
+                for (; lo != col[c].end() && *lo < g.t1; ++lo) work.push_back(make_int2(g.sys, *lo));
+            }
+        }
+        off.push_back(work.size());
         int2* d_work;
-        if ((r = dl.up(ctx, &d_work, work))) return r;
-        const int n = int(work.size());
-        near_kernel_lanes_batch<<<(n + NEAR_WARPS - 1) / NEAR_WARPS, 32 * NEAR_WARPS, near_smem, ctx->stream>>>(
-            d_args, d_work, n);
+        NearArgs* d_args = nullptr;
+        if ((r = dl.up(ctx, &d_work, work)) || (BATCH && (r = dl.up(ctx, &d_args, args)))) return r;
+        const NearArgs& a1 = args[pass[0].sys];
+        VP_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        vp_phase_begin(ctx, PH_NEAR);
+        const int lw = lane_warps(ctx, ntests, max_pairs);
+        near_kernel_lanes<BATCH><<<dim3(ntests, lw / NEAR_WARPS), 32 * NEAR_WARPS, near_smem, ctx->stream>>>(a1, d_args,
+                                                                                                            d_work);
         ctx->launches++;
-    }
-    // every system's rest list and block buffer; their pairs in one index space
-    std::vector<long long> base{0};
-    for (auto& j : jobs) {
-        if ((r = rest_list(ctx, j->ps.dl, j->na, &j->nrest))) return r;
-        double* d_pairs;
-        if ((r = j->ps.dl.alloc(ctx, &d_pairs, size_t(12) * size_t(std::max(j->nrest, 1LL))))) return r;
-        j->na.pair_out = d_pairs;
-        base.push_back(base.back() + j->nrest);
-    }
-    if ((r = upload_args(&d_args))) return r;
-    if (base.back() > 0) {
-        long long* d_base;
-        unsigned long long* d_next;
-        if ((r = dl.up(ctx, &d_base, base)) || (r = dl.alloc(ctx, &d_next, 1))) return r;
-        VP_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-        const int nb = persistent_blocks(ctx, near_kernel_pairs_batch, 32 * NEAR_WARPS, 0);
+        if (nfil > 0) {
+            near_kernel_filaments<BATCH><<<dim3((ntests + NEAR_WARPS - 1) / NEAR_WARPS, (nfil + 31) / 32), 32 * NEAR_WARPS, 0,
+                                           ctx->stream>>>(a1, d_args, d_work, ntests);
+            ctx->launches++;
+        }
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR_PAIRS);
-        near_kernel_pairs_batch<<<nb, 32 * NEAR_WARPS, 0, ctx->stream>>>(d_args, nsys, d_base, d_next);
+        near_kernel_pairs<BATCH><<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, nsys);
+        ctx->launches++;
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR);
-        ctx->launches++;
+        for (size_t c = 0; c < ncol; ++c) {
+            const int nb = int(off[c + 1] - off[c]);
+            if (!nb) continue;
+            near_kernel_gather<BATCH><<<nb, GATHER_NT, 0, ctx->stream>>>(a1, d_args, d_work + off[c]);
+            ctx->launches++;
+        }
+        vp_phase_end(ctx);
+        VP_CUDA(ctx, cudaGetLastError());
     }
-    for (size_t c = 0; c < ncol; ++c) {
-        std::vector<int2> work = colour_work(c);
-        if (work.empty()) continue;
-        int2* d_work;
-        if ((r = dl.up(ctx, &d_work, work))) return r;
-        const int n = int(work.size());
-        near_kernel_rest_batch<<<(n + NEAR_WARPS - 1) / NEAR_WARPS, 32 * NEAR_WARPS, 0, ctx->stream>>>(d_args, d_work,
-                                                                                                      n);
-        ctx->launches++;
-    }
-    vp_phase_end(ctx);
-    VP_CUDA(ctx, cudaGetLastError());
     return VP_OK;
 }
 
@@ -1196,7 +1221,7 @@ int vp_assemble_impl(vp_ctx* ctx, const vp_assembly_options* o, int nnode, const
     j.in = PairInput{o,     nnode, x,     ntri, tris,  corner_slot, nslot, ntouch, touch_pairs,
                      sigma, vinf,  nwnode, wx,  nwtri, wtris,       nfil,  fil,   body_sources != 0};
     int r;
-    if ((r = job_prepare(ctx, j)) || (r = far_dispatch(ctx, j)) || (r = near_launch(ctx, j))) return r;
+    if ((r = job_prepare(ctx, j)) || (r = far_dispatch(ctx, j)) || (r = near_launch<false>(ctx, {&j}, j.ps.dl))) return r;
     return job_finish(ctx, j, out, stats);
 }
 
@@ -1216,7 +1241,9 @@ int vp_assemble_batch_impl(vp_ctx* ctx, const vp_assembly_options* o, int nsys, 
                                     w.wtris, w.nfil,   w.fil,    true};
         if ((r = job_prepare(ctx, *jobs.back()))) return r;
     }
-    if ((r = far_dispatch_batch(ctx, jobs, dl)) || (r = near_launch_batch(ctx, jobs, dl))) return r;
+    std::vector<AsmJob*> all;
+    for (auto& j : jobs) all.push_back(j.get());
+    if ((r = far_dispatch_batch(ctx, jobs, dl)) || (r = near_launch<true>(ctx, all, dl))) return r;
     for (int k = 0; k < nsys; ++k)
         if ((r = job_finish(ctx, *jobs[k], &out[k], stats ? stats + k : nullptr))) {
             for (int i = 0; i < k; ++i) {

@@ -588,13 +588,13 @@ __device__ unsigned adj_chunk(PairCtx& pc, AdjChunkSh& ns, const AdjMulti& mx, i
     return __ballot_sync(FULL, valid && !near);
 }
 
+// blockIdx.x: the test triangle; its chunks go to NEAR_WARPS * gridDim.y warps, each with its own test-side sums (one
+// warp per test triangle left a 1,676-triangle wing at 11 warps per SM in one uneven wave: 159 ms in FP64)
 __global__ void __launch_bounds__(32 * NEAR_WARPS) adj_lanes_kernel(NearArgs a, AdjMulti mx) {
     extern __shared__ __align__(16) unsigned char adj_smem[];
     AdjChunkSh& ns = reinterpret_cast<AdjChunkSh*>(adj_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int idx = blockIdx.x * NEAR_WARPS + (threadIdx.x >> 5);
-    if (idx >= a.ntests) return;
-    const int t = a.tests[idx];
+    const int t = blockIdx.x, w = blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), nw = gridDim.y * NEAR_WARPS;
     const TriGeo& T = a.tri[t];
     const int K = mx.nadj;
     PairCtx pc;
@@ -614,20 +614,15 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) adj_lanes_kernel(NearArgs a, 
         fs[j] = 0;
     }
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
-    for (int set = 0; set < 2; ++set) {
-        const bool wake = set == 1;
-        const long long e0 = wake ? a.wf_ptr[t] : a.nf_ptr[t];
-        const long long e1 = wake ? a.wf_ptr[t + 1] : a.nf_ptr[t + 1];
-        const int* src = wake ? a.wf_src : a.nf_src;
-        int* rest = wake ? a.wrest_src : a.rest_src;
-        int nrest = 0;
-        for (long long c0 = e0; c0 < e1; c0 += 32) {
-            const int cnt = int(e1 - c0 < 32 ? e1 - c0 : 32);
-            unsigned m = adj_chunk(pc, ns, mx, t, src + c0, cnt, wake, Xg, U, fs, P, Q, Q64);
-            if ((m >> lane) & 1u) rest[e0 + nrest + __popc(m & ((1u << lane) - 1u))] = src[c0 + lane];
-            nrest += __popc(m);
-        }
-        if (lane == 0) a.rest_cnt[2 * t + set] = nrest;
+    const long long b0 = a.nf_ptr[t], nb = a.nf_ptr[t + 1] - b0, w0 = a.wf_ptr[t], nwk = a.wf_ptr[t + 1] - w0;
+    const int cb = int((nb + 31) >> 5), cw = int((nwk + 31) >> 5);
+    if (w >= cb + cw) return;
+    for (int c = w; c < cb + cw; c += nw) {
+        const bool wake = c >= cb;
+        const long long e = 32LL * (wake ? c - cb : c), n = (wake ? nwk : nb) - e, p0 = (wake ? w0 : b0) + e;
+        const int cnt = int(n < 32 ? n : 32);
+        const unsigned m = adj_chunk(pc, ns, mx, t, (wake ? a.wf_src : a.nf_src) + p0, cnt, wake, Xg, U, fs, P, Q, Q64);
+        rest_append(a, 2 * t + (wake ? 1 : 0), p0, m, lane);
     }
     // the test side, summed over the warp's pairs, per vector
     for (int j = 0; j < K; ++j) {
@@ -708,8 +703,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, 
         for (int z = 0; z < ADJ_LSTRIDE; ++z) mine[z] = 0.f;
         __syncwarp();
     }
-    const int n = 2 * a.ntri;
-    const long long total = a.rest_off[n];
+    const long long total = (long long)*a.rest_n;
     const int K = mx.nadj;
     PairCtx pc;
     pc.a = &a;
@@ -725,12 +719,10 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, 
     for (;;) {
         const long long idx = next_rest_pair(a.next, lane);
         if (idx >= total) break;
-        const int g = rest_entry(a.rest_off, n, idx);
-        const int t = g >> 1;
-        const int set = g & 1;
+        const unsigned long long item = a.rest_item[idx];
+        const int g = int(item >> REST_SHIFT), t = g >> 1, set = g & 1;
         const bool wake = set == 1;
-        const long long e0 = wake ? a.wf_ptr[t] : a.nf_ptr[t];
-        const int s = (wake ? a.wrest_src : a.rest_src)[e0 + (idx - a.rest_off[g])];
+        const int s = (wake ? a.wf_src : a.nf_src)[item & ((1ull << REST_SHIFT) - 1)];
         const TriGeo& T = a.tri[t];
         pc.T = &T;
         for (int k = 0; k < 3; ++k) {
@@ -1221,21 +1213,24 @@ int vp_adjoint_impl(vp_ctx* ctx, const vp_assembly_options* o, int nnode, const 
         NearArgs na = near_args(ps, in);
         na.tests = d_tests;
         na.ntests = ntri;
-        int *d_rest, *d_wrest, *d_rcnt;
-        if ((r = dl.alloc(ctx, &d_rest, size_t(std::max(ps.nfptr[ntri], 1LL)))) ||
-            (r = dl.alloc(ctx, &d_wrest, size_t(std::max(ps.wfptr[ntri], 1LL)))) ||
-            (r = dl.alloc(ctx, &d_rcnt, size_t(2) * ntri)))
+        unsigned long long *d_items, *d_cnt;
+        if ((r = dl.alloc(ctx, &d_items, size_t(std::max(ps.nfptr[ntri] + ps.wfptr[ntri], 1LL)))) ||
+            (r = dl.alloc(ctx, &d_cnt, 2)))
             return r;
-        na.rest_src = d_rest;
-        na.wrest_src = d_wrest;
-        na.rest_cnt = d_rcnt;
+        VP_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        na.rest_item = d_items;
+        na.rest_n = d_cnt;
+        na.next = d_cnt + 1;
+        long long max_pairs = 0;
+        for (int t = 0; t < ntri; ++t)
+            max_pairs = std::max(max_pairs, (ps.nfptr[t + 1] - ps.nfptr[t]) + (ps.wfptr[t + 1] - ps.wfptr[t]));
         const size_t smem = sizeof(AdjChunkSh) * NEAR_WARPS;
         VP_CUDA(ctx, cudaFuncSetAttribute(adj_lanes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         const int nb = (ntri + NEAR_WARPS - 1) / NEAR_WARPS;
         vp_phase_begin(ctx, PH_ADJ_NEAR);
         na.stats = d_stats;
-        adj_lanes_kernel<<<nb, 32 * NEAR_WARPS, smem, ctx->stream>>>(na, mx);  // every vector in one pass
-        if ((r = rest_list(ctx, dl, na, nullptr))) return r;
+        const int lw = lane_warps(ctx, ntri, max_pairs);
+        adj_lanes_kernel<<<dim3(ntri, lw / NEAR_WARPS), 32 * NEAR_WARPS, smem, ctx->stream>>>(na, mx);  // every vector in one pass
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_ADJ_PAIRS);
         if (na.mixed) {  // FP32 lane partials in shared memory, FP64 totals per warp

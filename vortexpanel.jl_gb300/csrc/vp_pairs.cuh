@@ -326,7 +326,7 @@ struct FarArgs {
 };
 
 // ------------------------------------------------------------------------------------------------------------------
-// device: the near, touching and contact tiers (assemble.jl:63-321), one warp per test triangle
+// device: the near, touching and contact tiers (assemble.jl:63-321)
 
 enum { TIER_SELF = 0, TIER_EDGE = 1, TIER_VERTEX = 2, TIER_CONTACT = 3, TIER_NEAR = 4, TIER_FAR = 5 };
 enum { R_NEAR = 0, R_SELF = 1, R_EDGE = 2, R_VERT = 3, R_FAR = 4 };
@@ -341,12 +341,17 @@ struct NearArgs {
     const int* nf_src;
     const long long* wf_ptr;
     const int* wf_src;
-    int* rest_src;   // per test, at the offsets of nf_src: the body sources left to the warp-cooperative path
-    int* wrest_src;  // the same for the wake sources
-    int* rest_cnt;   // per test: counts of both (2 x ntri)
-    const long long* rest_off;  // exclusive prefix sums of rest_cnt (2 x ntri + 1): a rest pair's place in the list
-    double* pair_out;           // forward: per rest pair, its 3 x 3 block (row-major) and its 3 right hand side terms
-    unsigned long long* next;   // work counter of the pair-parallel kernels
+    // the pairs the lanes kernels leave (self, touching, contact), as one list in any order: rest_item[i] = g << 38 |
+    // position, g = 2 t + set (0 body, 1 wake), position the pair's place in nf_src / wf_src; rest_sys[i] its system
+    // (batch; null for one system); rest_n entries, taken by the pair kernels from the counter next
+    unsigned long long* rest_item;
+    int* rest_sys;
+    unsigned long long *rest_n, *next;
+    int sys;                    // this system's index in a batch
+    double* blk[2];             // forward: per pair of nf_src / wf_src, at its position less blk0, its 3 x 3 block (row-
+    long long blk0[2];          // major) and (body) its 3 right hand side terms: BLK_B / BLK_W doubles a pair
+    double* fil_out;            // forward: per test triangle and filament, the columns of its two ends (6 doubles)
+    int fil_t0;                 // the test triangle of fil_out's first row
     const long long* touch;  // sorted keys t * ntri + s
     int ntouch;
     const RulePt* rule[5];
@@ -357,6 +362,11 @@ struct NearArgs {
     double* b;
     const int* tests;
     int ntests;
+    const int* slots[2];        // column slots of the body's / wake nodes of the wake's triangles (3 each)
+    const int* col_ptr[2];      // per column: its entries in col_ent, source * 3 + corner, ascending
+    const int* col_ent[2];
+    int nfnode;                 // wake nodes at filament ends, their entries filament * 2 + end, ascending
+    const int *fnode, *fnode_ptr, *fnode_ent;
     int test_mode, near_depth, mixed;
     double far_ratio, near_ratio, corner_angle, contact_rel, kernel_far;
     float kernel_far32;  // kernel_far in FP32 (the FP32 point evaluators)
@@ -2201,48 +2211,23 @@ int setup_pairs(vp_ctx* ctx, const PairInput& in, int ph_setup, int ph_classify,
 // the arguments of the near, touching and contact kernels that come from the set-up (A, b, tests, stats and the
 // rest lists are the caller's)
 // ---- the rest pairs (self, touching, contact) as one list, for the pair-parallel kernels ---------------------------
-// The lanes kernels leave, per test triangle t and source set (0 body, 1 wake), rest_cnt[2t + set] pairs at the
-// start of its segment of rest_src / wrest_src. Their exclusive prefix sums number the pairs 0 .. total - 1 in the
-// order (t, set, position); a warp of a pair-parallel kernel takes the next number from a counter.
+// A lanes kernel's warp appends the pairs it leaves of its chunk to one list (one atomic a chunk); a warp of a
+// pair-parallel kernel takes the next entry from a counter. The list's order differs from run to run and does not
+// matter: the forward writes each pair's block to the pair's own place, and the adjoint's sums are exact in any order.
 
-constexpr int SCAN_NT = 1024;
+constexpr int REST_SHIFT = 38;  // position bits of an entry
 
-// rest_off[i] = sum of cnt[0 .. i - 1] for i = 0 .. n (one block of SCAN_NT threads)
-__global__ void __launch_bounds__(SCAN_NT) rest_scan_kernel(const int* __restrict__ cnt, int n, long long* off) {
-    __shared__ long long s[SCAN_NT];
-    __shared__ long long carry;
-    const int i0 = threadIdx.x;
-    if (i0 == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < n; base += SCAN_NT) {
-        const int i = base + i0;
-        const long long v = i < n ? (long long)cnt[i] : 0;
-        s[i0] = v;
-        __syncthreads();
-        for (int o = 1; o < SCAN_NT; o <<= 1) {
-            const long long u = i0 >= o ? s[i0 - o] : 0;
-            __syncthreads();
-            s[i0] += u;
-            __syncthreads();
-        }
-        if (i < n) off[i] = carry + s[i0] - v;
-        __syncthreads();
-        if (i0 == SCAN_NT - 1) carry += s[SCAN_NT - 1];
-        __syncthreads();
+// append this chunk's pairs (the lanes of mask; list position p0 + lane) of entry g to the list; the whole warp calls
+__device__ __forceinline__ void rest_append(const NearArgs& a, int g, long long p0, unsigned mask, int lane) {
+    if (!mask) return;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(a.rest_n, (unsigned long long)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if ((mask >> lane) & 1u) {
+        at += __popc(mask & ((1u << lane) - 1u));
+        a.rest_item[at] = ((unsigned long long)g << REST_SHIFT) | (unsigned long long)(p0 + lane);
+        if (a.rest_sys) a.rest_sys[at] = a.sys;
     }
-    if (i0 == 0) off[n] = carry;
-}
-
-// the (t, set) entry g = 2 t + set of rest pair idx: the largest g with off[g] <= idx (0 <= idx < off[n], so g < n
-// and off[g + 1] > idx: empty entries are skipped)
-__device__ __forceinline__ int rest_entry(const long long* __restrict__ off, int n, long long idx) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (off[mid] <= idx) lo = mid;
-        else hi = mid;
-    }
-    return lo;
 }
 
 // the next rest pair of this warp (all lanes call it together)
@@ -2252,25 +2237,13 @@ __device__ __forceinline__ long long next_rest_pair(unsigned long long* next, in
     return (long long)__shfl_sync(0xffffffffu, v, 0);
 }
 
-// the offsets of the rest pairs (after the lanes kernel) and a zeroed work counter; with `total`, the number of rest
-// pairs is copied to the host (the stream is synchronised)
-int rest_list(vp_ctx* ctx, DevList& dl, NearArgs& na, long long* total) {
-    long long* d_off;
-    unsigned long long* d_next;
-    int r;
-    const int n = 2 * na.ntri;
-    if ((r = dl.alloc(ctx, &d_off, size_t(n) + 1)) || (r = dl.alloc(ctx, &d_next, 1))) return r;
-    rest_scan_kernel<<<1, SCAN_NT, 0, ctx->stream>>>(na.rest_cnt, n, d_off);
-    ctx->launches++;
-    VP_CUDA(ctx, cudaGetLastError());
-    VP_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), ctx->stream));
-    na.rest_off = d_off;
-    na.next = d_next;
-    if (total) {
-        VP_CUDA(ctx, vp_d2h(ctx, total, d_off + n, sizeof(long long)));
-        VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    }
-    return VP_OK;
+// warps per test triangle of a lanes kernel (each takes every so many chunks of 32 pairs): enough that the grid fills
+// the device about ten times over, no more than the longest list has chunks; a multiple of the warps of a CTA
+int lane_warps(vp_ctx* ctx, long long ntests, long long max_pairs) {
+    const long long want = (10LL * 12 * std::max(ctx->nsm, 1) + ntests - 1) / std::max(ntests, 1LL);
+    const long long have = (max_pairs + 31) / 32;
+    const long long w = std::max(1LL, std::min(want, have));
+    return int((w + NEAR_WARPS - 1) / NEAR_WARPS) * NEAR_WARPS;
 }
 
 // CTAs of a persistent pair-parallel kernel: as many as stay resident on every SM
