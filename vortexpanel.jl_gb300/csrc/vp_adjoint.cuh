@@ -18,10 +18,90 @@ struct ExactShape {
     T Om;        // solid angle
 };
 
+// sv_exact_vjp in FP64 by few FP64 instructions (vp_f64.cuh): one reciprocal of each denominator, the inverse lengths
+// from the square roots' reciprocal square roots
+__device__ __forceinline__ double sv_exact_vjp_f64(const SrcKern<double>& S, v3<double> r0, v3<double> r1, v3<double> r2,
+                                                   v3<double> r, v3<double> m, int side, double plane_tol,
+                                                   v3<double>& g0, v3<double>& g1, v3<double>& g2,
+                                                   ExactShape<double>& sh) {
+    const double i4pi = 1.0 / (4.0 * vp_pi<double>());
+    const v3<double> R[3] = {r0, r1, r2};
+    double l[3], il[3], p[3], lbar[3] = {0, 0, 0}, s = 0;
+    v3<double> gr[3] = {mk3(0.0, 0.0, 0.0), mk3(0.0, 0.0, 0.0), mk3(0.0, 0.0, 0.0)};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) l[a] = f64::sqrt_inv(dot(R[a], R[a]), il[a]);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const int i = e, j = (e + 1) % 3;
+        const v3<double> ri = R[i], rj = R[j];
+        p[e] = dot(ri, rj);
+        const double num = l[i] + l[j] + S.len[e], n2 = 2.0 * f64::rcp(num);
+        const double coef = dot(S.nu[e], m) * i4pi;
+        double rden, L;
+        if (p[e] < 0.0) {
+            const v3<double> c = cross(ri, rj);
+            const double den = l[i] * l[j] - p[e], rc2 = f64::rcp(norm2(c));
+            rden = f64::rcp(den);
+            L = f64::log<-1>(num * num * (den * rc2));
+            // d log q: li -> lj/den, lj -> li/den, p -> -1/den, c2 -> -1/c2; c2 = |ri x rj|^2: d/dri = 2 rj x c
+            const double k2 = (-2.0 * coef) * rc2;
+            gr[i] += k2 * cross(rj, c);
+            gr[j] += k2 * cross(c, ri);
+            lbar[i] += coef * (n2 + l[j] * rden);
+            lbar[j] += coef * (n2 + l[i] * rden);
+        } else {
+            rden = f64::rcp(l[i] * l[j] + p[e]);
+            L = f64::log<-1>(num * num * rden);
+            lbar[i] += coef * (n2 - l[j] * rden);
+            lbar[j] += coef * (n2 - l[i] * rden);
+        }
+        const double cp = -coef * rden;
+        gr[i] += cp * rj;
+        gr[j] += cp * ri;
+        s += L * coef;
+        sh.L[e] = L;
+        sh.dLdlen[e] = n2;
+    }
+    const double nm = dot(S.n, m) * i4pi;
+    const v3<double> c12 = cross(r1, r2);
+    const double N = dot(r0, c12);
+    const double D = l[0] * l[1] * l[2] + p[0] * l[2] + p[2] * l[1] + p[1] * l[0];
+    if (fabs(dot(r, S.n)) <= plane_tol * S.diam) {
+        const v3<double> q[3] = {-r0, -r1, -r2};
+        sh.Om = side == 0 ? 0.0 : double(side) * 2.0 * vp_pi<double>() * inplane_fraction_rel(q, S.n, S.area, plane_tol);
+    } else {
+        sh.Om = 2.0 * f64::atan2(N, D);
+    }
+    // as in the general form: the in-plane branch keeps the one-sided limit of the derivative along the normal
+    const double nd2 = N * N + D * D;
+    if (nd2 > 0.0) {
+        const double h = 2.0 * f64::rcp(nd2);
+        const double Nb = nm * D * h, Db = -nm * N * h;
+        gr[0] += Nb * c12;
+        gr[1] += Nb * cross(r2, r0);
+        gr[2] += Nb * cross(r0, r1);
+        lbar[0] += Db * (l[1] * l[2] + p[1]);
+        lbar[1] += Db * (l[0] * l[2] + p[2]);
+        lbar[2] += Db * (l[0] * l[1] + p[0]);
+        const double b0 = Db * l[0], b1 = Db * l[1], b2 = Db * l[2];
+        gr[0] += b2 * r1 + b1 * r2;
+        gr[1] += b2 * r0 + b0 * r2;
+        gr[2] += b1 * r0 + b0 * r1;
+    }
+    s += sh.Om * nm;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) gr[a] += (lbar[a] * il[a]) * R[a];
+    g0 = gr[0];
+    g1 = gr[1];
+    g2 = gr[2];
+    return s;
+}
+
 // s = w·m of the exact kernel at fixed shape (nu, len, n from the source) and ds/dr_a.
 template <class T, class M = KMath<T>>
 __device__ __forceinline__ T sv_exact_vjp(const SrcKern<T>& S, v3<T> r0, v3<T> r1, v3<T> r2, v3<T> r, v3<T> m,
                                           int side, T plane_tol, v3<T>& g0, v3<T>& g1, v3<T>& g2, ExactShape<T>& sh) {
+    if constexpr (kPlain64<T, M>) return sv_exact_vjp_f64(S, r0, r1, r2, r, m, side, plane_tol, g0, g1, g2, sh);
     const T i4pi = T(1) / (T(4) * vp_pi<T>());
     const v3<T> R[3] = {r0, r1, r2};
     T l[3] = {M::sqrt(dot(r0, r0)), M::sqrt(dot(r1, r1)), M::sqrt(dot(r2, r2))};
@@ -219,10 +299,55 @@ __device__ __forceinline__ bool sv_exact_vjp_split(const SrcKern<double>& S, v3<
     return true;
 }
 
+// The multipole form in FP64 with its derivatives, by few FP64 instructions (as sv_far_f64): with F·m = A r·m + sum_a c_a
+// d_a·m, everything unscaled by the area's factor k = area / 4pi, which is returned: w = k wu, s = k su, ds/dr = k gu,
+// ds/dd_a = k gdu_a, ds/darea = su / 4pi. e_a = dF·m/d(d_a·r) serves both ds/dr and ds/dd_a.
+__device__ __forceinline__ double sv_far_vjp_f64(const SrcKern<double>& S, v3<double> r, v3<double> m, v3<double>& wu,
+                                                 double& su, v3<double>& gu, v3<double>* gdu) {
+    double iR2, iR3;
+    inv_r23(dot(r, r), iR2, iR3);
+    const double iR5 = iR3 * iR2, iR7 = iR5 * iR2, iR9 = iR7 * iR2, iR11 = iR9 * iR2;
+    const double rm = dot(r, m);
+    double dr[3] = {dot(S.d[0], r), dot(S.d[1], r), 0}, dm[3] = {dot(S.d[0], m), dot(S.d[1], m), 0};
+    dr[2] = -(dr[0] + dr[1]);
+    dm[2] = -(dm[0] + dm[1]);
+    double S2 = 0, S3 = 0, T1 = 0, Sd = 0, B = 0, c[3], e[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double dd = dot(S.d[a], S.d[a]), dr2 = dr[a] * dr[a];
+        S2 += dr2;
+        S3 += dr2 * dr[a];
+        T1 += dd * dr[a];
+        Sd += dd;
+        const double q = dd * (1.0 / 20) - 0.25 * dr[a], u = iR7 * dr[a];
+        c[a] = iR5 * q - (0.25 * iR7) * dr2;
+        e[a] = rm * (1.25 * u - 0.25 * iR7 * dd + (1.75 * iR9) * dr2) - dm[a] * (0.25 * iR5 + 0.5 * u);
+        const double gdd2 = dm[a] * (0.1 * iR5) - rm * (0.25 * iR5 + 0.5 * u);  // 2 dF·m/d dd_a
+        B += dm[a] * ((0.875 * iR9) * dr2 - 2.5 * iR7 * q);
+        gdu[a] = e[a] * r + gdd2 * S.d[a] + c[a] * m;
+    }
+    const double P = 0.625 * S2 - 0.25 * T1, S7 = (7.0 / 12) * S3;
+    const double A = iR3 - iR5 * (Sd * 0.125) + iR7 * P + iR9 * S7;
+    B += rm * (-1.5 * iR5 + iR7 * (0.3125 * Sd) - 3.5 * iR9 * P - 4.5 * iR11 * S7);
+    wu = A * r + (c[0] - c[2]) * S.d[0] + (c[1] - c[2]) * S.d[1];
+    gu = A * m + (e[0] - e[2]) * S.d[0] + (e[1] - e[2]) * S.d[1] + (2.0 * B) * r;
+    su = A * rm + (c[0] - c[2]) * dm[0] + (c[1] - c[2]) * dm[1];
+    return S.area * (1.0 / (4.0 * vp_pi<double>()));
+}
+
 // s = w·m of the multipole form (source_triangle.jl:100-119) and its derivatives with respect to r = x - c, to the
 // corner offsets d_a (gd) and the area (ga)
 template <class T>
 __device__ __forceinline__ T sv_far_vjp(const SrcKern<T>& S, v3<T> r, v3<T> m, v3<T>& gr, v3<T>* gd, T& ga) {
+    if constexpr (sizeof(T) == 8) {
+        v3<double> w;
+        double su;
+        const double k = sv_far_vjp_f64(S, r, m, w, su, gr, gd);
+        gr = k * gr;
+        for (int a = 0; a < 3; ++a) gd[a] = k * gd[a];
+        ga = su * (1.0 / (4.0 * vp_pi<double>()));
+        return k * su;
+    }
     const T k = S.area / (T(4) * vp_pi<T>());
     T R2 = dot(r, r);
     T iR2, iR3;

@@ -142,6 +142,15 @@ template <class T>
 __device__ __forceinline__ T adj_point_far_multi(AdjSums<T>* acc, int nk, const T* Wn, const SrcKern<T>& S, T l0, T l1,
                                                  T l2, v3<T> r, v3<T> m, v3<T>& gx) {
     v3<T> gd[3];
+    if constexpr (sizeof(T) == 8) {  // unscaled; the area's factor goes to the weights
+        v3<T> w, gu;
+        T su, Wk[ADJ_VEC_MAX];
+        const T k = sv_far_vjp_f64(S, r, m, w, su, gu, gd);
+        for (int j = 0; j < ADJ_VEC_MAX; ++j) Wk[j] = k * Wn[j];
+        adj_acc_far(acc, nk, Wk, l0, l1, l2, w, gu, gd, su * f64::rcp(S.area));
+        gx = k * gu;
+        return k * su;
+    }
     T ga;
     T sv = sv_far_vjp(S, r, m, gx, gd, ga);
     const v3<T> w = sv_far(S, r);

@@ -114,13 +114,9 @@ __device__ __forceinline__ void far_body(const FarArgs& a, const int tile) {
                 const FarTest<T>& q = ts[i];
                 bool far = false;
                 if (sv && q.valid) {
-                    if (sizeof(T) == 8) {
-                        far = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
-                    } else {
-                        int f = far_test32(q.cf, scf, a.ratio32);
-                        if (f < 0) f = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
-                        far = f == 1;
-                    }
+                    int f = far_test32(q.cf, scf, a.ratio32);
+                    if (f < 0) f = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
+                    far = f == 1;
                 }
                 if (far) {
                     v3<T> P[3] = {mk3(T(0), T(0), T(0)), mk3(T(0), T(0), T(0)), mk3(T(0), T(0), T(0))};
@@ -133,12 +129,22 @@ __device__ __forceinline__ void far_body(const FarArgs& a, const int tile) {
                         P[2] += q.wpsi[p][2] * w;
                     }
                     v3<T> nT = mk3(q.n[0], q.n[1], q.n[2]);
+                    if constexpr (sizeof(T) == 8) {  // P.(n x gam_b) = gam_b.(P x n), and the gam_b sum to zero
 #pragma unroll
-                    for (int bb = 0; bb < 3; ++bb) {
-                        v3<T> m = cross(nT, gam[bb]);
-                        out[0 * 3 + bb] = dot(P[0], m);
-                        out[1 * 3 + bb] = dot(P[1], m);
-                        out[2 * 3 + bb] = dot(P[2], m);
+                        for (int aa = 0; aa < 3; ++aa) {
+                            const v3<T> C = cross(P[aa], nT);
+                            out[3 * aa] = dot(C, gam[0]);
+                            out[3 * aa + 1] = dot(C, gam[1]);
+                            out[3 * aa + 2] = -(out[3 * aa] + out[3 * aa + 1]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int bb = 0; bb < 3; ++bb) {
+                            v3<T> m = cross(nT, gam[bb]);
+                            out[0 * 3 + bb] = dot(P[0], m);
+                            out[1 * 3 + bb] = dot(P[1], m);
+                            out[2 * 3 + bb] = dot(P[2], m);
+                        }
                     }
                     rb[i][0] -= sig * dot(P[0], nT);
                     rb[i][1] -= sig * dot(P[1], nT);
@@ -230,7 +236,7 @@ struct NearChunkSh {
     double acc[32][9];     // per pair: sum of W psi_a w (FP64 evaluations)
     float accf[32][9];     // per pair: the same sums of the FP32 evaluations
     int off[33];           // points before each pair
-    int qp[64], qk[64];    // queued FP64 points: pair, point within the pair
+    int qp[64], qk[64];    // queued FP64 points (mixed): pair, point within the pair
 };
 
 constexpr int BLK_B = 12, BLK_W = 9;  // doubles of a pair's block: body pairs carry their right hand side terms
@@ -282,7 +288,48 @@ __device__ void near_point64(const NearArgs& a, const TriGeo& T, const TriGeo& S
     }
 }
 
+// FP64 path: the nr points of leaf `code` of a pair with frame E (x_T,k - v_S,a), summed: P[3a + z] = sum W psi_a w_z
+__device__ __forceinline__ void near_leaf64(const NearArgs& a, const TriGeo& T, const TriGeo& S, const double* E, int code,
+                                            double* P) {
+    float bf[9];
+    leaf_corners32(code, bf);
+    double b[9];
+    for (int z = 0; z < 9; ++z) b[z] = double(bf[z]);
+    SrcKern<double> K;
+    const v3<double> c = ld3(S.c);
+    for (int z = 0; z < 3; ++z) {
+        K.d[z] = ld3(S.x + 3 * z) - c;
+        K.nu[z] = ld3(S.nu + 3 * z);
+        K.len[z] = S.len[z];
+    }
+    K.n = ld3(S.n);
+    K.area = S.area;
+    K.diam = S.diam;
+    const double fd = a.kernel_far * K.diam, fd2 = fd * fd, frac = ldexp(1.0, -2 * (code >> 6)) * T.area;
+    const int nr = a.nrule[R_NEAR];
+#pragma unroll 1
+    for (int q = 0; q < nr; ++q) {
+        const RulePt m = a.rule[R_NEAR][q];
+        const double l0 = m.l0 * b[0] + m.l1 * b[3] + m.l2 * b[6];
+        const double l1 = m.l0 * b[1] + m.l1 * b[4] + m.l2 * b[7];
+        const double l2 = m.l0 * b[2] + m.l1 * b[5] + m.l2 * b[8];
+        const v3<double> ra = l0 * ld3(E + 0) + l1 * ld3(E + 9) + l2 * ld3(E + 18);
+        const v3<double> rb = l0 * ld3(E + 3) + l1 * ld3(E + 12) + l2 * ld3(E + 21);
+        const v3<double> rc = l0 * ld3(E + 6) + l1 * ld3(E + 15) + l2 * ld3(E + 24);
+        const v3<double> r = ra + K.d[0];
+        const v3<double> w = dot(r, r) > fd2 ? sv_far(K, r) : sv_exact3(K, ra, rb, rc, r, 0, 1e-12);
+        const v3<double> psi = test_weights(a.test_mode, l0, l1, l2);
+        const double W = m.w * frac, ps[3] = {W * psi.x, W * psi.y, W * psi.z};
+        for (int ai = 0; ai < 3; ++ai) {
+            P[3 * ai + 0] += ps[ai] * w.x;
+            P[3 * ai + 1] += ps[ai] * w.y;
+            P[3 * ai + 2] += ps[ai] * w.z;
+        }
+    }
+}
+
 // list: the chunk's sources, p0 the first one's place in nf_src / wf_src; returns the lanes of the rest pairs
+template <bool MIXED>
 __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* list, int cnt, bool wake, long long p0,
                                unsigned long long* P, unsigned long long* Q, unsigned long long& Q64) {
     const NearArgs& a = *pc.a;
@@ -315,23 +362,33 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
     const Fp32Guard g{PAIR_GUARD};
     int nq = 0;
     unsigned long long n64 = 0;
-    for (int i0 = 0; i0 < total; i0 += 32) {
+    if constexpr (!MIXED) {  // FP64: a lane takes a whole leaf, whose points' sums are added to the pair's once
+        for (int i0 = 0; i0 < total; i0 += 32 * nr) {
+            const int i = i0 + lane * nr;
+            int p = 32 + lane;
+            double P64[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            if (i < total) {
+                int lo = 0, hi = 31;
+                while (lo < hi) {
+                    int mid = (lo + hi + 1) >> 1;
+                    if (ns.off[mid] <= i) lo = mid;
+                    else hi = mid - 1;
+                }
+                p = lo;
+                near_leaf64(a, T, wake ? a.wtri[list[p]] : a.tri[list[p]], ns.pl.E64(p),
+                            ns.pl.leaf[p][(i - ns.off[p]) / nr], P64);
+            }
+            seg_accumulate<9>(ns.accf, ns.acc, lane, p, P64);
+        }
+        n64 = (unsigned long long)total;
+    }
+    for (int i0 = 0; MIXED && i0 < total; i0 += 32) {
         const int i = i0 + lane;
         const bool v = i < total;
         int p = 32 + lane, k = 0;
         float vals[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         bool need = false;
-        if (v && !a.mixed) {  // FP64: every point through the FP64 queue
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (ns.off[mid] <= i) lo = mid;
-                else hi = mid - 1;
-            }
-            p = lo;
-            k = i - ns.off[p];
-            need = true;
-        } else if (v) {
+        if (v) {
             int lo = 0, hi = 31;
             while (lo < hi) {
                 int mid = (lo + hi + 1) >> 1;
@@ -385,7 +442,7 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
                 need = true;
             }
         }
-        if (a.mixed) seg_accumulate<9>(ns.accf, ns.acc, lane, p, vals);  // flagged points add zero here, their FP64 value when drained
+        seg_accumulate<9>(ns.accf, ns.acc, lane, p, vals);  // flagged points add zero here, their FP64 value when drained
         unsigned m = __ballot_sync(FULL, need);
         if (m) {
             int pos = nq + __popc(m & ((1u << lane) - 1u));
@@ -449,6 +506,7 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
 
 // near tier, one pair per lane; the other pairs are listed for near_kernel_pairs. Warp w of nw of test triangle t: every
 // nw-th chunk of its body and wake lists.
+template <bool MIXED>
 __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, const int w, const int nw,
                                                 NearChunkSh& sh) {
     const int lane = threadIdx.x & 31;
@@ -465,7 +523,7 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
         const bool wake = c >= cb;
         const long long e = 32LL * (wake ? c - cb : c), n = (wake ? nwk : nb) - e, p0 = (wake ? w0 : b0) + e;
         const int cnt = int(n < 32 ? n : 32);
-        const unsigned m = near_chunk(pc, sh, t, (wake ? a.wf_src : a.nf_src) + p0, cnt, wake, p0, P, Q, Q64);
+        const unsigned m = near_chunk<MIXED>(pc, sh, t, (wake ? a.wf_src : a.nf_src) + p0, cnt, wake, p0, P, Q, Q64);
         rest_append(a, 2 * t + (wake ? 1 : 0), p0, m, lane);
         __syncwarp();
     }
@@ -478,14 +536,16 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
     }
 }
 
-// the kernels of the non-far tiers take one system's arguments by value, or (BATCH) those of system work[i].x from sys
-template <bool BATCH>
-__global__ void __launch_bounds__(32 * NEAR_WARPS) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
+// the kernels of the non-far tiers take one system's arguments by value, or (BATCH) those of system work[i].x from sys.
+// MIXED or FP64 by template: with both paths in one kernel the mixed one ran at 216 registers instead of 158 (near
+// phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles).
+template <bool BATCH, bool MIXED>
+__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
                                                                   const int2* __restrict__ work) {
     extern __shared__ __align__(16) unsigned char near_smem[];
     NearChunkSh* shm = reinterpret_cast<NearChunkSh*>(near_smem);
     const int2 wk = work[blockIdx.x];
-    near_lanes_body(BATCH ? sys[wk.x] : a, wk.y, blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), gridDim.y * NEAR_WARPS,
+    near_lanes_body<MIXED>(BATCH ? sys[wk.x] : a, wk.y, blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), gridDim.y * NEAR_WARPS,
                     shm[threadIdx.x >> 5]);
 }
 
@@ -1103,7 +1163,8 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         (BATCH && (r = dl.alloc(ctx, &d_sysof, most_items))))
         return r;
     const size_t near_smem = sizeof(NearChunkSh) * NEAR_WARPS;
-    VP_CUDA(ctx, cudaFuncSetAttribute(near_kernel_lanes<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(near_smem)));
+    auto lanes = jobs[0]->ps.mixed ? near_kernel_lanes<BATCH, true> : near_kernel_lanes<BATCH, false>;
+    VP_CUDA(ctx, cudaFuncSetAttribute(lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(near_smem)));
     const int npb = persistent_blocks(ctx, near_kernel_pairs<BATCH>, 32 * NEAR_WARPS, 0);
     for (auto& pass : passes) {
         // the systems' places in the workspace, the work lists: all test triangles, then by colour
@@ -1152,8 +1213,7 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         VP_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), ctx->stream));
         vp_phase_begin(ctx, PH_NEAR);
         const int lw = lane_warps(ctx, ntests, max_pairs);
-        near_kernel_lanes<BATCH><<<dim3(ntests, lw / NEAR_WARPS), 32 * NEAR_WARPS, near_smem, ctx->stream>>>(a1, d_args,
-                                                                                                            d_work);
+        lanes<<<dim3(ntests, lw / NEAR_WARPS), 32 * NEAR_WARPS, near_smem, ctx->stream>>>(a1, d_args, d_work);
         ctx->launches++;
         if (nfil > 0) {
             near_kernel_filaments<BATCH><<<dim3((ntests + NEAR_WARPS - 1) / NEAR_WARPS, (nfil + 31) / 32), 32 * NEAR_WARPS, 0,

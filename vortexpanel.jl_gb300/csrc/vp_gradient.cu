@@ -177,13 +177,9 @@ __global__ void __launch_bounds__(FAR_NT) adj_far_kernel(AdjFarArgs a) {
             const AdjFarTest<T>& q = ts[i];
             bool far = false;
             if (sv && q.t >= 0) {
-                if (sizeof(T) == 8) {
-                    far = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
-                } else {
-                    int f = far_test32(q.cf, scf, a.ratio32);
-                    if (f < 0) f = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
-                    far = f == 1;
-                }
+                int f = far_test32(q.cf, scf, a.ratio32);
+                if (f < 0) f = far_exact64(q.c64, q.diam64, a.sgeo[set][s].c, a.sgeo[set][s].diam, a.ratio);
+                far = f == 1;
             }
             v3<T> Xg[K][3], U[K];
             T fs[K];
@@ -371,19 +367,21 @@ __device__ void adj_point64(const NearArgs& a, const TriGeo& T, const TriGeo& S,
     double Wn[ADJ_MAX];
     for (int j = 0; j < ADJ_MAX; ++j) Wn[j] = W * (nu[j][0] * psi.x + nu[j][1] * psi.y + nu[j][2] * psi.z);
     v3<double> R[3];
-    for (int c = 0; c < 3; ++c)
-        R[c] = mk3(l0 * (T.x[0] - S.x[3 * c]) + l1 * (T.x[3] - S.x[3 * c]) + l2 * (T.x[6] - S.x[3 * c]),
+    if (!a.mixed) {
+        const double* E = ns.pl.E64(p);
+        for (int c = 0; c < 3; ++c) R[c] = l0 * ld3(E + 3 * c) + l1 * ld3(E + 9 + 3 * c) + l2 * ld3(E + 18 + 3 * c);
+    } else
+        for (int c = 0; c < 3; ++c)
+            R[c] = mk3(l0 * (T.x[0] - S.x[3 * c]) + l1 * (T.x[3] - S.x[3 * c]) + l2 * (T.x[6] - S.x[3 * c]),
                    l0 * (T.x[1] - S.x[3 * c + 1]) + l1 * (T.x[4] - S.x[3 * c + 1]) + l2 * (T.x[7] - S.x[3 * c + 1]),
                    l0 * (T.x[2] - S.x[3 * c + 2]) + l1 * (T.x[5] - S.x[3 * c + 2]) + l2 * (T.x[8] - S.x[3 * c + 2]));
-    v3<double> x = mk3(l0 * T.x[0] + l1 * T.x[3] + l2 * T.x[6], l0 * T.x[1] + l1 * T.x[4] + l2 * T.x[7],
-                       l0 * T.x[2] + l1 * T.x[5] + l2 * T.x[8]);
-    v3<double> r = x - ld3(S.c);
     SrcKern<double> Kd;
     for (int z = 0; z < 3; ++z) {
         Kd.d[z] = mk3(S.x[3 * z] - S.c[0], S.x[3 * z + 1] - S.c[1], S.x[3 * z + 2] - S.c[2]);
         Kd.nu[z] = ld3(S.nu + 3 * z);
         Kd.len[z] = S.len[z];
     }
+    const v3<double> r = R[0] + Kd.d[0];
     Kd.n = ld3(S.n);
     Kd.area = S.area;
     Kd.diam = S.diam;

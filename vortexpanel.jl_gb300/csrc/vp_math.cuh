@@ -7,6 +7,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "vp_f64.cuh"
+
 template <class T>
 struct v3 {
     T x, y, z;
@@ -40,20 +42,20 @@ template <class T> __device__ __forceinline__ T vnorm(v3<T> a) { return vsqrt(do
 
 // 1/R^2 and 1/R^3 of the multipole forms from R^2. FP32: one reciprocal square root (rsqrtf, a few ulp, far below the
 // multipole's truncation error and FP32's own rounding of the sums) instead of a square root and two IEEE divisions,
-// the far tiers' special-function bound. FP64: the square root and the divisions.
+// the far tiers' special-function bound. FP64: f64::rsqrt.
 __device__ __forceinline__ void inv_r23(float R2, float& iR2, float& iR3) {
     const float iR = rsqrtf(R2);
     iR2 = iR * iR;
     iR3 = iR2 * iR;
 }
 __device__ __forceinline__ void inv_r23(double R2, double& iR2, double& iR3) {
-    const double R = sqrt(R2);
-    iR2 = 1.0 / R2;
-    iR3 = iR2 / R;
+    const double iR = f64::rsqrt(R2);
+    iR2 = iR * iR;
+    iR3 = iR2 * iR;
 }
 
 // The scalar functions of the exact kernel and its derivatives, as a policy of the evaluation.
-// KMath<T>: the plain FP32 or FP64 functions.
+// KMath<T>: the plain FP32 functions, or FP64 ones of few FP64 instructions (vp_f64.cuh).
 // KMathHyb: the FP64 evaluation of the mixed-precision path, for the points that FP32 cannot take (near a source's
 // corners and edges, where the offsets, cross products and the solid angle's numerator and denominator cancel).
 // Those quantities stay FP64; the functions applied to them are FP32-based:
@@ -69,6 +71,18 @@ struct KMath {
     static __device__ __forceinline__ T log(T x) { return vlog(x); }
     static __device__ __forceinline__ T atan2(T y, T x) { return vatan2(y, x); }
 };
+
+template <>
+struct KMath<double> {
+    static constexpr bool hybrid = false;
+    static __device__ __forceinline__ double sqrt(double x) { return f64::sqrt(x); }
+    static __device__ __forceinline__ double div(double a, double b) { return f64::div(a, b); }
+    static __device__ __forceinline__ double log(double x) { return f64::log(x); }
+    static __device__ __forceinline__ double atan2(double y, double x) { return f64::atan2(y, x); }
+};
+// whether T and M are the plain FP64 evaluation
+template <class T, class M>
+constexpr bool kPlain64 = sizeof(T) == 8 && !M::hybrid;
 
 // the FP64 functions out of line, for KMathHyb's rare out-of-range arguments (kept off the hot path's registers)
 static __device__ __noinline__ double f64_sqrt(double x) { return sqrt(x); }
@@ -148,6 +162,9 @@ __device__ __forceinline__ T edge_log_n(v3<T> ri, v3<T> rj, T li, T lj, T d) {
     T num = li + lj + d;
     if constexpr (M::hybrid) {
         if (p >= T(0)) return M::log1p(M::div(d * num, li * lj + p));
+    } else if constexpr (sizeof(T) == 8) {
+        const T q = p < T(0) ? f64::div(li * lj - p, norm2(cross(ri, rj))) : f64::rcp(li * lj + p);
+        return f64::log<-1>(num * num * q);
     } else {
         if (sizeof(T) == 4 && p >= T(0)) return T(log1pf(float(d * num / (li * lj + p))));
     }
@@ -289,9 +306,34 @@ __device__ __forceinline__ bool sv_exact3_guarded(const SrcKern<float>& S, v3<fl
     return true;
 }
 
+// The multipole form in FP64, by few FP64 instructions (a third of the plain form's, which multiplies out every corner's
+// vectors: about 70 against 230 a point): with dr_a = d_a.r, dd_a = |d_a|^2 and the d_a summing to zero, the velocity is
+// area/4pi (A r + sum_a c_a d_a), A the sums' scalar and c_a a scalar per corner.
+__device__ __forceinline__ v3<double> sv_far_f64(const SrcKern<double>& S, v3<double> r) {
+    double iR2, iR3;
+    inv_r23(dot(r, r), iR2, iR3);
+    const double iR5 = iR3 * iR2, iR7 = iR5 * iR2, iR9 = iR7 * iR2;
+    double dr[3] = {dot(S.d[0], r), dot(S.d[1], r), 0};
+    dr[2] = -(dr[0] + dr[1]);
+    double S2 = 0, S3 = 0, T1 = 0, Sd = 0, c[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double dd = dot(S.d[a], S.d[a]), dr2 = dr[a] * dr[a];
+        S2 += dr2;
+        S3 += dr2 * dr[a];
+        T1 += dd * dr[a];
+        Sd += dd;
+        c[a] = iR5 * (dd * (1.0 / 20) - 0.25 * dr[a]) - (0.25 * iR7) * dr2;
+    }
+    const double A = iR3 - iR5 * (Sd * 0.125) + iR7 * (0.625 * S2 - 0.25 * T1) + iR9 * ((7.0 / 12) * S3);
+    const double k = S.area * (1.0 / (4.0 * vp_pi<double>()));
+    return (k * A) * r + (k * (c[0] - c[2])) * S.d[0] + (k * (c[1] - c[2])) * S.d[1];
+}
+
 // source_velocity_far (source_triangle.jl:100-119): monopole + quadrupole + octupole about the centroid
 template <class T>
 __device__ __forceinline__ v3<T> sv_far(const SrcKern<T>& S, v3<T> r) {
+    if constexpr (sizeof(T) == 8) return sv_far_f64(S, r);
     T R2 = dot(r, r);
     T iR2, iR3;
     inv_r23(R2, iR2, iR3);

@@ -534,7 +534,6 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, FwdAcc& acc, double
         v3<double> ra = l0 * ld3(sh.E + 0) + l1 * ld3(sh.E + 9) + l2 * ld3(sh.E + 18);
         v3<double> rb = l0 * ld3(sh.E + 3) + l1 * ld3(sh.E + 12) + l2 * ld3(sh.E + 21);
         v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
-        v3<double> r = l0 * ld3(sh.D) + l1 * ld3(sh.D + 3) + l2 * ld3(sh.D + 6);
         SrcKern<double> S;
         for (int k = 0; k < 3; ++k) {
             S.d[k] = ld3(sh.Sd + 3 * k);
@@ -544,6 +543,7 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, FwdAcc& acc, double
         S.n = ld3(sh.Sn);
         S.area = sh.Sarea;
         S.diam = sh.Sdiam;
+        const v3<double> r = ra + S.d[0];
         double fd = pc.a->kernel_far * S.diam;
         // the mixed path's FP64 points (where FP32 cancels): what cancels in FP64, the functions on it in FP32
         // (sv_exact3_split), or FP64 geometry with FP32-based functions (KMathHyb) where the split leaves FP32's range
@@ -793,8 +793,8 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, AdjAcc& acc, double
     double sv;
     if (pc.kind == 0) {
         v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
-        v3<double> r = l0 * ld3(sh.D) + l1 * ld3(sh.D + 3) + l2 * ld3(sh.D + 6);
         SrcKern<double> S = src64(sh);
+        const v3<double> r = ra + S.d[0];
         double fd = pc.a->kernel_far * S.diam;
         if (dot(r, r) > fd * fd)
             sv = adj_point_far_multi(acc.d, pc.nadj, Wn, S, l0, l1, l2, r, pc.m, gx);
@@ -1661,12 +1661,16 @@ __device__ void vertex_rule(PairCtx& pc, Acc& acc, int k) {
 // A warp takes up to 32 sources of its test triangle at once. Each lane decides its own pair's tier (FP32 with the
 // reference's FP64 test where FP32 cannot decide, exactly as pair_rule / wake_pair_rule) and, for a pair in the near
 // tier, walks near_pieces' quadtree to its leaves (assemble.jl:131-142), stored as codes, with the pair's FP32 frame.
-struct NearPlanSh {
+struct alignas(16) NearPlanSh {
     uint8_t leaf[32][64];  // leaf codes: level << 6 | path (level base-4 digits, most significant first)
     float E32[32][27];     // x_T,k - v_S,a
     float D32[32][9];      // x_T,k - c_S
     float S32[32][26];     // d (9), nu (9), len (3), n (3), area, diam
+    // FP64 path: x_T,k - v_S,a of every pair, in the place of the FP32 frames
+    __device__ __forceinline__ double* E64(int p) { return reinterpret_cast<double*>(&E32[0][0]) + 27 * p; }
+    __device__ __forceinline__ const double* E64(int p) const { return reinterpret_cast<const double*>(&E32[0][0]) + 27 * p; }
 };
+static_assert(sizeof(NearPlanSh) >= 32 * 64 + 32 * 27 * 8, "the FP64 frames fit in the FP32 frames' place");
 
 __device__ __forceinline__ void leaf_corners32(int code, float* b) {
     // the corners of a quadtree node in the test triangle's barycentrics (dyadic, exact in FP32)
@@ -1835,6 +1839,13 @@ __device__ bool near_plan(PairCtx& pc, NearPlanSh& pl, int t, const TriGeo& S, i
             }
             if (level == 0) break;
             path++;
+        }
+        if (!a.mixed) {
+            double* E = pl.E64(lane);
+            for (int k = 0; k < 3; ++k)
+                for (int q = 0; q < 3; ++q)
+                    for (int z = 0; z < 3; ++z) E[9 * k + 3 * q + z] = T.x[3 * k + z] - S.x[3 * q + z];
+            return true;
         }
         for (int k = 0; k < 3; ++k)
             for (int q = 0; q < 3; ++q)
