@@ -80,45 +80,52 @@ __device__ __forceinline__ T adj_point_far(AdjSums<T>& acc, const SrcKern<T>& S,
 
 // the sums of one exact-kernel point for nk adjoint vectors (weights Wn[k]): velocity w, ds/dx gx, ds/dr_a g_a, the
 // edge logs L, their length derivatives dL and the solid angle Om. The sums may be of a narrower type than the point.
+// (_one: of one vector.)
+template <class T>
+__device__ __forceinline__ void adj_acc_exact_one(AdjSums<T>& a, const T wn, T l0, T l1, T l2, v3<T> w, v3<T> gx, v3<T> g0,
+                                                  v3<T> g1, v3<T> g2, const T* L, const T* dL, T Om) {
+    a.Q += wn * w;
+    a.Xg[0] += (wn * l0) * gx;
+    a.Xg[1] += (wn * l1) * gx;
+    a.Xg[2] += (wn * l2) * gx;
+    a.Gr[0] += wn * g0;
+    a.Gr[1] += wn * g1;
+    a.Gr[2] += wn * g2;
+    for (int e = 0; e < 3; ++e) {
+        a.L[e] += wn * L[e];
+        a.N[e] += wn * dL[e];
+    }
+    a.O += wn * Om;
+}
 template <class T>
 __device__ __forceinline__ void adj_acc_exact(AdjSums<T>* acc, int nk, const T* Wn, T l0, T l1, T l2, v3<T> w,
                                               v3<T> gx, v3<T> g0, v3<T> g1, v3<T> g2, const T* L, const T* dL, T Om) {
 #pragma unroll
     for (int k = 0; k < ADJ_VEC_MAX; ++k) {
         if (k >= nk) break;
-        AdjSums<T>& a = acc[k];
-        const T wn = Wn[k];
-        a.Q += wn * w;
-        a.Xg[0] += (wn * l0) * gx;
-        a.Xg[1] += (wn * l1) * gx;
-        a.Xg[2] += (wn * l2) * gx;
-        a.Gr[0] += wn * g0;
-        a.Gr[1] += wn * g1;
-        a.Gr[2] += wn * g2;
-        for (int e = 0; e < 3; ++e) {
-            a.L[e] += wn * L[e];
-            a.N[e] += wn * dL[e];
-        }
-        a.O += wn * Om;
+        adj_acc_exact_one(acc[k], Wn[k], l0, l1, l2, w, gx, g0, g1, g2, L, dL, Om);
     }
 }
 
 // the sums of one multipole point: velocity w, ds/dr gx, ds/d(second moments) gd, ds/d(area) ga
+template <class T>
+__device__ __forceinline__ void adj_acc_far_one(AdjSums<T>& a, const T wn, T l0, T l1, T l2, v3<T> w, v3<T> gx,
+                                                const v3<T>* gd, T ga) {
+    a.Q += wn * w;
+    a.Xg[0] += (wn * l0) * gx;
+    a.Xg[1] += (wn * l1) * gx;
+    a.Xg[2] += (wn * l2) * gx;
+    a.Grf += wn * gx;
+    for (int b = 0; b < 3; ++b) a.Gd[b] += wn * gd[b];
+    a.A += wn * ga;
+}
 template <class T>
 __device__ __forceinline__ void adj_acc_far(AdjSums<T>* acc, int nk, const T* Wn, T l0, T l1, T l2, v3<T> w, v3<T> gx,
                                             const v3<T>* gd, T ga) {
 #pragma unroll
     for (int k = 0; k < ADJ_VEC_MAX; ++k) {
         if (k >= nk) break;
-        AdjSums<T>& a = acc[k];
-        const T wn = Wn[k];
-        a.Q += wn * w;
-        a.Xg[0] += (wn * l0) * gx;
-        a.Xg[1] += (wn * l1) * gx;
-        a.Xg[2] += (wn * l2) * gx;
-        a.Grf += wn * gx;
-        for (int b = 0; b < 3; ++b) a.Gd[b] += wn * gd[b];
-        a.A += wn * ga;
+        adj_acc_far_one(acc[k], Wn[k], l0, l1, l2, w, gx, gd, ga);
     }
 }
 

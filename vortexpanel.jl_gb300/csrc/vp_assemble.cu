@@ -540,18 +540,16 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
 // MIXED or FP64 by template: with both paths in one kernel the mixed one ran at 216 registers instead of 158 (near
 // phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles).
 template <bool BATCH, bool MIXED>
-__global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
+__global__ void __launch_bounds__(32, 12) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
                                                                   const int2* __restrict__ work) {
-    extern __shared__ __align__(16) unsigned char near_smem[];
-    NearChunkSh* shm = reinterpret_cast<NearChunkSh*>(near_smem);
+    __shared__ NearChunkSh sh;
     const int2 wk = work[blockIdx.x];
-    near_lanes_body<MIXED>(BATCH ? sys[wk.x] : a, wk.y, blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), gridDim.y * NEAR_WARPS,
-                    shm[threadIdx.x >> 5]);
+    near_lanes_body<MIXED>(BATCH ? sys[wk.x] : a, wk.y, blockIdx.y, gridDim.y, sh);
 }
 
 // the block of one pair: the per-lane sums reduced and contracted with n_T x gamma_b (9 values, row-major), and the
 // source part of the right hand side sigma_S (P_a . n_T) (3 values, subtracted when the pair is added)
-__device__ void pair_block_out(PairCtx& pc, FwdAcc& acc, const TriGeo& S, double* out, bool with_rhs) {
+__device__ __forceinline__ void pair_block_out(PairCtx& pc, FwdAcc& acc, const TriGeo& S, double* out, bool with_rhs) {
     fold32(acc);
     double P[9];
     for (int a = 0; a < 3; ++a) {
@@ -572,18 +570,200 @@ __device__ void pair_block_out(PairCtx& pc, FwdAcc& acc, const TriGeo& S, double
     __syncwarp();
 }
 
-// the self, touching and contact pairs, one warp per pair: a persistent grid whose warps take the next pair of the
-// list from a counter, so that test triangles with many contact pairs (thin panels at a sharp trailing edge) do not
-// hold a launch; each block goes to its pair's place in blk
-template <bool BATCH>
+// the mixed path's rare FP64 points, out of line: the multipole form, and the exact form in FP64 geometry with FP32-based
+// functions where the split evaluation leaves FP32's range
+__device__ __noinline__ v3<double> far64_sh(const WarpSh& sh, v3<double> r) { return sv_far(src64(sh), r); }
+__device__ __noinline__ v3<double> exact64_sh(const WarpSh& sh, v3<double> ra, v3<double> rb, v3<double> rc, v3<double> r,
+                                              int side) {
+    return sv_exact3<double, KMathHyb>(src64(sh), ra, rb, rc, r, side, 1e-12);
+}
+
+// one FP64 point of a triangle pair: every point of the FP64 path, the points the FP32 guard refuses of the mixed one
+template <bool MIXED>
+__device__ __forceinline__ void fwd_point64(const PairCtx& pc, FwdAcc& acc, double l0, double l1, double l2, double W) {
+    const WarpSh& sh = *pc.sh;
+    const v3<double> ra = l0 * ld3(sh.E + 0) + l1 * ld3(sh.E + 9) + l2 * ld3(sh.E + 18);
+    const v3<double> rb = l0 * ld3(sh.E + 3) + l1 * ld3(sh.E + 12) + l2 * ld3(sh.E + 21);
+    const v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
+    const SrcKern<double> S = src64(sh);
+    const v3<double> r = ra + S.d[0];
+    const double fd = pc.a->kernel_far * S.diam;
+    const bool far = dot(r, r) > fd * fd;
+    v3<double> w;
+    if constexpr (MIXED) {
+        v3<float> wf;
+        if (far)
+            w = far64_sh(sh, r);
+        else if (sv_exact3_split(S, ra, rb, rc, r, pc.side, 1e-12, wf))
+            w = mk3(double(wf.x), double(wf.y), double(wf.z));
+        else
+            w = exact64_sh(sh, ra, rb, rc, r, pc.side);
+    } else {
+        w = far ? sv_far(S, r) : sv_exact3(S, ra, rb, rc, r, pc.side, 1e-12);
+    }
+    const v3<double> psi = test_weights(pc.a->test_mode, l0, l1, l2);
+    acc.P[0] += (W * psi.x) * w;
+    acc.P[1] += (W * psi.y) * w;
+    acc.P[2] += (W * psi.z) * w;
+}
+
+// the records of a pair (walk_pair by one lane) evaluated by the warp. The buffer of leaves fills across the pair's pieces
+// and is evaluated when full, a rule piece at once, as when the walkers give the pieces to emit_leaf and emit_rule.
+// MIXED: a point is evaluated in FP32 under the guard; those it refuses are queued and evaluated 32 at a time.
+template <bool MIXED>
+__device__ __forceinline__ void eval_records(PairCtx& pc, FwdAcc& acc, const PieceRec* rec, int nrec,
+                                             const unsigned* leaf) {
+    WarpSh& sh = *pc.sh;
+    const int lane = pc.lane;
+    const double areaT = pc.T->area;
+    int ri = 0, lpos = 0, nl = 0;
+    for (;;) {
+        int rid = -1, slot0 = 0, nslot = 0;
+        while (ri < nrec) {
+            const PieceRec& r = rec[ri];
+            const int k = r.rid & (REC_DEP - 1);
+            if (k != R_NEAR) {
+                if (lane < 10) {
+                    const double v = lane < 9 ? r.b[lane] : r.frac;
+                    sh.leaf[LEAFBUF][lane] = v;
+                    sh.leaff[LEAFBUF][lane] = lane < 9 ? float(v) : float(v * areaT);
+                }
+                rid = k;
+                slot0 = LEAFBUF;
+                nslot = 1;
+                ++ri;
+                break;
+            }
+            const int take = min(LEAFBUF - nl, r.nleaf - lpos);
+            if (lane < take) {
+                const unsigned code = leaf[r.leaf0 + lpos + lane];
+                const int level = int(code >> LEAF_LEVEL);
+                double b[9];
+                quad_corners(r.b, level, code & ((1u << LEAF_LEVEL) - 1), b);
+                for (int z = 0; z < 9; ++z) {
+                    sh.leaf[nl + lane][z] = b[z];
+                    sh.leaff[nl + lane][z] = float(b[z]);
+                }
+                const double fr = r.frac * ldexp(1.0, -2 * level);
+                sh.leaf[nl + lane][9] = fr;
+                sh.leaff[nl + lane][9] = float(fr * areaT);
+            }
+            nl += take;
+            lpos += take;
+            if (lpos == r.nleaf) {
+                ++ri;
+                lpos = 0;
+            }
+            if (nl == LEAFBUF) break;
+        }
+        if (rid < 0) {
+            if (nl == 0) break;
+            rid = R_NEAR;
+            nslot = nl;
+            nl = 0;
+        }
+        __syncwarp();
+        const int n = pc.a->nrule[rid], tot = nslot * n;
+        const RulePt* R = pc.a->rule[rid];
+        const float4* Rf = pc.a->rulef[rid];
+        int nq = 0;
+        for (int i0 = 0; i0 < tot; i0 += 32) {
+            const int i = i0 + lane, k = nslot > 1 ? i / n : 0, q = i - k * n, lf = slot0 + k;
+            if constexpr (MIXED) {
+                bool need = false;
+                if (i < tot) {
+                    const float4 m = Rf[q];
+                    const float* bf = sh.leaff[lf];
+                    const float l0 = m.x * bf[0] + m.y * bf[3] + m.z * bf[6];
+                    const float l1 = m.x * bf[1] + m.y * bf[4] + m.z * bf[7];
+                    const float l2 = m.x * bf[2] + m.y * bf[5] + m.z * bf[8];
+                    need = !fwd_point32(pc, acc, l0, l1, l2, m.w * bf[9]);
+                }
+                const unsigned msk = __ballot_sync(0xffffffffu, need);
+                if (need) {
+                    const int pos = nq + __popc(msk & ((1u << lane) - 1u));
+                    sh.qi[pos] = q;
+                    sh.ql[pos] = lf;
+                }
+                nq += __popc(msk);
+                while (nq >= 32 || (nq > 0 && i0 + 32 >= tot)) {
+                    __syncwarp();
+                    const int take = nq < 32 ? nq : 32;
+                    if (lane < take) {
+                        const RulePt m = R[sh.qi[lane]];
+                        const double* b = sh.leaf[sh.ql[lane]];
+                        const double l0 = m.l0 * b[0] + m.l1 * b[3] + m.l2 * b[6];
+                        const double l1 = m.l0 * b[1] + m.l1 * b[4] + m.l2 * b[7];
+                        const double l2 = m.l0 * b[2] + m.l1 * b[5] + m.l2 * b[8];
+                        fwd_point64<true>(pc, acc, l0, l1, l2, (m.w * b[9]) * areaT);
+                    }
+                    nq -= take;
+                    int mi = 0, ml = 0;
+                    if (lane < nq) {
+                        mi = sh.qi[take + lane];
+                        ml = sh.ql[take + lane];
+                    }
+                    __syncwarp();
+                    if (lane < nq) {
+                        sh.qi[lane] = mi;
+                        sh.ql[lane] = ml;
+                    }
+                    pc.n64 += take;
+                }
+            } else {
+                if (i < tot) {
+                    const RulePt m = R[q];
+                    const double* b = sh.leaf[lf];
+                    const double l0 = m.l0 * b[0] + m.l1 * b[3] + m.l2 * b[6];
+                    const double l1 = m.l0 * b[1] + m.l1 * b[4] + m.l2 * b[7];
+                    const double l2 = m.l0 * b[2] + m.l1 * b[5] + m.l2 * b[8];
+                    fwd_point64<false>(pc, acc, l0, l1, l2, (m.w * b[9]) * areaT);
+                }
+            }
+        }
+        pc.npts += tot;
+        __syncwarp();
+    }
+    if (!MIXED) pc.n64 = pc.npts;
+}
+
+// a pair whose records do not fit, walked and evaluated piece by piece: its block to out; returns the tier
+__device__ __noinline__ int pair_direct(const NearArgs& a, WarpSh& sh, int t, int s, bool wake, double* out,
+                                        long long* npts, long long* n64) {
+    PairCtx pc;
+    pc.a = &a;
+    pc.T = &a.tri[t];
+    pc.sh = &sh;
+    pc.lane = threadIdx.x & 31;
+    pc.kind = 0;
+    pc.npts = pc.n64 = 0;
+    pc.nleaf = pc.nq64 = 0;
+    FwdAcc acc = {};
+    const int tier = tri_pair(pc, acc, t, s, wake);
+    pair_block_out(pc, acc, wake ? a.wtri[s] : a.tri[s], out, !wake);
+    *npts = pc.npts;
+    *n64 = pc.n64;
+    return tier;
+}
+
+// The self, touching and contact pairs: a persistent grid whose warps take the next pairs of the list from a counter, so
+// that test triangles with many contact pairs (thin panels at a sharp trailing edge) do not hold a launch. Each lane
+// walks one pair into records (in the warp's part of recs and leaves), then the warp evaluates the pairs one by one;
+// each block goes to its pair's place in blk. Mixed, 25k wing (1.1M pairs, 1.97G points): 189 ms, 358 ms when the warp
+// walked and evaluated piece by piece.
+template <bool BATCH, bool MIXED>
 __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs a1, const NearArgs* __restrict__ sys,
-                                                                     int nsys) {
+                                                                     PieceRec* recs, unsigned* leaves, int gmax) {
     __shared__ WarpSh shm[NEAR_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = (long long)*a1.rest_n;
+    const int warp = blockIdx.x * NEAR_WARPS + w;
+    recs += size_t(warp) * gmax * REC_MAX;
+    leaves += size_t(warp) * gmax * REC_LEAVES;
     PairCtx pc;
     pc.sh = &shm[w];
     pc.lane = lane;
+    pc.kind = 0;
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
     auto flush = [&](const NearArgs& a) {  // the counts of system a so far
         if (lane == 0) {
@@ -597,29 +777,65 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
         Q64 = 0;
     };
     for (;;) {
-        const long long idx = next_rest_pair(a1.next, lane);
-        if (idx >= total) break;
-        const NearArgs& a = BATCH ? sys[a1.rest_sys[idx]] : a1;
-        pc.a = &a;
-        const unsigned long long item = a1.rest_item[idx];
-        const int g = int(item >> REST_SHIFT), t = g >> 1;
-        const bool wake = (g & 1) != 0;
-        const long long p = (long long)(item & ((1ull << REST_SHIFT) - 1));
-        const int s = (wake ? a.wf_src : a.nf_src)[p];
-        pc.T = &a.tri[t];
-        FwdAcc acc = {};
-        pc.kind = 0;
-        pc.npts = 0;
-        pc.n64 = 0;
-        pc.nleaf = 0;
-        pc.nq64 = 0;
-        const int tier = tri_pair(pc, acc, t, s, wake);
-        pair_block_out(pc, acc, wake ? a.wtri[s] : a.tri[s],
-                       a.blk[wake ? 1 : 0] + size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B), !wake);
-        P[tier] += 1;
-        Q[tier] += pc.npts;
-        Q64 += pc.n64;
-        if (BATCH) flush(a);
+        int cnt;
+        const long long idx0 = next_rest_pairs(a1, total, gmax, lane, cnt);
+        if (cnt == 0) break;
+        // each lane walks its pair
+        unsigned long long item = 0;
+        int sy = 0, s = 0, tier = 0;
+        RecAcc ra;
+        ra.n = ra.nleaf = 0;
+        ra.over = false;
+        if (lane < cnt) {
+            item = a1.rest_item[idx0 + lane];
+            if (BATCH) sy = a1.rest_sys[idx0 + lane];
+            const NearArgs& a = BATCH ? sys[sy] : a1;
+            const int g = int(item >> REST_SHIFT), t = g >> 1;
+            const bool wake = (g & 1) != 0;
+            s = (wake ? a.wf_src : a.nf_src)[item & ((1ull << REST_SHIFT) - 1)];
+            PairCtx wc;
+            wc.a = &a;
+            wc.T = &a.tri[t];
+            wc.lane = 0;
+            ra.rec = recs + lane * REC_MAX;
+            ra.leaf = leaves + lane * REC_LEAVES;
+            ra.dep = ra.moves = false;
+            tier = walk_pair(wc, ra, t, s, wake ? a.wtri[s] : a.tri[s], wake);
+        }
+        __syncwarp();
+        for (int q = 0; q < cnt; ++q) {
+            const unsigned long long it = __shfl_sync(0xffffffffu, item, q);
+            const NearArgs& a = BATCH ? sys[__shfl_sync(0xffffffffu, sy, q)] : a1;
+            const int sq = __shfl_sync(0xffffffffu, s, q), nrec = __shfl_sync(0xffffffffu, ra.n, q);
+            const bool over = __shfl_sync(0xffffffffu, int(ra.over), q) != 0;
+            int tq = __shfl_sync(0xffffffffu, tier, q);
+            const int g = int(it >> REST_SHIFT), t = g >> 1;
+            const bool wake = (g & 1) != 0;
+            const long long p = (long long)(it & ((1ull << REST_SHIFT) - 1));
+            const TriGeo& S = wake ? a.wtri[sq] : a.tri[sq];
+            double* out = a.blk[wake ? 1 : 0] + size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B);
+            pc.npts = 0;
+            pc.n64 = 0;
+            if (over) {
+                long long np, n64;
+                tq = pair_direct(a, shm[w], t, sq, wake, out, &np, &n64);
+                pc.npts = np;
+                pc.n64 = n64;
+            } else {
+                pc.a = &a;
+                pc.T = &a.tri[t];
+                setup_tri_source(pc, S);
+                pc.side = (!wake && sq == t) ? 1 : 0;
+                FwdAcc acc = {};
+                eval_records<MIXED>(pc, acc, recs + q * REC_MAX, nrec, leaves + q * REC_LEAVES);
+                pair_block_out(pc, acc, S, out, !wake);
+            }
+            P[tq] += 1;
+            Q[tq] += pc.npts;
+            Q64 += pc.n64;
+            if (BATCH) flush(a);
+        }
+        __syncwarp();
     }
     if (!BATCH) flush(a1);
 }
@@ -1162,10 +1378,16 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         (r = dl.alloc(ctx, &d_items, most_items)) || (r = dl.alloc(ctx, &d_cnt, 2)) ||
         (BATCH && (r = dl.alloc(ctx, &d_sysof, most_items))))
         return r;
-    const size_t near_smem = sizeof(NearChunkSh) * NEAR_WARPS;
     auto lanes = jobs[0]->ps.mixed ? near_kernel_lanes<BATCH, true> : near_kernel_lanes<BATCH, false>;
-    VP_CUDA(ctx, cudaFuncSetAttribute(lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(near_smem)));
-    const int npb = persistent_blocks(ctx, near_kernel_pairs<BATCH>, 32 * NEAR_WARPS, 0);
+    auto pairs = jobs[0]->ps.mixed ? near_kernel_pairs<BATCH, true> : near_kernel_pairs<BATCH, false>;
+    const int npb = persistent_blocks(ctx, pairs, 32 * NEAR_WARPS, 0);
+    // pairs a warp walks at once: no more than there can be for every warp
+    const int gmax = int(std::max<size_t>(1, std::min<size_t>(32, most_items / (size_t(npb) * NEAR_WARPS))));
+    PieceRec* d_recs;
+    unsigned* d_leaves;
+    if ((r = dl.alloc(ctx, &d_recs, size_t(npb) * NEAR_WARPS * gmax * REC_MAX)) ||
+        (r = dl.alloc(ctx, &d_leaves, size_t(npb) * NEAR_WARPS * gmax * REC_LEAVES)))
+        return r;
     for (auto& pass : passes) {
         // the systems' places in the workspace, the work lists: all test triangles, then by colour
         std::vector<NearArgs> args(nsys);
@@ -1213,7 +1435,7 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         VP_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), ctx->stream));
         vp_phase_begin(ctx, PH_NEAR);
         const int lw = lane_warps(ctx, ntests, max_pairs);
-        lanes<<<dim3(ntests, lw / NEAR_WARPS), 32 * NEAR_WARPS, near_smem, ctx->stream>>>(a1, d_args, d_work);
+        lanes<<<dim3(ntests, lw), 32, 0, ctx->stream>>>(a1, d_args, d_work);
         ctx->launches++;
         if (nfil > 0) {
             near_kernel_filaments<BATCH><<<dim3((ntests + NEAR_WARPS - 1) / NEAR_WARPS, (nfil + 31) / 32), 32 * NEAR_WARPS, 0,
@@ -1222,7 +1444,7 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         }
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR_PAIRS);
-        near_kernel_pairs<BATCH><<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, nsys);
+        pairs<<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, d_recs, d_leaves, gmax);
         ctx->launches++;
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR);

@@ -586,13 +586,10 @@ __device__ unsigned adj_chunk(PairCtx& pc, AdjChunkSh& ns, const AdjMulti& mx, i
     return __ballot_sync(FULL, valid && !near);
 }
 
-// blockIdx.x: the test triangle; its chunks go to NEAR_WARPS * gridDim.y warps, each with its own test-side sums (one
-// warp per test triangle left a 1,676-triangle wing at 11 warps per SM in one uneven wave: 159 ms in FP64)
-__global__ void __launch_bounds__(32 * NEAR_WARPS) adj_lanes_kernel(NearArgs a, AdjMulti mx) {
-    extern __shared__ __align__(16) unsigned char adj_smem[];
-    AdjChunkSh& ns = reinterpret_cast<AdjChunkSh*>(adj_smem)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int t = blockIdx.x, w = blockIdx.y * NEAR_WARPS + (threadIdx.x >> 5), nw = gridDim.y * NEAR_WARPS;
+// blockIdx.x: the test triangle; its chunks go to gridDim.y warps (CTAs), each with its own test-side sums
+__global__ void __launch_bounds__(32, 8) adj_lanes_kernel(NearArgs a, AdjMulti mx) {
+    __shared__ AdjChunkSh ns;
+    const int lane = threadIdx.x, t = blockIdx.x, w = blockIdx.y, nw = gridDim.y;
     const TriGeo& T = a.tri[t];
     const int K = mx.nadj;
     PairCtx pc;
@@ -685,14 +682,83 @@ __device__ __forceinline__ void acc_init(AdjAccW& acc, unsigned char* smem, int 
     acc.me = acc.lanes + lane;
 }
 
-// the pairs the lanes kernel left (self, touching, contact), one warp per pair, for up to ADJ_MAX adjoint vectors at
-// once: every point's kernel and derivatives are evaluated once, and each vector keeps its sums. A persistent grid
-// whose warps take the next pair of the list from a counter, so that test triangles with many contact pairs do not
-// leave the end of the launch to a few warps. The test side of a pair goes to TA, the source side to SA (atomics).
+// the pair's context for the adjoint: test side values, direction m
+__device__ __forceinline__ void adj_pair_ctx(PairCtx& pc, const NearArgs& a, const AdjMulti& mx, int t, int s, bool wake,
+                                             v3<double>& nT, v3<double>& G, double& sig) {
+    const TriGeo& T = a.tri[t];
+    const int K = mx.nadj;
+    pc.T = &T;
+    for (int k = 0; k < 3; ++k) {
+        for (int j = 0; j < ADJ_MAX; ++j) {
+            pc.nuk[j][k] = j < K ? mx.x[j].nu[T.slot[k]] : 0.0;
+            pc.nukf[j][k] = float(pc.nuk[j][k]);
+        }
+        pc.nu[k] = pc.nuk[0][k];
+        pc.Xc[k] = ld3(T.x + 3 * k) - ld3(T.c);
+        pc.Xcf[k] = mk3(float(pc.Xc[k].x), float(pc.Xc[k].y), float(pc.Xc[k].z));
+    }
+    pc.dep = 0;
+    nT = ld3(T.n);
+    const double* gp = (wake ? mx.x[0].gam_w : mx.x[0].gam_b) + 3 * size_t(s);
+    G = mk3(gp[0], gp[1], gp[2]);
+    sig = wake ? 0.0 : a.tri[s].sigma;
+    pc.m = cross(nT, G) + sig * nT;
+    pc.mf = mk3(float(pc.m.x), float(pc.m.y), float(pc.m.z));
+    pc.kind = 0;
+    pc.npts = 0;
+    pc.n64 = 0;
+    pc.nleaf = 0;
+    pc.nq64 = 0;
+}
+
+// a pair's sums to TA and SA
+template <class Acc>
+__device__ __noinline__ void adj_pair_out(PairCtx& pc, Acc& acc, const AdjMulti& mx, int t, int s, const TriGeo& S, int set,
+                                          v3<double> nT, v3<double> G, double sig) {
+    const int lane = pc.lane, K = mx.nadj;
+    AdjSums<double> dsum[ADJ_MAX];
+    pair_sums(pc, acc, dsum, K);
+    v3<double> xS[3];
+    tri_corners(S, xS);
+    for (int j = 0; j < K; ++j) {
+        const AdjSums<double>& d = dsum[j];
+        // the test side: lane k adds field k of the pair's (Xg, U, fs)
+        const v3<double> U = cross(G, d.Q) + sig * d.Q;
+        const double v[NTA] = {d.Xg[0].x, d.Xg[0].y, d.Xg[0].z, d.Xg[1].x, d.Xg[1].y, d.Xg[1].z,
+                               d.Xg[2].x, d.Xg[2].y, d.Xg[2].z, U.x,       U.y,       U.z,       dot(d.Q, pc.m)};
+        double tmine = 0;
+#pragma unroll
+        for (int k = 0; k < NTA; ++k)
+            if (k == lane) tmine = v[k];
+        if (lane < NTA) fx_add(mx.x[j].TA + size_t(t) * NTA + lane, tmine);
+        // the source side: lane k adds field k
+        SrcAdj<double> sa = src_of_pair(xS, d, pc.m, nT);
+        double f[NSA];
+        sa_flat(sa, f);
+        vp_fx* dst = mx.x[j].SA[set] + size_t(s) * NSA;
+        double mine = 0, mine2 = 0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+            if (k == lane) mine = f[k];
+#pragma unroll
+        for (int k = 32; k < NSA; ++k)
+            if (k - 32 == lane) mine2 = f[k];
+        fx_add(dst + lane, mine);
+        if (lane < NSA - 32) fx_add(dst + 32 + lane, mine2);
+    }
+    __syncwarp();
+}
+
+// The pairs the lanes kernel left (self, touching, contact), for up to ADJ_MAX adjoint vectors at once: every point's
+// kernel and derivatives are evaluated once, and each vector keeps its sums. A persistent grid whose warps take the next
+// pairs of the list from a counter (as near_kernel_pairs): each lane walks one pair into records, the warp evaluates
+// the pairs one by one, and last, for the pairs with moving pieces, walks them once more with the tangents. The test side
+// of a pair goes to TA, the source side to SA (fixed-point sums).
 // Acc: AdjAcc (FP64 path: FP64 sums per lane) or AdjAccW (mixed path: FP32 lane partials in dynamic shared memory,
 // NEAR_WARPS x 32 AdjLane, folded into the warp's FP64 totals).
 template <class Acc>
-__global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, AdjMulti mx) {
+__global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, AdjMulti mx, PieceRec* recs,
+                                                                  unsigned* leaves, double* deps, int gmax) {
     __shared__ WarpSh shm[NEAR_WARPS];
     extern __shared__ __align__(16) unsigned char adjw_smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -702,87 +768,90 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, 
         __syncwarp();
     }
     const long long total = (long long)*a.rest_n;
-    const int K = mx.nadj;
+    const int warp = blockIdx.x * NEAR_WARPS + w;
+    recs += size_t(warp) * gmax * REC_MAX;
+    leaves += size_t(warp) * gmax * REC_LEAVES;
+    deps += size_t(warp) * gmax * REC_MAX * ADJ_NDEP;
     PairCtx pc;
     pc.a = &a;
     pc.sh = &shm[w];
     pc.lane = lane;
-    pc.nleaf = 0;
-    pc.nq64 = 0;
-    pc.fp32 = 0;
-    pc.nadj = K;
-    pc.dep = 0;
+    pc.nadj = mx.nadj;
     for (int j = 0; j < ADJ_MAX; ++j) pc.gdir[j] = 0;
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
     for (;;) {
-        const long long idx = next_rest_pair(a.next, lane);
-        if (idx >= total) break;
-        const unsigned long long item = a.rest_item[idx];
-        const int g = int(item >> REST_SHIFT), t = g >> 1, set = g & 1;
-        const bool wake = set == 1;
-        const int s = (wake ? a.wf_src : a.nf_src)[item & ((1ull << REST_SHIFT) - 1)];
-        const TriGeo& T = a.tri[t];
-        pc.T = &T;
-        for (int k = 0; k < 3; ++k) {
-            for (int j = 0; j < ADJ_MAX; ++j) {
-                pc.nuk[j][k] = j < K ? mx.x[j].nu[T.slot[k]] : 0.0;
-                pc.nukf[j][k] = float(pc.nuk[j][k]);
-            }
-            pc.nu[k] = pc.nuk[0][k];
-            pc.Xc[k] = ld3(T.x + 3 * k) - ld3(T.c);
-            pc.Xcf[k] = mk3(float(pc.Xc[k].x), float(pc.Xc[k].y), float(pc.Xc[k].z));
-        }
-        pc.dep = 0;
-        const v3<double> nT = ld3(T.n);
-        const TriGeo& S = wake ? a.wtri[s] : a.tri[s];
-        const double* gp = (wake ? mx.x[0].gam_w : mx.x[0].gam_b) + 3 * size_t(s);
-        const v3<double> G = mk3(gp[0], gp[1], gp[2]);
-        const double sig = wake ? 0.0 : S.sigma;
-        pc.m = cross(nT, G) + sig * nT;
-        pc.mf = mk3(float(pc.m.x), float(pc.m.y), float(pc.m.z));
-        Acc acc = {};
-        acc_init(acc, adjw_smem, w, lane);
-        pc.kind = 0;
-        pc.npts = 0;
-        pc.n64 = 0;
-        pc.nleaf = 0;
-        pc.nq64 = 0;
-        const int tier = tri_pair(pc, acc, t, s, wake);
-        flush_gdir(pc, mx, T, &S, wake);
-        AdjSums<double> dsum[ADJ_MAX];
-        pair_sums(pc, acc, dsum, K);
-        v3<double> xS[3];
-        tri_corners(S, xS);
-        for (int j = 0; j < K; ++j) {
-            const AdjSums<double>& d = dsum[j];
-            // the test side: lane k adds field k of the pair's (Xg, U, fs)
-            const v3<double> U = cross(G, d.Q) + sig * d.Q;
-            const double v[NTA] = {d.Xg[0].x, d.Xg[0].y, d.Xg[0].z, d.Xg[1].x, d.Xg[1].y, d.Xg[1].z,
-                                   d.Xg[2].x, d.Xg[2].y, d.Xg[2].z, U.x,       U.y,       U.z,       dot(d.Q, pc.m)};
-            double tmine = 0;
-#pragma unroll
-            for (int k = 0; k < NTA; ++k)
-                if (k == lane) tmine = v[k];
-            if (lane < NTA) fx_add(mx.x[j].TA + size_t(t) * NTA + lane, tmine);
-            // the source side: lane k adds field k
-            SrcAdj<double> sa = src_of_pair(xS, d, pc.m, nT);
-            double f[NSA];
-            sa_flat(sa, f);
-            vp_fx* dst = mx.x[j].SA[set] + size_t(s) * NSA;
-            double mine = 0, mine2 = 0;
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-                if (k == lane) mine = f[k];
-#pragma unroll
-            for (int k = 32; k < NSA; ++k)
-                if (k - 32 == lane) mine2 = f[k];
-            fx_add(dst + lane, mine);
-            if (lane < NSA - 32) fx_add(dst + 32 + lane, mine2);
+        int cnt;
+        const long long idx0 = next_rest_pairs(a, total, gmax, lane, cnt);
+        if (cnt == 0) break;
+        // each lane walks its pair
+        int g = 0, s = 0, tier = 0;
+        RecAcc ra;
+        ra.n = ra.nleaf = 0;
+        ra.over = false;
+        bool moves = false;
+        if (lane < cnt) {
+            const unsigned long long item = a.rest_item[idx0 + lane];
+            g = int(item >> REST_SHIFT);
+            const bool wake = (g & 1) != 0;
+            s = (wake ? a.wf_src : a.nf_src)[item & ((1ull << REST_SHIFT) - 1)];
+            PairCtx wc;
+            wc.a = &a;
+            wc.T = &a.tri[g >> 1];
+            wc.lane = 0;
+            ra.rec = recs + lane * REC_MAX;
+            ra.leaf = leaves + lane * REC_LEAVES;
+            ra.dep = ra.moves = false;
+            tier = walk_pair(wc, ra, g >> 1, s, wake ? a.wtri[s] : a.tri[s], wake);
+            if (!ra.over)
+                for (int k = 0; k < ra.n; ++k) moves |= (ra.rec[k].rid & REC_DEP) != 0;
         }
         __syncwarp();
-        P[tier] += 1;
-        Q[tier] += pc.npts;
-        Q64 += pc.n64;
+        // the warp evaluates them
+        for (int q = 0; q < cnt; ++q) {
+            const int gq = __shfl_sync(0xffffffffu, g, q), sq = __shfl_sync(0xffffffffu, s, q);
+            const int nrec = __shfl_sync(0xffffffffu, ra.n, q);
+            const bool over = __shfl_sync(0xffffffffu, int(ra.over), q) != 0;
+            int tq = __shfl_sync(0xffffffffu, tier, q);
+            const int t = gq >> 1;
+            const bool wake = (gq & 1) != 0;
+            const TriGeo& S = wake ? a.wtri[sq] : a.tri[sq];
+            v3<double> nT, G;
+            double sig;
+            adj_pair_ctx(pc, a, mx, t, sq, wake, nT, G, sig);
+            Acc acc = {};
+            acc_init(acc, adjw_smem, w, lane);
+            if (over) {
+                tq = tri_pair(pc, acc, t, sq, wake);
+                flush_gdir(pc, mx, a.tri[t], &S, wake);
+            } else {
+                setup_tri_source(pc, S);
+                pc.side = (!wake && sq == t) ? 1 : 0;
+                pc.fp32 = a.mixed;
+                adj_eval_records(pc, acc, recs + q * REC_MAX, nrec, leaves + q * REC_LEAVES,
+                                 deps + size_t(q) * REC_MAX * ADJ_NDEP);
+            }
+            adj_pair_out(pc, acc, mx, t, sq, S, wake ? 1 : 0, nT, G, sig);
+            P[tq] += 1;
+            Q[tq] += pc.npts;
+            Q64 += pc.n64;
+        }
+        // the moving pieces' tangents
+        unsigned mv = __ballot_sync(0xffffffffu, moves);
+        while (mv) {
+            const int q = __ffs(mv) - 1;
+            mv &= mv - 1;
+            const int gq = __shfl_sync(0xffffffffu, g, q), sq = __shfl_sync(0xffffffffu, s, q);
+            const bool wake = (gq & 1) != 0;
+            const TriGeo& T = a.tri[gq >> 1];
+            const TriGeo& S = wake ? a.wtri[sq] : a.tri[sq];
+            pc.T = &T;
+            for (int k = 0; k < 3; ++k) pc.Xc[k] = ld3(T.x + 3 * k) - ld3(T.c);
+            pc.dep = 0;
+            TanAcc ta{deps + size_t(q) * REC_MAX * ADJ_NDEP, 0};
+            walk_pair(pc, ta, gq >> 1, sq, S, wake);
+            flush_gdir(pc, mx, T, &S, wake);
+        }
+        __syncwarp();
     }
     if (lane == 0) {
         for (int k = 0; k < 6; ++k) {
@@ -1222,25 +1291,28 @@ int vp_adjoint_impl(vp_ctx* ctx, const vp_assembly_options* o, int nnode, const 
         long long max_pairs = 0;
         for (int t = 0; t < ntri; ++t)
             max_pairs = std::max(max_pairs, (ps.nfptr[t + 1] - ps.nfptr[t]) + (ps.wfptr[t + 1] - ps.wfptr[t]));
-        const size_t smem = sizeof(AdjChunkSh) * NEAR_WARPS;
-        VP_CUDA(ctx, cudaFuncSetAttribute(adj_lanes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         const int nb = (ntri + NEAR_WARPS - 1) / NEAR_WARPS;
         vp_phase_begin(ctx, PH_ADJ_NEAR);
         na.stats = d_stats;
         const int lw = lane_warps(ctx, ntri, max_pairs);
-        adj_lanes_kernel<<<dim3(ntri, lw / NEAR_WARPS), 32 * NEAR_WARPS, smem, ctx->stream>>>(na, mx);  // every vector in one pass
+        adj_lanes_kernel<<<dim3(ntri, lw), 32, 0, ctx->stream>>>(na, mx);  // every vector in one pass
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_ADJ_PAIRS);
-        if (na.mixed) {  // FP32 lane partials in shared memory, FP64 totals per warp
-            const size_t wsm = sizeof(AdjLane) * 32 * NEAR_WARPS;
-            VP_CUDA(ctx, cudaFuncSetAttribute(adj_pairs_kernel<AdjAccW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              int(wsm)));
-            const int npb = persistent_blocks(ctx, adj_pairs_kernel<AdjAccW>, 32 * NEAR_WARPS, wsm);
-            adj_pairs_kernel<AdjAccW><<<npb, 32 * NEAR_WARPS, wsm, ctx->stream>>>(na, mx);
-        } else {
-            const int npb = persistent_blocks(ctx, adj_pairs_kernel<AdjAcc>, 32 * NEAR_WARPS, 0);
-            adj_pairs_kernel<AdjAcc><<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(na, mx);
-        }
+        // mixed: FP32 lane partials in shared memory, FP64 totals per warp
+        auto pairs = na.mixed ? adj_pairs_kernel<AdjAccW> : adj_pairs_kernel<AdjAcc>;
+        const size_t wsm = na.mixed ? sizeof(AdjLane) * 32 * NEAR_WARPS : 0;
+        VP_CUDA(ctx, cudaFuncSetAttribute(pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wsm)));
+        const int npb = persistent_blocks(ctx, pairs, 32 * NEAR_WARPS, wsm);
+        // pairs a warp walks at once: no more than there can be for every warp
+        const size_t nwarp = size_t(npb) * NEAR_WARPS;
+        const int gmax = int(std::max<size_t>(1, std::min<size_t>(32, size_t(ps.nfptr[ntri] + ps.wfptr[ntri]) / nwarp)));
+        PieceRec* d_recs;
+        unsigned* d_leaves;
+        double* d_deps;
+        if ((r = dl.alloc(ctx, &d_recs, nwarp * gmax * REC_MAX)) || (r = dl.alloc(ctx, &d_leaves, nwarp * gmax * REC_LEAVES)) ||
+            (r = dl.alloc(ctx, &d_deps, nwarp * gmax * REC_MAX * ADJ_NDEP)))
+            return r;
+        pairs<<<npb, 32 * NEAR_WARPS, wsm, ctx->stream>>>(na, mx, d_recs, d_leaves, d_deps, gmax);
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_ADJ_NEAR);
         adj_near_kernel<<<nb, 32 * NEAR_WARPS, 0, ctx->stream>>>(na, mx);

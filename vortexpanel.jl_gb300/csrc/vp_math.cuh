@@ -133,8 +133,9 @@ struct SrcKern {
 };
 
 // inplane_fraction (source_triangle.jl:52-64) with the vertices given relative to the point (q_k = v_k - x)
+// (out of line: few points lie in a source's plane)
 template <class T>
-__device__ T inplane_fraction_rel(const v3<T> q[3], v3<T> n, T area, T tol) {
+__device__ __noinline__ T inplane_fraction_rel(const v3<T> q[3], v3<T> n, T area, T tol) {
     T A2 = T(2) * area;
     T l[3] = {dot(cross(q[1], q[2]), n) / A2, dot(cross(q[2], q[0]), n) / A2, dot(cross(q[0], q[1]), n) / A2};
     for (int k = 0; k < 3; ++k)

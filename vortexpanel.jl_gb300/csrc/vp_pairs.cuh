@@ -386,8 +386,8 @@ struct WarpSh {
     float E32[27];         // E in FP32
     float D32[9];          // D in FP32
     float Sdf[9], Snf[3], Snuf[9], Slenf[3], Sareaf, Sdiamf;
-    double leaf[LEAFBUF][10];
-    float leaff[LEAFBUF][10];  // the leaves in FP32: corners, and frac x the test triangle's area
+    double leaf[LEAFBUF + 1][10];   // the buffered leaves; the last place: the current rule piece of a record
+    float leaff[LEAFBUF + 1][10];   // the same in FP32: corners, and frac x the test triangle's area
     int qi[64], ql[64];    // points waiting for FP64: rule point, and leaf (-1: the current piece)
 };
 
@@ -577,7 +577,7 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, FwdAcc& acc, double
 }
 
 // evaluate one point in FP32 (triangle sources in VP_MIXED); false when it lies where FP32 cancels
-__device__ __noinline__ bool eval_point32(const PairCtx& pc, FwdAcc& acc, float l0, float l1, float l2, float W) {
+__device__ __forceinline__ bool fwd_point32(const PairCtx& pc, FwdAcc& acc, float l0, float l1, float l2, float W) {
     if (pc.a->test_mode == 2) return false;  // the dual test's ties are decided in FP64
     const WarpSh& sh = *pc.sh;
     SrcKern<float> S;
@@ -609,6 +609,9 @@ __device__ __noinline__ bool eval_point32(const PairCtx& pc, FwdAcc& acc, float 
     acc.Pf[2] += (W * psi.z) * w;
     if (++acc.nf == 16) fold32(acc);
     return true;
+}
+__device__ __noinline__ bool eval_point32(const PairCtx& pc, FwdAcc& acc, float l0, float l1, float l2, float W) {
+    return fwd_point32(pc, acc, l0, l1, l2, W);
 }
 
 // ---- adjoint accumulation of a pair (warp-cooperative path) --------------------------------------------------------
@@ -691,6 +694,7 @@ __device__ __noinline__ void fold_w(AdjAccW& acc, int lane) {
         const int z = lane + 32 * j;
         if (z < ADJ_NFIELD) {
             float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
             for (int l = 0; l < 16; ++l) {
                 float* p0 = base + l * ADJ_LSTRIDE + z;
                 float* p1 = base + (l + 16) * ADJ_LSTRIDE + z;
@@ -715,6 +719,7 @@ __device__ __noinline__ void fold_piece(AdjAccW& acc, int lane) {
         const int z = lane + 32 * j;
         if (z >= ADJ_BB0 && z < ADJ_NFIELD) {
             float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
             for (int l = 0; l < 16; ++l) {
                 float* p0 = base + l * ADJ_LSTRIDE + z;
                 float* p1 = base + (l + 16) * ADJ_LSTRIDE + z;
@@ -859,100 +864,141 @@ __device__ __noinline__ bool eval_point32(const PairCtx& pc, AdjAcc& acc, float 
 }
 
 
-// the exact kernel and its derivatives wholly in FP64 geometry (KMathHyb), added to this lane's FP32 partials: the
-// split evaluation's fallback, kept out of line so that the common path's code stays small
-__device__ __noinline__ double exact_vjp64_acc(const PairCtx& pc, AdjAccW& acc, const SrcKern<double>& S,
-                                               v3<double> ra, v3<double> rb, v3<double> rc, v3<double> r,
-                                               const float* Wn, float fl0, float fl1, float fl2, v3<double>& gx) {
-    v3<double> h0, h1, h2;
-    ExactShape<double> shd;
-    const double sv = sv_exact_vjp<double, KMathHyb>(S, ra, rb, rc, r, pc.m, pc.side, 1e-12, h0, h1, h2, shd);
-    const double i4pi = 1.0 / (4.0 * vp_pi<double>());
-    const v3<double> w = (shd.L[0] * S.nu[0] + shd.L[1] * S.nu[1] + shd.L[2] * S.nu[2] + shd.Om * S.n) * i4pi;
-    gx = h0 + h1 + h2;
-    const float Lf[3] = {float(shd.L[0]), float(shd.L[1]), float(shd.L[2])};
-    const float dLf[3] = {float(shd.dLdlen[0]), float(shd.dLdlen[1]), float(shd.dLdlen[2])};
-    adj_acc_exact(acc.me->f, pc.nadj, Wn, fl0, fl1, fl2, f3(w), f3(gx), f3(h0), f3(h1), f3(h2), Lf, dLf,
-                  float(shd.Om));
-    return sv;
+// The mixed adjoint's points, warp sums. The two evaluators alternate in the hot loop of a warp, so their code is kept
+// small: the sums' loop over the adjoint vectors is not unrolled, what few points take is out of line.
+
+// one point's sums of every vector into this lane's FP32 partials: the exact form's (gd null) or the multipole form's
+__device__ __forceinline__ float point_weight(const PairCtx& pc, int k, float W, v3<float> psi) {
+    return W * (pc.nukf[k][0] * psi.x + pc.nukf[k][1] * psi.y + pc.nukf[k][2] * psi.z);
+}
+__device__ __forceinline__ void point_rule(const PairCtx& pc, AdjAccW& acc, int k, float W, float l0, float l1, float l2,
+                                           float sv, v3<float> gx) {
+    if (pc.dep) rule_point(pc, pc.nukf[k], pc.binvf, acc.me->Bbf[k], acc.me->Fbf[k], W, l0, l1, l2, sv, gx, pc.Xcf);
 }
 
-// the mixed path's FP64 point (a triangle source's point the FP32 guard refused), warp sums: the kernel and its
-// derivatives in FP64 geometry with the FP32-based functions, added to this lane's FP32 partials
-__device__ __noinline__ void eval_point64(const PairCtx& pc, AdjAccW& acc, double l0, double l1, double l2, double W) {
+// the weights W nu(q) of an FP64 point, formed in FP64
+__device__ __forceinline__ float point_weight64(const PairCtx& pc, int k, double W, v3<double> psi) {
+    return float(W * (pc.nuk[k][0] * psi.x + pc.nuk[k][1] * psi.y + pc.nuk[k][2] * psi.z));
+}
+
+// an FP64 point of the multipole form, or of the exact form wholly in FP64 geometry (KMathHyb, the split evaluation's
+// fallback): rare, out of line
+__device__ __noinline__ void eval_point64_rare(const PairCtx& pc, AdjAccW& acc, bool far, double l0, double l1, double l2,
+                                               double W) {
     const WarpSh& sh = *pc.sh;
     const v3<double> psi = test_weights(pc.a->test_mode, l0, l1, l2);
-    float Wn[ADJ_MAX];
-    for (int k = 0; k < ADJ_MAX; ++k)
-        Wn[k] = float(W * (pc.nuk[k][0] * psi.x + pc.nuk[k][1] * psi.y + pc.nuk[k][2] * psi.z));
-    const v3<double> ra = l0 * ld3(sh.E + 0) + l1 * ld3(sh.E + 9) + l2 * ld3(sh.E + 18);
-    const v3<double> rb = l0 * ld3(sh.E + 3) + l1 * ld3(sh.E + 12) + l2 * ld3(sh.E + 21);
-    const v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
-    const v3<double> r = l0 * ld3(sh.D) + l1 * ld3(sh.D + 3) + l2 * ld3(sh.D + 6);
-    const SrcKern<double> S = src64(sh);
     const float fl0 = float(l0), fl1 = float(l1), fl2 = float(l2);
-    const double fd = pc.a->kernel_far * S.diam;
+    const SrcKern<double> S = src64(sh);
+    const v3<double> ra = l0 * ld3(sh.E + 0) + l1 * ld3(sh.E + 9) + l2 * ld3(sh.E + 18);
+    const v3<double> r = ra + S.d[0];
     v3<double> gx;
     double sv;
-    if (dot(r, r) > fd * fd) {
+    if (far) {
         v3<double> gd[3];
         double ga;
         sv = sv_far_vjp(S, r, pc.m, gx, gd, ga);
-        const v3<float> gdf[3] = {f3(gd[0]), f3(gd[1]), f3(gd[2])};
-        adj_acc_far(acc.me->f, pc.nadj, Wn, fl0, fl1, fl2, f3(sv_far(S, r)), f3(gx), gdf, float(ga));
-    } else {
-        v3<float> g0, g1, g2;
-        ExactShape<float> shp;
-        float svf;
-        if (sv_exact_vjp_split(S, ra, rb, rc, r, pc.mf, pc.side, 1e-12, svf, g0, g1, g2, shp)) {
-            const float i4pi = 1.f / (4.f * vp_pi<float>());
-            const v3<float> w =
-                (shp.L[0] * f3(S.nu[0]) + shp.L[1] * f3(S.nu[1]) + shp.L[2] * f3(S.nu[2]) + shp.Om * f3(S.n)) * i4pi;
-            const v3<float> gxf = g0 + g1 + g2;
-            adj_acc_exact(acc.me->f, pc.nadj, Wn, fl0, fl1, fl2, w, gxf, g0, g1, g2, shp.L, shp.dLdlen, shp.Om);
-            if (pc.dep)
-                for (int k = 0; k < pc.nadj; ++k)
-                    rule_point(pc, pc.nukf[k], pc.binvf, acc.me->Bbf[k], acc.me->Fbf[k], float(W), fl0, fl1, fl2,
-                               svf, gxf, pc.Xcf);
-            return;
-        }
-        // offsets outside FP32's range: all in FP64, out of line (rare)
-        sv = exact_vjp64_acc(pc, acc, S, ra, rb, rc, r, Wn, fl0, fl1, fl2, gx);
-    }
-    if (pc.dep)
+        const v3<float> gdf[3] = {f3(gd[0]), f3(gd[1]), f3(gd[2])}, w = f3(sv_far(S, r));
+#pragma unroll 1
         for (int k = 0; k < pc.nadj; ++k)
-            rule_point(pc, pc.nukf[k], pc.binvf, acc.me->Bbf[k], acc.me->Fbf[k], float(W), fl0, fl1, fl2, float(sv),
-                       f3(gx), pc.Xcf);
+            adj_acc_far_one(acc.me->f[k], point_weight64(pc, k, W, psi), fl0, fl1, fl2, w, f3(gx), gdf, float(ga));
+    } else {
+        const v3<double> rb = l0 * ld3(sh.E + 3) + l1 * ld3(sh.E + 12) + l2 * ld3(sh.E + 21);
+        const v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
+        v3<double> h0, h1, h2;
+        ExactShape<double> shd;
+        sv = sv_exact_vjp<double, KMathHyb>(S, ra, rb, rc, r, pc.m, pc.side, 1e-12, h0, h1, h2, shd);
+        const double i4pi = 1.0 / (4.0 * vp_pi<double>());
+        const v3<float> w = f3((shd.L[0] * S.nu[0] + shd.L[1] * S.nu[1] + shd.L[2] * S.nu[2] + shd.Om * S.n) * i4pi);
+        gx = h0 + h1 + h2;
+        const float Lf[3] = {float(shd.L[0]), float(shd.L[1]), float(shd.L[2])};
+        const float dLf[3] = {float(shd.dLdlen[0]), float(shd.dLdlen[1]), float(shd.dLdlen[2])};
+#pragma unroll 1
+        for (int k = 0; k < pc.nadj; ++k)
+            adj_acc_exact_one(acc.me->f[k], point_weight64(pc, k, W, psi), fl0, fl1, fl2, w, f3(gx), f3(h0), f3(h1), f3(h2),
+                              Lf, dLf, float(shd.Om));
+    }
+    for (int k = 0; k < pc.nadj; ++k) point_rule(pc, acc, k, float(W), fl0, fl1, fl2, float(sv), f3(gx));
 }
 
-// one point in FP32 under the guard, warp sums; false when it must be evaluated in FP64
+// the mixed path's FP64 point (a triangle source's point the FP32 guard refused): the kernel and its derivatives split
+// by what cancels (sv_exact_vjp_split), added to this lane's FP32 partials
+__device__ __noinline__ void eval_point64(const PairCtx& pc, AdjAccW& acc, double l0, double l1, double l2, double W) {
+    const WarpSh& sh = *pc.sh;
+    const v3<double> ra = l0 * ld3(sh.E + 0) + l1 * ld3(sh.E + 9) + l2 * ld3(sh.E + 18);
+    const v3<double> rb = l0 * ld3(sh.E + 3) + l1 * ld3(sh.E + 12) + l2 * ld3(sh.E + 21);
+    const v3<double> rc = l0 * ld3(sh.E + 6) + l1 * ld3(sh.E + 15) + l2 * ld3(sh.E + 24);
+    const SrcKern<double> S = src64(sh);
+    const v3<double> r = ra + S.d[0];
+    const double fd = pc.a->kernel_far * S.diam;
+    const bool far = dot(r, r) > fd * fd;
+    v3<float> g0, g1, g2;
+    ExactShape<float> shp;
+    float svf;
+    if (far || !sv_exact_vjp_split(S, ra, rb, rc, r, pc.mf, pc.side, 1e-12, svf, g0, g1, g2, shp)) {
+        eval_point64_rare(pc, acc, far, l0, l1, l2, W);
+        return;
+    }
+    const float i4pi = 1.f / (4.f * vp_pi<float>());
+    const v3<float> w = (shp.L[0] * f3(S.nu[0]) + shp.L[1] * f3(S.nu[1]) + shp.L[2] * f3(S.nu[2]) + shp.Om * f3(S.n)) * i4pi;
+    const v3<float> gx = g0 + g1 + g2;
+    const v3<double> psi = test_weights(pc.a->test_mode, l0, l1, l2);
+    const float fl0 = float(l0), fl1 = float(l1), fl2 = float(l2);
+#pragma unroll 1
+    for (int k = 0; k < pc.nadj; ++k) {
+        adj_acc_exact_one(acc.me->f[k], point_weight64(pc, k, W, psi), fl0, fl1, fl2, w, gx, g0, g1, g2, shp.L, shp.dLdlen,
+                          shp.Om);
+        point_rule(pc, acc, k, float(W), fl0, fl1, fl2, svf, gx);
+    }
+}
+
+// an FP32 point of the multipole form
+__device__ __noinline__ void eval_point32_far(const PairCtx& pc, AdjAccW& acc, float l0, float l1, float l2, float W,
+                                              v3<float> r) {
+    const SrcKern<float> S = src32(*pc.sh);
+    const v3<float> psi = pc.a->test_mode == 0 ? mk3(l0, l1, l2) : mk3(1.f, 1.f, 1.f);
+    v3<float> gx, gd[3];
+    float ga;
+    const float sv = sv_far_vjp(S, r, pc.mf, gx, gd, ga);
+    const v3<float> w = sv_far(S, r);
+#pragma unroll 1
+    for (int k = 0; k < pc.nadj; ++k) {
+        adj_acc_far_one(acc.me->f[k], point_weight(pc, k, W, psi), l0, l1, l2, w, gx, gd, ga);
+        point_rule(pc, acc, k, W, l0, l1, l2, sv, gx);
+    }
+}
+
+// one point in FP32 under the guard; false when it must be evaluated in FP64
 __device__ __noinline__ bool eval_point32(const PairCtx& pc, AdjAccW& acc, float l0, float l1, float l2, float W) {
     if (pc.a->test_mode == 2) return false;
     const WarpSh& sh = *pc.sh;
-    SrcKern<float> S = src32(sh);
-    v3<float> r = l0 * mk3(sh.D32[0], sh.D32[1], sh.D32[2]) + l1 * mk3(sh.D32[3], sh.D32[4], sh.D32[5]) +
-                  l2 * mk3(sh.D32[6], sh.D32[7], sh.D32[8]);
-    v3<float> psi = pc.a->test_mode == 0 ? mk3(l0, l1, l2) : mk3(1.f, 1.f, 1.f);
-    float Wn[ADJ_MAX];
-    for (int k = 0; k < ADJ_MAX; ++k)
-        Wn[k] = W * (pc.nukf[k][0] * psi.x + pc.nukf[k][1] * psi.y + pc.nukf[k][2] * psi.z);
-    float fd = pc.a->kernel_far32 * S.diam;
-    v3<float> gx;
-    float sv;
+    const v3<float> r = l0 * mk3(sh.D32[0], sh.D32[1], sh.D32[2]) + l1 * mk3(sh.D32[3], sh.D32[4], sh.D32[5]) +
+                        l2 * mk3(sh.D32[6], sh.D32[7], sh.D32[8]);
+    const float fd = pc.a->kernel_far32 * sh.Sdiamf;
     if (dot(r, r) > fd * fd) {
-        sv = adj_point_far_multi(acc.me->f, pc.nadj, Wn, S, l0, l1, l2, r, pc.mf, gx);
-    } else {
-        const float* E = sh.E32;
-        v3<float> ra = l0 * mk3(E[0], E[1], E[2]) + l1 * mk3(E[9], E[10], E[11]) + l2 * mk3(E[18], E[19], E[20]);
-        v3<float> rb = l0 * mk3(E[3], E[4], E[5]) + l1 * mk3(E[12], E[13], E[14]) + l2 * mk3(E[21], E[22], E[23]);
-        v3<float> rc = l0 * mk3(E[6], E[7], E[8]) + l1 * mk3(E[15], E[16], E[17]) + l2 * mk3(E[24], E[25], E[26]);
-        if (!fp32_guard_ok(S, ra, rb, rc, pc.side, Fp32Guard{ADJ_GUARD})) return false;
-        sv = adj_point_exact_multi(acc.me->f, pc.nadj, Wn, S, l0, l1, l2, ra, rb, rc, r, pc.mf, pc.side,
-                                   pc.side ? 1e-4f : 1e-12f, gx);
+        eval_point32_far(pc, acc, l0, l1, l2, W, r);
+        return true;
     }
-    if (pc.dep)
-        for (int k = 0; k < pc.nadj; ++k)
-            rule_point(pc, pc.nukf[k], pc.binvf, acc.me->Bbf[k], acc.me->Fbf[k], W, l0, l1, l2, sv, gx, pc.Xcf);
+    const SrcKern<float> S = src32(sh);
+    const float* E = sh.E32;
+    const v3<float> ra = l0 * mk3(E[0], E[1], E[2]) + l1 * mk3(E[9], E[10], E[11]) + l2 * mk3(E[18], E[19], E[20]);
+    const v3<float> rb = l0 * mk3(E[3], E[4], E[5]) + l1 * mk3(E[12], E[13], E[14]) + l2 * mk3(E[21], E[22], E[23]);
+    const v3<float> rc = l0 * mk3(E[6], E[7], E[8]) + l1 * mk3(E[15], E[16], E[17]) + l2 * mk3(E[24], E[25], E[26]);
+    if (!fp32_guard_ok(S, ra, rb, rc, pc.side, Fp32Guard{ADJ_GUARD})) return false;
+    // the self pair's points lie in the source's plane up to FP32 rounding: its in-plane branch (solid angle side 2 pi,
+    // as the forward's FP32 kernel takes it) must not depend on the sign of that rounding
+    v3<float> g0, g1, g2;
+    ExactShape<float> shp;
+    const float sv = sv_exact_vjp(S, ra, rb, rc, r, pc.mf, pc.side, pc.side ? 1e-4f : 1e-12f, g0, g1, g2, shp);
+    const float i4pi = 1.f / (4.f * vp_pi<float>());
+    const v3<float> w = (shp.L[0] * S.nu[0] + shp.L[1] * S.nu[1] + shp.L[2] * S.nu[2] + shp.Om * S.n) * i4pi;
+    const v3<float> gx = g0 + g1 + g2;
+    const v3<float> psi = pc.a->test_mode == 0 ? mk3(l0, l1, l2) : mk3(1.f, 1.f, 1.f);
+#pragma unroll 1
+    for (int k = 0; k < pc.nadj; ++k) {
+        adj_acc_exact_one(acc.me->f[k], point_weight(pc, k, W, psi), l0, l1, l2, w, gx, g0, g1, g2, shp.L, shp.dLdlen,
+                          shp.Om);
+        point_rule(pc, acc, k, W, l0, l1, l2, sv, gx);
+    }
     return true;
 }
 
@@ -1115,41 +1161,140 @@ __device__ void emit_leaf(PairCtx& pc, Acc& acc, const double* b, double frac) {
     if (pc.nleaf == LEAFBUF) flush_leaves(pc, acc);
 }
 
+// ---- a pair's pieces as records ---------------------------------------------------------------------------------------
+// The pair-parallel kernels build a pair's rule and evaluate it in two steps. One lane walks the rule (the tiers, splits
+// and quadtrees, FP64 geometry on which every lane of a warp would agree) and writes its pieces as records; 32 lanes
+// walk 32 pairs. Then the warp takes the pairs one after another and evaluates each one's records across its lanes.
+// When a warp walked and evaluated piece by piece, the walkers' geometry took an FP64 instruction of the whole warp per
+// operation, and walkers and evaluators together (over 400 KB of code, of which warps in different places execute
+// different parts) did not fit the instruction caches: 13.7 of near_kernel_pairs' 22.7 cycles per issue were "no
+// instruction", 18.2 of 26 in adj_pairs_kernel.
+struct PieceRec {
+    double b[9], frac;  // corners in the test triangle's barycentrics, fraction
+    int rid;            // R_SELF, R_EDGE, R_VERT: the whole rule; R_NEAR: the leaves; | REC_DEP: moves with the geometry
+    int nleaf;          // R_NEAR: leaves of the quadtree below the piece, their codes from leaf0
+    int leaf0, pad;
+};
+constexpr int REC_DEP = 256;
+// records and leaf codes a lane has room for; a pair that needs more (deep subdivision options) is walked and
+// evaluated piece by piece by its warp
+constexpr int REC_MAX = 32, REC_LEAVES = 512;
+constexpr int LEAF_LEVEL = 28;  // leaf code: level << 28 | path (level base-4 digits), levels up to 13
+
+struct RecAcc {
+    PieceRec* rec;
+    unsigned* leaf;
+    int n, nleaf;
+    bool dep, moves, over;
+};
+
+template <class Acc>
+constexpr bool kRec = std::is_same<Acc, RecAcc>::value;
+
+__device__ __forceinline__ PieceRec* rec_add(RecAcc& o, int rid, const double* b, double frac) {
+    if (o.n == REC_MAX) {
+        o.over = true;
+        return nullptr;
+    }
+    PieceRec* r = o.rec + o.n++;
+    for (int k = 0; k < 9; ++k) r->b[k] = b[k];
+    r->frac = frac;
+    r->rid = rid | (o.dep ? REC_DEP : 0);
+    r->nleaf = 0;
+    r->leaf0 = o.nleaf;
+    return r;
+}
+__device__ void emit_rule(PairCtx&, RecAcc& o, int rid, const double* b, double frac) { rec_add(o, rid, b, frac); }
+__device__ __forceinline__ void flush_leaves(PairCtx&, RecAcc&) {}
+
+// the quadtree node `path` (level base-4 digits, most significant first) below b0, as near_pieces subdivides
+__device__ __forceinline__ void quad_corners(const double* b0, int level, unsigned path, double* b) {
+    for (int k = 0; k < 9; ++k) b[k] = b0[k];
+    for (int l = 0; l < level; ++l) {
+        const int digit = (path >> (2 * (level - 1 - l))) & 3;
+        double m[9], nb[9];  // midpoints of sides 12, 23, 31
+        for (int z = 0; z < 3; ++z) {
+            m[z] = 0.5 * b[z] + 0.5 * b[3 + z];
+            m[3 + z] = 0.5 * b[3 + z] + 0.5 * b[6 + z];
+            m[6 + z] = 0.5 * b[6 + z] + 0.5 * b[z];
+        }
+        for (int z = 0; z < 3; ++z) {  // quarters (assemble.jl:79-82)
+            nb[z] = digit == 0 ? b[z] : (digit == 2 ? m[6 + z] : m[z]);
+            nb[3 + z] = digit == 1 ? b[3 + z] : (digit == 0 ? m[z] : m[3 + z]);
+            nb[6 + z] = digit == 2 ? b[6 + z] : (digit == 1 ? m[3 + z] : m[6 + z]);
+        }
+        for (int k = 0; k < 9; ++k) b[k] = nb[k];
+    }
+}
+
+// near_pieces! (assemble.jl:131-142) as one record and its leaves' codes
+__device__ __noinline__ void near_pieces(PairCtx& pc, RecAcc& o, const SrcRef& src, const double* b0, double frac0,
+                                         int depth) {
+    PieceRec* r = rec_add(o, R_NEAR, b0, frac0);
+    if (!r) return;
+    int level = 0;
+    unsigned path = 0;
+    const double ratio = pc.a->near_ratio;
+    for (int guard = 0; guard < (1 << 22); ++guard) {
+        double b[9];
+        quad_corners(b0, level, path, b);
+        v3<double> p1 = tpoint(*pc.T, b), p2 = tpoint(*pc.T, b + 3), p3 = tpoint(*pc.T, b + 6);
+        double size = fmax(vnorm(p2 - p1), fmax(vnorm(p3 - p2), vnorm(p1 - p3)));
+        if (level < depth && dist_src(src, (p1 + p2 + p3) / 3.0) < ratio * size) {
+            level++;
+            path = path * 4;
+            continue;
+        }
+        if (o.nleaf == REC_LEAVES) {
+            o.over = true;
+            return;
+        }
+        o.leaf[o.nleaf++] = (unsigned(level) << LEAF_LEVEL) | path;
+        r->nleaf++;
+        while (level > 0 && (path & 3) == 3) {
+            path >>= 2;
+            level--;
+        }
+        if (level == 0) break;
+        path++;
+    }
+}
+
 // ---- adjoint: pieces whose corners move with the geometry ---------------------------------------------------------
 // The contact splits and the wide-corner wedges place their pieces from the pair's geometry, so the points' positions
 // in the test triangle and the pieces' weights move with it. Each lane carries the tangent of the current piece along
 // one geometry coordinate (lane < 18); the points of a dependent piece sum sum W beta_j dphi/dl and sum W phi
 // (rule_point), and piece_end contracts those with the lanes' tangents.
 template <class Acc>
-constexpr bool kAdj = std::is_same<Acc, AdjAcc>::value || std::is_same<Acc, AdjAccW>::value;
+constexpr bool kAdj = std::is_same<Acc, AdjAcc>::value || std::is_same<Acc, AdjAccW>::value || std::is_same<Acc, struct TanAcc>::value;
 
 __device__ __forceinline__ void piece_begin(PairCtx&, FwdAcc&, const double*, double, const double*) {}
 __device__ __forceinline__ void piece_end(PairCtx&, FwdAcc&) {}
 
-// c: the piece's corners (9, test barycentrics), frac, tan: this lane's tangent (10) or null for a fixed piece
-__device__ void piece_begin(PairCtx& pc, AdjAcc& acc, const double* c, double frac, const double* tan) {
-    if (pc.nleaf) flush_leaves(pc, acc);
-    if (!tan) {
-        pc.dep = 0;
-        return;
-    }
+// the current piece moves: its frac and the map of a point's barycentrics to the piece's own, binv = M^-1,
+// M[k][j] = c[3j + k]: l = M beta
+__device__ void piece_moving(PairCtx& pc, const double* c, double frac) {
     pc.dep = 1;
     pc.pfrac = frac;
-    for (int k = 0; k < 10; ++k) pc.tb[k] = tan[k];
-    // binv = M^-1, M[k][j] = c[3j + k]: l = M beta
     const double a = c[0], b = c[3], cc = c[6], d = c[1], e = c[4], f = c[7], g = c[2], h = c[5], i = c[8];
     const double A = e * i - f * h, B = -(d * i - f * g), C = d * h - e * g;
     const double id = 1.0 / (a * A + b * B + cc * C);
-    pc.binv[0] = A * id;
-    pc.binv[1] = -(b * i - cc * h) * id;
-    pc.binv[2] = (b * f - cc * e) * id;
-    pc.binv[3] = B * id;
-    pc.binv[4] = (a * i - cc * g) * id;
-    pc.binv[5] = -(a * f - cc * d) * id;
-    pc.binv[6] = C * id;
-    pc.binv[7] = -(a * h - b * g) * id;
-    pc.binv[8] = (a * e - b * d) * id;
-    for (int k = 0; k < 9; ++k) pc.binvf[k] = float(pc.binv[k]);
+    const double bi[9] = {A * id, -(b * i - cc * h) * id, (b * f - cc * e) * id, B * id, (a * i - cc * g) * id,
+                          -(a * f - cc * d) * id, C * id, -(a * h - b * g) * id, (a * e - b * d) * id};
+    for (int k = 0; k < 9; ++k) {
+        pc.binv[k] = bi[k];
+        pc.binvf[k] = float(bi[k]);
+    }
+}
+
+// c: the piece's corners (9, test barycentrics), frac, tan: this lane's tangent (10) or null for a fixed piece
+template <class Acc>
+__device__ void piece_begin(PairCtx& pc, Acc& acc, const double* c, double frac, const double* tan) {
+    if (pc.nleaf) flush_leaves(pc, acc);
+    pc.dep = 0;
+    if (!tan) return;
+    piece_moving(pc, c, frac);
+    for (int k = 0; k < 10; ++k) pc.tb[k] = tan[k];
 }
 
 __device__ void piece_end(PairCtx& pc, AdjAcc& acc) {
@@ -1167,26 +1312,6 @@ __device__ void piece_end(PairCtx& pc, AdjAcc& acc) {
         if (pc.lane < 18) pc.gdir[j] += v;
     }
     pc.dep = 0;
-}
-
-__device__ void piece_begin(PairCtx& pc, AdjAccW& acc, const double* c, double frac, const double* tan) {
-    if (pc.nleaf) flush_leaves(pc, acc);
-    if (!tan) {
-        pc.dep = 0;
-        return;
-    }
-    pc.dep = 1;
-    pc.pfrac = frac;
-    for (int k = 0; k < 10; ++k) pc.tb[k] = tan[k];
-    const double a = c[0], b = c[3], cc = c[6], d = c[1], e = c[4], f = c[7], g = c[2], h = c[5], i = c[8];
-    const double A = e * i - f * h, B = -(d * i - f * g), C = d * h - e * g;
-    const double id = 1.0 / (a * A + b * B + cc * C);
-    const double bi[9] = {A * id, -(b * i - cc * h) * id, (b * f - cc * e) * id, B * id, (a * i - cc * g) * id,
-                          -(a * f - cc * d) * id, C * id, -(a * h - b * g) * id, (a * e - b * d) * id};
-    for (int k = 0; k < 9; ++k) {
-        pc.binv[k] = bi[k];
-        pc.binvf[k] = float(bi[k]);
-    }
 }
 
 // the piece's rule-geometry totals (folded first) contracted with this lane's tangent; the totals are then cleared
@@ -1209,6 +1334,113 @@ __device__ void piece_end(PairCtx& pc, AdjAccW& acc) {
         if (z >= ADJ_BB0 && z < ADJ_NFIELD) acc.tot[j] = 0;
     }
     pc.dep = 0;
+}
+
+// The derivative with respect to the moving pieces of a pair evaluated by records: the evaluation leaves each moving
+// record's sums (the Bb of every vector, then the Fb) in dep, and the warp walks the rule once more, with tangents and
+// without evaluating, contracting them.
+constexpr int ADJ_NDEP = ADJ_MAX * 10;
+
+struct TanAcc {
+    const double* dep;  // ADJ_NDEP per record
+    int rec;            // records so far
+};
+
+__device__ __forceinline__ void emit_rule(PairCtx&, TanAcc& o, int, const double*, double) { o.rec++; }
+__device__ __forceinline__ void near_pieces(PairCtx&, TanAcc& o, const SrcRef&, const double*, double, int) { o.rec++; }
+__device__ __forceinline__ void flush_leaves(PairCtx&, TanAcc&) {}
+__device__ __forceinline__ void piece_begin(PairCtx& pc, TanAcc&, const double*, double frac, const double* tan) {
+    pc.dep = tan ? 1 : 0;
+    if (!tan) return;
+    pc.pfrac = frac;
+    for (int k = 0; k < 10; ++k) pc.tb[k] = tan[k];
+}
+__device__ __forceinline__ void piece_end(PairCtx& pc, TanAcc& o) {
+    if (!pc.dep) return;
+    const double* D = o.dep + size_t(o.rec - 1) * ADJ_NDEP;
+    for (int j = 0; j < pc.nadj; ++j) {
+        double v = 0;
+        for (int k = 0; k < 9; ++k) v += D[9 * j + k] * pc.tb[k];
+        v += D[9 * ADJ_MAX + j] * pc.tb[9] / pc.pfrac;
+        if (pc.lane < 18) pc.gdir[j] += v;
+    }
+    pc.dep = 0;
+}
+
+// the moving record's sums to D (ADJ_NDEP), cleared
+__device__ void dep_out(PairCtx& pc, AdjAcc& acc, double* D) {
+    fold32(acc);
+    for (int j = 0; j < pc.nadj; ++j) {
+        for (int k = 0; k < 9; ++k) {
+            const double v = wsum_d(acc.Bb[j][k]);
+            if (pc.lane == 0) D[9 * j + k] = v;
+            acc.Bb[j][k] = 0;
+        }
+        const double v = wsum_d(acc.Fb[j]);
+        if (pc.lane == 0) D[9 * ADJ_MAX + j] = v;
+        acc.Fb[j] = 0;
+    }
+}
+__device__ void dep_out(PairCtx& pc, AdjAccW& acc, double* D) {
+    fold_piece(acc, pc.lane);
+#pragma unroll
+    for (int j = 0; j < ADJ_TSLOT; ++j) {
+        const int z = pc.lane + 32 * j;
+        if (z >= ADJ_BB0 && z < ADJ_NFIELD) {
+            D[z - ADJ_BB0] = acc.tot[j];
+            acc.tot[j] = 0;
+        }
+    }
+}
+
+// The records of a pair evaluated by the warp for the adjoint, in the walkers' order: the buffered leaves are evaluated
+// before each piece, a moving piece ends with its sums going to dep.
+template <class Acc>
+__device__ __noinline__ void adj_eval_records(PairCtx& pc, Acc& acc, const PieceRec* rec, int nrec, const unsigned* leaf,
+                                              double* dep) {
+    WarpSh& sh = *pc.sh;
+    const int lane = pc.lane;
+    for (int ri = 0; ri < nrec; ++ri) {
+        const PieceRec& r = rec[ri];
+        const int rid = r.rid & (REC_DEP - 1);
+        const bool moves = (r.rid & REC_DEP) != 0;
+        if (pc.nleaf) flush_leaves(pc, acc);
+        pc.dep = 0;
+        __syncwarp();
+        if (lane < 10) sh.leaf[LEAFBUF][lane] = lane < 9 ? r.b[lane] : r.frac;
+        __syncwarp();
+        const double* b = sh.leaf[LEAFBUF];
+        if (moves) piece_moving(pc, b, r.frac);
+        if (rid != R_NEAR) {
+            emit_rule(pc, acc, rid, b, r.frac);
+        } else {
+            for (int lpos = 0; lpos < r.nleaf;) {
+                const int take = min(LEAFBUF - pc.nleaf, r.nleaf - lpos);
+                if (lane < take) {
+                    const unsigned code = leaf[r.leaf0 + lpos + lane];
+                    const int level = int(code >> LEAF_LEVEL), at = pc.nleaf + lane;
+                    double c[9];
+                    quad_corners(r.b, level, code & ((1u << LEAF_LEVEL) - 1), c);
+                    for (int z = 0; z < 9; ++z) {
+                        sh.leaf[at][z] = c[z];
+                        sh.leaff[at][z] = float(c[z]);
+                    }
+                    const double fr = r.frac * ldexp(1.0, -2 * level);
+                    sh.leaf[at][9] = fr;
+                    sh.leaff[at][9] = float(fr * pc.T->area);
+                }
+                lpos += take;
+                pc.nleaf += take;
+                if (pc.nleaf == LEAFBUF) flush_leaves(pc, acc);
+            }
+        }
+        if (moves) {
+            if (pc.nleaf) flush_leaves(pc, acc);
+            dep_out(pc, acc, dep + size_t(ri) * ADJ_NDEP);
+            pc.dep = 0;
+        }
+    }
+    if (pc.nleaf) flush_leaves(pc, acc);
 }
 
 // the warp's FP64 sums of the pair's d[j], j < nadj, in every lane (after the last fold)
@@ -1317,6 +1549,7 @@ __device__ __noinline__ void vertex_pieces(PairCtx& pc, Acc& acc, const v3<doubl
             }
             piece_begin(pc, acc, c, frac, tan ? ct : nullptr);
         }
+        if constexpr (kRec<Acc>) acc.dep = acc.moves;
         emit_rule(pc, acc, R_VERT, c, frac);
         if constexpr (kAdj<Acc>) piece_end(pc, acc);
         return;
@@ -1364,6 +1597,7 @@ __device__ __noinline__ void vertex_pieces(PairCtx& pc, Acc& acc, const v3<doubl
             ct[9] = tp[9] * (t1 - t0) + frac * (dt1 - dt0);
             piece_begin(pc, acc, c, frac * (t1 - t0), ct);
         }
+        if constexpr (kRec<Acc>) acc.dep = true;
         emit_rule(pc, acc, R_VERT, c, frac * (t1 - t0));
         if constexpr (kAdj<Acc>) piece_end(pc, acc);
         t0 = t1;
@@ -1461,10 +1695,7 @@ __device__ __noinline__ bool contact_rule(PairCtx& pc, Acc& acc, const TriGeo& S
                 }
                 // push in reverse so that the pieces are processed in order
                 for (int i = nts; i >= 0; --i) {
-                    if (sp >= 16) {
-                        if (pc.lane == 0) atomicExch((int*)&pc.sh->leaf[0][0], 0);  // never: depth-bounded
-                        break;
-                    }
+                    if (sp >= 16) break;  // never: depth-bounded
                     if constexpr (kAdj<Acc>) {
                         double* te = tstk[sp];
                         for (int z = 0; z < 3; ++z) {
@@ -1487,6 +1718,7 @@ __device__ __noinline__ bool contact_rule(PairCtx& pc, Acc& acc, const TriGeo& S
         }
         // pieces below a split move with the geometry
         const double* tan = (kAdj<Acc> && level > 0) ? tb : nullptr;
+        if constexpr (kRec<Acc>) acc.dep = acc.moves = level > 0;
         bool on[3];
         int nc = 0;
         for (int q = 0; q < 3; ++q) {
@@ -1532,109 +1764,39 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// the pair's offsets and the source's data to shared memory, by the warp
 __device__ void setup_tri_source(PairCtx& pc, const TriGeo& S) {
-    if (pc.lane == 0) {
-        WarpSh& sh = *pc.sh;
-        const TriGeo& T = *pc.T;
-        for (int k = 0; k < 3; ++k)
-            for (int q = 0; q < 3; ++q)
-                for (int z = 0; z < 3; ++z) {
-                    sh.E[9 * k + 3 * q + z] = T.x[3 * k + z] - S.x[3 * q + z];
-                    sh.E32[9 * k + 3 * q + z] = float(sh.E[9 * k + 3 * q + z]);
-                }
-        for (int k = 0; k < 3; ++k)
-            for (int z = 0; z < 3; ++z) {
-                sh.D[3 * k + z] = T.x[3 * k + z] - S.c[z];
-                sh.D32[3 * k + z] = float(sh.D[3 * k + z]);
-            }
-        for (int k = 0; k < 9; ++k) {
-            sh.Sd[k] = S.x[k] - S.c[k % 3];
-            sh.Snu[k] = S.nu[k];
-            sh.Sdf[k] = float(sh.Sd[k]);
-            sh.Snuf[k] = float(S.nu[k]);
-        }
-        for (int k = 0; k < 3; ++k) {
-            sh.Sn[k] = S.n[k];
-            sh.Slen[k] = S.len[k];
-            sh.Snf[k] = float(S.n[k]);
-            sh.Slenf[k] = float(S.len[k]);
-        }
+    WarpSh& sh = *pc.sh;
+    const TriGeo& T = *pc.T;
+    const int i = pc.lane;
+    __syncwarp();
+    if (i < 27) {  // i = 9 k + 3 q + z
+        const double e = T.x[3 * (i / 9) + i % 3] - S.x[i % 9];
+        sh.E[i] = e;
+        sh.E32[i] = float(e);
+    }
+    if (i < 9) {
+        const double d = T.x[i] - S.c[i % 3], sd = S.x[i] - S.c[i % 3];
+        sh.D[i] = d;
+        sh.D32[i] = float(d);
+        sh.Sd[i] = sd;
+        sh.Sdf[i] = float(sd);
+        sh.Snu[i] = S.nu[i];
+        sh.Snuf[i] = float(S.nu[i]);
+    }
+    if (i < 3) {
+        sh.Sn[i] = S.n[i];
+        sh.Snf[i] = float(S.n[i]);
+        sh.Slen[i] = S.len[i];
+        sh.Slenf[i] = float(S.len[i]);
+    }
+    if (i == 0) {
         sh.Sarea = S.area;
-        sh.Sdiam = S.diam;
         sh.Sareaf = float(S.area);
+        sh.Sdiam = S.diam;
         sh.Sdiamf = float(S.diam);
     }
     __syncwarp();
-}
-
-// the rule of one triangle pair and its evaluation; returns the tier. Sources: body (wake = 0) or wake triangle.
-template <class Acc>
-__device__ int tri_pair(PairCtx& pc, Acc& acc, int t, int s, bool wake) {
-    const NearArgs& a = *pc.a;
-    const TriGeo& T = *pc.T;
-    const TriGeo& S = wake ? a.wtri[s] : a.tri[s];
-    setup_tri_source(pc, S);
-    const double corners[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    pc.side = (!wake && s == t) ? 1 : 0;
-    pc.fp32 = a.mixed;
-    if (!wake && s == t) {
-        emit_rule(pc, acc, R_SELF, corners, 1.0);
-        return TIER_SELF;
-    }
-    bool shared[3] = {false, false, false};
-    int ns = 0;
-    if (!wake)
-        for (int k = 0; k < 3; ++k) {
-            shared[k] = T.node[k] == S.node[0] || T.node[k] == S.node[1] || T.node[k] == S.node[2];
-            ns += shared[k];
-        }
-    if (contact_rule(pc, acc, S, shared)) {
-        flush_leaves(pc, acc);
-        return TIER_CONTACT;
-    }
-    if (ns == 2) {
-        int k = (shared[0] && shared[1]) ? 0 : ((shared[1] && shared[2]) ? 1 : 2);
-        double c[9];
-        for (int z = 0; z < 3; ++z) {
-            c[z] = corners[3 * k + z];
-            c[3 + z] = corners[3 * ((k + 1) % 3) + z];
-            c[6 + z] = corners[3 * ((k + 2) % 3) + z];
-        }
-        emit_rule(pc, acc, R_EDGE, c, 1.0);
-        return TIER_EDGE;
-    }
-    if (ns == 1) {
-        int k = shared[0] ? 0 : (shared[1] ? 1 : 2);
-        v3<double> p[3] = {ld3(T.x), ld3(T.x + 3), ld3(T.x + 6)};
-        v3<double> u = p[(k + 1) % 3] - p[k], v = p[(k + 2) % 3] - p[k];
-        if (dot(u, v) >= 0) {  // vertex_rule (assemble.jl:119-125): the stored rotation
-            double c[9];
-            for (int z = 0; z < 3; ++z) {
-                c[z] = corners[3 * k + z];
-                c[3 + z] = corners[3 * ((k + 1) % 3) + z];
-                c[6 + z] = corners[3 * ((k + 2) % 3) + z];
-            }
-            emit_rule(pc, acc, R_VERT, c, 1.0);
-        } else {
-            vertex_pieces(pc, acc, p, k, corners, 1.0, nullptr);
-        }
-        return TIER_VERTEX;
-    }
-    int depth = a.near_depth;
-    if (!wake && a.ntouch > 0) {
-        long long key = (long long)t * a.ntri + s;
-        int lo = 0, hi = a.ntouch;
-        while (lo < hi) {
-            int mid = (lo + hi) >> 1;
-            if (a.touch[mid] < key) lo = mid + 1;
-            else hi = mid;
-        }
-        if (lo < a.ntouch && a.touch[lo] == key) depth += 4;
-    }
-    SrcRef src{0, S.x, {}, {}};
-    near_pieces(pc, acc, src, corners, 1.0, depth);
-    flush_leaves(pc, acc);
-    return TIER_NEAR;
 }
 
 // vertex_rule (assemble.jl:119-125) toward corner k of the whole test triangle
@@ -1655,6 +1817,72 @@ __device__ void vertex_rule(PairCtx& pc, Acc& acc, int k) {
     } else {
         vertex_pieces(pc, acc, p, k, corners, 1.0, nullptr);
     }
+}
+
+// the rule of one triangle pair (pair_rule, assemble.jl:266-282; wake_pair_rule, :288-293) given to acc; returns the
+// tier. Sources: body (wake = 0) or wake triangle.
+template <class Acc>
+__device__ int walk_pair(PairCtx& pc, Acc& acc, int t, int s, const TriGeo& S, bool wake) {
+    const NearArgs& a = *pc.a;
+    const TriGeo& T = *pc.T;
+    const double corners[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+    if (!wake && s == t) {
+        emit_rule(pc, acc, R_SELF, corners, 1.0);
+        return TIER_SELF;
+    }
+    bool shared[3] = {false, false, false};
+    int ns = 0;
+    if (!wake)
+        for (int k = 0; k < 3; ++k) {
+            shared[k] = T.node[k] == S.node[0] || T.node[k] == S.node[1] || T.node[k] == S.node[2];
+            ns += shared[k];
+        }
+    if (contact_rule(pc, acc, S, shared)) {
+        flush_leaves(pc, acc);
+        return TIER_CONTACT;
+    }
+    if constexpr (kRec<Acc>) acc.dep = acc.moves = false;
+    if (ns == 2) {
+        int k = (shared[0] && shared[1]) ? 0 : ((shared[1] && shared[2]) ? 1 : 2);
+        double c[9];
+        for (int z = 0; z < 3; ++z) {
+            c[z] = corners[3 * k + z];
+            c[3 + z] = corners[3 * ((k + 1) % 3) + z];
+            c[6 + z] = corners[3 * ((k + 2) % 3) + z];
+        }
+        emit_rule(pc, acc, R_EDGE, c, 1.0);
+        return TIER_EDGE;
+    }
+    if (ns == 1) {
+        vertex_rule(pc, acc, shared[0] ? 0 : (shared[1] ? 1 : 2));
+        return TIER_VERTEX;
+    }
+    int depth = a.near_depth;
+    if (!wake && a.ntouch > 0) {
+        long long key = (long long)t * a.ntri + s;
+        int lo = 0, hi = a.ntouch;
+        while (lo < hi) {
+            int mid = (lo + hi) >> 1;
+            if (a.touch[mid] < key) lo = mid + 1;
+            else hi = mid;
+        }
+        if (lo < a.ntouch && a.touch[lo] == key) depth += 4;
+    }
+    SrcRef src{0, S.x, {}, {}};
+    near_pieces(pc, acc, src, corners, 1.0, depth);
+    flush_leaves(pc, acc);
+    return TIER_NEAR;
+}
+
+// a pair walked and evaluated piece by piece by its warp
+template <class Acc>
+__device__ __noinline__ int tri_pair(PairCtx& pc, Acc& acc, int t, int s, bool wake) {
+    const NearArgs& a = *pc.a;
+    const TriGeo& S = wake ? a.wtri[s] : a.tri[s];
+    setup_tri_source(pc, S);
+    pc.side = (!wake && s == t) ? 1 : 0;
+    pc.fp32 = a.mixed;
+    return walk_pair(pc, acc, t, s, S, wake);
 }
 
 // ---- the near tier, one pair per lane: the plan shared by the assembly and the adjoint -------------------------------
@@ -2241,20 +2469,32 @@ __device__ __forceinline__ void rest_append(const NearArgs& a, int g, long long 
     }
 }
 
-// the next rest pair of this warp (all lanes call it together)
-__device__ __forceinline__ long long next_rest_pair(unsigned long long* next, int lane) {
-    unsigned long long v = 0;
-    if (lane == 0) v = atomicAdd(next, 1ull);
-    return (long long)__shfl_sync(0xffffffffu, v, 0);
+// the next rest pairs of this warp, taken from a counter (all lanes call it together): the first one's index, cnt of them
+// (none left: cnt 0). A warp takes up to gmax pairs while there are many left, fewer toward the end, so that the last
+// pairs spread over all warps (a fixed 12 left the SMs idle for 13% of a 65k-pair launch).
+__device__ __forceinline__ long long next_rest_pairs(const NearArgs& a, long long total, int gmax, int lane, int& cnt) {
+    unsigned long long idx = 0;
+    int g = 0;
+    if (lane == 0) {
+        const long long left = total - (long long)*(volatile unsigned long long*)a.next;
+        const long long share = left / (4LL * gridDim.x * (blockDim.x >> 5));
+        g = int(share < 1 ? 1 : (share > gmax ? gmax : share));
+        idx = atomicAdd(a.next, (unsigned long long)g);
+    }
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    g = __shfl_sync(0xffffffffu, g, 0);
+    const long long n = total - (long long)idx;
+    cnt = int(n < 0 ? 0 : (n < g ? n : g));
+    return (long long)idx;
 }
 
 // warps per test triangle of a lanes kernel (each takes every so many chunks of 32 pairs): enough that the grid fills
-// the device about ten times over, no more than the longest list has chunks; a multiple of the warps of a CTA
+// the device about ten times over, no more than the longest list has chunks. A CTA is one warp: chunks differ in work,
+// and warps that share a CTA hold its slot until the slowest is done.
 int lane_warps(vp_ctx* ctx, long long ntests, long long max_pairs) {
     const long long want = (10LL * 12 * std::max(ctx->nsm, 1) + ntests - 1) / std::max(ntests, 1LL);
     const long long have = (max_pairs + 31) / 32;
-    const long long w = std::max(1LL, std::min(want, have));
-    return int((w + NEAR_WARPS - 1) / NEAR_WARPS) * NEAR_WARPS;
+    return int(std::max(1LL, std::min(want, have)));
 }
 
 // CTAs of a persistent pair-parallel kernel: as many as stay resident on every SM
