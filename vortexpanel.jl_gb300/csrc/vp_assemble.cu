@@ -14,9 +14,9 @@
 //      for bit;
 //   3. near, touching and contact tiers: the near pairs one per lane in chunks of 32, the others (self, edge, vertex
 //      with wide-corner wedges, contact splits) one warp per pair with the reference's rules, all test triangles in one
-//      launch each. Every pair's block goes to the pair's own place in a workspace, and one kernel per colour of test
-//      triangles adds the blocks to A, column by column in a fixed order. FP64 for the touching and contact tiers, FP32
-//      or FP64 for the near tier, FP64 for the wake's tip filaments.
+//      launch each. Every pair's block goes to the pair's own place in a workspace, and one kernel adds the blocks to
+//      A row by row, each column's in a fixed order. FP64 for the touching and contact tiers, FP32 or FP64 for the near
+//      tier, FP64 for the wake's tip filaments.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -872,7 +872,7 @@ __device__ void far_filament_fwd(const NearArgs& a, const TriGeo& T, v3<double> 
 // the tip filaments (assemble.jl:344-354): segment_rule (:299-306) and segment_block (:312-321), FP64. A warp takes 32
 // filaments of one test triangle: a far one (the far rule's few points) is summed by its own lane, the others by the
 // whole warp. Every (test triangle, filament) writes the columns of its two ends to fil_out; near_kernel_gather adds
-// them, so all test triangles share one launch.
+// them.
 template <bool BATCH>
 __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_filaments(NearArgs a1, const NearArgs* __restrict__ sys,
                                                                          const int2* __restrict__ work, int nwork) {
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_filaments(Near
     pc.fp32 = 0;
     unsigned long long P[6] = {0, 0, 0, 0, 0, 0}, Q[6] = {0, 0, 0, 0, 0, 0}, Q64 = 0;
     const double corners[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    double* out = a.fil_out + 6 * (size_t(t - a.fil_t0) * a.nfil + f0);
+    double* out = a.fil_out + 6 * (size_t(t - a.t0) * a.nfil + f0);
     const int cnt = a.nfil - f0 < 32 ? a.nfil - f0 : 32;
     bool mfar = false;
     if (lane < cnt) {
@@ -985,81 +985,76 @@ __device__ __forceinline__ int find_source(const int* list, int n, int s) {
 constexpr int GATHER_NT = 128;
 constexpr int GATHER_LIST = 2048;  // sources of a list staged in shared memory (8 KB); longer lists are searched in place
 
-// One CTA per test triangle, one launch per colour (no two test triangles of a launch share a row): the blocks of its
-// non-far pairs and its filaments' columns added to its three rows of A, its right hand side to b, in a fixed order.
-// A thread takes a (pair, source corner) and adds its column's whole sum if no earlier pair of the list has that
-// column: the pairs with the column are those of the column's triangles that binary search finds in the list. Every
-// entry of A is read and written once, by one thread, all columns in parallel; bound by reading the blocks.
+// One CTA per row slot: the blocks of its triangles' non-far pairs and their filaments' columns added to its row of A, its
+// right hand side to b, in a fixed order. Per triangle, a thread takes a (pair, source corner) and adds its column's
+// whole sum if no earlier pair of the list has that column: the pairs with the column are those of the column's
+// triangles that binary search finds in the list. Latency of the searches and of the row's read-modify-writes bounds
+// it, so all rows share one launch (one CTA per test triangle, a launch per colour: 2.0 ms on a 1,676-triangle wing).
 template <bool BATCH>
 __global__ void __launch_bounds__(GATHER_NT) near_kernel_gather(NearArgs a1, const NearArgs* __restrict__ sys,
                                                               const int2* __restrict__ work) {
     __shared__ int s_list[GATHER_LIST];
-    __shared__ double red[3][GATHER_NT];
+    __shared__ double red[GATHER_NT];
     const int2 wk = work[blockIdx.x];
     const NearArgs& a = BATCH ? sys[wk.x] : a1;
-    const int t = wk.y, tid = threadIdx.x;
-    const TriGeo& T = a.tri[t];
-    double* row[3];
-    for (int k = 0; k < 3; ++k) row[k] = a.A + size_t(T.slot[k]) * size_t(a.lda);
-    double rb[3] = {0, 0, 0};
-    for (int set = 0; set < 2; ++set) {
-        const long long p0 = (set ? a.wf_ptr : a.nf_ptr)[t];
-        const int n = int((set ? a.wf_ptr : a.nf_ptr)[t + 1] - p0);
-        const int* src = (set ? a.wf_src : a.nf_src) + p0;
-        const int nb = set ? BLK_W : BLK_B;
-        const double* blk = a.blk[set] + size_t(p0 - a.blk0[set]) * nb;
-        const int col0 = set ? a.nslot : 0;
-        const int *slots = a.slots[set], *ptr = a.col_ptr[set], *ent = a.col_ent[set];
-        const bool staged = n <= GATHER_LIST;
-        __syncthreads();
-        if (staged)
-            for (int i = tid; i < n; i += GATHER_NT) s_list[i] = src[i];
-        __syncthreads();
-        const int* list = staged ? s_list : src;
-        for (int i = tid; i < 3 * n; i += GATHER_NT) {
-            const int p = i / 3, b = i - 3 * p, s = list[p], c = slots[3 * s + b];
-            double v[3] = {0, 0, 0};
-            bool own = false;
-            for (int u = ptr[c]; u < ptr[c + 1]; ++u) {
-                const int e = ent[u], se = e / 3, be = e - 3 * se;
-                const bool me = e == 3 * s + b;
-                const int q = me ? p : find_source(list, n, se);
-                if (q < 0) continue;
-                if (!me && !own) break;  // an earlier pair has this column
-                own = true;
-                const double* pb = blk + size_t(q) * nb + be;
-                v[0] += pb[0];
-                v[1] += pb[3];
-                v[2] += pb[6];
+    const int slot = wk.y, tid = threadIdx.x;
+    double* row = a.A + size_t(slot) * size_t(a.lda);
+    double rb = 0, free = 0;
+    for (int ue = a.col_ptr[0][slot]; ue < a.col_ptr[0][slot + 1]; ++ue) {
+        const int et = a.col_ent[0][ue], t = et / 3, ta = et - 3 * t;
+        if (t < a.t0 || t >= a.t1) continue;
+        const TriGeo& T = a.tri[t];
+        for (int set = 0; set < 2; ++set) {
+            const long long p0 = (set ? a.wf_ptr : a.nf_ptr)[t];
+            const int n = int((set ? a.wf_ptr : a.nf_ptr)[t + 1] - p0);
+            if (n == 0) continue;
+            const int* src = (set ? a.wf_src : a.nf_src) + p0;
+            const int nb = set ? BLK_W : BLK_B;
+            const double* blk = a.blk[set] + size_t(p0 - a.blk0[set]) * nb + 3 * ta;
+            const int col0 = set ? a.nslot : 0;
+            const int *slots = a.slots[set], *ptr = a.col_ptr[set], *ent = a.col_ent[set];
+            const bool staged = n <= GATHER_LIST;
+            __syncthreads();
+            if (staged)
+                for (int i = tid; i < n; i += GATHER_NT) s_list[i] = src[i];
+            __syncthreads();
+            const int* list = staged ? s_list : src;
+            for (int i = tid; i < 3 * n; i += GATHER_NT) {
+                const int p = i / 3, b = i - 3 * p, s = list[p], c = slots[3 * s + b];
+                double v = 0;
+                bool own = false;
+                for (int u = ptr[c]; u < ptr[c + 1]; ++u) {
+                    const int e = ent[u], se = e / 3, be = e - 3 * se;
+                    const bool me = e == 3 * s + b;
+                    const int q = me ? p : find_source(list, n, se);
+                    if (q < 0) continue;
+                    if (!me && !own) break;  // an earlier pair has this column
+                    own = true;
+                    v += blk[size_t(q) * nb + be];
+                }
+                if (own) row[col0 + c] += v;
             }
-            if (own)
-                for (int k = 0; k < 3; ++k) row[k][col0 + c] += v[k];
+            if (!set)
+                for (int p = tid; p < n; p += GATHER_NT) rb -= blk[size_t(p) * nb + 9 - 2 * ta];
         }
-        if (!set)
-            for (int p = tid; p < n; p += GATHER_NT)
-                for (int k = 0; k < 3; ++k) rb[k] -= blk[size_t(p) * nb + 9 + k];
-    }
-    if (a.nfil > 0) {
-        __syncthreads();  // the wake's columns are the filaments' too
-        const double* fo = a.fil_out + 6 * size_t(t - a.fil_t0) * a.nfil;
-        for (int i = tid; i < a.nfnode; i += GATHER_NT) {
-            double v[3] = {0, 0, 0};
-            for (int u = a.fnode_ptr[i]; u < a.fnode_ptr[i + 1]; ++u)
-                for (int k = 0; k < 3; ++k) v[k] += fo[3 * a.fnode_ent[u] + k];
-            for (int k = 0; k < 3; ++k) row[k][a.nslot + a.fnode[i]] += v[k];
+        if (a.nfil > 0) {
+            __syncthreads();  // the wake's columns are the filaments' too
+            const double* fo = a.fil_out + 6 * size_t(t - a.t0) * a.nfil + ta;
+            for (int i = tid; i < a.nfnode; i += GATHER_NT) {
+                double v = 0;
+                for (int u = a.fnode_ptr[i]; u < a.fnode_ptr[i + 1]; ++u) v += fo[3 * a.fnode_ent[u]];
+                row[a.nslot + a.fnode[i]] += v;
+            }
         }
+        // the freestream, exact (assemble.jl:422)
+        free += (a.vinf[0] * T.n[0] + a.vinf[1] * T.n[1] + a.vinf[2] * T.n[2]) * T.area * a.tint[ta];
     }
-    // the right hand side: the pairs' terms, and the freestream, exact (assemble.jl:422)
-    for (int k = 0; k < 3; ++k) red[k][tid] = rb[k];
+    red[tid] = rb;
     for (int o = GATHER_NT / 2; o > 0; o >>= 1) {
         __syncthreads();
-        if (tid < o)
-            for (int k = 0; k < 3; ++k) red[k][tid] += red[k][tid + o];
+        if (tid < o) red[tid] += red[tid + o];
     }
-    if (tid == 0) {
-        const double vn = (a.vinf[0] * T.n[0] + a.vinf[1] * T.n[1] + a.vinf[2] * T.n[2]) * T.area;
-        for (int k = 0; k < 3; ++k) a.b[T.slot[k]] += red[k][0] - vn * a.tint[k];
-    }
+    if (tid == 0) a.b[slot] += red[0] - free;
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -1108,7 +1103,6 @@ struct AsmJob {
     vp_system* sys = nullptr;
     FarArgs fa{};
     std::vector<std::vector<int>> far_col;   // far test tiles, per colour
-    std::vector<std::vector<int>> near_col;  // test triangles, per colour
     NearArgs na{};
     unsigned long long* d_stats = nullptr;
     std::chrono::steady_clock::time_point t0;
@@ -1118,7 +1112,7 @@ struct AsmJob {
 };
 
 // classification, pair lists, the zeroed system, the far tier's source tiles and arrays, its test tiles and their
-// colours, the near tier's colours and arguments
+// colours, the near tier's arguments
 int job_prepare(vp_ctx* ctx, AsmJob& j) {
     j.t0 = std::chrono::steady_clock::now();
     const PairInput& in = j.in;
@@ -1197,10 +1191,6 @@ int job_prepare(vp_ctx* ctx, AsmJob& j) {
     // near, touching and contact tiers
     if ((r = dl.alloc(ctx, &j.d_stats, 13))) return r;
     VP_CUDA(ctx, cudaMemsetAsync(j.d_stats, 0, sizeof(unsigned long long) * 13, ctx->stream));
-    std::vector<std::vector<int>> groups(ntri);
-    for (int t = 0; t < ntri; ++t)
-        groups[t] = {in.corner_slot[3 * t], in.corner_slot[3 * t + 1], in.corner_slot[3 * t + 2]};
-    j.near_col = colour_groups(groups, nslot);
     j.na = near_args(ps, in);
     j.na.A = sys->A;
     j.na.b = sys->b;
@@ -1334,7 +1324,7 @@ constexpr size_t NEAR_PASS_BYTES = size_t(1) << 30;
 
 // The non-far tiers of the jobs (one: BATCH false). The test triangles go in passes whose pair blocks fit the workspace;
 // a pass is: the lanes kernel over all its test triangles (blocks of the near pairs, the list of the rest), the
-// persistent pair kernel (blocks of the rest), the filaments, and per colour the kernel that adds the blocks to A.
+// persistent pair kernel (blocks of the rest), the filaments, and the kernel that adds the blocks to A's rows.
 template <bool BATCH>
 int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
     int r;
@@ -1389,11 +1379,10 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         (r = dl.alloc(ctx, &d_leaves, size_t(npb) * NEAR_WARPS * gmax * REC_LEAVES)))
         return r;
     for (auto& pass : passes) {
-        // the systems' places in the workspace, the work lists: all test triangles, then by colour
+        // the systems' places in the workspace, the work lists: all test triangles, then all rows
         std::vector<NearArgs> args(nsys);
         std::vector<int2> work;
-        std::vector<size_t> off;
-        size_t at = 0, fat = 0, ncol = 0;
+        size_t at = 0, fat = 0;
         int nfil = 0;
         for (const Range& g : pass) {
             AsmJob& j = *jobs[g.sys];
@@ -1410,24 +1399,17 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
             na.blk[1] = d_blk + at;
             at += size_t(BLK_W) * size_t(j.ps.wfptr[g.t1] - j.ps.wfptr[g.t0]);
             na.fil_out = d_fil + fat;
-            na.fil_t0 = g.t0;
+            na.t0 = g.t0;
+            na.t1 = g.t1;
             fat += 6 * size_t(na.nfil) * size_t(g.t1 - g.t0);
             nfil = std::max(nfil, na.nfil);
             args[g.sys] = na;
-            ncol = std::max(ncol, j.near_col.size());
             for (int t = g.t0; t < g.t1; ++t) work.push_back(make_int2(g.sys, t));
         }
         const int ntests = int(work.size());
-        for (size_t c = 0; c < ncol; ++c) {
-            off.push_back(work.size());
-            for (const Range& g : pass) {
-                const auto& col = jobs[g.sys]->near_col;
-                if (c >= col.size()) continue;
-                auto lo = std::lower_bound(col[c].begin(), col[c].end(), g.t0);
-                for (; lo != col[c].end() && *lo < g.t1; ++lo) work.push_back(make_int2(g.sys, *lo));
-            }
-        }
-        off.push_back(work.size());
+        for (const Range& g : pass)
+            for (int i = 0; i < jobs[g.sys]->in.nslot; ++i) work.push_back(make_int2(g.sys, i));
+        const int nrows = int(work.size()) - ntests;
         int2* d_work;
         NearArgs* d_args = nullptr;
         if ((r = dl.up(ctx, &d_work, work)) || (BATCH && (r = dl.up(ctx, &d_args, args)))) return r;
@@ -1448,12 +1430,8 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         ctx->launches++;
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR);
-        for (size_t c = 0; c < ncol; ++c) {
-            const int nb = int(off[c + 1] - off[c]);
-            if (!nb) continue;
-            near_kernel_gather<BATCH><<<nb, GATHER_NT, 0, ctx->stream>>>(a1, d_args, d_work + off[c]);
-            ctx->launches++;
-        }
+        near_kernel_gather<BATCH><<<nrows, GATHER_NT, 0, ctx->stream>>>(a1, d_args, d_work + ntests);
+        ctx->launches++;
         vp_phase_end(ctx);
         VP_CUDA(ctx, cudaGetLastError());
     }

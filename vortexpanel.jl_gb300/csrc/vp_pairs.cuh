@@ -351,7 +351,7 @@ struct NearArgs {
     double* blk[2];             // forward: per pair of nf_src / wf_src, at its position less blk0, its 3 x 3 block (row-
     long long blk0[2];          // major) and (body) its 3 right hand side terms: BLK_B / BLK_W doubles a pair
     double* fil_out;            // forward: per test triangle and filament, the columns of its two ends (6 doubles)
-    int fil_t0;                 // the test triangle of fil_out's first row
+    int t0, t1;                 // the pass's test triangles (fil_out's first row: t0)
     const long long* touch;  // sorted keys t * ntri + s
     int ntouch;
     const RulePt* rule[5];
