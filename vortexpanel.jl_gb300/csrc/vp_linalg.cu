@@ -4,9 +4,9 @@
 //  - reduction + border: one kernel gathers M = C' A Cf (A row-major FP64, C and Cf sparse) into a column-major FP64
 //    matrix through a shared-memory transpose, then the border rows/columns (scaled to the mean |diagonal|) are set;
 //  - LU with partial pivoting (the reference calls LAPACK dgetrf): recursive (left half, swap, TRSM, GEMM, right
-//    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster of 8 CTAs that holds the panel
-//    in distributed shared memory: per column, every CTA finds its pivot candidate, one cluster barrier, every CTA
-//    reads the 8 candidates and the pivot row through DSMEM, swaps and updates its rows. TRSM is cuBLAS; the
+//    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster of 8 CTAs that holds the panel in
+//    registers: per column, every CTA sends its pivot candidate's row to all, one cluster barrier, every thread picks
+//    the pivot, swaps and updates its rows. TRSM is cuBLAS; the
 //    trailing-update GEMM is cuBLAS DGEMM for VP_FP64 and, for VP_MIXED, the tensor-core GEMM of vp_tcgemm.cu
 //    (three-piece bf16 split, six tcgen05 products accumulated in FP32 in TMEM) for updates of at least one
 //    128 x 128 x 64 tile, cuBLAS SGEMM for the smaller ones;
@@ -82,11 +82,178 @@ __global__ void col_abs_sum_kernel(int n, const T* __restrict__ M, double* __res
     if (threadIdx.x == 0) out[c] = red[0];
 }
 
-// LU leaf: rows [c0, c0 + m) x columns [c0, c0 + w) (w <= W) of the column-major matrix (ld lda), partial pivoting.
-// Rows are split over the 8 CTAs of the cluster (R rows each) and held in shared memory for the whole panel.
+// the largest |v| of a warp's candidates, the smallest index on ties; NaN is no candidate (index INT_MAX where there is
+// none). Returns the winner's index; best receives its value.
+__device__ __forceinline__ int warp_best(float v, int i, float& best) {
+    if (!(v >= 0.f)) {
+        v = 0.f;
+        i = INT_MAX;
+    }
+    const unsigned key = __float_as_uint(v), m = __reduce_max_sync(0xffffffffu, i == INT_MAX ? 0u : key);
+    best = __uint_as_float(m);
+    return __reduce_min_sync(0xffffffffu, key == m ? i : INT_MAX);
+}
+__device__ __forceinline__ int warp_best(double v, int i, double& best) {
+    if (!(v >= 0.0)) {
+        v = 0.0;
+        i = INT_MAX;
+    }
+    const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, i == INT_MAX ? 0u : hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh && i != INT_MAX ? lo : 0u);
+    best = __hiloint2double(mh, ml);
+    return __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? i : INT_MAX);
+}
+
+// LU leaf: rows [c0, c0 + m) x columns [c0, c0 + w) (w <= W) of the column-major matrix (ld lda), partial pivoting, by a
+// cluster of CL CTAs. Rows are split over the CTAs (R each) and stay in registers for the whole panel, RPT rows a
+// thread. A column is one chain of latencies - search, exchange, elimination - so what bounds a leaf is the steps in
+// that chain: each warp finds its candidate and writes that row to shared memory, one warp reduces the CTA's candidates
+// and stores the winner and its row to every CTA's shared memory, and after one cluster barrier all threads pick the
+// pivot among the 8 from their own shared memory, swap and eliminate. (With the panel in shared memory, the candidates
+// and the pivot row read from the other CTAs after the barrier, and three more block barriers: 7 us a column.)
+template <class T, int W>
+struct LeafCand {
+    T best;
+    int idx, pad;
+    alignas(16) T row[W];
+};
+template <class T, int W, int RPT, int CL>
+__global__ void __launch_bounds__(LU_THREADS)
+    lu_leaf_kernel(T* __restrict__ A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
+                   int* __restrict__ info) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    __shared__ LeafCand<T, W> s_cand[2][CL];  // written by every CTA of the cluster
+    __shared__ alignas(16) T s_rowj[2][W];       // row j, written by its owner
+    __shared__ LeafCand<T, W> s_warp[LU_THREADS / 32];
+    __shared__ alignas(16) T s_mine[W];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    const int row0 = rank * R;
+    const int nloc = max(0, min(R, m - row0));
+    T a[RPT][W];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int li = tid + r * nt;
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            a[r][k] = li < nloc && k < w ? A[size_t(c0 + k) * size_t(lda) + size_t(c0 + row0 + li)] : T(0);
+    }
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        if (j >= w) break;
+        const int buf = j & 1;
+        // 1. this warp's candidate: the largest |a(i, j)| over its rows i >= j (smallest index on ties)
+        T best = T(-1);
+        int bi = INT_MAX;
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) {
+            const int li = tid + r * nt, i = row0 + li;
+            const T v = fabs(a[r][j]);
+            if (li < nloc && i >= j && v > best) {
+                best = v;
+                bi = i;
+            }
+        }
+        T wb;
+        const int wi = warp_best(best, bi, wb);
+        if (bi == wi && wi != INT_MAX) {
+            s_warp[wid].best = wb;
+            s_warp[wid].idx = wi;
+#pragma unroll
+            for (int r = 0; r < RPT; ++r)
+                if (row0 + tid + r * nt == wi)
+#pragma unroll
+                    for (int k = 0; k < W; ++k) s_warp[wid].row[k] = a[r][k];
+        } else if (wi == INT_MAX && lane == 0) {
+            s_warp[wid].best = T(-1);
+            s_warp[wid].idx = INT_MAX;
+        }
+        const bool own_j = j >= row0 && j < row0 + nloc;
+        if (own_j)
+#pragma unroll
+            for (int r = 0; r < RPT; ++r)
+                if (row0 + tid + r * nt == j)
+#pragma unroll
+                    for (int k = 0; k < W; ++k) s_mine[k] = a[r][k];
+        __syncthreads();
+        // 2. the CTA's candidate and its row, and row j, to every CTA of the cluster
+        if (wid == 0) {
+            T cb;
+            const T v = lane < nw ? s_warp[lane].best : T(-1);
+            const int ci = warp_best(v, lane < nw ? s_warp[lane].idx : INT_MAX, cb);
+            const unsigned who = __ballot_sync(0xffffffffu, lane < nw && ci != INT_MAX && s_warp[lane].idx == ci);
+            const T* src = s_warp[who ? __ffs(who) - 1 : 0].row;
+            for (int e = lane; e < CL * W; e += 32) {
+                const int dst = e / W, k = e - dst * W;
+                LeafCand<T, W>* c = cl.map_shared_rank(&s_cand[buf][rank], dst);
+                c->row[k] = src[k];
+                if (k == 0) {
+                    c->best = ci == INT_MAX ? T(-1) : cb;
+                    c->idx = ci;
+                }
+                if (own_j) cl.map_shared_rank(&s_rowj[buf][0], dst)[k] = s_mine[k];
+            }
+        }
+        cl.sync();
+        // 3. the pivot over the cluster
+        T gb = T(-1);
+        int p = INT_MAX, pr = 0;
+#pragma unroll
+        for (int r = 0; r < CL; ++r) {
+            const T v = s_cand[buf][r].best;
+            const int ix = s_cand[buf][r].idx;
+            if (ix != INT_MAX && (v > gb || (v == gb && ix < p))) {
+                gb = v;
+                p = ix;
+                pr = r;
+            }
+        }
+        if (!(gb > T(0)) || p == INT_MAX) {
+            if (rank == 0 && tid == 0) {
+                if (*info == 0) *info = c0 + j + 1;
+                ipiv[c0 + j] = c0 + j;
+            }
+            continue;
+        }
+        if (rank == 0 && tid == 0) ipiv[c0 + j] = c0 + p;
+        const T* piv = s_cand[buf][pr].row;
+        // 4. swap rows j and p, eliminate below the pivot (l = 0 leaves a row alone)
+        T l[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) {
+            const int li = tid + r * nt, i = row0 + li;
+            if (i == p && p != j && li < nloc)
+#pragma unroll
+                for (int k = 0; k < W; ++k) a[r][k] = s_rowj[buf][k];
+            if (i == j && li < nloc)
+#pragma unroll
+                for (int k = 0; k < W; ++k) a[r][k] = piv[k];
+            l[r] = T(0);
+            if (i > j && li < nloc) a[r][j] = l[r] = a[r][j] / piv[j];
+        }
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (k > j) {
+                const T pk = piv[k];
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) a[r][k] -= l[r] * pk;
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int li = tid + r * nt;
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (li < nloc && k < w) A[size_t(c0 + k) * size_t(lda) + size_t(c0 + row0 + li)] = a[r][k];
+    }
+    cl.sync();  // no CTA leaves while another may still write its shared memory
+}
+
+// The LU leaf for panels too tall for the cluster's registers (over 16,384 rows): the panel in shared memory.
 template <class T, int W>
 __global__ void __cluster_dims__(LU_CL, 1, 1) __launch_bounds__(LU_THREADS)
-    lu_leaf_kernel(T* __restrict__ A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
+    lu_leaf_tall_kernel(T* __restrict__ A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
                    int* __restrict__ info) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -207,19 +374,52 @@ __global__ void __cluster_dims__(LU_CL, 1, 1) __launch_bounds__(LU_THREADS)
     cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// apply the row swaps ipiv[j0..j1) (in order) to the columns [cs, ce)
+// apply the row swaps ipiv[j0..j1) (in order) to the columns [cs, ce). The swaps go in groups of 16: a group touches at
+// most 32 rows (its own 16 and their partners), and one thread works out which row each of them ends up with; then a warp
+// takes a column at a time, a lane a row: one load and one store, where a thread that swaps along its column waits for
+// one swap after another (and reads a 32-byte sector per element).
+constexpr int SWAP_G = 16, SWAP_WARPS = 8;
 template <class T>
-__global__ void laswp_kernel(T* __restrict__ A, long long lda, int cs, int ce, int j0, int j1, const int* __restrict__ ipiv) {
-    int c = cs + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ce) return;
-    T* col = A + size_t(c) * size_t(lda);
-    for (int j = j0; j < j1; ++j) {
-        int p = ipiv[j];
-        if (p != j) {
-            T t = col[j];
-            col[j] = col[p];
-            col[p] = t;
+__global__ void __launch_bounds__(32 * SWAP_WARPS) laswp_kernel(T* __restrict__ A, long long lda, int cs, int ce, int j0, int j1,
+                                                              const int* __restrict__ ipiv) {
+    __shared__ int s_row[2 * SWAP_G], s_src[2 * SWAP_G], s_n;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int g = j0; g < j1; g += SWAP_G) {
+        const int ng = min(SWAP_G, j1 - g);
+        if (w == 0) {
+            // rows: g .. g + ng - 1 in places 0 .. ng - 1, then the partners outside that range, each once
+            const int p = lane < ng ? ipiv[g + lane] : -1;
+            int row = lane < ng ? g + lane : -1, n = ng;
+            for (int k = 0; k < ng; ++k) {
+                const int pk = __shfl_sync(0xffffffffu, p, k);
+                if (!__any_sync(0xffffffffu, row == pk)) {
+                    if (lane == n) row = pk;
+                    ++n;
+                }
+            }
+            int src = row;  // the row whose value this place ends up with
+            for (int k = 0; k < ng; ++k) {
+                const int pk = __shfl_sync(0xffffffffu, p, k);
+                const int at = __ffs(__ballot_sync(0xffffffffu, row == pk)) - 1;
+                const int a = __shfl_sync(0xffffffffu, src, k), b = __shfl_sync(0xffffffffu, src, at);
+                if (lane == k) src = b;
+                else if (lane == at) src = a;
+            }
+            s_row[lane] = row;
+            s_src[lane] = src;
+            if (lane == 0) s_n = n;
         }
+        __syncthreads();
+        const int row = s_row[lane], src = s_src[lane];
+        const bool on = lane < s_n && src != row;
+        for (int c = cs + blockIdx.x * SWAP_WARPS + w; c < ce; c += gridDim.x * SWAP_WARPS) {
+            T* col = A + size_t(c) * size_t(lda);
+            const T v = on ? col[src] : T(0);
+            __syncwarp();
+            if (on) col[row] = v;
+            __syncwarp();
+        }
+        __syncthreads();
     }
 }
 
@@ -302,24 +502,61 @@ int trsm<float>(vp_ctx* ctx, cublasFillMode_t uplo, cublasOperation_t op, cublas
 
 template <class T>
 int leaf_width(int m) {
-    // the widest leaf whose panel fits the cluster's shared memory (200 KB per CTA)
+    // FP64: the widest leaf that a cluster of 16 holds in registers (16 columns up to 8,192 rows, 8 up to 16,384); else,
+    // and in FP32, the widest whose panel fits the shared memory of 8 CTAs (200 KB each)
     int R = (m + LU_CL - 1) / LU_CL;
+    if (sizeof(T) == 8 && m <= 32 * LU_THREADS) return m <= 16 * LU_THREADS ? 16 : 8;
     for (int w : {16, 8, 4})
         if (size_t(R) * w * sizeof(T) <= 200 * 1024) return w;
     return 0;
 }
 
 template <class T, int W>
-int launch_leaf(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
-    if (w < 1 || w > W || w > m) return vp_fail(ctx, VP_ERR_ARG, "LU leaf width out of range");
+int launch_leaf_tall(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
     int R = (m + LU_CL - 1) / LU_CL;
     size_t smem = size_t(R) * W * sizeof(T);
     if (smem > 227 * 1024) return vp_fail(ctx, VP_ERR_ARG, "LU leaf panel does not fit shared memory");
-    VP_CUDA(ctx, cudaFuncSetAttribute(lu_leaf_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    lu_leaf_kernel<T, W><<<LU_CL, LU_THREADS, smem, ctx->stream>>>(A, lda, c0, m, w, R, ipiv, info);
+    VP_CUDA(ctx, cudaFuncSetAttribute(lu_leaf_tall_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    lu_leaf_tall_kernel<T, W><<<LU_CL, LU_THREADS, smem, ctx->stream>>>(A, lda, c0, m, w, R, ipiv, info);
     ctx->launches++;
     VP_CUDA(ctx, cudaGetLastError());
     return VP_OK;
+}
+
+// rows a thread holds at most: 32 words of panel a row pair fit its 128 registers
+template <class T, int W>
+constexpr int leaf_rpt_max = W * sizeof(T) <= 64 ? 2 : 1;
+
+template <class T, int W, int RPT, int CL>
+int launch_leaf_cl(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int R, int nt, int* ipiv, int* info) {
+    auto kern = lu_leaf_kernel<T, W, RPT, CL>;
+    if (CL > 8) VP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CL);
+    cfg.blockDim = dim3(nt);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    VP_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, A, (long long)lda, c0, m, w, R, ipiv, info));
+    ctx->launches++;
+    return VP_OK;
+}
+
+// A cluster of 8 CTAs where the panel fits its registers, of 16 (the largest) above that, the tall kernel beyond.
+template <class T, int W>
+int launch_leaf(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
+    if (w < 1 || w > W || w > m) return vp_fail(ctx, VP_ERR_ARG, "LU leaf width out of range");
+    constexpr int RM = leaf_rpt_max<T, W>;
+    const int cl = m <= 8 * RM * LU_THREADS ? 8 : 16, R = (m + cl - 1) / cl;
+    const int nt = std::min(LU_THREADS, (R + 31) / 32 * 32), rpt = (R + nt - 1) / nt;
+    if (rpt > RM) return launch_leaf_tall<T, W>(ctx, A, lda, c0, m, w, ipiv, info);
+    if (cl == 16) return launch_leaf_cl<T, W, RM, 16>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
+    if (rpt == 1) return launch_leaf_cl<T, W, 1, 8>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
+    return launch_leaf_cl<T, W, RM, 8>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
 }
 
 // factor a leaf of w columns with the smallest kernel instance that holds it
@@ -327,9 +564,7 @@ template <class T>
 int leaf(vp_ctx* ctx, T* A, int lda, int c0, int w, int m, int* ipiv, int* info) {
     if (w > 8) return launch_leaf<T, 16>(ctx, A, lda, c0, m, w, ipiv, info);
     if (w > 4) return launch_leaf<T, 8>(ctx, A, lda, c0, m, w, ipiv, info);
-    if (w > 2) return launch_leaf<T, 4>(ctx, A, lda, c0, m, w, ipiv, info);
-    if (w > 1) return launch_leaf<T, 2>(ctx, A, lda, c0, m, w, ipiv, info);
-    return launch_leaf<T, 1>(ctx, A, lda, c0, m, w, ipiv, info);
+    return launch_leaf<T, 4>(ctx, A, lda, c0, m, w, ipiv, info);
 }
 
 __global__ void iota_kernel(int n, int* __restrict__ a) {
@@ -341,7 +576,8 @@ template <class T>
 int laswp(vp_ctx* ctx, T* A, int lda, int cs, int ce, int j0, int j1, const int* ipiv) {
     if (ce <= cs || j1 <= j0) return VP_OK;
     int nc = ce - cs;
-    laswp_kernel<T><<<(nc + 127) / 128, 128, 0, ctx->stream>>>(A, lda, cs, ce, j0, j1, ipiv);
+    laswp_kernel<T><<<std::min((nc + SWAP_WARPS - 1) / SWAP_WARPS, 8 * ctx->nsm), 32 * SWAP_WARPS, 0, ctx->stream>>>(
+        A, lda, cs, ce, j0, j1, ipiv);
     ctx->launches++;
     VP_CUDA(ctx, cudaGetLastError());
     return VP_OK;
