@@ -40,8 +40,6 @@ __global__ void __launch_bounds__(128) blob_rhs_kernel(BlobRhsArgs a) {
     }
 }
 
-int points_grid(int n) { return (n + NB_THREADS - 1) / NB_THREADS; }
-
 }  // namespace
 
 extern "C" int vp_blob_velocities(vp_ctx* ctx, int precision, int nblob, const double* blobs, int npts, const double* X,
@@ -60,14 +58,16 @@ extern "C" int vp_blob_velocities(vp_ctx* ctx, int precision, int nblob, const d
     std::vector<double> hb(blobs, blobs + 7 * size_t(nblob));
     std::vector<double> hx(X, X + 3 * size_t(npts));
     if ((r = dl.up(ctx, &db, hb)) || (r = dl.up(ctx, &dx, hx)) || (r = dl.alloc(ctx, &du, 3 * size_t(npts)))) return r;
+    double* dp;
+    if ((r = dl.alloc(ctx, &dp, sum_parts(ctx, npts, precision == VP_FP64 ? NB_THREADS : NB_THREADS * NB_PTS,
+                                          (nblob + NB_TILE - 1) / NB_TILE))))
+        return r;
     vp_phase_begin(ctx, PH_WAKE);
     if (precision == VP_FP64)
-        blob_kernel<double><<<points_grid(npts), NB_THREADS, 0, ctx->stream>>>(nblob, db, npts, dx, du);
+        launch_blobs<double>(ctx, nblob, db, npts, dx, du, dp);
     else
-        blob_kernel<float><<<(npts + NB_THREADS * NB_PTS - 1) / (NB_THREADS * NB_PTS), NB_THREADS, 0, ctx->stream>>>(
-            nblob, db, npts, dx, du);
+        launch_blobs<float>(ctx, nblob, db, npts, dx, du, dp);
     vp_phase_end(ctx);
-    ctx->launches++;
     VP_CUDA(ctx, cudaGetLastError());
     VP_CUDA(ctx, vp_d2h(ctx, U, du, sizeof(double) * 3 * npts));
     VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -107,13 +107,14 @@ extern "C" int vp_body_velocity(vp_ctx* ctx, int precision, int ntri, const doub
     int r;
     std::vector<double> hx(X, X + 3 * size_t(npts));
     if ((r = dl.up(ctx, &ds, hs)) || (r = dl.up(ctx, &dx, hx)) || (r = dl.alloc(ctx, &du, 3 * size_t(npts)))) return r;
+    double* dp;
+    if ((r = dl.alloc(ctx, &dp, sum_parts(ctx, npts, NB_THREADS, (ntri + BODY_TILE - 1) / BODY_TILE)))) return r;
     vp_phase_begin(ctx, PH_WAKE);
     if (precision == VP_FP64)
-        body_kernel<double><<<points_grid(npts), NB_THREADS, 0, ctx->stream>>>(ntri, ds, kernel_far, npts, dx, du);
+        launch_body<double>(ctx, ntri, ds, kernel_far, npts, dx, du, dp);
     else
-        body_kernel<float><<<points_grid(npts), NB_THREADS, 0, ctx->stream>>>(ntri, ds, kernel_far, npts, dx, du);
+        launch_body<float>(ctx, ntri, ds, kernel_far, npts, dx, du, dp);
     vp_phase_end(ctx);
-    ctx->launches++;
     VP_CUDA(ctx, cudaGetLastError());
     VP_CUDA(ctx, vp_d2h(ctx, U, du, sizeof(double) * 3 * npts));
     VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -1120,6 +1120,7 @@ struct vp_freewake {
     double *blobs = nullptr, *X = nullptr, *ub = nullptr, *uw = nullptr, *umax_part = nullptr;
     double *trow = nullptr, *rhs = nullptr, *x = nullptr, *mu = nullptr, *mu_prev = nullptr, *dmu = nullptr;
     double *cp = nullptr, *surf_part = nullptr, *mom_part = nullptr, *rec = nullptr;
+    double* sum_parts = nullptr;  // the parts of split point sums
     // the mixed path's FP32 N-body kernels: the particles as FP32 splits, the chunks' partial sums, the body sources
     float4 *ph = nullptr, *pl = nullptr, *pa = nullptr;
     double *prhs = nullptr, *bvel = nullptr;
@@ -1423,6 +1424,7 @@ extern "C" int vp_freewake_create(vp_ctx* ctx, const vp_freewake_setup* s, vp_fr
         (r = own_alloc(fw, &fw->mu, size_t(s->nslot))) || (r = own_alloc(fw, &fw->mu_prev, size_t(s->nslot))) ||
         (r = own_alloc(fw, &fw->dmu, size_t(s->nslot))) || (r = own_alloc(fw, &fw->cp, size_t(s->ntri))) ||
         (r = own_alloc(fw, &fw->surf_part, 6 * size_t((s->ntri + 255) / 256 + 1))) ||
+        (r = own_alloc(fw, &fw->sum_parts, sum_parts_max(ctx->nsm, NB_THREADS * NB_PTS))) ||
         (r = own_alloc(fw, &fw->rec, 32 + size_t(nte))) || (r = own_alloc(fw, &fw->src32, size_t(BS32) * s->ntri)))
         return fail(r);
     if ((r = vp_solve_work_alloc(ctx, F, &fw->sw))) return fail(r);
@@ -1565,18 +1567,12 @@ extern "C" int vp_freewake_step(vp_freewake* fw, vp_freewake_record* rec) {
             VP_CUDA(ctx, cudaMemsetAsync(fw->ub, 0, sizeof(double) * 3 * npts, ctx->stream));
             add_chunks_kernel<<<(3 * npts + 255) / 256, 256, 0, ctx->stream>>>(3 * npts, ba.nchunk, fw->bvel, fw->ub);
             ctx->launches += 3;
-            if (nblob > 0)
-                blob_kernel<float><<<(npts + NB_THREADS * NB_PTS - 1) / (NB_THREADS * NB_PTS), NB_THREADS, 0,
-                                     ctx->stream>>>(nblob, fw->blobs, npts, fw->X, fw->uw);
+            if (nblob > 0) launch_blobs<float>(ctx, nblob, fw->blobs, npts, fw->X, fw->uw, fw->sum_parts);
         } else {
-            body_kernel<double><<<(npts + NB_THREADS - 1) / NB_THREADS, NB_THREADS, 0, ctx->stream>>>(
-                ntri, fw->bs, o.kernel_far, npts, fw->X, fw->ub);
-            if (nblob > 0)
-                blob_kernel<double><<<(npts + NB_THREADS - 1) / NB_THREADS, NB_THREADS, 0, ctx->stream>>>(
-                    nblob, fw->blobs, npts, fw->X, fw->uw);
+            launch_body<double>(ctx, ntri, fw->bs, o.kernel_far, npts, fw->X, fw->ub, fw->sum_parts);
+            if (nblob > 0) launch_blobs<double>(ctx, nblob, fw->blobs, npts, fw->X, fw->uw, fw->sum_parts);
         }
         if (nblob == 0) VP_CUDA(ctx, cudaMemsetAsync(fw->uw, 0, sizeof(double) * 3 * npts, ctx->stream));
-        ctx->launches += 2;
     }
     vp_phase_end(ctx);
     vp_phase_begin(ctx, PH_WAKE);
