@@ -30,13 +30,15 @@ enum {
     PH_COUNT
 };
 
-// buffers of the tensor-core GEMM of the LU's trailing updates (vp_tcgemm.cu): the bf16 pieces of its operands,
-// grown to the largest update seen, and its error word
+// buffers of the tensor-core GEMMs of the LU's trailing updates (vp_tcgemm.cu): the bf16 pieces of their operands, grown
+// to the largest update seen, and their error word
 struct TcWork {
     void* pieces = nullptr;  // bf16 elements
     size_t cap = 0;          // elements
+    int* exps = nullptr;     // FP64: the rows' and columns' exponents
+    size_t nexp = 0;
     int* err = nullptr;
-    bool attr_set = false;
+    bool attr_set = false, attr64_set = false;
 };
 
 struct vp_ctx {
@@ -186,6 +188,10 @@ bool vp_tc_gemm_enabled();
 bool vp_tc_gemm_fits(int m, int n, int k);
 int vp_tc_gemm_sub(vp_ctx* ctx, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C,
                    int ldc);
+// the same for FP64 operands, as exact products of 7-bit digits: FP64-class accuracy
+bool vp_tc_gemm64_fits(int m, int n, int k);
+int vp_tc_gemm_sub64(vp_ctx* ctx, int m, int n, int k, const double* A, int lda, const double* B, int ldb, double* C,
+                     int ldc);
 int vp_tc_gemm_check(vp_ctx* ctx);
 void vp_tc_work_free(TcWork* w);
 

@@ -6,10 +6,9 @@
 //  - LU with partial pivoting (the reference calls LAPACK dgetrf): recursive (left half, swap, TRSM, GEMM, right
 //    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster of 8 CTAs that holds the panel in
 //    registers: per column, every CTA sends its pivot candidate's row to all, one cluster barrier, every thread picks
-//    the pivot, swaps and updates its rows. TRSM is cuBLAS; the
-//    trailing-update GEMM is cuBLAS DGEMM for VP_FP64 and, for VP_MIXED, the tensor-core GEMM of vp_tcgemm.cu
-//    (three-piece bf16 split, six tcgen05 products accumulated in FP32 in TMEM) for updates of at least one
-//    128 x 128 x 64 tile, cuBLAS SGEMM for the smaller ones;
+//    the pivot, swaps and updates its rows. The trailing updates run on the tensor cores (vp_tcgemm.cu): VP_MIXED by
+//    three-piece bf16 splits (FP32-class), VP_FP64 by exact products of 7-bit digits (FP64-class), for updates of at
+//    least a tile of the kernels, cuBLAS for the smaller ones; TRSM is cuBLAS, in FP64 on 64 x 64 diagonal blocks only;
 //  - VP_MIXED keeps the FP64 bordered matrix and refines every solve with FP64 residuals (iterative refinement) to
 //    FP64 accuracy;
 //  - the 1-norm condition estimate of dgecon (Hager/Higham, as LAPACK dlacn2) from solves with M and M'.
@@ -467,6 +466,7 @@ int gemm_sub(vp_ctx* ctx, int m, int n, int k, const T* A, int lda, const T* B, 
 template <>
 int gemm_sub<double>(vp_ctx* ctx, int m, int n, int k, const double* A, int lda, const double* B, int ldb, double* C,
                      int ldc) {
+    if (vp_tc_gemm_enabled() && vp_tc_gemm64_fits(m, n, k)) return vp_tc_gemm_sub64(ctx, m, n, k, A, lda, B, ldb, C, ldc);
     const double one = 1.0, mone = -1.0;
     VP_BLAS(ctx, cublasDgemm(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &mone, A, lda, B, ldb, &one, C, ldc));
     return VP_OK;
@@ -498,6 +498,19 @@ int trsm<float>(vp_ctx* ctx, cublasFillMode_t uplo, cublasOperation_t op, cublas
     const float one = 1.0f;
     VP_BLAS(ctx, cublasStrsm(ctx->blas, CUBLAS_SIDE_LEFT, uplo, op, diag, m, n, &one, A, lda, B, ldb));
     return VP_OK;
+}
+
+// X = L^-1 B for the factorization's unit lower triangle L (m x m), in place of B (m x n). FP64: recursive, so that the
+// products go to gemm_sub (tensor cores); cuBLAS's DTRSM, at the FP64 pipe's rate, keeps the 64 x 64 diagonal blocks
+template <class T>
+int trsm_lower(vp_ctx* ctx, int m, int n, const T* L, int ldl, T* B, int ldb) {
+    if (sizeof(T) == 4 || m <= 64 || !vp_tc_gemm64_fits(m, n, m / 2))
+        return trsm<T>(ctx, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, CUBLAS_DIAG_UNIT, m, n, L, ldl, B, ldb);
+    const int h = (m / 2 + 31) / 32 * 32;
+    int r;
+    if ((r = trsm_lower<T>(ctx, h, n, L, ldl, B, ldb))) return r;
+    if ((r = gemm_sub<T>(ctx, m - h, n, h, L + h, ldl, B, ldb, B + h, ldb))) return r;
+    return trsm_lower<T>(ctx, m - h, n, L + size_t(h) * ldl + h, ldl, B + h, ldb);
 }
 
 template <class T>
@@ -593,9 +606,7 @@ int rgetrf(vp_ctx* ctx, T* A, int n, int c0, int w, int lw, int* ipiv, int* info
     int w2 = w - w1;
     if ((r = rgetrf<T>(ctx, A, n, c0, w1, lw, ipiv, info))) return r;
     if ((r = laswp<T>(ctx, A, n, c0 + w1, c0 + w, c0, c0 + w1, ipiv))) return r;
-    if ((r = trsm<T>(ctx, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, CUBLAS_DIAG_UNIT, w1, w2, A + size_t(c0) * n + c0, n,
-                     A + size_t(c0 + w1) * n + c0, n)))
-        return r;
+    if ((r = trsm_lower<T>(ctx, w1, w2, A + size_t(c0) * n + c0, n, A + size_t(c0 + w1) * n + c0, n))) return r;
     if (n - c0 - w1 > 0 &&
         (r = gemm_sub<T>(ctx, n - c0 - w1, w2, w1, A + size_t(c0) * n + (c0 + w1), n, A + size_t(c0 + w1) * n + c0, n,
                          A + size_t(c0 + w1) * n + (c0 + w1), n)))
@@ -643,6 +654,7 @@ int vp_lu_factor(vp_ctx* ctx, int precision, int n, double* M64, vp_factor* F) {
         int lw = leaf_width<double>(n);
         if (!lw) return vp_fail(ctx, VP_ERR_ARG, "matrix too large for the LU panel");
         r = rgetrf<double>(ctx, F->LU64, n, 0, n, lw, F->ipiv, d_info);
+        if (!r) r = vp_tc_gemm_check(ctx);
     } else {
         if ((r = vp_alloc(ctx, &F->LU32, size_t(n) * n))) return r;
         convert_kernel<double, float><<<4 * ctx->nsm, 256, 0, ctx->stream>>>(size_t(n) * n, M64, F->LU32);

@@ -19,9 +19,21 @@
 //     sum from C (coalesced along C's columns).
 // Every mbarrier wait has an iteration limit: a wait that gives up sets the error word, the CTA skips the rest of its
 // work and still frees its TMEM; the host reports VP_ERR_TIMEOUT.
+//
+// FP64 (vp_tc_gemm_sub64, the trailing updates of the FP64 LU): the same tensor cores through exact integer products
+// (Ozaki, Ogita, Oishi and Rump's error-free splitting, Numer. Algorithms 59, 2012; its fixed-point form on low-precision
+// tensor cores). Each row of A and column of B is scaled by a power of two to |x| <= 1 and rounded to 62 bits, cut into
+// nine signed 7-bit digits d_p (x = sum d_p 2^(-6-7p), |d_p| <= 64), bf16 integers. The products of digits p and q are
+// integers of at most 2^12; those of equal p + q = s are summed in one FP32 accumulator, exactly while 9 k 2^12 < 2^24,
+// k <= 448 (longer sums go in slices). The 45 products with s <= 8 are kept: what is dropped is below 2^-59 of
+// |A_i||B_j| (the row's and the column's largest), so that sums whose terms are far below that still come out at DGEMM's
+// accuracy (eight digits were measured 10 times worse than DGEMM on rows graded over five decades, nine are better than
+// it there and elsewhere). The nine accumulators (48 columns each) are combined in FP64 at the end: 11 FP64 instructions
+// an element whatever k, where the FP64 pipe takes k.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 
@@ -260,6 +272,220 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
 }
 
+// ---- FP64 ------------------------------------------------------------------------------------------------------------
+
+constexpr int TD_BN = 48, TD_BK = 32, TD_DIGITS = 9, TD_PAIRS = (TD_DIGITS + 1) / 2, TD_STAGES = 2;
+constexpr int TD_A_BYTES = TC_BM * 128, TD_B_BYTES = TD_BN * 128;  // a tile of two digits of 32 k: rows of 128 bytes
+constexpr int TD_STAGE_BYTES = TD_PAIRS * (TD_A_BYTES + TD_B_BYTES);  // 110 KB
+constexpr int TD_SMEM = TD_STAGES * TD_STAGE_BYTES + 1024;
+constexpr int TD_KMAX = 448;       // exact integer sums in FP32
+constexpr int TD_TMEM_COLS = 512;  // nine accumulators of 48 columns
+constexpr int TD_EMIN = -900;      // exponents below are taken as this (the values' digits vanish)
+
+// the largest exponent field of every row of A (m x k, column-major), or (rows = 0) of every column: into ex (zeroed).
+// Exponent fields order as the numbers; 2047 marks an infinity or NaN.
+__global__ void row_exp_kernel(int m, int k, const double* __restrict__ A, int lda, int* __restrict__ ex) {
+    const int r = blockIdx.x * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
+    int e = 0;
+    if (r < m)
+        for (int c = blockIdx.y * 64 + w; c < min(k, int(blockIdx.y) * 64 + 64); c += 8)
+            e = max(e, (__double2hiint(A[size_t(c) * lda + r]) >> 20) & 2047);
+    __shared__ int s[8][32];
+    s[w][threadIdx.x & 31] = e;
+    __syncthreads();
+    if (w == 0 && r < m) {
+        for (int q = 1; q < 8; ++q) e = max(e, s[q][threadIdx.x]);
+        atomicMax(ex + r, e);
+    }
+}
+__global__ void col_exp_kernel(int k, int n, const double* __restrict__ B, int ldb, int* __restrict__ ex) {
+    const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= n) return;
+    int e = 0;
+    for (int r = lane; r < k; r += 32) e = max(e, (__double2hiint(B[size_t(c) * ldb + r]) >> 20) & 2047);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) ex[c] = e;
+}
+
+// 2^e for the exponents of normal numbers
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+__device__ __forceinline__ int scale_exp(int field) { return max(field - 1022, TD_EMIN); }  // |x| < 2^this
+
+// the digits of x, |x| < 2^e, to dst[q * plane + par * 32], digit 2 q + par
+__device__ __forceinline__ void put_digits(double x, int e, __nv_bfloat16* dst, size_t plane) {
+    long long u = __double2ll_rn(x * pow2(62 - e));
+#pragma unroll
+    for (int p = TD_DIGITS - 1; p >= 0; --p) {
+        const int d = p ? (int(u + 64) & 127) - 64 : int(u);
+        dst[(p >> 1) * plane + (p & 1) * 32] = __float2bfloat16_rn(float(d));
+        u = (u - d) >> 7;
+    }
+}
+
+// A (m x k, column-major) -> digits dst[q][row][k / 32][digit parity][k % 32] (TD_PAIRS planes q of rows_pad rows of 2 k_pad
+// elements), through a 32 x 32 shared-memory transpose; the odd place of the last pair stays unwritten and unread
+__global__ void digits_a_kernel(int m, int k, const double* __restrict__ A, int lda, int rows_pad, int k_pad,
+                                const int* __restrict__ ex, __nv_bfloat16* __restrict__ dst) {
+    __shared__ double t[32][33];
+    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    for (int yy = ty; yy < 32; yy += 8) {
+        const int r = r0 + tx, c = c0 + yy;
+        t[yy][tx] = (r < m && c < k) ? A[size_t(c) * lda + r] : 0.0;
+    }
+    __syncthreads();
+    const size_t plane = size_t(rows_pad) * 2 * k_pad;
+    for (int yy = ty; yy < 32; yy += 8) {
+        const int r = r0 + yy;
+        put_digits(t[tx][yy], r < m ? scale_exp(ex[r]) : 0, dst + size_t(r) * 2 * k_pad + 2 * c0 + tx, plane);
+    }
+}
+// B (k x n, column-major) -> digits dst[q][column][..] in the same layout
+__global__ void digits_b_kernel(int k, int n, const double* __restrict__ B, int ldb, int cols_pad, int k_pad,
+                                const int* __restrict__ ex, __nv_bfloat16* __restrict__ dst) {
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= size_t(cols_pad) * k_pad) return;
+    const int j = int(i / k_pad), kk = int(i % k_pad);
+    const double x = (j < n && kk < k) ? B[size_t(j) * ldb + kk] : 0.0;
+    put_digits(x, j < n ? scale_exp(ex[j]) : 0, dst + size_t(j) * 2 * k_pad + 2 * (kk & ~31) + (kk & 31),
+               size_t(cols_pad) * 2 * k_pad);
+}
+
+constexpr uint32_t TD_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(TD_BN >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
+
+__device__ __forceinline__ void mma_digits(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem), "l"(ad), "l"(bd), "r"(TD_IDESC), "r"(acc)
+        : "memory");
+}
+
+// 8 consecutive FP32 columns of this warp's 32 TMEM lanes (one row per thread)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+// C (m x n) -= A B for one slice of k <= TD_KMAX: one CTA per 128 x 48 tile of C, as tc_gemm_kernel
+__global__ void __launch_bounds__(TC_THREADS, 1)
+    tc_gemm64_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int m, int n,
+                     int ktiles, int m_pad, int n_pad, const int* __restrict__ exA, const int* __restrict__ exB,
+                     double* __restrict__ C, int ldc, int* err) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full_bar[TD_STAGES], empty_bar[TD_STAGES], done_bar;
+    __shared__ uint32_t tmem_holder;
+    __shared__ int s_fail;
+    __shared__ double s_scale[TD_BN];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TD_BN;
+    const uint32_t sbase = smem_u32(smem);
+    auto tileA = [&](int s, int q) { return sbase + uint32_t(s * TD_STAGE_BYTES + q * TD_A_BYTES); };
+    auto tileB = [&](int s, int q) { return sbase + uint32_t(s * TD_STAGE_BYTES + TD_PAIRS * TD_A_BYTES + q * TD_B_BYTES); };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TD_STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        mbar_init(smem_u32(&done_bar), 1);
+        s_fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // the columns' scales: 2^(e - 68), so that a row's 2^e makes C's; NaN for a column with an infinity or NaN
+    for (int j = threadIdx.x; j < TD_BN; j += TC_THREADS) {
+        const int f = n0 + j < n ? exB[n0 + j] : 0;
+        s_scale[j] = f == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : pow2(scale_exp(f) - 68);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
+                     "r"(TD_TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_holder;
+
+    if (threadIdx.x == 0) {  // TMA producer
+        for (int kt = 0; kt < ktiles; ++kt) {
+            const int s = kt % TD_STAGES;
+            if (kt >= TD_STAGES && !mbar_wait(smem_u32(&empty_bar[s]), uint32_t((kt / TD_STAGES - 1) & 1), err)) {
+                s_fail = 1;
+                break;
+            }
+            const uint32_t fb = smem_u32(&full_bar[s]);
+            mbar_expect_tx(fb, TD_STAGE_BYTES);
+            for (int q = 0; q < TD_PAIRS; ++q) {
+                tma_load_2d(tileA(s, q), &mapA, kt * 2 * TD_BK, q * m_pad + m0, fb);
+                tma_load_2d(tileB(s, q), &mapB, kt * 2 * TD_BK, q * n_pad + n0, fb);
+            }
+        }
+    } else if (threadIdx.x == 32) {  // MMA issuer
+        for (int kt = 0; kt < ktiles; ++kt) {
+            const int s = kt % TD_STAGES;
+            if (!mbar_wait(smem_u32(&full_bar[s]), uint32_t((kt / TD_STAGES) & 1), err)) {
+                s_fail = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int kk = 0; kk < TD_BK / 16; ++kk)
+                for (int g = 0; g < TD_DIGITS; ++g)
+                    for (int p = 0; p <= g; ++p) {
+                        const int q = g - p;
+                        const uint64_t ad = smem_desc(tileA(s, p >> 1) + uint32_t((p & 1) * 64 + kk * 32));
+                        const uint64_t bd = smem_desc(tileB(s, q >> 1) + uint32_t((q & 1) * 64 + kk * 32));
+                        mma_digits(tmem + uint32_t(g * TD_BN), ad, bd, (kt | kk | p) ? 1u : 0u);
+                    }
+            mma_commit(smem_u32(&empty_bar[s]));
+        }
+        mma_commit(smem_u32(&done_bar));  // arrives when every MMA issued above has completed
+    }
+    __syncwarp();
+    // epilogue: the accumulators (integers) combined, C -= D
+    const bool done = mbar_wait(smem_u32(&done_bar), 0u, err);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (done && !s_fail) {
+        const int row = m0 + warp * 32 + lane;
+        const int f = row < m ? exA[row] : 0;
+        const double sr = f == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : pow2(scale_exp(f));
+        for (int c0 = 0; c0 < TD_BN; c0 += 8) {
+            uint32_t v[TD_DIGITS][8];
+            const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0);
+#pragma unroll
+            for (int g = 0; g < TD_DIGITS; ++g) tmem_ld8(taddr + uint32_t(g * TD_BN), v[g]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (row < m)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int col = n0 + c0 + j;
+                    int t[4];  // groups 2 h and 2 h + 1: below 2^31 (group g is at most (g + 1) 448 2^12)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h)
+                        t[h] = __float2int_rn(__uint_as_float(v[2 * h][j])) * 128 + __float2int_rn(__uint_as_float(v[2 * h + 1][j]));
+                    double x = double(t[0]);
+                    x = fma(x, 16384.0, double(t[1]));
+                    x = fma(x, 16384.0, double(t[2]));
+                    x = fma(x, 16384.0, double(t[3]));
+                    x = fma(x, 128.0, double(__uint_as_float(v[8][j])));
+                    if (col < n) {
+                        double* c = C + size_t(col) * ldc + row;
+                        *c = fma(-x, sr * s_scale[c0 + j], *c);
+                    }
+                }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TD_TMEM_COLS) : "memory");
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -278,13 +504,14 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// the tensor map of three stacked K-major pieces (3 rows_pad rows of k_pad bf16), box 64 x 128, 128-byte swizzle
-bool make_map(CUtensorMap* map, void* base, int rows_pad, int k_pad) {
+// the tensor map of `planes` stacked K-major planes (rows_pad rows of `cols` bf16 each), box 64 x box_rows, 128-byte
+// swizzle
+bool make_map(CUtensorMap* map, void* base, int planes, int rows_pad, int cols, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
-    const cuuint64_t gdim[2] = {cuuint64_t(k_pad), cuuint64_t(TC_PIECES) * cuuint64_t(rows_pad)};
-    const cuuint64_t gstride[1] = {cuuint64_t(k_pad) * 2};
-    const cuuint32_t box[2] = {TC_BK, TC_BM};
+    const cuuint64_t gdim[2] = {cuuint64_t(cols), cuuint64_t(planes) * cuuint64_t(rows_pad)};
+    const cuuint64_t gstride[1] = {cuuint64_t(cols) * 2};
+    const cuuint32_t box[2] = {64, cuuint32_t(box_rows)};
     const cuuint32_t estride[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
@@ -302,8 +529,81 @@ bool vp_tc_gemm_fits(int m, int n, int k) { return m >= TC_BM && n >= TC_BN && k
 
 void vp_tc_work_free(TcWork* w) {
     if (w->pieces) cudaFree(w->pieces);
+    if (w->exps) cudaFree(w->exps);
     if (w->err) cudaFree(w->err);
     *w = TcWork();
+}
+
+namespace {
+
+// room for `elems` bf16 elements and `nexp` exponents, and the error word (kept as it is when the rest grows)
+int tc_reserve(vp_ctx* ctx, size_t elems, size_t nexp) {
+    TcWork* w = &ctx->tc;
+    int r;
+    if (!w->err) {
+        if ((r = vp_alloc(ctx, &w->err, 1))) return r;
+        VP_CUDA(ctx, cudaMemsetAsync(w->err, 0, sizeof(int), ctx->stream));
+    }
+    if (elems > w->cap) {
+        if (w->pieces) cudaFree(w->pieces);
+        w->pieces = nullptr;
+        w->cap = 0;
+        __nv_bfloat16* p = nullptr;
+        if ((r = vp_alloc(ctx, &p, elems))) return r;
+        w->pieces = p;
+        w->cap = elems;
+    }
+    if (nexp > w->nexp) {
+        if (w->exps) cudaFree(w->exps);
+        w->exps = nullptr;
+        w->nexp = 0;
+        if ((r = vp_alloc(ctx, &w->exps, nexp))) return r;
+        w->nexp = nexp;
+    }
+    return VP_OK;
+}
+
+}  // namespace
+
+// k >= 64, and enough work: below about 8M multiply-adds the five launches (58 us) take longer than cuBLAS's DGEMM
+// (1000 x 64 x 64: 58 against 25 us; 6000 x 64 x 64: 63 against 81; 6000 x 128 x 128: 70 against 226)
+bool vp_tc_gemm64_fits(int m, int n, int k) {
+    return m >= TC_BM && n >= TD_BN && k >= 64 && double(m) * n * k >= 1.6e7;
+}
+
+int vp_tc_gemm_sub64(vp_ctx* ctx, int m, int n, int k, const double* A, int lda, const double* B, int ldb, double* C,
+                     int ldc) {
+    if (m <= 0 || n <= 0 || k <= 0) return VP_OK;
+    const int m_pad = (m + TC_BM - 1) / TC_BM * TC_BM, n_pad = (n + TD_BN - 1) / TD_BN * TD_BN;
+    const int kc = std::min(k, TD_KMAX), kc_pad = (kc + TD_BK - 1) / TD_BK * TD_BK;
+    const size_t na = size_t(2 * TD_PAIRS) * m_pad * kc_pad, nb = size_t(2 * TD_PAIRS) * n_pad * kc_pad;
+    int r = tc_reserve(ctx, na + nb, size_t(m_pad) + n_pad);
+    if (r) return r;
+    TcWork* w = &ctx->tc;
+    if (!w->attr64_set) {
+        VP_CUDA(ctx, cudaFuncSetAttribute(tc_gemm64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TD_SMEM));
+        w->attr64_set = true;
+    }
+    __nv_bfloat16* da = static_cast<__nv_bfloat16*>(w->pieces);
+    __nv_bfloat16* db = da + na;
+    int *ea = w->exps, *eb = w->exps + m_pad;
+    for (int k0 = 0; k0 < k; k0 += TD_KMAX) {
+        const int kk = std::min(TD_KMAX, k - k0), k_pad = (kk + TD_BK - 1) / TD_BK * TD_BK;
+        const double *a = A + size_t(k0) * lda, *b = B + k0;
+        VP_CUDA(ctx, cudaMemsetAsync(ea, 0, sizeof(int) * m_pad, ctx->stream));
+        row_exp_kernel<<<dim3(m_pad / 32, (kk + 63) / 64), 256, 0, ctx->stream>>>(m, kk, a, lda, ea);
+        col_exp_kernel<<<(n + 7) / 8, 256, 0, ctx->stream>>>(kk, n, b, ldb, eb);
+        digits_a_kernel<<<dim3(m_pad / 32, k_pad / 32), 256, 0, ctx->stream>>>(m, kk, a, lda, m_pad, k_pad, ea, da);
+        digits_b_kernel<<<int((size_t(n_pad) * k_pad + 255) / 256), 256, 0, ctx->stream>>>(kk, n, b, ldb, n_pad, k_pad, eb, db);
+        CUtensorMap ma, mb;
+        if (!make_map(&ma, da, TD_PAIRS, m_pad, 2 * k_pad, TC_BM) || !make_map(&mb, db, TD_PAIRS, n_pad, 2 * k_pad, TD_BN))
+            return vp_fail(ctx, VP_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+        tc_gemm64_kernel<<<dim3(m_pad / TC_BM, n_pad / TD_BN), TC_THREADS, TD_SMEM, ctx->stream>>>(
+            ma, mb, m, n, k_pad / TD_BK, m_pad, n_pad, ea, eb, C, ldc, w->err);
+        ctx->launches += 5;
+    }
+    VP_CUDA(ctx, cudaGetLastError());
+    return VP_OK;
 }
 
 int vp_tc_gemm_sub(vp_ctx* ctx, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C,
@@ -313,15 +613,8 @@ int vp_tc_gemm_sub(vp_ctx* ctx, int m, int n, int k, const float* A, int lda, co
     const int m_pad = (m + TC_BM - 1) / TC_BM * TC_BM, n_pad = (n + TC_BN - 1) / TC_BN * TC_BN;
     const int k_pad = (k + TC_BK - 1) / TC_BK * TC_BK;
     const size_t na = size_t(TC_PIECES) * m_pad * k_pad, nb = size_t(TC_PIECES) * n_pad * k_pad;
-    if (na + nb > w->cap) {
-        vp_tc_work_free(w);
-        int r;
-        __nv_bfloat16* pieces = nullptr;
-        if ((r = vp_alloc(ctx, &pieces, na + nb)) || (r = vp_alloc(ctx, &w->err, 1))) return r;
-        w->pieces = pieces;
-        w->cap = na + nb;
-        VP_CUDA(ctx, cudaMemsetAsync(w->err, 0, sizeof(int), ctx->stream));
-    }
+    int r = tc_reserve(ctx, na + nb, 0);
+    if (r) return r;
     if (!w->attr_set) {
         VP_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
         w->attr_set = true;
@@ -331,7 +624,7 @@ int vp_tc_gemm_sub(vp_ctx* ctx, int m, int n, int k, const float* A, int lda, co
     split_a_kernel<<<dim3(m_pad / 32, k_pad / 32), 256, 0, ctx->stream>>>(m, k, A, lda, m_pad, k_pad, a3);
     split_b_kernel<<<int((size_t(n_pad) * k_pad + 255) / 256), 256, 0, ctx->stream>>>(k, n, B, ldb, n_pad, k_pad, b3);
     CUtensorMap ma, mb;
-    if (!make_map(&ma, a3, m_pad, k_pad) || !make_map(&mb, b3, n_pad, k_pad))
+    if (!make_map(&ma, a3, TC_PIECES, m_pad, k_pad, TC_BM) || !make_map(&mb, b3, TC_PIECES, n_pad, k_pad, TC_BN))
         return vp_fail(ctx, VP_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     tc_gemm_kernel<<<dim3(m_pad / TC_BM, n_pad / TC_BN), TC_THREADS, TC_SMEM, ctx->stream>>>(
         ma, mb, m, n, k_pad / TC_BK, m_pad, n_pad, C, ldc, w->err);
