@@ -4,9 +4,9 @@
 //  - reduction + border: one kernel gathers M = C' A Cf (A row-major FP64, C and Cf sparse) into a column-major FP64
 //    matrix through a shared-memory transpose, then the border rows/columns (scaled to the mean |diagonal|) are set;
 //  - LU with partial pivoting (the reference calls LAPACK dgetrf): recursive (left half, swap, TRSM, GEMM, right
-//    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster of 8 CTAs that holds the panel in
-//    registers: per column, every CTA sends its pivot candidate's row to all, one cluster barrier, every thread picks
-//    the pivot, swaps and updates its rows. The trailing updates run on the tensor cores (vp_tcgemm.cu): VP_MIXED by
+//    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster (1 to 16 CTAs) that holds the panel in
+//    registers: per column, every CTA sends its pivot candidate's row to all, every thread picks the pivot, swaps and
+//    updates its rows. The trailing updates run on the tensor cores (vp_tcgemm.cu): VP_MIXED by
 //    three-piece bf16 splits (FP32-class), VP_FP64 by exact products of 7-bit digits (FP64-class), for updates of at
 //    least a tile of the kernels, cuBLAS for the smaller ones; TRSM is cuBLAS, in FP64 on 64 x 64 diagonal blocks only;
 //  - VP_MIXED keeps the FP64 bordered matrix and refines every solve with FP64 residuals (iterative refinement) to
@@ -81,55 +81,80 @@ __global__ void col_abs_sum_kernel(int n, const T* __restrict__ M, double* __res
     if (threadIdx.x == 0) out[c] = red[0];
 }
 
-// the largest |v| of a warp's candidates, the smallest index on ties; NaN is no candidate (index INT_MAX where there is
-// none). Returns the winner's index; best receives its value.
-__device__ __forceinline__ int warp_best(float v, int i, float& best) {
-    if (!(v >= 0.f)) {
-        v = 0.f;
-        i = INT_MAX;
-    }
-    const unsigned key = __float_as_uint(v), m = __reduce_max_sync(0xffffffffu, i == INT_MAX ? 0u : key);
-    best = __uint_as_float(m);
+// |v| as an unsigned key that orders as the magnitudes (above the infinity's: NaN)
+__device__ __forceinline__ unsigned mag_key(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long mag_key(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ bool key_nan(unsigned k) { return k > 0x7f800000u; }
+__device__ __forceinline__ bool key_nan(unsigned long long k) { return k > 0x7ff0000000000000ull; }
+
+// the index of the largest key of a warp's candidates (key, i), the smallest index on ties; INT_MAX: no candidate
+__device__ __forceinline__ int warp_best(unsigned key, int i) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, i == INT_MAX ? 0u : key);
     return __reduce_min_sync(0xffffffffu, key == m ? i : INT_MAX);
 }
-__device__ __forceinline__ int warp_best(double v, int i, double& best) {
-    if (!(v >= 0.0)) {
-        v = 0.0;
-        i = INT_MAX;
-    }
-    const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+__device__ __forceinline__ int warp_best(unsigned long long key, int i) {
+    const unsigned hi = unsigned(key >> 32), lo = unsigned(key);
     const unsigned mh = __reduce_max_sync(0xffffffffu, i == INT_MAX ? 0u : hi);
     const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh && i != INT_MAX ? lo : 0u);
-    best = __hiloint2double(mh, ml);
     return __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? i : INT_MAX);
 }
+
+// a CTA's pivot candidate of a column: its row, the reciprocal of its pivot (FP64), its index (INT_MAX: none)
+template <class T, int W>
+struct alignas(16) LeafCand {
+    T row[W];
+    T rcp;
+    int idx;
+};
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ unsigned cluster_addr(unsigned a, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+// 16 bytes to another CTA's shared memory, counted on its mbarrier
+__device__ __forceinline__ void send16(unsigned dst, uint4 v, unsigned bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
+}
+
+constexpr long long LEAF_WAIT_LIMIT = 1LL << 20;  // tries of a bounded wait
 
 // LU leaf: rows [c0, c0 + m) x columns [c0, c0 + w) (w <= W) of the column-major matrix (ld lda), partial pivoting, by a
 // cluster of CL CTAs. Rows are split over the CTAs (R each) and stay in registers for the whole panel, RPT rows a
 // thread. A column is one chain of latencies - search, exchange, elimination - so what bounds a leaf is the steps in
-// that chain: each warp finds its candidate and writes that row to shared memory, one warp reduces the CTA's candidates
-// and stores the winner and its row to every CTA's shared memory, and after one cluster barrier all threads pick the
-// pivot among the 8 from their own shared memory, swap and eliminate. (With the panel in shared memory, the candidates
-// and the pivot row read from the other CTAs after the barrier, and three more block barriers: 7 us a column.)
-template <class T, int W>
-struct LeafCand {
-    T best;
-    int idx, pad;
-    alignas(16) T row[W];
-};
-template <class T, int W, int RPT, int CL>
-__global__ void __launch_bounds__(LU_THREADS)
-    lu_leaf_kernel(T* __restrict__ A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
+// that chain: each warp finds its candidate and writes that row to shared memory, one warp picks the CTA's and sends it
+// to every CTA's shared memory, where an mbarrier counts the bytes; all threads wait for the candidates on their own
+// mbarrier, pick the pivot, swap and eliminate. (With the panel in shared memory, reads from the other CTAs after a
+// cluster barrier and three more block barriers a column took 7 us; with the candidates pushed and a cluster barrier
+// 2.3 us.) A panel that one CTA holds needs block barriers only. FP64 multiplies by the pivot's reciprocal, computed once
+// by the CTA that sends it: a division per row is ten FP64 instructions of each warp.
+template <class T, int W, int RPT, int CL, int NT>
+__global__ void __launch_bounds__(NT)
+    lu_leaf_kernel(T* A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
                    int* __restrict__ info) {
     cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    __shared__ LeafCand<T, W> s_cand[2][CL];  // written by every CTA of the cluster
-    __shared__ alignas(16) T s_rowj[2][W];       // row j, written by its owner
-    __shared__ LeafCand<T, W> s_warp[LU_THREADS / 32];
+    const int rank = CL > 1 ? (int)cl.block_rank() : 0;
+    constexpr int NV = sizeof(LeafCand<T, W>) / 16, NR = W * sizeof(T) / 16;
+    __shared__ LeafCand<T, W> s_cand[2][CL];         // written by every CTA of the cluster
+    __shared__ alignas(16) T s_rowj[2][W];           // row j, written by its owner
+    __shared__ LeafCand<T, W> s_warp[NT / 32];
     __shared__ alignas(16) T s_mine[W];
+    __shared__ alignas(8) unsigned long long s_bar[2];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
     const int row0 = rank * R;
     const int nloc = max(0, min(R, m - row0));
+    if (CL > 1) {
+        if (tid == 0) {
+            for (int b = 0; b < 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[b])) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        cl.sync();
+    }
     T a[RPT][W];
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
@@ -138,35 +163,37 @@ __global__ void __launch_bounds__(LU_THREADS)
         for (int k = 0; k < W; ++k)
             a[r][k] = li < nloc && k < w ? A[size_t(c0 + k) * size_t(lda) + size_t(c0 + row0 + li)] : T(0);
     }
+    bool lost = false;
 #pragma unroll
     for (int j = 0; j < W; ++j) {
         if (j >= w) break;
         const int buf = j & 1;
+        if (CL > 1 && tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_bar[buf])),
+                         "r"(unsigned(CL * sizeof(LeafCand<T, W>) + W * sizeof(T)))
+                         : "memory");
         // 1. this warp's candidate: the largest |a(i, j)| over its rows i >= j (smallest index on ties)
-        T best = T(-1);
+        decltype(mag_key(T(0))) bk = 0;
         int bi = INT_MAX;
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
             const int li = tid + r * nt, i = row0 + li;
-            const T v = fabs(a[r][j]);
-            if (li < nloc && i >= j && v > best) {
-                best = v;
+            const auto k = mag_key(a[r][j]);
+            if (li < nloc && i >= j && !key_nan(k) && (k > bk || bi == INT_MAX)) {
+                bk = k;
                 bi = i;
             }
         }
-        T wb;
-        const int wi = warp_best(best, bi, wb);
-        if (bi == wi && wi != INT_MAX) {
-            s_warp[wid].best = wb;
+        const int wi = warp_best(bk, bi);
+        if (wi == INT_MAX) {
+            if (lane == 0) s_warp[wid].idx = INT_MAX;
+        } else if (bi == wi) {
             s_warp[wid].idx = wi;
 #pragma unroll
             for (int r = 0; r < RPT; ++r)
                 if (row0 + tid + r * nt == wi)
 #pragma unroll
                     for (int k = 0; k < W; ++k) s_warp[wid].row[k] = a[r][k];
-        } else if (wi == INT_MAX && lane == 0) {
-            s_warp[wid].best = T(-1);
-            s_warp[wid].idx = INT_MAX;
         }
         const bool own_j = j >= row0 && j < row0 + nloc;
         if (own_j)
@@ -174,41 +201,65 @@ __global__ void __launch_bounds__(LU_THREADS)
             for (int r = 0; r < RPT; ++r)
                 if (row0 + tid + r * nt == j)
 #pragma unroll
-                    for (int k = 0; k < W; ++k) s_mine[k] = a[r][k];
+                    for (int k = 0; k < W; ++k) (CL > 1 ? s_mine : s_rowj[buf])[k] = a[r][k];
         __syncthreads();
-        // 2. the CTA's candidate and its row, and row j, to every CTA of the cluster
+        // 2. the CTA's candidate, to every CTA of the cluster, and row j
         if (wid == 0) {
-            T cb;
-            const T v = lane < nw ? s_warp[lane].best : T(-1);
-            const int ci = warp_best(v, lane < nw ? s_warp[lane].idx : INT_MAX, cb);
-            const unsigned who = __ballot_sync(0xffffffffu, lane < nw && ci != INT_MAX && s_warp[lane].idx == ci);
-            const T* src = s_warp[who ? __ffs(who) - 1 : 0].row;
-            for (int e = lane; e < CL * W; e += 32) {
-                const int dst = e / W, k = e - dst * W;
-                LeafCand<T, W>* c = cl.map_shared_rank(&s_cand[buf][rank], dst);
-                c->row[k] = src[k];
-                if (k == 0) {
-                    c->best = ci == INT_MAX ? T(-1) : cb;
-                    c->idx = ci;
+            const int ix = lane < nw ? s_warp[lane].idx : INT_MAX;
+            const int ci = warp_best(ix != INT_MAX ? mag_key(s_warp[lane].row[j]) : 0, ix);
+            const unsigned who = __ballot_sync(0xffffffffu, ix == ci);
+            LeafCand<T, W>* c = &s_warp[__ffs(who) - 1];
+            if (sizeof(T) == 8) {
+                const T rc = ci != INT_MAX ? T(1) / c->row[j] : T(0);
+                if (lane == 0) c->rcp = rc;
+                __syncwarp();
+            }
+            const uint4* src = reinterpret_cast<const uint4*>(c);
+            if (CL > 1) {
+                for (int e = lane; e < CL * NV; e += 32) {
+                    const int dst = e / NV, k = e - dst * NV;
+                    send16(cluster_addr(smem_addr(&s_cand[buf][rank]) + 16 * k, dst), src[k],
+                           cluster_addr(smem_addr(&s_bar[buf]), dst));
                 }
-                if (own_j) cl.map_shared_rank(&s_rowj[buf][0], dst)[k] = s_mine[k];
+                if (own_j)
+                    for (int e = lane; e < CL * NR; e += 32) {
+                        const int dst = e / NR, k = e - dst * NR;
+                        send16(cluster_addr(smem_addr(&s_rowj[buf][0]) + 16 * k, dst), reinterpret_cast<const uint4*>(s_mine)[k],
+                               cluster_addr(smem_addr(&s_bar[buf]), dst));
+                    }
+            } else {
+                for (int k = lane; k < NV; k += 32) reinterpret_cast<uint4*>(&s_cand[buf][0])[k] = src[k];
             }
         }
-        cl.sync();
+        if (CL > 1) {
+            unsigned done = 0;
+            for (long long t = 0; t < LEAF_WAIT_LIMIT && !done && !lost; ++t)
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                    "selp.u32 %0, 1, 0, p;\n\t}"
+                    : "=r"(done)
+                    : "r"(smem_addr(&s_bar[buf])), "r"(unsigned(j >> 1) & 1u)
+                    : "memory");
+            if (!done) lost = true;  // the loop goes on without waits, so that the other barriers end; the factors are dropped
+        } else {
+            __syncthreads();
+        }
         // 3. the pivot over the cluster
-        T gb = T(-1);
+        decltype(mag_key(T(0))) gk = 0;
         int p = INT_MAX, pr = 0;
 #pragma unroll
         for (int r = 0; r < CL; ++r) {
-            const T v = s_cand[buf][r].best;
             const int ix = s_cand[buf][r].idx;
-            if (ix != INT_MAX && (v > gb || (v == gb && ix < p))) {
-                gb = v;
+            const auto k = mag_key(s_cand[buf][r].row[j]);
+            if (ix != INT_MAX && (k > gk || p == INT_MAX || (k == gk && ix < p))) {
+                gk = k;
                 p = ix;
                 pr = r;
             }
         }
-        if (!(gb > T(0)) || p == INT_MAX) {
+        if (gk == 0 || lost) {
+            if (lost) atomicExch(info, -1);
             if (rank == 0 && tid == 0) {
                 if (*info == 0) *info = c0 + j + 1;
                 ipiv[c0 + j] = c0 + j;
@@ -218,6 +269,8 @@ __global__ void __launch_bounds__(LU_THREADS)
         if (rank == 0 && tid == 0) ipiv[c0 + j] = c0 + p;
         const T* piv = s_cand[buf][pr].row;
         // 4. swap rows j and p, eliminate below the pivot (l = 0 leaves a row alone)
+        const T pj = piv[j], rj = s_cand[buf][pr].rcp;
+        const bool mul = sizeof(T) == 8 && fabs(pj) > T(1e-300);
         T l[RPT];
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {
@@ -229,7 +282,7 @@ __global__ void __launch_bounds__(LU_THREADS)
 #pragma unroll
                 for (int k = 0; k < W; ++k) a[r][k] = piv[k];
             l[r] = T(0);
-            if (i > j && li < nloc) a[r][j] = l[r] = a[r][j] / piv[j];
+            if (i > j && li < nloc) a[r][j] = l[r] = mul ? a[r][j] * rj : a[r][j] / pj;
         }
 #pragma unroll
         for (int k = 0; k < W; ++k)
@@ -239,6 +292,7 @@ __global__ void __launch_bounds__(LU_THREADS)
                 for (int r = 0; r < RPT; ++r) a[r][k] -= l[r] * pk;
             }
     }
+    asm volatile("" : "+l"(A));  // the store addresses computed anew, not kept in registers since the loads
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
         const int li = tid + r * nt;
@@ -246,7 +300,7 @@ __global__ void __launch_bounds__(LU_THREADS)
         for (int k = 0; k < W; ++k)
             if (li < nloc && k < w) A[size_t(c0 + k) * size_t(lda) + size_t(c0 + row0 + li)] = a[r][k];
     }
-    cl.sync();  // no CTA leaves while another may still write its shared memory
+    if (CL > 1) cl.sync();  // no CTA leaves while another may still write its shared memory
 }
 
 // The LU leaf for panels too tall for the cluster's registers (over 16,384 rows): the panel in shared memory.
@@ -378,6 +432,34 @@ __global__ void __cluster_dims__(LU_CL, 1, 1) __launch_bounds__(LU_THREADS)
 // takes a column at a time, a lane a row: one load and one store, where a thread that swaps along its column waits for
 // one swap after another (and reads a 32-byte sector per element).
 constexpr int SWAP_G = 16, SWAP_WARPS = 8;
+constexpr int PANEL_W = 64;  // columns of a panel that is factored leaf by leaf
+
+// one warp: the rows that the ng swaps ipiv[g..g + ng) touch (g .. g + ng - 1 in places 0 .. ng - 1, then the partners
+// outside that range, each once; -1 in the other places), and the row whose value each of them ends up with
+__device__ __forceinline__ void swap_rows(const int* __restrict__ ipiv, int g, int ng, int lane, int* s_row, int* s_src,
+                                          int* s_n) {
+    const int p = lane < ng ? ipiv[g + lane] : -1;
+    int row = lane < ng ? g + lane : -1, n = ng;
+    for (int k = 0; k < ng; ++k) {
+        const int pk = __shfl_sync(0xffffffffu, p, k);
+        if (!__any_sync(0xffffffffu, row == pk)) {
+            if (lane == n) row = pk;
+            ++n;
+        }
+    }
+    int src = row;
+    for (int k = 0; k < ng; ++k) {
+        const int pk = __shfl_sync(0xffffffffu, p, k);
+        const int at = __ffs(__ballot_sync(0xffffffffu, row == pk)) - 1;
+        const int a = __shfl_sync(0xffffffffu, src, k), b = __shfl_sync(0xffffffffu, src, at);
+        if (lane == k) src = b;
+        else if (lane == at) src = a;
+    }
+    s_row[lane] = row;
+    s_src[lane] = src;
+    if (lane == 0) *s_n = n;
+}
+
 template <class T>
 __global__ void __launch_bounds__(32 * SWAP_WARPS) laswp_kernel(T* __restrict__ A, long long lda, int cs, int ce, int j0, int j1,
                                                               const int* __restrict__ ipiv) {
@@ -385,29 +467,7 @@ __global__ void __launch_bounds__(32 * SWAP_WARPS) laswp_kernel(T* __restrict__ 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int g = j0; g < j1; g += SWAP_G) {
         const int ng = min(SWAP_G, j1 - g);
-        if (w == 0) {
-            // rows: g .. g + ng - 1 in places 0 .. ng - 1, then the partners outside that range, each once
-            const int p = lane < ng ? ipiv[g + lane] : -1;
-            int row = lane < ng ? g + lane : -1, n = ng;
-            for (int k = 0; k < ng; ++k) {
-                const int pk = __shfl_sync(0xffffffffu, p, k);
-                if (!__any_sync(0xffffffffu, row == pk)) {
-                    if (lane == n) row = pk;
-                    ++n;
-                }
-            }
-            int src = row;  // the row whose value this place ends up with
-            for (int k = 0; k < ng; ++k) {
-                const int pk = __shfl_sync(0xffffffffu, p, k);
-                const int at = __ffs(__ballot_sync(0xffffffffu, row == pk)) - 1;
-                const int a = __shfl_sync(0xffffffffu, src, k), b = __shfl_sync(0xffffffffu, src, at);
-                if (lane == k) src = b;
-                else if (lane == at) src = a;
-            }
-            s_row[lane] = row;
-            s_src[lane] = src;
-            if (lane == 0) s_n = n;
-        }
+        if (w == 0) swap_rows(ipiv, g, ng, lane, s_row, s_src, &s_n);
         __syncthreads();
         const int row = s_row[lane], src = s_src[lane];
         const bool on = lane < s_n && src != row;
@@ -540,9 +600,10 @@ int launch_leaf_tall(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv
 template <class T, int W>
 constexpr int leaf_rpt_max = W * sizeof(T) <= 64 ? 2 : 1;
 
-template <class T, int W, int RPT, int CL>
-int launch_leaf_cl(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int R, int nt, int* ipiv, int* info) {
-    auto kern = lu_leaf_kernel<T, W, RPT, CL>;
+template <class T, int W, int RPT, int CL, int NT>
+int launch_leaf_cl(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
+    auto kern = lu_leaf_kernel<T, W, RPT, CL, NT>;
+    const int R = (m + CL - 1) / CL, nt = std::min(NT, ((R + RPT - 1) / RPT + 31) / 32 * 32);
     if (CL > 8) VP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(CL);
@@ -559,17 +620,22 @@ int launch_leaf_cl(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int R, int 
     return VP_OK;
 }
 
-// A cluster of 8 CTAs where the panel fits its registers, of 16 (the largest) above that, the tall kernel beyond.
+// The smallest cluster that holds the panel, as fewer CTAs exchange faster: FP32, one CTA up to 1,024 rows, 8 CTAs up to
+// 8,192, 16 (the largest) up to 16,384; FP64, whose elimination is bound by each SM's two FP64 operations a clock, one CTA
+// up to 256 rows, 8 up to 2,048, then 16; the tall kernel beyond.
 template <class T, int W>
 int launch_leaf(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
     if (w < 1 || w > W || w > m) return vp_fail(ctx, VP_ERR_ARG, "LU leaf width out of range");
     constexpr int RM = leaf_rpt_max<T, W>;
-    const int cl = m <= 8 * RM * LU_THREADS ? 8 : 16, R = (m + cl - 1) / cl;
-    const int nt = std::min(LU_THREADS, (R + 31) / 32 * 32), rpt = (R + nt - 1) / nt;
-    if (rpt > RM) return launch_leaf_tall<T, W>(ctx, A, lda, c0, m, w, ipiv, info);
-    if (cl == 16) return launch_leaf_cl<T, W, RM, 16>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
-    if (rpt == 1) return launch_leaf_cl<T, W, 1, 8>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
-    return launch_leaf_cl<T, W, RM, 8>(ctx, A, lda, c0, m, w, R, nt, ipiv, info);
+    if constexpr (sizeof(T) == 4) {
+        if (m <= 1024) return launch_leaf_cl<T, W, 1, 1, 1024>(ctx, A, lda, c0, m, w, ipiv, info);
+        if (m <= 8 * RM * LU_THREADS) return launch_leaf_cl<T, W, RM, 8, LU_THREADS>(ctx, A, lda, c0, m, w, ipiv, info);
+    } else {
+        if (m <= 256) return launch_leaf_cl<T, W, 1, 1, 256>(ctx, A, lda, c0, m, w, ipiv, info);
+        if (m <= 2048) return launch_leaf_cl<T, W, 1, 8, 256>(ctx, A, lda, c0, m, w, ipiv, info);
+    }
+    if (m <= 16 * RM * LU_THREADS) return launch_leaf_cl<T, W, RM, 16, LU_THREADS>(ctx, A, lda, c0, m, w, ipiv, info);
+    return launch_leaf_tall<T, W>(ctx, A, lda, c0, m, w, ipiv, info);
 }
 
 // factor a leaf of w columns with the smallest kernel instance that holds it
@@ -596,13 +662,97 @@ int laswp(vp_ctx* ctx, T* A, int lda, int cs, int ce, int j0, int j1, const int*
     return VP_OK;
 }
 
+// After a leaf of the columns [j0, j1) inside the panel [c0, c1): its row swaps on the panel's other columns and, for those
+// to its right, U = L^-1 A of the leaf's rows (L: its unit lower triangle). A warp takes a column, a lane one of the at
+// most 32 rows that the swaps touch (as laswp_kernel); the first j1 - j0 lanes then hold the column's leaf rows and solve
+// by shuffles.
+template <class T>
+__global__ void __launch_bounds__(32 * SWAP_WARPS) panel_swap_kernel(T* __restrict__ A, long long lda, int c0, int c1, int j0,
+                                                                   int j1, const int* __restrict__ ipiv) {
+    __shared__ int s_row[2 * SWAP_G], s_src[2 * SWAP_G], s_n;
+    __shared__ T s_L[SWAP_G][SWAP_G + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ng = j1 - j0;
+    if (w == 0) swap_rows(ipiv, j0, ng, lane, s_row, s_src, &s_n);
+    for (int e = threadIdx.x; e < ng * ng; e += blockDim.x) {
+        const int i = e % ng, k = e / ng;
+        s_L[i][k] = i > k ? A[size_t(j0 + k) * size_t(lda) + j0 + i] : T(0);
+    }
+    __syncthreads();
+    const int row = s_row[lane], src = s_src[lane];
+    const bool on = lane < s_n;
+    for (int q = blockIdx.x * SWAP_WARPS + w; q < c1 - c0 - ng; q += gridDim.x * SWAP_WARPS) {
+        const int c = c0 + q < j0 ? c0 + q : c0 + q + ng;
+        T* col = A + size_t(c) * size_t(lda);
+        T v = on ? col[src] : T(0);
+        if (c >= j1)
+            for (int k = 0; k < ng; ++k) {
+                const T x = __shfl_sync(0xffffffffu, v, k);
+                if (lane > k && lane < ng) v -= s_L[lane][k] * x;
+            }
+        __syncwarp();
+        if (on) col[row] = v;
+        __syncwarp();
+    }
+}
+
+// C -= L U for the panel's columns [j1, c1) and the rows below the leaf: L = A(j1.., j0..j1), U = A(j0..j1, j1..c1). A thread
+// takes a row: its ng values of L in registers, U in shared memory; the row's columns are read and written once.
+template <class T>
+__global__ void __launch_bounds__(128) panel_update_kernel(T* __restrict__ A, long long lda, int n, int c1, int j0, int j1) {
+    __shared__ T s_U[PANEL_W][SWAP_G];
+    const int ng = j1 - j0, nc = c1 - j1;
+    for (int e = threadIdx.x; e < nc * SWAP_G; e += blockDim.x) {
+        const int k = e % SWAP_G, c = e / SWAP_G;
+        s_U[c][k] = k < ng ? A[size_t(j1 + c) * size_t(lda) + j0 + k] : T(0);
+    }
+    const int i = j1 + blockIdx.x * blockDim.x + threadIdx.x;
+    T l[SWAP_G];
+#pragma unroll
+    for (int k = 0; k < SWAP_G; ++k) l[k] = k < ng && i < n ? A[size_t(j0 + k) * size_t(lda) + i] : T(0);
+    __syncthreads();
+    if (i >= n) return;
+    // blockIdx.y: every gridDim.y-th column
+    for (int c = blockIdx.y; c < nc; c += gridDim.y) {
+        T* x = A + size_t(j1 + c) * size_t(lda) + i;
+        T v = T(0);
+#pragma unroll
+        for (int k = 0; k < SWAP_G; ++k) v += l[k] * s_U[c][k];
+        *x -= v;
+    }
+}
+
+// LU of a panel of at most PANEL_W columns [c0, c0 + w): leaf by leaf, each followed by its swaps, triangular solve and
+// update inside the panel. Three launches a leaf of 16 columns, where the recursion down to leaves takes a leaf, two row
+// swap kernels, a cuBLAS TRSM and a cuBLAS GEMM (of 28 us each at 6,600 rows). With the leaf's exchange by mbarriers: LU
+// 99.6 -> 75.3 ms at 6.6k unknowns FP64, 78 -> 68 at 12.8k mixed, 4.4 -> 3.2 at 643 FP64.
+template <class T>
+int panel(vp_ctx* ctx, T* A, int n, int c0, int w, int lw, int* ipiv, int* info) {
+    const int c1 = c0 + w;
+    int r;
+    for (int j0 = c0; j0 < c1; j0 += lw) {
+        const int j1 = std::min(j0 + lw, c1);
+        if ((r = leaf<T>(ctx, A, n, j0, j1 - j0, n - j0, ipiv, info))) return r;
+        if (w == j1 - j0) break;
+        panel_swap_kernel<T><<<(w - (j1 - j0) + SWAP_WARPS - 1) / SWAP_WARPS, 32 * SWAP_WARPS, 0, ctx->stream>>>(A, n, c0, c1,
+                                                                                                                j0, j1, ipiv);
+        ctx->launches++;
+        if (j1 < c1 && j1 < n) {
+            const int gx = (n - j1 + 127) / 128, gy = std::max(1, std::min(c1 - j1, 4 * ctx->nsm / gx));
+            panel_update_kernel<T><<<dim3(gx, gy), 128, 0, ctx->stream>>>(A, n, n, c1, j0, j1);
+            ctx->launches++;
+        }
+    }
+    VP_CUDA(ctx, cudaGetLastError());
+    return VP_OK;
+}
+
 // recursive LU of the columns [c0, c0 + w) (rows c0..n-1)
 template <class T>
 int rgetrf(vp_ctx* ctx, T* A, int n, int c0, int w, int lw, int* ipiv, int* info) {
     int r;
-    if (w <= lw) return leaf<T>(ctx, A, n, c0, w, n - c0, ipiv, info);
-    int w1 = ((w / 2 + lw - 1) / lw) * lw;
-    if (w1 >= w) w1 = w - lw;
+    if (w <= PANEL_W) return panel<T>(ctx, A, n, c0, w, lw, ipiv, info);
+    int w1 = ((w / 2 + PANEL_W - 1) / PANEL_W) * PANEL_W;
+    if (w1 >= w) w1 = w - PANEL_W;
     int w2 = w - w1;
     if ((r = rgetrf<T>(ctx, A, n, c0, w1, lw, ipiv, info))) return r;
     if ((r = laswp<T>(ctx, A, n, c0 + w1, c0 + w, c0, c0 + w1, ipiv))) return r;
@@ -675,6 +825,7 @@ int vp_lu_factor(vp_ctx* ctx, int precision, int n, double* M64, vp_factor* F) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_info);
     if (e != cudaSuccess) return vp_fail(ctx, VP_ERR_CUDA, std::string("LU: ") + cudaGetErrorString(e));
+    if (info < 0) return vp_fail(ctx, VP_ERR_TIMEOUT, "LU leaf: a bounded wait gave up");
     if (info > 0) return vp_fail(ctx, VP_ERR_SINGULAR, "zero pivot in column " + std::to_string(info));
     return VP_OK;
 }
