@@ -363,18 +363,35 @@ __device__ __forceinline__ v3<T> sv_rel(const SrcKern<T>& S, v3<T> r, int side, 
 // segment_velocity (segment.jl:15-25)
 template <class T>
 __device__ __forceinline__ void segment_velocity(v3<T> ra, v3<T> rb, v3<T>& va, v3<T>& vb) {
-    T Ra = vnorm(ra), Rb = vnorm(rb);
+    T Ra, Rb, iRa, iRb;
+    if constexpr (std::is_same<T, double>::value) {  // the reciprocal roots come with the roots: no FP64 division
+        Ra = f64::sqrt_inv(norm2(ra), iRa);
+        Rb = f64::sqrt_inv(norm2(rb), iRb);
+    } else {
+        Ra = vnorm(ra);
+        Rb = vnorm(rb);
+    }
     v3<T> c = cross(ra, rb);
     T p = dot(ra, rb);
-    T den = p >= T(0) ? Ra * Rb + p : norm2(c) / (Ra * Rb - p);
+    T den;
+    if constexpr (std::is_same<T, double>::value)
+        den = p >= 0.0 ? Ra * Rb + p : f64::div(norm2(c), Ra * Rb - p);
+    else
+        den = p >= T(0) ? Ra * Rb + p : norm2(c) / (Ra * Rb - p);
     if (den == T(0) || Ra == T(0) || Rb == T(0)) {
         va = mk3<T>(0, 0, 0);
         vb = va;
         return;
     }
-    v3<T> f = c / (T(4) * vp_pi<T>() * den);
-    va = f / Ra;
-    vb = f / Rb;
+    if constexpr (std::is_same<T, double>::value) {
+        const v3<T> f = f64::rcp(T(4) * vp_pi<T>() * den) * c;
+        va = iRa * f;
+        vb = iRb * f;
+    } else {
+        v3<T> f = c / (T(4) * vp_pi<T>() * den);
+        va = f / Ra;
+        vb = f / Rb;
+    }
 }
 
 // test_weights (assemble.jl:52-58): 0 hat, 1 onering, 2 dual

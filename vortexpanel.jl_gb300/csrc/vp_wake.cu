@@ -30,7 +30,26 @@
 
 namespace {
 
-constexpr int RHS_WARPS = 4;    // warps (test triangles) per block of the right hand side kernel
+// explicit right hand side: warps (test triangle, chunk of sources) of a launch that are enough to fill the chip evenly,
+// and the sheets or filaments a warp takes at least (one a lane)
+constexpr int RHS_ROWS = 24576, RHS_MIN = 32;
+constexpr int NB_TPB = 128;     // targets per block of the body velocity's 2-D grid
+constexpr int NB_BLOCKS = 8;    // such blocks an SM that a grid aims at
+constexpr int P_TILE = 128;     // particles whose FP32 sum is added in FP64
+
+// the source chunks of an N-body grid: n chunks of `per` sources, a multiple of the tile, so that a tile's FP32 sum does not
+// depend on the split; enough of them for NB_BLOCKS blocks an SM. (Chunks of 1,024 left 52 blocks for 3,136 triangles and
+// 2,000 particles: 8.0 ms, 3.0 with chunks of 128.)
+struct NbSplit {
+    int per, n;
+};
+inline NbSplit nb_split(int nsm, int targets, int sources, int tile) {
+    const int blocks = std::max(1, (targets + NB_TPB - 1) / NB_TPB), tiles = (sources + tile - 1) / tile;
+    const int n = std::max(1, std::min(tiles, NB_BLOCKS * nsm / blocks)), per = std::max(1, (tiles + n - 1) / n) * tile;
+    return {per, (sources + per - 1) / per};
+}
+// rows of partial sums of any such grid up to this many targets: n targets <= max(targets, NB_BLOCKS nsm NB_TPB)
+inline size_t nb_rows(int nsm, size_t targets) { return std::max(targets, size_t(NB_BLOCKS) * nsm * NB_TPB); }
 constexpr int BK_THREADS = 1024;  // the single-block bookkeeping kernels
 constexpr int ELEM_THREADS = 128;
 
@@ -244,8 +263,16 @@ struct RhsArgs {
     const double* seg;   // nsg x 8
     const double* part;  // npart x 7
     ParticleRule pr;
-    double* trow;        // ntri x 3: the rows of every test triangle
+    int csh, csg, cpt;   // chunks of the sheets, the filaments, the particles (of pper each)
+    int pper;
+    double* part_rows;   // (csh + csg) x ntri x 3: the sheets' and filaments' rows of every test triangle
+    double* prow;        // cpt x ntri x 3: the particles'
 };
+
+// chunks of n sources: one lane a source, as many as RHS_ROWS allows
+inline int rhs_chunks(int ntri, int n) {
+    return std::min((n + RHS_MIN - 1) / RHS_MIN, std::max(1, RHS_ROWS / std::max(ntri, 1)));
+}
 
 // the source velocity w of sheet S at the point x: the multipole beyond kernel_far diameters, else the exact kernel;
 // FP32 under the guard in mixed precision, FP64 where the guard refuses (source_velocity, source_triangle.jl:134-138)
@@ -287,31 +314,290 @@ __device__ v3<double> sheet_w(const TriGeo& S, v3<double> x, double kfar) {
     return sv_exact3(K, r64 - K.d[0], r64 - K.d[1], r64 - K.d[2], r64, 0, 1e-12);
 }
 
-// one warp per body test triangle: rows_a = -sum over the sheets of the pair block times their doublets, - the
-// filaments' end parts times their circulations, - the particles' normal velocity, each against psi_a
+// a warp's work space of the right hand side: the close sheets waiting, the plans of 32 of them (see near_plan) with
+// n_T x G, their points, and the points the FP32 guard refused
+struct RhsSh {
+    WarpSh warp;
+    NearPlanSh pl;
+    double g[32][3];
+    int list[64], off[33], qp[64], qk[64];
+};
+
+// point k of pair p of the plans in FP32 (as fwd_point32): v[3 a + z] = W psi_a w_z; false where the guard refuses
+__device__ __forceinline__ bool near_eval32(const NearArgs& a, const NearPlanSh& pl, float areaT, int nr, int p, int k,
+                                            v3<float>& w, float* ps) {
+    const int leaf = k / nr, q = k - leaf * nr, code = pl.leaf[p][leaf];
+    float b[9];
+    leaf_corners32(code, b);
+    const float4 m = a.rulef[R_NEAR][q];
+    const float l0 = m.x * b[0] + m.y * b[3] + m.z * b[6];
+    const float l1 = m.x * b[1] + m.y * b[4] + m.z * b[7];
+    const float l2 = m.x * b[2] + m.y * b[5] + m.z * b[8];
+    const float W = m.w * (ldexpf(1.f, -2 * (code >> 6)) * areaT);
+    const float *E = pl.E32[p], *D = pl.D32[p], *Sf = pl.S32[p];
+    SrcKern<float> K;
+    for (int z = 0; z < 3; ++z) {
+        K.d[z] = mk3(Sf[3 * z], Sf[3 * z + 1], Sf[3 * z + 2]);
+        K.nu[z] = mk3(Sf[9 + 3 * z], Sf[10 + 3 * z], Sf[11 + 3 * z]);
+        K.len[z] = Sf[18 + z];
+    }
+    K.n = mk3(Sf[21], Sf[22], Sf[23]);
+    K.area = Sf[24];
+    K.diam = Sf[25];
+    const v3<float> r = l0 * mk3(D[0], D[1], D[2]) + l1 * mk3(D[3], D[4], D[5]) + l2 * mk3(D[6], D[7], D[8]);
+    const float fd = a.kernel_far32 * K.diam;
+    if (dot(r, r) > fd * fd) {
+        w = sv_far(K, r);
+    } else {
+        const v3<float> ra = l0 * mk3(E[0], E[1], E[2]) + l1 * mk3(E[9], E[10], E[11]) + l2 * mk3(E[18], E[19], E[20]);
+        const v3<float> rb = l0 * mk3(E[3], E[4], E[5]) + l1 * mk3(E[12], E[13], E[14]) + l2 * mk3(E[21], E[22], E[23]);
+        const v3<float> rc = l0 * mk3(E[6], E[7], E[8]) + l1 * mk3(E[15], E[16], E[17]) + l2 * mk3(E[24], E[25], E[26]);
+        const Fp32Guard g{PAIR_GUARD};
+        if (!sv_exact3_guarded(K, ra, rb, rc, 0, g, w)) return false;
+    }
+    const v3<float> psi = a.test_mode == 0 ? mk3(l0, l1, l2) : mk3(1.f, 1.f, 1.f);
+    ps[0] = W * psi.x;
+    ps[1] = W * psi.y;
+    ps[2] = W * psi.z;
+    return true;
+}
+
+// the points of leaf `code`, or (q >= 0) its point q alone, of sheet S in FP64: rows_a -= W psi_a w . g. MIXED: as
+// eval_point64, what cancels in FP64 and the functions on it in FP32
+template <bool MIXED>
+__device__ __noinline__ void near_rows64(const NearArgs& a, const TriGeo& T, const TriGeo& S, int code, int q,
+                                         const double* g, double* rows) {
+    float bf[9];
+    leaf_corners32(code, bf);
+    SrcKern<double> K;
+    const v3<double> c = ld3(S.c);
+    for (int z = 0; z < 3; ++z) {
+        K.d[z] = ld3(S.x + 3 * z) - c;
+        K.nu[z] = ld3(S.nu + 3 * z);
+        K.len[z] = S.len[z];
+    }
+    K.n = ld3(S.n);
+    K.area = S.area;
+    K.diam = S.diam;
+    const double fd = a.kernel_far * K.diam, frac = ldexp(1.0, -2 * (code >> 6));
+    v3<double> E[9];
+    for (int k = 0; k < 3; ++k)
+        for (int z = 0; z < 3; ++z) E[3 * k + z] = ld3(T.x + 3 * k) - ld3(S.x + 3 * z);
+    const int q1 = q < 0 ? a.nrule[R_NEAR] : q + 1;
+#pragma unroll 1
+    for (q = max(q, 0); q < q1; ++q) {
+        const RulePt m = a.rule[R_NEAR][q];
+        const double l0 = m.l0 * double(bf[0]) + m.l1 * double(bf[3]) + m.l2 * double(bf[6]);
+        const double l1 = m.l0 * double(bf[1]) + m.l1 * double(bf[4]) + m.l2 * double(bf[7]);
+        const double l2 = m.l0 * double(bf[2]) + m.l1 * double(bf[5]) + m.l2 * double(bf[8]);
+        const v3<double> ra = l0 * E[0] + l1 * E[3] + l2 * E[6], rb = l0 * E[1] + l1 * E[4] + l2 * E[7];
+        const v3<double> rc = l0 * E[2] + l1 * E[5] + l2 * E[8], r = ra + K.d[0];
+        v3<double> w;
+        v3<float> wf;
+        if (dot(r, r) > fd * fd)
+            w = sv_far(K, r);
+        else if (!MIXED)
+            w = sv_exact3(K, ra, rb, rc, r, 0, 1e-12);
+        else if (sv_exact3_split(K, ra, rb, rc, r, 0, 1e-12, wf))
+            w = mk3(double(wf.x), double(wf.y), double(wf.z));
+        else
+            w = exact64_hyb(K, ra, rb, rc, r, 0);
+        const v3<double> psi = test_weights(a.test_mode, l0, l1, l2);
+        const double v = ((m.w * frac) * T.area) * dot(w, ld3(g));
+        rows[0] -= v * psi.x;
+        rows[1] -= v * psi.y;
+        rows[2] -= v * psi.z;
+    }
+}
+
+// the largest p < 32 with off[p] <= i
+__device__ __forceinline__ int place_of(const int* off, int i) {
+    int lo = 0, hi = 31;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= i) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// the first cnt sheets of the list, which are not far from the test triangle: the near tier's pairs by their points, one a
+// lane (a pair has 7 points in most cases: 4.5 pairs to a round of the warp), the other tiers' by the warp, pair by pair.
+// A pair of more than 32 points takes the rounds of a warp for itself, as FP32 sums over its points need their order.
 template <class T>
-__global__ void __launch_bounds__(32 * RHS_WARPS) wake_rhs_kernel(RhsArgs ra) {
-    __shared__ WarpSh shm[RHS_WARPS];
+__device__ void sheet_rows_close(PairCtx& pc, RhsSh& sh, const RhsArgs& ra, int t, int cnt, double* rows) {
+    constexpr bool MIXED = sizeof(T) == 4;
+    const unsigned FULL = 0xffffffffu;
     const NearArgs& a = ra.na;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * RHS_WARPS + w;
-    if (t >= a.ntri) return;
+    const TriGeo& Tr = *pc.T;
+    const int lane = pc.lane;
+    const v3<double> nT = ld3(Tr.n);
+    __syncwarp();
+    const bool valid = lane < cnt;
+    const int s = valid ? sh.list[lane] : 0;
+    int nleaf = 0;
+    const bool near = near_plan(pc, sh.pl, t, a.wtri[s], s, valid, true, nleaf);
+    const int nr = a.nrule[R_NEAR];
+    const int np = near ? nleaf * nr : 0, packed = MIXED ? (np <= 32 ? np : 0) : (near ? nleaf : 0);
+    if (near) {
+        const v3<double> g = cross(nT, ld3(ra.sheet_G + 3 * size_t(s)));
+        sh.g[lane][0] = g.x;
+        sh.g[lane][1] = g.y;
+        sh.g[lane][2] = g.z;
+    }
+    int incl = packed;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    sh.off[lane + 1] = incl;
+    if (lane == 0) sh.off[0] = 0;
+    const int total = __shfl_sync(FULL, incl, 31);
+    unsigned big = __ballot_sync(FULL, MIXED && np > 32);
+    __syncwarp();
+    if constexpr (!MIXED) {
+        for (int i = lane; i < total; i += 32) {
+            const int p = place_of(sh.off, i);
+            near_rows64<false>(a, Tr, a.wtri[sh.list[p]], sh.pl.leaf[p][i - sh.off[p]], -1, sh.g[p], rows);
+        }
+    } else {
+        const float areaT = float(Tr.area);
+        int nq = 0;
+        auto drain = [&](bool all) {
+            while (nq >= 32 || (all && nq > 0)) {
+                __syncwarp();
+                const int take = nq < 32 ? nq : 32;
+                if (lane < take) {
+                    const int p = sh.qp[lane], k = sh.qk[lane];
+                    near_rows64<true>(a, Tr, a.wtri[sh.list[p]], sh.pl.leaf[p][k / nr], k % nr, sh.g[p], rows);
+                }
+                nq -= take;
+                int mp = 0, mk = 0;
+                if (lane < nq) {
+                    mp = sh.qp[take + lane];
+                    mk = sh.qk[take + lane];
+                }
+                __syncwarp();
+                if (lane < nq) {
+                    sh.qp[lane] = mp;
+                    sh.qk[lane] = mk;
+                }
+                __syncwarp();
+            }
+        };
+        auto queue = [&](bool need, int p, int k) {
+            const unsigned m = __ballot_sync(FULL, need);
+            if (need) {
+                const int pos = nq + __popc(m & ((1u << lane) - 1u));
+                sh.qp[pos] = p;
+                sh.qk[pos] = k;
+            }
+            nq += __popc(m);
+            drain(false);
+        };
+        auto add = [&](const float* F, const double* g) {
+            for (int k = 0; k < 3; ++k)
+                rows[k] -= double(F[3 * k]) * g[0] + double(F[3 * k + 1]) * g[1] + double(F[3 * k + 2]) * g[2];
+        };
+        // rounds of the packed pairs' points, then of each large pair's
+        int i0 = 0, pb = -1, nf = 0;
+        float F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        int tot = total;
+        for (;;) {
+            if (i0 >= tot) {
+                if (pb >= 0) {
+                    add(F, sh.g[pb]);
+                    for (int k = 0; k < 9; ++k) F[k] = 0.f;
+                }
+                if (!big) break;
+                pb = __ffs(big) - 1;
+                big &= big - 1;
+                tot = __shfl_sync(FULL, np, pb);
+                i0 = nf = 0;
+            }
+            const int i = i0 + lane;
+            int p = pb, k = i;
+            bool need = false;
+            if (i < tot) {
+                if (pb < 0) {
+                    p = place_of(sh.off, i);
+                    k = i - sh.off[p];
+                }
+                v3<float> w;
+                float ps[3];
+                if (near_eval32(a, sh.pl, areaT, nr, p, k, w, ps)) {
+                    for (int z = 0; z < 3; ++z) {
+                        F[3 * z] += ps[z] * w.x;
+                        F[3 * z + 1] += ps[z] * w.y;
+                        F[3 * z + 2] += ps[z] * w.z;
+                    }
+                    if (pb < 0 || ++nf == 16) {
+                        add(F, sh.g[p]);
+                        for (int z = 0; z < 9; ++z) F[z] = 0.f;
+                        nf = 0;
+                    }
+                } else {
+                    need = true;
+                }
+            }
+            queue(need, p, k);
+            i0 += 32;
+        }
+        drain(true);
+    }
+    unsigned rest = __ballot_sync(FULL, valid && !near);
+    while (rest) {
+        const int q = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const int sq = sh.list[q];
+        FwdAcc acc = {};
+        pc.kind = 0;
+        pc.npts = 0;
+        pc.n64 = 0;
+        tri_pair(pc, acc, t, sq, true);
+        fold32(acc);
+        const v3<double> G = ld3(ra.sheet_G + 3 * size_t(sq));
+        for (int k = 0; k < 3; ++k) {
+            const v3<double> P = mk3(warp_sum(acc.P[k].x), warp_sum(acc.P[k].y), warp_sum(acc.P[k].z));
+            if (lane == 0) rows[k] -= dot(cross(P, nT), G);
+        }
+        __syncwarp();
+    }
+}
+
+// One warp per body test triangle and chunk of sources: rows_a = -sum over the sheets of the pair block times their
+// doublets (this kernel), - the filaments' end parts times their circulations (fil_rhs_kernel), - the particles' normal
+// velocity (particle kernels), each against psi_a. A far sheet is its lane's; the close ones are gathered and taken 32 at a
+// time. A chunk takes every csh-th sheet, which spreads the sheets close to a test triangle over all chunks; the chunks'
+// rows are added in chunk order. Bound by latency and instruction fetch at 8 warps an SM (registers). A step's right hand
+// side on 3,136 triangles with 1,700 sheets, 116 filaments and 2,000 particles: 24.4 ms when a warp took all sources of its
+// triangle and close sheets and filaments one by one, 18.5 with the sources in chunks, 4.0 with the close ones by their
+// points (sheets 1.55, filaments 0.59).
+template <class T>
+__global__ void __launch_bounds__(32) sheet_rhs_kernel(RhsArgs ra) {
+    __shared__ RhsSh shm;
+    const NearArgs& a = ra.na;
+    const int lane = threadIdx.x & 31;
+    const int t = blockIdx.x, chunk = blockIdx.y;
+    double* out = ra.part_rows + 3 * (size_t(chunk) * a.ntri + t);
     const TriGeo& Tr = a.tri[t];
     const v3<double> nT = ld3(Tr.n);
     PairCtx pc;
     pc.a = &a;
     pc.T = &Tr;
-    pc.sh = &shm[w];
+    pc.sh = &shm.warp;
     pc.lane = lane;
     pc.nleaf = 0;
     pc.nq64 = 0;
     double rows[3] = {0, 0, 0};
     const RulePt* RF = a.rule[R_FAR];
     const int nfar = a.nrule[R_FAR];
-    // sheets (wake_pair_rule, assemble.jl:288-293): a far one by its lane, the others by the warp
-    for (int s0 = 0; s0 < ra.nsh; s0 += 32) {
-        const int s = s0 + lane;
-        bool nonfar = false;
+    // sheets (wake_pair_rule, assemble.jl:288-293)
+    int nl = 0;
+    for (int s0 = chunk; s0 < ra.nsh; s0 += 32 * ra.csh) {
+        const int s = s0 + lane * ra.csh;
+        bool close = false;
         if (s < ra.nsh && ra.sheet_ok[s]) {
             const TriGeo& S = a.wtri[s];
             const double dc = vnorm(ld3(S.c) - ld3(Tr.c));
@@ -327,33 +613,187 @@ __global__ void __launch_bounds__(32 * RHS_WARPS) wake_rhs_kernel(RhsArgs ra) {
                     rows[2] -= c * psi.z;
                 }
             } else {
-                nonfar = true;
+                close = true;
             }
         }
-        unsigned msk = __ballot_sync(0xffffffffu, nonfar);
-        while (msk) {
-            const int q = __ffs(msk) - 1;
-            msk &= msk - 1;
-            const int sq = s0 + q;
-            FwdAcc acc = {};
-            pc.kind = 0;
-            pc.npts = 0;
-            pc.n64 = 0;
-            tri_pair(pc, acc, t, sq, true);
-            fold32(acc);
-            const v3<double> G = ld3(ra.sheet_G + 3 * size_t(sq));
-            for (int k = 0; k < 3; ++k) {
-                const v3<double> P = mk3(warp_sum(acc.P[k].x), warp_sum(acc.P[k].y), warp_sum(acc.P[k].z));
-                if (lane == 0) rows[k] -= dot(cross(P, nT), G);
-            }
+        const unsigned msk = __ballot_sync(0xffffffffu, close);
+        if (close) shm.list[nl + __popc(msk & ((1u << lane) - 1u))] = s;
+        nl += __popc(msk);
+        if (nl >= 32) {
+            sheet_rows_close<T>(pc, shm, ra, t, 32, rows);
+            nl -= 32;
+            __syncwarp();
+            if (lane < nl) shm.list[lane] = shm.list[32 + lane];
             __syncwarp();
         }
     }
-    // filaments (segment_rule, assemble.jl:299-306; segment_block, :312-321): far by the lane, vertex or near by the warp
+    if (nl) sheet_rows_close<T>(pc, shm, ra, t, nl, rows);
+    for (int k = 0; k < 3; ++k) {
+        const double v = warp_sum(rows[k]);
+        if (lane == 0) out[k] = v;
+    }
+}
+
+struct FilSh {
+    WarpSh warp;
+    uint8_t leaf[32][64];  // leaf codes: level << 6 | path, as NearPlanSh
+    int list[64], off[33];
+};
+
+// near_pieces' leaves of the filament fa, fb (assemble.jl:131-142), decided in FP32 unless a node is too close to the
+// threshold (as near_plan for a sheet); returns their number
+__device__ int fil_leaves(const NearArgs& a, const TriGeo& T, v3<double> fa, v3<double> fb, uint8_t* leaf) {
+    v3<float> tv[3], sb = mk3(float(fb.x - fa.x), float(fb.y - fa.y), float(fb.z - fa.z));
+    float e32 = vnorm(sb);
+    for (int q = 0; q < 3; ++q) {
+        tv[q] = mk3(float(T.x[3 * q] - fa.x), float(T.x[3 * q + 1] - fa.y), float(T.x[3 * q + 2] - fa.z));
+        e32 = fmaxf(e32, vnorm(tv[q]));
+    }
+    e32 *= 1e-4f;
+    const float ratiof = float(a.near_ratio), isb = 1.f / dot(sb, sb);
+    int level = 0, path = 0, n = 0;
+    for (int guard = 0; guard < 1024; ++guard) {
+        float bf[9];
+        leaf_corners32((level << 6) | path, bf);
+        const v3<float> p1 = bf[0] * tv[0] + bf[1] * tv[1] + bf[2] * tv[2];
+        const v3<float> p2 = bf[3] * tv[0] + bf[4] * tv[1] + bf[5] * tv[2];
+        const v3<float> p3 = bf[6] * tv[0] + bf[7] * tv[1] + bf[8] * tv[2];
+        const float size = fmaxf(vnorm(p2 - p1), fmaxf(vnorm(p3 - p2), vnorm(p1 - p3)));
+        const v3<float> pc = (p1 + p2 + p3) * (1.f / 3.f);
+        const float d = vnorm(pc - fminf(fmaxf(dot(pc, sb) * isb, 0.f), 1.f) * sb);
+        int split = level < a.near_depth ? lt32(d, ratiof * size, 2.f * e32) : 0;
+        if (split < 0) {  // the reference's FP64 test at this node
+            double b[9], dd, tt;
+            for (int z = 0; z < 9; ++z) b[z] = double(bf[z]);
+            const v3<double> q1 = tpoint(T, b), q2 = tpoint(T, b + 3), q3 = tpoint(T, b + 6);
+            const double sz = fmax(vnorm(q2 - q1), fmax(vnorm(q3 - q2), vnorm(q1 - q3)));
+            seg_proj((q1 + q2 + q3) / 3.0, fa, fb, dd, tt);
+            split = dd < a.near_ratio * sz ? 1 : 0;
+        }
+        if (split) {
+            level++;
+            path *= 4;
+            continue;
+        }
+        leaf[n++] = uint8_t((level << 6) | path);
+        while (level > 0 && (path & 3) == 3) {
+            path >>= 2;
+            level--;
+        }
+        if (level == 0) break;
+        path++;
+    }
+    return n;
+}
+
+// the first cnt filaments of the list, which are not far: each lane takes its own's leaves, then the points of all of
+// them are evaluated, one a lane; a filament that ends at a corner of the test triangle (vertex_rule), and depths beyond the
+// leaf codes' room, by the warp
+__device__ void fil_rows_close(PairCtx& pc, FilSh& sh, const RhsArgs& ra, int cnt, double* rows) {
+    const unsigned FULL = 0xffffffffu;
+    const NearArgs& a = ra.na;
+    const TriGeo& Tr = *pc.T;
+    const int lane = pc.lane;
+    const v3<double> nT = ld3(Tr.n);
     const double corners[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    for (int f0 = 0; f0 < ra.nsg; f0 += 32) {
-        const int f = f0 + lane;
-        bool nonfar = false;
+    __syncwarp();
+    int nleaf = 0, kv = -1;
+    if (lane < cnt) {
+        const double* sg = ra.seg + 8 * size_t(sh.list[lane]);
+        const v3<double> fa = ld3(sg), fb = ld3(sg + 3);
+        for (int k = 2; k >= 0; --k)
+            if (fmin(vnorm(ld3(Tr.x + 3 * k) - fa), vnorm(ld3(Tr.x + 3 * k) - fb)) <= 1e-12 * Tr.diam) kv = k;
+        if (kv < 0 && a.near_depth <= 3) {
+            nleaf = fil_leaves(a, Tr, fa, fb, sh.leaf[lane]);
+        }
+    }
+    const int nr = a.nrule[R_NEAR];
+    int incl = nleaf * nr;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    sh.off[lane + 1] = incl;
+    if (lane == 0) sh.off[0] = 0;
+    const int total = __shfl_sync(FULL, incl, 31);
+    __syncwarp();
+    for (int i = lane; i < total; i += 32) {
+        const int p = place_of(sh.off, i), k = i - sh.off[p], lf = k / nr;
+        const int code = sh.leaf[p][lf], level = code >> 6;
+        const double* sg = ra.seg + 8 * size_t(sh.list[p]);
+        const v3<double> fa = ld3(sg), fb = ld3(sg + 3);
+        float bf[9];
+        leaf_corners32(code, bf);
+        const RulePt m = a.rule[R_NEAR][k - lf * nr];
+        const double l0 = m.l0 * double(bf[0]) + m.l1 * double(bf[3]) + m.l2 * double(bf[6]);
+        const double l1 = m.l0 * double(bf[1]) + m.l1 * double(bf[4]) + m.l2 * double(bf[7]);
+        const double l2 = m.l0 * double(bf[2]) + m.l1 * double(bf[5]) + m.l2 * double(bf[8]);
+        const v3<double> t0 = ld3(Tr.x), t1 = ld3(Tr.x + 3), t2 = ld3(Tr.x + 6);
+        v3<double> va, vb;
+        segment_velocity(l0 * (t0 - fa) + l1 * (t1 - fa) + l2 * (t2 - fa), l0 * (t0 - fb) + l1 * (t1 - fb) + l2 * (t2 - fb),
+                         va, vb);
+        const double c = (m.w * ldexp(Tr.area, -2 * level)) * (dot(va, nT) * sg[6] + dot(vb, nT) * sg[7]);
+        const v3<double> psi = test_weights(a.test_mode, l0, l1, l2);
+        rows[0] -= c * psi.x;
+        rows[1] -= c * psi.y;
+        rows[2] -= c * psi.z;
+    }
+    unsigned rest = __ballot_sync(FULL, lane < cnt && nleaf == 0);
+    while (rest) {
+        const int q = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const int kq = __shfl_sync(FULL, kv, q);
+        const double* sg = ra.seg + 8 * size_t(sh.list[q]);
+        const v3<double> fa = ld3(sg), fb = ld3(sg + 3);
+        if (lane == 0)
+            for (int k = 0; k < 3; ++k)
+                for (int z = 0; z < 3; ++z) {
+                    pc.sh->E[9 * k + z] = Tr.x[3 * k + z] - sg[z];
+                    pc.sh->E[9 * k + 3 + z] = Tr.x[3 * k + z] - sg[3 + z];
+                }
+        __syncwarp();
+        FwdAcc acc = {};
+        pc.kind = 1;
+        pc.npts = 0;
+        pc.n64 = 0;
+        pc.side = 0;
+        pc.fp32 = 0;
+        if (kq >= 0) {
+            vertex_rule(pc, acc, kq);
+        } else {
+            near_pieces(pc, acc, SrcRef{1, nullptr, fa, fb}, corners, 1.0, a.near_depth);
+            flush_leaves(pc, acc);
+        }
+        for (int k = 0; k < 3; ++k) {
+            const double ca = warp_sum(acc.ca[k]), cb = warp_sum(acc.cb[k]);
+            if (lane == 0) rows[k] -= ca * sg[6] + cb * sg[7];
+        }
+        __syncwarp();
+    }
+}
+
+// the filaments (segment_rule, assemble.jl:299-306; segment_block, :312-321), FP64; chunks as in sheet_rhs_kernel
+__global__ void __launch_bounds__(32) fil_rhs_kernel(RhsArgs ra) {
+    __shared__ FilSh shm;
+    const NearArgs& a = ra.na;
+    const int lane = threadIdx.x & 31, t = blockIdx.x;
+    const TriGeo& Tr = a.tri[t];
+    const v3<double> nT = ld3(Tr.n);
+    PairCtx pc;
+    pc.a = &a;
+    pc.T = &Tr;
+    pc.sh = &shm.warp;
+    pc.lane = lane;
+    pc.nleaf = 0;
+    pc.nq64 = 0;
+    double rows[3] = {0, 0, 0};
+    const RulePt* RF = a.rule[R_FAR];
+    const int nfar = a.nrule[R_FAR];
+    int nl = 0;
+    for (int f0 = blockIdx.y; f0 < ra.nsg; f0 += 32 * ra.csg) {
+        const int f = f0 + lane * ra.csg;
+        bool close = false;
         if (f < ra.nsg) {
             const double* sg = ra.seg + 8 * size_t(f);
             const v3<double> fa = ld3(sg), fb = ld3(sg + 3);
@@ -370,53 +810,39 @@ __global__ void __launch_bounds__(32 * RHS_WARPS) wake_rhs_kernel(RhsArgs ra) {
                     rows[2] -= c * psi.z;
                 }
             } else {
-                nonfar = true;
+                close = true;
             }
         }
-        unsigned msk = __ballot_sync(0xffffffffu, nonfar);
-        while (msk) {
-            const int q = __ffs(msk) - 1;
-            msk &= msk - 1;
-            const double* sg = ra.seg + 8 * size_t(f0 + q);
-            const v3<double> fa = ld3(sg), fb = ld3(sg + 3);
-            if (lane == 0)
-                for (int k = 0; k < 3; ++k) {
-                    pc.sh->E[9 * k + 0] = Tr.x[3 * k + 0] - fa.x;
-                    pc.sh->E[9 * k + 1] = Tr.x[3 * k + 1] - fa.y;
-                    pc.sh->E[9 * k + 2] = Tr.x[3 * k + 2] - fa.z;
-                    pc.sh->E[9 * k + 3] = Tr.x[3 * k + 0] - fb.x;
-                    pc.sh->E[9 * k + 4] = Tr.x[3 * k + 1] - fb.y;
-                    pc.sh->E[9 * k + 5] = Tr.x[3 * k + 2] - fb.z;
-                }
+        const unsigned msk = __ballot_sync(0xffffffffu, close);
+        if (close) shm.list[nl + __popc(msk & ((1u << lane) - 1u))] = f;
+        nl += __popc(msk);
+        if (nl >= 32) {
+            fil_rows_close(pc, shm, ra, 32, rows);
+            nl -= 32;
             __syncwarp();
-            FwdAcc acc = {};
-            pc.kind = 1;
-            pc.npts = 0;
-            pc.n64 = 0;
-            pc.side = 0;
-            pc.fp32 = 0;
-            int kv = -1;
-            for (int k = 0; k < 3 && kv < 0; ++k)
-                if (fmin(vnorm(ld3(Tr.x + 3 * k) - fa), vnorm(ld3(Tr.x + 3 * k) - fb)) <= 1e-12 * Tr.diam) kv = k;
-            if (kv >= 0) {
-                vertex_rule(pc, acc, kv);
-            } else {
-                SrcRef src{1, nullptr, fa, fb};
-                near_pieces(pc, acc, src, corners, 1.0, a.near_depth);
-                flush_leaves(pc, acc);
-            }
-            for (int k = 0; k < 3; ++k) {
-                const double ca = warp_sum(acc.ca[k]), cb = warp_sum(acc.cb[k]);
-                if (lane == 0) rows[k] -= ca * sg[6] + cb * sg[7];
-            }
+            if (lane < nl) shm.list[lane] = shm.list[32 + lane];
             __syncwarp();
         }
     }
-    // particles (explicit.jl:63-76)
-    for (int k = lane; k < ra.npart; k += 32) particle_rows<T>(ra.pr, Tr, ra.part + 7 * size_t(k), rows);
+    if (nl) fil_rows_close(pc, shm, ra, nl, rows);
+    double* out = ra.part_rows + 3 * (size_t(ra.csh + blockIdx.y) * a.ntri + t);
     for (int k = 0; k < 3; ++k) {
         const double v = warp_sum(rows[k]);
-        if (lane == 0) ra.trow[3 * size_t(t) + k] = v;
+        if (lane == 0) out[k] = v;
+    }
+}
+
+// the particles in FP64 (explicit.jl:63-76; in mixed precision particle_rhs_kernel), a chunk a warp
+__global__ void __launch_bounds__(32) particle_rhs64_kernel(RhsArgs ra) {
+    const int lane = threadIdx.x & 31, t = blockIdx.x, chunk = blockIdx.y;
+    const TriGeo& Tr = ra.na.tri[t];
+    double rows[3] = {0, 0, 0};
+    const int k1 = min((chunk + 1) * ra.pper, ra.npart);
+    for (int k = chunk * ra.pper + lane; k < k1; k += 32) particle_rows<double>(ra.pr, Tr, ra.part + 7 * size_t(k), rows);
+    double* out = ra.prow + 3 * (size_t(chunk) * ra.na.ntri + t);
+    for (int k = 0; k < 3; ++k) {
+        const double v = warp_sum(rows[k]);
+        if (lane == 0) out[k] = v;
     }
 }
 
@@ -449,9 +875,6 @@ __global__ void csr_mv_kernel(int nrow, const int* __restrict__ p, const int* __
 // need the reference's near rule or FP64 (a particle within far_ratio of a test triangle, a point where the FP32 exact
 // kernel cancels, a distance within rounding of a switch) take the FP64 path of the same pair.
 
-constexpr int NB_CHUNK = 1024;  // sources per chunk of the 2-D N-body grids
-constexpr int NB_TPB = 128;     // targets per block
-
 __device__ __forceinline__ void split_hi_lo(double x, float& hi, float& lo) {
     hi = float(x);
     lo = float(x - double(hi));
@@ -472,7 +895,7 @@ __global__ void particle_prep_kernel(int n, const double* __restrict__ part, flo
 }
 
 struct PRhsArgs {
-    int ntri, npart, nchunk;
+    int ntri, npart, nchunk, per;
     const TriGeo* tri;
     const double* part;  // npart x 7 (the FP64 path of near and ambiguous pairs)
     const float4* ph;
@@ -482,20 +905,141 @@ struct PRhsArgs {
     double* out;         // nchunk x ntri x 3
 };
 
-// one thread per body test triangle (its far-rule points), the block's chunk of particles through shared memory:
-// -int psi_a n.u dA of every particle of the chunk (explicit.jl:63-76)
-__global__ void __launch_bounds__(NB_TPB) particle_rhs_kernel(PRhsArgs a) {
-    __shared__ float4 sh[NB_TPB], sl[NB_TPB], sa[NB_TPB];
-    const int t = blockIdx.x * NB_TPB + threadIdx.x;
+// a warp's near (test triangle, particle) pairs waiting: the triangle's lane, the particle's place in the tile; then the
+// leaves, points and rows of 32 of them
+struct PNearSh {
+    int lane[64], k[64], off[33];
+    uint8_t leaf[32][64];  // leaf codes: level << 6 | path, as NearPlanSh
+    double row[32][3];
+};
+
+// near_rule's leaves about the particle x (assemble.jl:69-91 with distance_to(b, p) = |p - x_b|), decided in FP32 unless a
+// node is too close to the threshold (as near_plan); returns their number
+__device__ int particle_leaves(const ParticleRule& a, const TriGeo& T, v3<double> x, uint8_t* leaf) {
+    v3<float> tv[3];
+    float e32 = 0.f;
+    for (int q = 0; q < 3; ++q) {
+        tv[q] = mk3(float(T.x[3 * q] - x.x), float(T.x[3 * q + 1] - x.y), float(T.x[3 * q + 2] - x.z));
+        e32 = fmaxf(e32, vnorm(tv[q]));
+    }
+    e32 *= 1e-4f;
+    const float ratiof = float(a.near_ratio);
+    int level = 0, path = 0, n = 0;
+    for (int guard = 0; guard < 1024; ++guard) {
+        float bf[9];
+        leaf_corners32((level << 6) | path, bf);
+        const v3<float> p1 = bf[0] * tv[0] + bf[1] * tv[1] + bf[2] * tv[2];
+        const v3<float> p2 = bf[3] * tv[0] + bf[4] * tv[1] + bf[5] * tv[2];
+        const v3<float> p3 = bf[6] * tv[0] + bf[7] * tv[1] + bf[8] * tv[2];
+        const float size = fmaxf(vnorm(p2 - p1), fmaxf(vnorm(p3 - p2), vnorm(p1 - p3)));
+        int split = level < a.near_depth ? lt32(vnorm((p1 + p2 + p3) * (1.f / 3.f)), ratiof * size, 2.f * e32) : 0;
+        if (split < 0) {  // the reference's FP64 test at this node
+            double b[9];
+            for (int z = 0; z < 9; ++z) b[z] = double(bf[z]);
+            const v3<double> q1 = tpoint(T, b), q2 = tpoint(T, b + 3), q3 = tpoint(T, b + 6);
+            const double sz = fmax(vnorm(q2 - q1), fmax(vnorm(q3 - q2), vnorm(q1 - q3)));
+            split = vnorm((q1 + q2 + q3) / 3.0 - x) < a.near_ratio * sz ? 1 : 0;
+        }
+        if (split) {
+            level++;
+            path *= 4;
+            continue;
+        }
+        leaf[n++] = uint8_t((level << 6) | path);
+        while (level > 0 && (path & 3) == 3) {
+            path >>= 2;
+            level--;
+        }
+        if (level == 0) break;
+        path++;
+    }
+    return n;
+}
+
+// the first `take` waiting pairs (particle_rows<float> of each): every lane takes its pair's leaves, then the points of all
+// of them are evaluated, one a lane, and summed per pair; each lane adds its triangle's pairs to rows in the list's order
+__device__ __noinline__ void near_particles(const ParticleRule& a, const TriGeo* tri, const double* part, PNearSh& sn, int take,
+                                            int lane, double* rows) {
+    const unsigned FULL = 0xffffffffu;
+    __syncwarp();
+    int np = 0;
+    bool far = false;
+    if (lane < take) {
+        const TriGeo& T = tri[sn.lane[lane]];
+        const double* bl = part + 7 * size_t(sn.k[lane]);
+        const double dx = bl[0] - T.c[0], dy = bl[1] - T.c[1], dz = bl[2] - T.c[2];
+        far = sqrt(dx * dx + dy * dy + dz * dz) > a.far_ratio * fmax(T.diam, bl[6]);
+        np = far ? a.nfar : a.near_depth <= 3 ? a.nnear * particle_leaves(a, T, ld3(bl), sn.leaf[lane]) : 0;
+        sn.row[lane][0] = sn.row[lane][1] = sn.row[lane][2] = 0.0;
+        if (np == 0) particle_rows<float>(a, T, bl, sn.row[lane]);  // deeper than the leaf codes
+    }
+    const unsigned farm = __ballot_sync(FULL, far);
+    int incl = np;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    sn.off[lane + 1] = incl;
+    if (lane == 0) sn.off[0] = 0;
+    const int total = __shfl_sync(FULL, incl, 31);
+    __syncwarp();
+    for (int i0 = 0; i0 < total; i0 += 32) {
+        const int i = i0 + lane;
+        int p = 32 + lane;
+        double r[3] = {0, 0, 0};
+        if (i < total) {
+            p = place_of(sn.off, i);
+            const int k = i - sn.off[p];
+            const bool fp = (farm >> p) & 1;
+            const int lf = fp ? 0 : k / a.nnear, code = fp ? 0 : sn.leaf[p][lf];
+            const RulePt m = fp ? a.rfar[k] : a.rnear[k - lf * a.nnear];
+            float bf[9];
+            leaf_corners32(code, bf);
+            const double l0 = m.l0 * double(bf[0]) + m.l1 * double(bf[3]) + m.l2 * double(bf[6]);
+            const double l1 = m.l0 * double(bf[1]) + m.l1 * double(bf[4]) + m.l2 * double(bf[7]);
+            const double l2 = m.l0 * double(bf[2]) + m.l1 * double(bf[5]) + m.l2 * double(bf[8]);
+            const TriGeo& T = tri[sn.lane[p]];
+            particle_point<float>(a, T, l0, l1, l2, m.w * ldexp(1.0, -2 * (code >> 6)) * T.area, part + 7 * size_t(sn.k[p]), r);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int po = __shfl_down_sync(FULL, p, o);
+            for (int z = 0; z < 3; ++z) {
+                const double v = __shfl_down_sync(FULL, r[z], o);
+                if (lane + o < 32 && po == p) r[z] += v;
+            }
+        }
+        const int before = __shfl_up_sync(FULL, p, 1);
+        if (p < 32 && (lane == 0 || before != p))
+            for (int z = 0; z < 3; ++z) sn.row[p][z] += r[z];
+        __syncwarp();
+    }
+    for (int e = 0; e < take; ++e)
+        if (sn.lane[e] == lane)
+            for (int z = 0; z < 3; ++z) rows[z] += sn.row[e][z];
+    __syncwarp();
+}
+
+// One thread per body test triangle (its far-rule points), a warp's 32 triangles and chunk of particles through shared
+// memory: -int psi_a n.u dA of every particle of the chunk (explicit.jl:63-76). The near pairs (a quadtree about the
+// particle each) are gathered and taken 32 at a time. They are concentrated on the triangles and particles beside the
+// trailing edge, hence CTAs of one warp. NQ: room for the far rule's points (its registers). 3,136 triangles, 2,000
+// particles: 3.0 ms with each near pair evaluated by its thread at once and CTAs of 128 triangles, 2.0 so.
+template <int NQ>
+__global__ void __launch_bounds__(32) particle_rhs_kernel(PRhsArgs a) {
+    __shared__ float4 sh[P_TILE], sl[P_TILE], sa[P_TILE];
+    __shared__ PNearSh sn;
+    const int t = blockIdx.x * 32 + threadIdx.x, lane = threadIdx.x & 31;
     const bool valid = t < a.ntri;
     const TriGeo& Tr = a.tri[valid ? t : 0];
     const int nf = a.pr.nfar;
-    float qh[NQMAX][3], ql[NQMAX][3];
-    double U[NQMAX][3];
+    float qh[NQ][3], ql[NQ][3];
+    double U[NQ][3];
     float ch[3], cl[3];
     for (int z = 0; z < 3; ++z) split_hi_lo(Tr.c[z], ch[z], cl[z]);
 #pragma unroll
-    for (int q = 0; q < NQMAX; ++q) {
+    for (int q = 0; q < NQ; ++q) {
         const RulePt m = a.pr.rfar[q < nf ? q : 0];
         const v3<double> x = tpoint(Tr, &m.l0);
         split_hi_lo(x.x, qh[q][0], ql[q][0]);
@@ -505,29 +1049,44 @@ __global__ void __launch_bounds__(NB_TPB) particle_rhs_kernel(PRhsArgs a) {
     }
     const float diam = float(Tr.diam), fr = float(a.pr.far_ratio);
     double rows[3] = {0, 0, 0};
-    const int j0 = blockIdx.y * NB_CHUNK, j1 = min(a.npart, j0 + NB_CHUNK);
-    for (int b0 = j0; b0 < j1; b0 += NB_TPB) {
-        const int nb = min(NB_TPB, j1 - b0);
-        __syncthreads();
-        if (threadIdx.x < nb) {
-            sh[threadIdx.x] = a.ph[b0 + threadIdx.x];
-            sl[threadIdx.x] = a.pl[b0 + threadIdx.x];
-            sa[threadIdx.x] = a.pa[b0 + threadIdx.x];
+    const int j0 = blockIdx.y * a.per, j1 = min(a.npart, j0 + a.per);
+    for (int b0 = j0; b0 < j1; b0 += P_TILE) {
+        const int nb = min(P_TILE, j1 - b0);
+        __syncwarp();
+        for (int k = lane; k < nb; k += 32) {
+            sh[k] = a.ph[b0 + k];
+            sl[k] = a.pl[b0 + k];
+            sa[k] = a.pa[b0 + k];
         }
-        __syncthreads();
-        if (!valid) continue;
-        float u[NQMAX][3];
+        __syncwarp();
+        int nq = 0;  // near pairs waiting
+        auto drain = [&](bool all) {
+            while (nq >= 32 || (all && nq > 0)) {
+                const int take = min(nq, 32);
+                near_particles(a.pr, a.tri + (t - lane), a.part + 7 * size_t(b0), sn, take, lane, rows);
+                nq -= take;
+                const int ml = lane < nq ? sn.lane[take + lane] : 0, mk = lane < nq ? sn.k[take + lane] : 0;
+                __syncwarp();
+                if (lane < nq) {
+                    sn.lane[lane] = ml;
+                    sn.k[lane] = mk;
+                }
+                __syncwarp();
+            }
+        };
+        float u[NQ][3];
 #pragma unroll
-        for (int q = 0; q < NQMAX; ++q) u[q][0] = u[q][1] = u[q][2] = 0.f;
+        for (int q = 0; q < NQ; ++q) u[q][0] = u[q][1] = u[q][2] = 0.f;
         for (int k = 0; k < nb; ++k) {
             const float4 h = sh[k], l = sl[k], al = sa[k];
             const float dx = (ch[0] - h.x) + (cl[0] - l.x), dy = (ch[1] - h.y) + (cl[1] - l.y),
                         dz = (ch[2] - h.z) + (cl[2] - l.z);
             const float d2 = dx * dx + dy * dy + dz * dz;
             const float thr = fr * fmaxf(diam, l.w);
-            if (d2 > thr * thr * 1.00001f) {  // far, beyond rounding: the far rule's points in FP32
+            const bool far = d2 > thr * thr * 1.00001f;  // beyond rounding: the far rule's points in FP32
+            if (valid && far) {
 #pragma unroll
-                for (int q = 0; q < NQMAX; ++q) {
+                for (int q = 0; q < NQ; ++q) {
                     if (q >= nf) break;
                     const float rx = (qh[q][0] - h.x) + (ql[q][0] - l.x), ry = (qh[q][1] - h.y) + (ql[q][1] - l.y),
                                 rz = (qh[q][2] - h.z) + (ql[q][2] - l.z);
@@ -538,17 +1097,27 @@ __global__ void __launch_bounds__(NB_TPB) particle_rhs_kernel(PRhsArgs a) {
                     u[q][1] = fmaf(sc, al.z * rx - al.x * rz, u[q][1]);
                     u[q][2] = fmaf(sc, al.x * ry - al.y * rx, u[q][2]);
                 }
-            } else {  // near, or within rounding of the switch: the reference's decision and rule in FP64
-                particle_rows<float>(a.pr, Tr, a.part + 7 * size_t(b0 + k), rows);
+            }
+            // near, or within rounding of the switch: the reference's decision and rule in FP64
+            const unsigned m = __ballot_sync(0xffffffffu, valid && !far);
+            if (m) {
+                if (valid && !far) {
+                    const int e = nq + __popc(m & ((1u << lane) - 1u));
+                    sn.lane[e] = lane;
+                    sn.k[e] = k;
+                }
+                nq += __popc(m);
+                drain(false);
             }
         }
+        drain(true);
 #pragma unroll
-        for (int q = 0; q < NQMAX; ++q)
+        for (int q = 0; q < NQ; ++q)
             for (int z = 0; z < 3; ++z) U[q][z] += double(u[q][z]);
     }
     if (!valid) return;
 #pragma unroll
-    for (int q = 0; q < NQMAX; ++q) {
+    for (int q = 0; q < NQ; ++q) {
         if (q >= nf) break;
         const RulePt m = a.pr.rfar[q];
         const double un = (m.w * Tr.area) * (U[q][0] * Tr.n[0] + U[q][1] * Tr.n[1] + U[q][2] * Tr.n[2]);
@@ -597,7 +1166,7 @@ __global__ void body_src32_kernel(int ntri, const BodySrc* __restrict__ bs, floa
 }
 
 struct BVelArgs {
-    int ntri, npts, nchunk;
+    int ntri, npts, nchunk, per;
     const float* src32;    // ntri x BS32
     const BodySrc* src64;  // the FP64 sources (guarded points, ambiguous far tests)
     const double* X;       // npts x 3
@@ -622,7 +1191,7 @@ __global__ void __launch_bounds__(NB_TPB) body_vel_kernel(BVelArgs a) {
     const float kf = float(a.kernel_far);
     const Fp32Guard g{PAIR_GUARD};
     v3<double> acc = mk3(0.0, 0.0, 0.0);
-    const int s0 = blockIdx.y * NB_CHUNK, s1 = min(a.ntri, s0 + NB_CHUNK);
+    const int s0 = blockIdx.y * a.per, s1 = min(a.ntri, s0 + a.per);
     for (int t0 = s0; t0 < s1; t0 += BV_TILE) {
         const int nt = min(BV_TILE, s1 - t0);
         __syncthreads();
@@ -1118,7 +1687,7 @@ struct vp_freewake {
     double *sheet_G = nullptr, *seg = nullptr;
     int* sheet_ok = nullptr;
     double *blobs = nullptr, *X = nullptr, *ub = nullptr, *uw = nullptr, *umax_part = nullptr;
-    double *trow = nullptr, *rhs = nullptr, *x = nullptr, *mu = nullptr, *mu_prev = nullptr, *dmu = nullptr;
+    double *trow = nullptr, *rhs_parts = nullptr, *rhs = nullptr, *x = nullptr, *mu = nullptr, *mu_prev = nullptr, *dmu = nullptr;
     double *cp = nullptr, *surf_part = nullptr, *mom_part = nullptr, *rec = nullptr;
     double* sum_parts = nullptr;  // the parts of split point sums
     // the mixed path's FP32 N-body kernels: the particles as FP32 splits, the chunks' partial sums, the body sources
@@ -1171,15 +1740,14 @@ int ensure_capacity(vp_freewake* fw, int need) {
     signed char* group;
     int r;
     const size_t nb = blob_cap(fw, cap), npnt = point_cap(fw, cap);
-    const size_t pchunks = (size_t(cap) + NB_CHUNK - 1) / NB_CHUNK, bchunks = (size_t(fw->ntri) + NB_CHUNK - 1) / NB_CHUNK;
     if ((r = own_alloc(fw, &part, 7 * size_t(cap))) || (r = own_alloc(fw, &tag, size_t(cap))) ||
         (r = own_alloc(fw, &group, size_t(cap))) || (r = own_alloc(fw, &blobs, 7 * nb)) ||
         (r = own_alloc(fw, &X, 3 * npnt)) || (r = own_alloc(fw, &ub, 3 * npnt)) || (r = own_alloc(fw, &uw, 3 * npnt)) ||
         (r = own_alloc(fw, &umax_part, (npnt + 255) / 256 + 1)) ||
         (r = own_alloc(fw, &mom_part, 6 * ((size_t(fw->ntri) + nb + 255) / 256 + 1))) ||
         (r = own_alloc(fw, &ph, size_t(cap))) || (r = own_alloc(fw, &pl, size_t(cap))) ||
-        (r = own_alloc(fw, &pa, size_t(cap))) || (r = own_alloc(fw, &prhs, pchunks * fw->ntri * 3)) ||
-        (r = own_alloc(fw, &bvel, bchunks * npnt * 3)))
+        (r = own_alloc(fw, &pa, size_t(cap))) || (r = own_alloc(fw, &prhs, 3 * nb_rows(ctx->nsm, fw->ntri))) ||
+        (r = own_alloc(fw, &bvel, 3 * nb_rows(ctx->nsm, npnt))))
         return r;
     if (fw->np > 0) {
         VP_CUDA(ctx, cudaMemcpyAsync(part, fw->part, sizeof(double) * 7 * fw->np, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1420,6 +1988,8 @@ extern "C" int vp_freewake_create(vp_ctx* ctx, const vp_freewake_setup* s, vp_fr
         (r = own_alloc(fw, &fw->sheet_G, 3 * size_t(std::max(fw->ns_cap, 1)))) ||
         (r = own_alloc(fw, &fw->sheet_ok, size_t(std::max(fw->ns_cap, 1)))) ||
         (r = own_alloc(fw, &fw->seg, 8 * size_t(fw->nsg_cap))) || (r = own_alloc(fw, &fw->trow, 3 * size_t(s->ntri))) ||
+        (r = own_alloc(fw, &fw->rhs_parts,
+                       3 * size_t(s->ntri) * size_t(rhs_chunks(s->ntri, fw->ns_cap) + rhs_chunks(s->ntri, fw->nsg_cap)))) ||
         (r = own_alloc(fw, &fw->rhs, size_t(s->nslot))) || (r = own_alloc(fw, &fw->x, size_t(F->n))) ||
         (r = own_alloc(fw, &fw->mu, size_t(s->nslot))) || (r = own_alloc(fw, &fw->mu_prev, size_t(s->nslot))) ||
         (r = own_alloc(fw, &fw->dmu, size_t(s->nslot))) || (r = own_alloc(fw, &fw->cp, size_t(s->ntri))) ||
@@ -1488,24 +2058,45 @@ extern "C" int vp_freewake_step(vp_freewake* fw, vp_freewake_record* rec) {
         ra.na = wake_near_args(fw, o);
         // mixed: the particles go to the FP32 N-body kernel below; FP64: they stay in the warp kernel
         ra.sheet_G = fw->sheet_G, ra.sheet_ok = fw->sheet_ok, ra.nsh = nsh, ra.nsg = nsg, ra.npart = mixed ? 0 : fw->np;
-        ra.seg = fw->seg, ra.part = fw->part, ra.trow = fw->trow;
+        ra.seg = fw->seg, ra.part = fw->part;
         ra.pr.rfar = fw->rule[R_FAR], ra.pr.nfar = fw->nrule[R_FAR], ra.pr.rnear = fw->rule[R_NEAR];
         ra.pr.nnear = fw->nrule[R_NEAR], ra.pr.test_mode = o.test, ra.pr.near_depth = o.near_depth;
         ra.pr.far_ratio = o.far_ratio, ra.pr.near_ratio = o.near_ratio;
-        const int nb = (ntri + RHS_WARPS - 1) / RHS_WARPS;
+        const NbSplit ps = nb_split(ctx->nsm, ntri, fw->np, P_TILE);
+        ra.csh = rhs_chunks(ntri, nsh), ra.csg = rhs_chunks(ntri, nsg), ra.cpt = mixed ? 0 : ps.n, ra.pper = ps.per;
+        ra.part_rows = fw->rhs_parts, ra.prow = fw->prhs;
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_WAKE_RHS);
-        if (mixed)
-            wake_rhs_kernel<float><<<nb, 32 * RHS_WARPS, 0, ctx->stream>>>(ra);
-        else
-            wake_rhs_kernel<double><<<nb, 32 * RHS_WARPS, 0, ctx->stream>>>(ra);
+        VP_CUDA(ctx, cudaMemsetAsync(fw->trow, 0, sizeof(double) * 3 * ntri, ctx->stream));
+        if (ra.csh > 0) {
+            if (mixed)
+                sheet_rhs_kernel<float><<<dim3(ntri, ra.csh), 32, 0, ctx->stream>>>(ra);
+            else
+                sheet_rhs_kernel<double><<<dim3(ntri, ra.csh), 32, 0, ctx->stream>>>(ra);
+            ctx->launches++;
+        }
+        if (ra.csg > 0) {
+            fil_rhs_kernel<<<dim3(ntri, ra.csg), 32, 0, ctx->stream>>>(ra);
+            ctx->launches++;
+        }
+        if (ra.csh + ra.csg > 0) {
+            add_chunks_kernel<<<(3 * ntri + 255) / 256, 256, 0, ctx->stream>>>(3 * ntri, ra.csh + ra.csg, ra.part_rows,
+                                                                               fw->trow);
+            ctx->launches++;
+        }
+        if (ra.cpt > 0) {
+            particle_rhs64_kernel<<<dim3(ntri, ra.cpt), 32, 0, ctx->stream>>>(ra);
+            add_chunks_kernel<<<(3 * ntri + 255) / 256, 256, 0, ctx->stream>>>(3 * ntri, ra.cpt, ra.prow, fw->trow);
+            ctx->launches += 2;
+        }
         if (mixed && fw->np > 0) {
             particle_prep_kernel<<<(fw->np + 255) / 256, 256, 0, ctx->stream>>>(fw->np, fw->part, fw->ph, fw->pl, fw->pa);
             PRhsArgs pa{};
-            pa.ntri = ntri, pa.npart = fw->np, pa.nchunk = (fw->np + NB_CHUNK - 1) / NB_CHUNK;
+            pa.ntri = ntri, pa.npart = fw->np, pa.nchunk = ps.n, pa.per = ps.per;
             pa.tri = fw->tg, pa.part = fw->part, pa.ph = fw->ph, pa.pl = fw->pl, pa.pa = fw->pa, pa.pr = ra.pr;
             pa.out = fw->prhs;
-            particle_rhs_kernel<<<dim3((ntri + NB_TPB - 1) / NB_TPB, pa.nchunk), NB_TPB, 0, ctx->stream>>>(pa);
+            (ra.pr.nfar <= 3 ? particle_rhs_kernel<3> : particle_rhs_kernel<NQMAX>)<<<dim3((ntri + 31) / 32, pa.nchunk), 32, 0,
+                                                                                      ctx->stream>>>(pa);
             add_chunks_kernel<<<(3 * ntri + 255) / 256, 256, 0, ctx->stream>>>(3 * ntri, pa.nchunk, fw->prhs, fw->trow);
             ctx->launches += 3;
         }
@@ -1513,7 +2104,7 @@ extern "C" int vp_freewake_step(vp_freewake* fw, vp_freewake_record* rec) {
         vp_phase_begin(ctx, PH_WAKE);
         slot_gather_kernel<<<(nslot + 255) / 256, 256, 0, ctx->stream>>>(nslot, fw->sg_ptr, fw->sg_ent, fw->trow, fw->b0,
                                                                           fw->rhs);
-        ctx->launches += 2;
+        ctx->launches++;
         VP_CUDA(ctx, cudaGetLastError());
     }
     vp_phase_end(ctx);
@@ -1560,8 +2151,9 @@ extern "C" int vp_freewake_step(vp_freewake* fw, vp_freewake_record* rec) {
     if (!freestream) {
         if (mixed) {
             body_src32_kernel<<<(ntri + 255) / 256, 256, 0, ctx->stream>>>(ntri, fw->bs, fw->src32);
+            const NbSplit bs = nb_split(ctx->nsm, npts, ntri, BV_TILE);
             BVelArgs ba{};
-            ba.ntri = ntri, ba.npts = npts, ba.nchunk = (ntri + NB_CHUNK - 1) / NB_CHUNK, ba.src32 = fw->src32;
+            ba.ntri = ntri, ba.npts = npts, ba.nchunk = bs.n, ba.per = bs.per, ba.src32 = fw->src32;
             ba.src64 = fw->bs, ba.X = fw->X, ba.kernel_far = o.kernel_far, ba.out = fw->bvel;
             body_vel_kernel<<<dim3((npts + NB_TPB - 1) / NB_TPB, ba.nchunk), NB_TPB, 0, ctx->stream>>>(ba);
             VP_CUDA(ctx, cudaMemsetAsync(fw->ub, 0, sizeof(double) * 3 * npts, ctx->stream));
