@@ -172,7 +172,7 @@ int vp_lu_factor(vp_ctx* ctx, int precision, int n, double* M64, vp_factor* F);
 // steps): vp_solve_work_alloc sizes them for the factorization, vp_solve_work_free releases them.
 struct SolveWork {
     int n = 0;
-    double *work64 = nullptr, *rhs = nullptr, *res = nullptr;
+    double *work64 = nullptr, *rhs = nullptr, *res = nullptr, *norms = nullptr;
     float *f = nullptr, *fw = nullptr;
 };
 int vp_solve_work_alloc(vp_ctx* ctx, const vp_factor* F, SolveWork* w);

@@ -26,6 +26,9 @@ namespace {
 
 constexpr int LU_CL = 8;       // CTAs per cluster of the leaf kernel
 constexpr int LU_THREADS = 512;
+// right hand sides from which the FP64 residual is one product on the tensor cores: its cost hardly depends on them (the
+// digits of M), a matrix-vector product takes 0.1 ms each at 6.6k unknowns: 64 of them 6.9 ms an iteration, one product 2
+constexpr int RES_TC = 24;
 
 // M(q, q') = sum_{i in C[:,q]} C[i,q] sum_{j in Cf[:,q']} A[i, j] Cf[j,q'], written column-major (ld n)
 __global__ void reduce_kernel(int nq, int n, const double* __restrict__ A, long long lda, const int* __restrict__ ctp,
@@ -765,6 +768,29 @@ int rgetrf(vp_ctx* ctx, T* A, int n, int c0, int w, int lw, int* ipiv, int* info
     return laswp<T>(ctx, A, n, c0, c0 + w1, c0 + w1, c0 + w, ipiv);
 }
 
+// out[2 k], out[2 k + 1] = the largest |r|, |x| of column k (n rows): one CTA a column, all columns in one launch and one
+// copy to the host (cuBLAS IDAMAX and two copies a column, each with its synchronization, took 60 us a column)
+__global__ void __launch_bounds__(512) col_max_kernel(int n, const double* __restrict__ r, const double* __restrict__ x,
+                                                      double* __restrict__ out) {
+    __shared__ unsigned long long s_m[2][16];
+    const size_t o = size_t(blockIdx.x) * n;
+    unsigned long long m[2] = {0, 0};
+    for (int i = threadIdx.x; i < n; i += 512) {
+        m[0] = max(m[0], mag_key(r[o + i]));
+        m[1] = max(m[1], mag_key(x[o + i]));
+    }
+    for (int d = 16; d; d >>= 1)
+        for (int k = 0; k < 2; ++k) m[k] = max(m[k], __shfl_xor_sync(0xffffffffu, m[k], d));
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 2; ++k) s_m[k][threadIdx.x >> 5] = m[k];
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long v = 0;
+        for (int w = 0; w < 16; ++w) v = max(v, s_m[threadIdx.x][w]);
+        out[2 * size_t(blockIdx.x) + threadIdx.x] = __longlong_as_double((long long)v);
+    }
+}
+
 // solve with the factors: op = N: M x = b; op = T: M' x = b (b, x: n x nrhs column-major, device; may alias)
 template <class T>
 int lu_solve(vp_ctx* ctx, const vp_factor* F, const T* LU, const int* d_perm, int nrhs, T* b, T* work, bool trans) {
@@ -1046,7 +1072,7 @@ int vp_solve_work_alloc(vp_ctx* ctx, const vp_factor* F, SolveWork* w) {
     int r;
     w->n = F->n;
     if ((r = vp_alloc(ctx, &w->work64, n)) || (r = vp_alloc(ctx, &w->rhs, n)) || (r = vp_alloc(ctx, &w->res, n)) ||
-        (r = vp_alloc(ctx, &w->f, n)) || (r = vp_alloc(ctx, &w->fw, n))) {
+        (r = vp_alloc(ctx, &w->f, n)) || (r = vp_alloc(ctx, &w->fw, n)) || (r = vp_alloc(ctx, &w->norms, 2))) {
         vp_solve_work_free(w);
         return r;
     }
@@ -1059,6 +1085,7 @@ void vp_solve_work_free(SolveWork* w) {
     cudaFree(w->res);
     cudaFree(w->f);
     cudaFree(w->fw);
+    cudaFree(w->norms);
     *w = SolveWork();
 }
 
@@ -1084,9 +1111,10 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
         return r;
     }
     // mixed: x0 = LU32^-1 rhs; r = rhs - M x; x += LU32^-1 r until the residual is at FP64 rounding level
-    double *rhs, *res;
+    double *rhs, *res, *norms;
     float *f, *fw;
     if (ws) {
+        norms = ws->norms;
         rhs = ws->rhs;
         res = ws->res;
         f = ws->f;
@@ -1096,6 +1124,7 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
         if ((r = vp_alloc(ctx, &res, tot))) { cudaFree(rhs); return r; }
         if ((r = vp_alloc(ctx, &f, tot))) { cudaFree(rhs); cudaFree(res); return r; }
         if ((r = vp_alloc(ctx, &fw, tot))) { cudaFree(rhs); cudaFree(res); cudaFree(f); return r; }
+        if ((r = vp_alloc(ctx, &norms, 2 * size_t(nrhs)))) { cudaFree(rhs); cudaFree(res); cudaFree(f); cudaFree(fw); return r; }
     }
     auto cleanup = [&]() {
         if (ws) return;
@@ -1103,6 +1132,7 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
         cudaFree(res);
         cudaFree(f);
         cudaFree(fw);
+        cudaFree(norms);
     };
     VP_CUDA(ctx, cudaMemcpyAsync(rhs, x, sizeof(double) * tot, cudaMemcpyDeviceToDevice, ctx->stream));
     int g = std::min<int>(4 * ctx->nsm, int((tot + 255) / 256));
@@ -1113,30 +1143,30 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
     ctx->launches++;
     const double one = 1.0, mone = -1.0;
     const cublasOperation_t op = trans ? CUBLAS_OP_T : CUBLAS_OP_N;
-    std::vector<double> rn(nrhs), xn(nrhs);
+    std::vector<double> mx(2 * size_t(nrhs));
     int it = 0;
     bool conv = false;
     double prev = INFINITY;
     for (it = 1; it <= 30; ++it) {
         VP_CUDA(ctx, cudaMemcpyAsync(res, rhs, sizeof(double) * tot, cudaMemcpyDeviceToDevice, ctx->stream));
-        // a matrix-vector product per column: M is read once per column at the HBM rate (a GEMM with a few columns
-        // takes a tile shape that reads it far slower)
-        for (int k = 0; k < nrhs; ++k)
+        // one product on the tensor cores (nine-digit FP64) from RES_TC columns on, below and for M' a matrix-vector product
+        // per column: each reads M once at the HBM rate (a DGEMM with a few columns takes a tile shape that reads it far
+        // slower, with many it runs at the FP64 pipe's rate)
+        const bool tc = nrhs >= RES_TC && !trans && vp_tc_gemm_enabled() && n >= 1024;
+        if (tc && (r = vp_tc_gemm_sub64(ctx, n, nrhs, n, F->M, n, x, n, res, n))) { cleanup(); return r; }
+        for (int k = 0; k < nrhs && !tc; ++k)
             VP_BLAS(ctx, cublasDgemv(ctx->blas, op, n, n, &mone, F->M, n, x + size_t(k) * n, 1, &one,
                                      res + size_t(k) * n, 1));
         // convergence: every column's residual at FP64 rounding of |M| |x|
+        col_max_kernel<<<nrhs, 512, 0, ctx->stream>>>(n, res, x, norms);
+        ctx->launches++;
+        VP_CUDA(ctx, vp_d2h(ctx, mx.data(), norms, sizeof(double) * 2 * nrhs));
+        if (tc && (r = vp_tc_gemm_check(ctx))) { cleanup(); return r; }
+        VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         bool ok = true;
         double worst = 0;
         for (int k = 0; k < nrhs; ++k) {
-            int ir, ix;
-            cublasSetPointerMode(ctx->blas, CUBLAS_POINTER_MODE_HOST);
-            VP_BLAS(ctx, cublasIdamax(ctx->blas, n, res + size_t(k) * n, 1, &ir));
-            VP_BLAS(ctx, cublasIdamax(ctx->blas, n, x + size_t(k) * n, 1, &ix));
-            double a, bx;
-            VP_CUDA(ctx, vp_d2h(ctx, &a, res + size_t(k) * n + (ir - 1), sizeof(double)));
-            VP_CUDA(ctx, vp_d2h(ctx, &bx, x + size_t(k) * n + (ix - 1), sizeof(double)));
-            VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            double ratio = std::fabs(a) / (norm1 * std::fabs(bx) + 1e-300);
+            const double ratio = mx[2 * size_t(k)] / (norm1 * mx[2 * size_t(k) + 1] + 1e-300);
             worst = std::max(worst, ratio);
             if (ratio > 4 * std::sqrt(double(n)) * 1.1102230246251565e-16) ok = false;
         }
