@@ -183,6 +183,109 @@ __device__ __forceinline__ T sv_exact_vjp(const SrcKern<T>& S, v3<T> r0, v3<T> r
     return s;
 }
 
+// The mixed adjoint's two evaluators of the touching and contact pairs with the three edges as a loop, their operands rotated
+// in registers, the edge's constants read from shared memory (nu: 3 x 3, len: 3). A warp alternates between the two, and
+// with the edges unrolled their code (75 KB) did not stay in the instruction caches: 13 of 20 cycles per issue were "no
+// instruction". The operations of a point, their order and their fusing (written out where the compiler has a choice) are
+// those of the unrolled forms.
+
+// sv_exact_vjp in FP32 under the guard (fp32_guard_ok); false where it refuses
+__device__ __forceinline__ bool sv_exact_vjp32(const float* __restrict__ snu, const float* __restrict__ slen, v3<float> n,
+                                               float area, float diam, v3<float> r0, v3<float> r1, v3<float> r2,
+                                               v3<float> r, v3<float> m, int side, float plane_tol, const Fp32Guard& gd,
+                                               float& so, v3<float>& g0, v3<float>& g1, v3<float>& g2,
+                                               ExactShape<float>& sh) {
+    using M = KMath<float>;
+    const float i4pi = 1.f / (4.f * vp_pi<float>());
+    float l0 = M::sqrt(dot(r0, r0)), l1 = M::sqrt(dot(r1, r1)), l2 = M::sqrt(dot(r2, r2));
+    if (fminf(l0, fminf(l1, l2)) < gd.corner * diam) return false;
+    const float N = dot(r0, cross(r1, r2));
+    const float l01 = __fmul_rn(l0, l1), P3 = l01 * l2, d01 = dot(r0, r1);
+    const float D = fmaf(dot(r1, r2), l0, fmaf(dot(r0, r2), l1, fmaf(l01, l2, __fmul_rn(d01, l2))));
+    if (side == 0) {
+        if (fabsf(N) < gd.plane * P3 && (D < 0.f || fabsf(D) < gd.plane * P3)) return false;
+    }
+    g0 = g1 = g2 = mk3(0.f, 0.f, 0.f);
+    float b0 = 0.f, b1 = 0.f, b2 = 0.f, s = 0.f;
+#pragma unroll 1
+    for (int e = 0; e < 3; ++e) {  // the edge from corner offset r0 to r1
+        const v3<float> nu = mk3(snu[3 * e], snu[3 * e + 1], snu[3 * e + 2]);
+        const float len = slen[e];
+        const float p = dot(r0, r1);
+        const float num = l0 + l1 + len;
+        const float coef = dot(nu, m) * i4pi;
+        float L, dLdli, dLdlj, dLdp;
+        if (p < 0.f) {
+            const v3<float> c = cross(r0, r1);
+            const float c2 = norm2(c);
+            if (c2 < gd.edge_sin2 * (l0 * l0) * (l1 * l1)) return false;
+            const float den = l0 * l1 - p;
+            const float q = M::div(den, 2.f * c2);
+            L = M::log(num * num * q);
+            dLdli = M::div(2.f, num) + M::div(l1, den);
+            dLdlj = M::div(2.f, num) + M::div(l0, den);
+            dLdp = M::div(-1.f, den);
+            const float dLdc2 = M::div(-1.f, c2);
+            g0 += (coef * dLdc2 * 2.f) * cross(r1, c);
+            g1 += (coef * dLdc2 * 2.f) * cross(c, r0);
+        } else {
+            const float den = l0 * l1 + p;
+            L = log1pf(len * num / den);
+            dLdli = M::div(2.f, num) - M::div(l1, den);
+            dLdlj = M::div(2.f, num) - M::div(l0, den);
+            dLdp = M::div(-1.f, den);
+        }
+        s += L * coef;
+        b0 += coef * dLdli;
+        b1 += coef * dLdlj;
+        g0 += (coef * dLdp) * r1;
+        g1 += (coef * dLdp) * r0;
+        sh.L[0] = sh.L[1];
+        sh.L[1] = sh.L[2];
+        sh.L[2] = L;
+        sh.dLdlen[0] = sh.dLdlen[1];
+        sh.dLdlen[1] = sh.dLdlen[2];
+        sh.dLdlen[2] = M::div(2.f, num);
+        const v3<float> tr = r0, tg = g0;
+        const float tl = l0, tb = b0;
+        r0 = r1, r1 = r2, r2 = tr;
+        g0 = g1, g1 = g2, g2 = tg;
+        l0 = l1, l1 = l2, l2 = tl;
+        b0 = b1, b1 = b2, b2 = tb;
+    }
+    const float z = dot(r, n);
+    const float nm = dot(n, m) * i4pi;
+    if (fabs(z) <= plane_tol * diam) {
+        const v3<float> q[3] = {-r0, -r1, -r2};
+        sh.Om = side == 0 ? 0.f : float(side) * 2.f * vp_pi<float>() * inplane_fraction_rel(q, n, area, plane_tol);
+    } else {
+        sh.Om = 2.f * M::atan2(N, D);
+    }
+    auto lin = [](float a, v3<float> x, float b, v3<float> y) {
+        return mk3(fmaf(a, x.x, __fmul_rn(b, y.x)), fmaf(a, x.y, __fmul_rn(b, y.y)), fmaf(a, x.z, __fmul_rn(b, y.z)));
+    };
+    const float nd = fmaf(N, N, __fmul_rn(D, D));
+    if (nd > 0.f) {
+        const float h = M::div(2.f, nd);
+        const float Nb = nm * D * h, Db = -nm * N * h;
+        g0 += Nb * cross(r1, r2);
+        g1 += Nb * cross(r2, r0);
+        g2 += Nb * cross(r0, r1);
+        b0 += Db * fmaf(l1, l2, dot(r1, r2));
+        b1 += Db * fmaf(l0, l2, dot(r0, r2));
+        b2 += Db * __fadd_rn(l01, d01);
+        g0 += Db * lin(l2, r1, l1, r2);
+        g1 += Db * lin(l2, r0, l0, r2);
+        g2 += Db * lin(l1, r0, l0, r1);
+    }
+    s += sh.Om * nm;
+    g0 += M::div(b0, l0) * r0;
+    g1 += M::div(b1, l1) * r1;
+    g2 += M::div(b2, l2) * r2;
+    so = s;
+    return true;
+}
+
 // The mixed path's FP64 points (where FP32 cancels), split by what cancels: the offsets' lengths, the edges' dot and
 // cross products, the stable forms l_i l_j + r_i.r_j, the solid angle's numerator and denominator and the vectors
 // l_k r_j + l_j r_k are formed in FP64 (with KMathHyb's square root), and the functions and the derivative algebra on
@@ -190,112 +293,107 @@ __device__ __forceinline__ T sv_exact_vjp(const SrcKern<T>& S, v3<T> r0, v3<T> r
 // sv_exact_vjp<double, KMathHyb>, at FP32 accuracy, with about a quarter of its FP64 work. Returns false, with the
 // outputs unset, for a point so near a corner or an edge's line that the terms leave FP32's range (a corner offset
 // under 1e-10, an edge cross product |c|^2 under 1e-30); the caller takes that point wholly in FP64.
-__device__ __forceinline__ bool sv_exact_vjp_split(const SrcKern<double>& S, v3<double> r0, v3<double> r1,
+__device__ __forceinline__ bool sv_exact_vjp_split(const double* __restrict__ snu, const double* __restrict__ slen,
+                                                   v3<double> n, double area, double diam, v3<double> r0, v3<double> r1,
                                                    v3<double> r2, v3<double> r, v3<float> m, int side, double plane_tol,
                                                    float& svo, v3<float>& g0, v3<float>& g1, v3<float>& g2,
                                                    ExactShape<float>& sh) {
-    const v3<double> R[3] = {r0, r1, r2};
-    double l64[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) l64[a] = KMathHyb::sqrt(dot(R[a], R[a]));
-    if (!(fmin(l64[0], fmin(l64[1], l64[2])) > 1e-10)) return false;
-    float l[3], p[3], s2[3], c2[3];
-    v3<float> c[3], Rf[3];
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const int i = e, j = (e + 1) % 3;
-        const double pe = dot(R[i], R[j]);
-        const v3<double> ce = cross(R[i], R[j]);
-        const double lilj = l64[i] * l64[j];
-        // l_i l_j + p without cancellation: |c|^2 / (l_i l_j - p) where p < 0
-        const double c2e = norm2(ce);
-        if (pe < 0.0 && !(c2e > 1e-30)) return false;
-        const double se = pe < 0.0 ? KMathHyb::div(c2e, lilj - pe) : lilj + pe;
-        c2[e] = float(c2e);
-        l[e] = float(l64[e]);
-        p[e] = float(pe);
-        s2[e] = float(se);
-        c[e] = f3(ce);
-        Rf[e] = f3(R[e]);
-    }
+    double L0 = KMathHyb::sqrt(dot(r0, r0)), L1 = KMathHyb::sqrt(dot(r1, r1)), L2 = KMathHyb::sqrt(dot(r2, r2));
+    if (!(fmin(L0, fmin(L1, L2)) > 1e-10)) return false;
     const double N64 = dot(r0, cross(r1, r2));
-    const double D64 = l64[0] * l64[1] * l64[2] + dot(r0, r1) * l64[2] + dot(r0, r2) * l64[1] + dot(r1, r2) * l64[0];
-    const v3<float> V[3] = {f3(l64[2] * r1 + l64[1] * r2), f3(l64[2] * r0 + l64[0] * r2), f3(l64[1] * r0 + l64[0] * r1)};
-    const double z = dot(r, S.n);
+    const double D64 = L0 * L1 * L2 + dot(r0, r1) * L2 + dot(r0, r2) * L1 + dot(r1, r2) * L0;
+    const v3<float> V0 = f3(L2 * r1 + L1 * r2), V1 = f3(L2 * r0 + L0 * r2), V2 = f3(L1 * r0 + L0 * r1);
+    const double z = dot(r, n);
     const float N = float(N64), D = float(D64);
     // the solid angle's derivative factors 2 (D, N) / (N^2 + D^2), formed in FP64: the squares of N and D leave
     // FP32's range where the offsets are small
     const double nd2 = N64 * N64 + D64 * D64;
     const double hnd = nd2 > 0.0 ? KMathHyb::div(2.0, nd2) : 0.0;
     const float hD = float(hnd * D64), hN = float(hnd * N64);
-    // FP32 from here
     const float i4pi = 1.f / (4.f * vp_pi<float>());
-    v3<float> gr[3] = {mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 0.f)};
-    float lbar[3] = {0.f, 0.f, 0.f};
-    float sv = 0.f;
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const int i = e, j = (e + 1) % 3;
-        const float len = float(S.len[e]);
-        const float num = l[i] + l[j] + len;
-        const v3<float> nu = f3(S.nu[e]);
+    float b0 = 0.f, b1 = 0.f, b2 = 0.f, sv = 0.f, t0 = 0.f, t1 = 0.f, t2 = 0.f;
+    v3<float> h0 = mk3(0.f, 0.f, 0.f), h1 = h0, h2 = h0, c0 = h0, c1 = h0, c2 = h0;
+#pragma unroll 1
+    for (int e = 0; e < 3; ++e) {  // the edge from corner offset r0 to r1
+        const double pe = dot(r0, r1);
+        const v3<double> ce = cross(r0, r1);
+        const double lilj = L0 * L1;
+        // l_i l_j + p without cancellation: |c|^2 / (l_i l_j - p) where p < 0
+        const double c2e = norm2(ce);
+        if (pe < 0.0 && !(c2e > 1e-30)) return false;
+        const double se = pe < 0.0 ? KMathHyb::div(c2e, lilj - pe) : lilj + pe;
+        const float cc = float(c2e), p = float(pe), st = float(se), li = float(L0), lj = float(L1);
+        const v3<float> c = f3(ce), ri = f3(r0), rj = f3(r1);
+        // FP32 from here
+        const float len = float(slen[e]);
+        const float num = li + lj + len;
+        const v3<float> nu = mk3(float(snu[3 * e]), float(snu[3 * e + 1]), float(snu[3 * e + 2]));
         const float coef = dot(nu, m) * i4pi;
         float L, dLdli, dLdlj, dLdp;
-        if (p[e] < 0.f) {
-            const float den = l[i] * l[j] - p[e];
-            L = logf(num * num * (den / (2.f * c2[e])));
-            dLdli = 2.f / num + l[j] / den;
-            dLdlj = 2.f / num + l[i] / den;
+        if (p < 0.f) {
+            const float den = li * lj - p;
+            L = logf(num * num * (den / (2.f * cc)));
+            dLdli = 2.f / num + lj / den;
+            dLdlj = 2.f / num + li / den;
             dLdp = -1.f / den;
-            const float k2 = coef * (-1.f / c2[e]) * 2.f;
-            gr[i] += k2 * cross(Rf[j], c[e]);
-            gr[j] += k2 * cross(c[e], Rf[i]);
+            const float k2 = coef * (-1.f / cc) * 2.f;
+            h0 += k2 * cross(rj, c);
+            h1 += k2 * cross(c, ri);
         } else {
-            const float den = s2[e];
+            const float den = st;
             L = log1pf(len * num / den);
-            dLdli = 2.f / num - l[j] / den;
-            dLdlj = 2.f / num - l[i] / den;
+            dLdli = 2.f / num - lj / den;
+            dLdlj = 2.f / num - li / den;
             dLdp = -1.f / den;
         }
         sv += L * coef;
-        lbar[i] += coef * dLdli;
-        lbar[j] += coef * dLdlj;
-        gr[i] += (coef * dLdp) * Rf[j];
-        gr[j] += (coef * dLdp) * Rf[i];
-        sh.L[e] = L;
-        sh.dLdlen[e] = 2.f / num;
+        b0 += coef * dLdli;
+        b1 += coef * dLdlj;
+        h0 += (coef * dLdp) * rj;
+        h1 += (coef * dLdp) * ri;
+        sh.L[0] = sh.L[1];
+        sh.L[1] = sh.L[2];
+        sh.L[2] = L;
+        sh.dLdlen[0] = sh.dLdlen[1];
+        sh.dLdlen[1] = sh.dLdlen[2];
+        sh.dLdlen[2] = 2.f / num;
+        const v3<double> tr = r0;
+        const v3<float> th = h0;
+        const double tl = L0;
+        const float tb = b0;
+        r0 = r1, r1 = r2, r2 = tr;
+        h0 = h1, h1 = h2, h2 = th;
+        L0 = L1, L1 = L2, L2 = tl;
+        b0 = b1, b1 = b2, b2 = tb;
+        c0 = c1, c1 = c2, c2 = c;
+        t0 = t1, t1 = t2, t2 = st;
     }
-    const float nm = dot(f3(S.n), m) * i4pi;
-    if (fabs(z) <= plane_tol * S.diam) {
-        const v3<double> q[3] = {-r0, -r1, -r2};
-        sh.Om = side == 0 ? 0.f
-                          : float(side) * 2.f * vp_pi<float>() *
-                                float(inplane_fraction_rel(q, S.n, S.area, plane_tol));
-    } else {
+    const float nm = dot(f3(n), m) * i4pi;
+    if (fabs(z) <= plane_tol * diam)
+        sh.Om = side == 0 ? 0.f : float(side) * 2.f * vp_pi<float>() * inplane_fraction32(r0, r1, r2, n, area, plane_tol);
+    else
         sh.Om = 2.f * atan2f(N, D);
-    }
     if (nd2 > 0.0) {
         const float Nb = nm * hD, Db = -nm * hN;
-        gr[0] += Nb * c[1];
-        gr[1] += Nb * c[2];
-        gr[2] += Nb * c[0];
-        lbar[0] += Db * s2[1];
-        lbar[1] += Db * s2[2];
-        lbar[2] += Db * s2[0];
-        gr[0] += Db * V[0];
-        gr[1] += Db * V[1];
-        gr[2] += Db * V[2];
+        h0 += Nb * c1;
+        h1 += Nb * c2;
+        h2 += Nb * c0;
+        b0 += Db * t1;
+        b1 += Db * t2;
+        b2 += Db * t0;
+        h0 += Db * V0;
+        h1 += Db * V1;
+        h2 += Db * V2;
     }
     sv += sh.Om * nm;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) gr[a] += (lbar[a] / l[a]) * Rf[a];
-    if (!(isfinite(sv) && isfinite(gr[0].x + gr[0].y + gr[0].z + gr[1].x + gr[1].y + gr[1].z + gr[2].x + gr[2].y +
-                                   gr[2].z)))
-        return false;
+    h0 += (b0 / float(L0)) * f3(r0);
+    h1 += (b1 / float(L1)) * f3(r1);
+    h2 += (b2 / float(L2)) * f3(r2);
+    if (!(isfinite(sv) && isfinite(h0.x + h0.y + h0.z + h1.x + h1.y + h1.z + h2.x + h2.y + h2.z))) return false;
     svo = sv;
-    g0 = gr[0];
-    g1 = gr[1];
-    g2 = gr[2];
+    g0 = h0;
+    g1 = h1;
+    g2 = h2;
     return true;
 }
 

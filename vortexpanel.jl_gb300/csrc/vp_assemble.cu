@@ -594,7 +594,7 @@ __device__ __forceinline__ void fwd_point64(const PairCtx& pc, FwdAcc& acc, doub
         v3<float> wf;
         if (far)
             w = far64_sh(sh, r);
-        else if (sv_exact3_split(S, ra, rb, rc, r, pc.side, 1e-12, wf))
+        else if (sv_exact3_split(sh.Snu, sh.Slen, S.n, S.area, S.diam, ra, rb, rc, r, pc.side, 1e-12, wf))
             w = mk3(double(wf.x), double(wf.y), double(wf.z));
         else
             w = exact64_sh(sh, ra, rb, rc, r, pc.side);

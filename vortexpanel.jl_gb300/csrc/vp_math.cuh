@@ -194,6 +194,13 @@ __device__ __forceinline__ v3<T> sv_exact3(const SrcKern<T>& S, v3<T> ra, v3<T> 
     return (wt + Om * S.n) * (T(1) / (T(4) * vp_pi<T>()));
 }
 
+// inplane_fraction_rel of the self pair's points in the split evaluations, out of line
+static __device__ __noinline__ float inplane_fraction32(v3<double> r0, v3<double> r1, v3<double> r2, v3<double> n, double area,
+                                                        double plane_tol) {
+    const v3<double> q[3] = {-r0, -r1, -r2};
+    return float(inplane_fraction_rel(q, n, area, plane_tol));
+}
+
 // The mixed path's FP64 points of the exact kernel, split by what cancels: the offsets' lengths (KMathHyb's square
 // root), the edges' dot products and squared cross products, and the solid angle's numerator and denominator are
 // formed in FP64; the logs, the atan2 and the sums on them run in FP32, where no difference of nearly equal terms is
@@ -201,41 +208,41 @@ __device__ __forceinline__ v3<T> sv_exact3(const SrcKern<T>& S, v3<T> ra, v3<T> 
 // sv_exact3<double, KMathHyb> at FP32 accuracy, with about half its FP64 work. Returns false, with w unset, for a
 // point so near a corner or an edge's line that the terms leave FP32's range (a corner offset under 1e-10, an edge
 // cross product |c|^2 under 1e-30); the caller takes that point wholly in FP64.
-__device__ __forceinline__ bool sv_exact3_split(const SrcKern<double>& S, v3<double> ra, v3<double> rb, v3<double> rc,
-                                                v3<double> r, int side, double plane_tol, v3<float>& w) {
-    const v3<double> R[3] = {ra, rb, rc};
-    double l64[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) l64[a] = KMathHyb::sqrt(dot(R[a], R[a]));
-    if (!(fmin(l64[0], fmin(l64[1], l64[2])) > 1e-10)) return false;
+__device__ __forceinline__ bool sv_exact3_split(const double* __restrict__ snu, const double* __restrict__ slen,
+                                                v3<double> n, double area, double diam, v3<double> ra, v3<double> rb,
+                                                v3<double> rc, v3<double> r, int side, double plane_tol, v3<float>& w) {
+    double la = KMathHyb::sqrt(dot(ra, ra)), lb = KMathHyb::sqrt(dot(rb, rb)), lc = KMathHyb::sqrt(dot(rc, rc));
+    if (!(fmin(la, fmin(lb, lc)) > 1e-10)) return false;
     v3<float> wt = mk3(0.f, 0.f, 0.f);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const int i = e, j = (e + 1) % 3;
-        const double pe = dot(R[i], R[j]);
-        const float li = float(l64[i]), lj = float(l64[j]), p = float(pe), len = float(S.len[e]);
+#pragma unroll 1
+    for (int e = 0; e < 3; ++e) {  // the edge from corner offset ra to rb
+        const double pe = dot(ra, rb);
+        const float li = float(la), lj = float(lb), p = float(pe), len = float(slen[e]);
         const float num = li + lj + len;
         float L;
         if (pe < 0.0) {
-            const double c2e = norm2(cross(R[i], R[j]));
+            const double c2e = norm2(cross(ra, rb));
             if (!(c2e > 1e-30)) return false;
             const float c2 = float(c2e);
             L = logf(num * num * ((li * lj - p) / (2.f * c2)));
         } else {
             L = log1pf(len * num / (li * lj + p));
         }
-        wt += L * f3(S.nu[e]);
+        wt += L * mk3(float(snu[3 * e]), float(snu[3 * e + 1]), float(snu[3 * e + 2]));
+        const v3<double> tr = ra;
+        const double tl = la;
+        ra = rb, rb = rc, rc = tr;
+        la = lb, lb = lc, lc = tl;
     }
     float Om;
-    if (fabs(dot(r, S.n)) <= plane_tol * S.diam) {
-        const v3<double> q[3] = {-ra, -rb, -rc};
-        Om = side == 0 ? 0.f : float(side) * 2.f * vp_pi<float>() * float(inplane_fraction_rel(q, S.n, S.area, plane_tol));
+    if (fabs(dot(r, n)) <= plane_tol * diam) {
+        Om = side == 0 ? 0.f : float(side) * 2.f * vp_pi<float>() * inplane_fraction32(ra, rb, rc, n, area, plane_tol);
     } else {
         const double N = dot(ra, cross(rb, rc));
-        const double D = l64[0] * l64[1] * l64[2] + dot(ra, rb) * l64[2] + dot(ra, rc) * l64[1] + dot(rb, rc) * l64[0];
+        const double D = la * lb * lc + dot(ra, rb) * lc + dot(ra, rc) * lb + dot(rb, rc) * la;
         Om = 2.f * atan2f(float(N), float(D));
     }
-    w = (wt + Om * f3(S.n)) * (1.f / (4.f * vp_pi<float>()));
+    w = (wt + Om * f3(n)) * (1.f / (4.f * vp_pi<float>()));
     return isfinite(w.x + w.y + w.z);
 }
 
@@ -304,6 +311,49 @@ __device__ __forceinline__ bool sv_exact3_guarded(const SrcKern<float>& S, v3<fl
         Om = 2.f * atan2f(N, D);
     }
     w = (wt + Om * S.n) * (1.f / (4.f * vp_pi<float>()));
+    return true;
+}
+
+// sv_exact3_guarded with the edges as a loop, their constants read from shared memory (nu: 3 x 3, len: 3), for the pair
+// kernels, whose code must stay in the instruction caches beside the FP64 evaluation's (as sv_exact3_split). The same
+// operations in the same order.
+__device__ __forceinline__ bool sv_exact3_guarded_loop(const float* __restrict__ snu, const float* __restrict__ slen,
+                                                       v3<float> n, float diam, v3<float> ra, v3<float> rb, v3<float> rc,
+                                                       int side, const Fp32Guard& g, v3<float>& w) {
+    float la = vnorm(ra), lb = vnorm(rb), lc = vnorm(rc);
+    if (fminf(la, fminf(lb, lc)) < g.corner * diam) return false;
+    v3<float> wt = mk3(0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int e = 0; e < 3; ++e) {  // the edge from corner offset ra to rb
+        const v3<float> nu = mk3(snu[3 * e], snu[3 * e + 1], snu[3 * e + 2]);
+        const float len = slen[e];
+        float p = dot(ra, rb);
+        float num = la + lb + len;
+        float q;
+        if (p < 0.f) {
+            float c2 = norm2(cross(ra, rb));
+            if (c2 < g.edge_sin2 * (la * la) * (lb * lb)) return false;
+            q = (la * lb - p) / (2.f * c2);
+            wt += logf(num * num * q) * nu;
+        } else {
+            wt += log1pf(len * num / (la * lb + p)) * nu;
+        }
+        const v3<float> tr = ra;
+        const float tl = la;
+        ra = rb, rb = rc, rc = tr;
+        la = lb, lb = lc, lc = tl;
+    }
+    float Om;
+    if (side != 0) {
+        Om = float(side) * 2.f * vp_pi<float>();
+    } else {
+        float P3 = la * lb * lc;
+        float N = dot(ra, cross(rb, rc));
+        float D = P3 + dot(ra, rb) * lc + dot(ra, rc) * lb + dot(rb, rc) * la;
+        if (fabsf(N) < g.plane * P3 && (D < 0.f || fabsf(D) < g.plane * P3)) return false;
+        Om = 2.f * atan2f(N, D);
+    }
+    w = (wt + Om * n) * (1.f / (4.f * vp_pi<float>()));
     return true;
 }
 

@@ -553,7 +553,7 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, FwdAcc& acc, double
             w = sv_far(S, r);
         else if (!pc.fp32)
             w = sv_exact3(S, ra, rb, rc, r, pc.side, 1e-12);
-        else if (sv_exact3_split(S, ra, rb, rc, r, pc.side, 1e-12, wf))
+        else if (sv_exact3_split(sh.Snu, sh.Slen, S.n, S.area, S.diam, ra, rb, rc, r, pc.side, 1e-12, wf))
             w = mk3(double(wf.x), double(wf.y), double(wf.z));
         else
             w = exact64_hyb(S, ra, rb, rc, r, pc.side);
@@ -601,7 +601,7 @@ __device__ __forceinline__ bool fwd_point32(const PairCtx& pc, FwdAcc& acc, floa
         v3<float> rb = l0 * mk3(E[3], E[4], E[5]) + l1 * mk3(E[12], E[13], E[14]) + l2 * mk3(E[21], E[22], E[23]);
         v3<float> rc = l0 * mk3(E[6], E[7], E[8]) + l1 * mk3(E[15], E[16], E[17]) + l2 * mk3(E[24], E[25], E[26]);
         const Fp32Guard g{PAIR_GUARD};
-        if (!sv_exact3_guarded(S, ra, rb, rc, pc.side, g, w)) return false;
+        if (!sv_exact3_guarded_loop(sh.Snuf, sh.Slenf, S.n, S.diam, ra, rb, rc, pc.side, g, w)) return false;
     }
     v3<float> psi = pc.a->test_mode == 0 ? mk3(l0, l1, l2) : mk3(1.f, 1.f, 1.f);
     acc.Pf[0] += (W * psi.x) * w;
@@ -934,7 +934,7 @@ __device__ __noinline__ void eval_point64(const PairCtx& pc, AdjAccW& acc, doubl
     v3<float> g0, g1, g2;
     ExactShape<float> shp;
     float svf;
-    if (far || !sv_exact_vjp_split(S, ra, rb, rc, r, pc.mf, pc.side, 1e-12, svf, g0, g1, g2, shp)) {
+    if (far || !sv_exact_vjp_split(sh.Snu, sh.Slen, S.n, S.area, S.diam, ra, rb, rc, r, pc.mf, pc.side, 1e-12, svf, g0, g1, g2, shp)) {
         eval_point64_rare(pc, acc, far, l0, l1, l2, W);
         return;
     }
@@ -983,12 +983,14 @@ __device__ __noinline__ bool eval_point32(const PairCtx& pc, AdjAccW& acc, float
     const v3<float> ra = l0 * mk3(E[0], E[1], E[2]) + l1 * mk3(E[9], E[10], E[11]) + l2 * mk3(E[18], E[19], E[20]);
     const v3<float> rb = l0 * mk3(E[3], E[4], E[5]) + l1 * mk3(E[12], E[13], E[14]) + l2 * mk3(E[21], E[22], E[23]);
     const v3<float> rc = l0 * mk3(E[6], E[7], E[8]) + l1 * mk3(E[15], E[16], E[17]) + l2 * mk3(E[24], E[25], E[26]);
-    if (!fp32_guard_ok(S, ra, rb, rc, pc.side, Fp32Guard{ADJ_GUARD})) return false;
     // the self pair's points lie in the source's plane up to FP32 rounding: its in-plane branch (solid angle side 2 pi,
     // as the forward's FP32 kernel takes it) must not depend on the sign of that rounding
     v3<float> g0, g1, g2;
     ExactShape<float> shp;
-    const float sv = sv_exact_vjp(S, ra, rb, rc, r, pc.mf, pc.side, pc.side ? 1e-4f : 1e-12f, g0, g1, g2, shp);
+    float sv;
+    if (!sv_exact_vjp32(sh.Snuf, sh.Slenf, S.n, S.area, S.diam, ra, rb, rc, r, pc.mf, pc.side, pc.side ? 1e-4f : 1e-12f,
+                        Fp32Guard{ADJ_GUARD}, sv, g0, g1, g2, shp))
+        return false;
     const float i4pi = 1.f / (4.f * vp_pi<float>());
     const v3<float> w = (shp.L[0] * S.nu[0] + shp.L[1] * S.nu[1] + shp.L[2] * S.nu[2] + shp.Om * S.n) * i4pi;
     const v3<float> gx = g0 + g1 + g2;

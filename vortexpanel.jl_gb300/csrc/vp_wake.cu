@@ -398,7 +398,7 @@ __device__ __noinline__ void near_rows64(const NearArgs& a, const TriGeo& T, con
             w = sv_far(K, r);
         else if (!MIXED)
             w = sv_exact3(K, ra, rb, rc, r, 0, 1e-12);
-        else if (sv_exact3_split(K, ra, rb, rc, r, 0, 1e-12, wf))
+        else if (sv_exact3_split(S.nu, S.len, K.n, K.area, K.diam, ra, rb, rc, r, 0, 1e-12, wf))
             w = mk3(double(wf.x), double(wf.y), double(wf.z));
         else
             w = exact64_hyb(K, ra, rb, rc, r, 0);
