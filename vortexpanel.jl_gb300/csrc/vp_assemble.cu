@@ -538,9 +538,10 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
 
 // the kernels of the non-far tiers take one system's arguments by value, or (BATCH) those of system work[i].x from sys.
 // MIXED or FP64 by template: with both paths in one kernel the mixed one ran at 216 registers instead of 158 (near
-// phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles).
+// phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles). Ten CTAs an SM: 106 ms on a 25k wing, 110 with
+// twelve (spills), 127 with eight, 135 with sixteen.
 template <bool BATCH, bool MIXED>
-__global__ void __launch_bounds__(32, 12) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
+__global__ void __launch_bounds__(32, 10) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
                                                                   const int2* __restrict__ work) {
     __shared__ NearChunkSh sh;
     const int2 wk = work[blockIdx.x];

@@ -756,9 +756,13 @@ __device__ __noinline__ void adj_pair_out(PairCtx& pc, Acc& acc, const AdjMulti&
 // of a pair goes to TA, the source side to SA (fixed-point sums).
 // Acc: AdjAcc (FP64 path: FP64 sums per lane) or AdjAccW (mixed path: FP32 lane partials in dynamic shared memory,
 // NEAR_WARPS x 32 AdjLane, folded into the warp's FP64 totals).
+// Three CTAs an SM in the mixed path (168 registers; 255 and two: 418 instead of 391 ms on a 13k wing), as many as the
+// partials' shared memory allows: more warps cover the instruction fetches.
 template <class Acc>
-__global__ void __launch_bounds__(32 * NEAR_WARPS) adj_pairs_kernel(NearArgs a, AdjMulti mx, PieceRec* recs,
-                                                                  unsigned* leaves, double* deps, int gmax) {
+constexpr int adj_pairs_ctas = std::is_same<Acc, AdjAccW>::value ? 3 : 2;
+template <class Acc>
+__global__ void __launch_bounds__(32 * NEAR_WARPS, adj_pairs_ctas<Acc>)
+    adj_pairs_kernel(NearArgs a, AdjMulti mx, PieceRec* recs, unsigned* leaves, double* deps, int gmax) {
     __shared__ WarpSh shm[NEAR_WARPS];
     extern __shared__ __align__(16) unsigned char adjw_smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
