@@ -237,6 +237,7 @@ struct NearChunkSh {
     float accf[32][9];     // per pair: the same sums of the FP32 evaluations
     int off[33];           // points before each pair
     int qp[64], qk[64];    // queued FP64 points (mixed): pair, point within the pair
+    unsigned char nz[32];  // the pairs with points, in order
 };
 
 constexpr int BLK_B = 12, BLK_W = 9;  // doubles of a pair's block: body pairs carry their right hand side terms
@@ -382,30 +383,25 @@ __device__ unsigned near_chunk(PairCtx& pc, NearChunkSh& ns, int t, const int* l
         }
         n64 = (unsigned long long)total;
     }
+    PointWalk wk{};
+    if (MIXED) {
+        wk = point_walk(incl - (near ? nleaf * nr : 0), near ? nleaf * nr : 0, lane, ns.nz);
+        __syncwarp();
+    }
     for (int i0 = 0; MIXED && i0 < total; i0 += 32) {
         const int i = i0 + lane;
         const bool v = i < total;
+        const int pw = walk_point(wk, i0, lane, ns.nz);
         int p = 32 + lane, k = 0;
         float vals[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         bool need = false;
         if (v) {
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (ns.off[mid] <= i) lo = mid;
-                else hi = mid - 1;
-            }
-            p = lo;
+            p = pw;
             k = i - ns.off[p];
             int leaf = k / nr, q = k - leaf * nr;
             int code = ns.pl.leaf[p][leaf];
-            float b[9];
-            leaf_corners32(code, b);
-            float4 m = a.rulef[R_NEAR][q];
-            float l0 = m.x * b[0] + m.y * b[3] + m.z * b[6];
-            float l1 = m.x * b[1] + m.y * b[4] + m.z * b[7];
-            float l2 = m.x * b[2] + m.y * b[5] + m.z * b[8];
-            float W = m.w * ldexpf(1.f, -2 * (code >> 6)) * areaT;
+            const float4 m = a.leafpt[leaf_node(code) * nr + q];
+            const float l0 = m.x, l1 = m.y, l2 = m.z, W = m.w * areaT;
             const float* E = ns.pl.E32[p];
             const float* Dp = ns.pl.D32[p];
             const float* Sf = ns.pl.S32[p];

@@ -345,6 +345,7 @@ struct AdjChunkSh {
     double m64[32][3];              // the pair's direction m
     int off[33];                    // points before each pair
     int qp[64], qk[64];             // queued FP64 points: pair, point within the pair
+    unsigned char nz[32];           // the pairs with points, in order
 };
 
 // the FP64 adjoint evaluation of point k of pair p (queued by the FP32 guard) for the K vectors with test-corner
@@ -450,34 +451,26 @@ __device__ unsigned adj_chunk(PairCtx& pc, AdjChunkSh& ns, const AdjMulti& mx, i
         for (int c = 0; c < 3; ++c) nuf[j][c] = float(pc.nuk[j][c]);
     int nq = 0;
     unsigned long long n64 = 0;
+    PointWalk wk = point_walk(incl - (near ? nleaf * nr : 0), near ? nleaf * nr : 0, lane, ns.nz);
+    __syncwarp();
     for (int i0 = 0; i0 < total; i0 += 32) {
         const int i = i0 + lane;
         const bool v = i < total;
+        const int pw = walk_point(wk, i0, lane, ns.nz);
         int p = 32 + lane, k = 0;
         AdjSums<float> as[ADJ_MAX];
         for (int j = 0; j < ADJ_MAX; ++j) adj_zero(as[j]);
         bool need = false;
         if (v) {
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (ns.off[mid] <= i) lo = mid;
-                else hi = mid - 1;
-            }
-            p = lo;
+            p = pw;
             k = i - ns.off[p];
             need = !a.mixed;
         }
         if (v && a.mixed) {
             int leaf = k / nr, q = k - leaf * nr;
             int code = ns.pl.leaf[p][leaf];
-            float b[9];
-            leaf_corners32(code, b);
-            float4 m = a.rulef[R_NEAR][q];
-            float l0 = m.x * b[0] + m.y * b[3] + m.z * b[6];
-            float l1 = m.x * b[1] + m.y * b[4] + m.z * b[7];
-            float l2 = m.x * b[2] + m.y * b[5] + m.z * b[8];
-            float W = m.w * ldexpf(1.f, -2 * (code >> 6)) * areaT;
+            const float4 m = a.leafpt[leaf_node(code) * nr + q];
+            const float l0 = m.x, l1 = m.y, l2 = m.z, W = m.w * areaT;
             float Wn[ADJ_MAX];
             for (int j = 0; j < ADJ_MAX; ++j)
                 Wn[j] = W * (a.test_mode == 0 ? nuf[j][0] * l0 + nuf[j][1] * l1 + nuf[j][2] * l2

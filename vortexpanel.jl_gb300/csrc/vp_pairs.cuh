@@ -356,6 +356,7 @@ struct NearArgs {
     int ntouch;
     const RulePt* rule[5];
     const float4* rulef[5];  // the same rules in FP32 (l0, l1, l2, w)
+    const float4* leafpt;    // the near rule's points of every quadtree node of levels 0 to 3 (leaf_points_kernel)
     int nrule[5];
     double* A;
     long long lda;
@@ -2096,6 +2097,50 @@ __device__ bool near_plan(PairCtx& pc, NearPlanSh& pl, int t, const TriGeo& S, i
     return near;
 }
 
+// The near rule's points of every node a leaf code can name: (barycentrics on the test triangle, weight x 4^-level), node
+// (4^level - 1) / 3 + path, its nr points in turn. The lanes kernels read a point (16 bytes, 9.5 KB in all) where they
+// formed the node's corners and the three products for every point of every pair: with PointWalk, near phase of a 25k
+// wing 106 -> 91 ms, of five wings in a batch 52.8 -> 44.7, adj_near of a 13k wing 177 -> 165.
+constexpr int LEAF_NODES = 1 + 4 + 16 + 64;
+__device__ __forceinline__ int leaf_node(int code) { return ((0x15050100 >> (8 * (code >> 6))) & 255) + (code & 63); }
+
+__global__ void leaf_points_kernel(int nr, const float4* __restrict__ rule, float4* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= LEAF_NODES * nr) return;
+    const int node = i / nr, q = i - node * nr;
+    const int level = node < 1 ? 0 : node < 5 ? 1 : node < 21 ? 2 : 3;
+    const int code = (level << 6) | (node - ((0x15050100 >> (8 * level)) & 255));
+    float b[9];
+    leaf_corners32(code, b);
+    const float4 m = rule[q];
+    out[i] = make_float4(m.x * b[0] + m.y * b[3] + m.z * b[6], m.x * b[1] + m.y * b[4] + m.z * b[7],
+                         m.x * b[2] + m.y * b[5] + m.z * b[8], m.w * ldexpf(1.f, -2 * level));
+}
+inline void leaf_points(vp_ctx* ctx, int nr, const float4* rule, float4* out) {
+    leaf_points_kernel<<<(LEAF_NODES * nr + 127) / 128, 128, 0, ctx->stream>>>(nr, rule, out);
+    ctx->launches++;
+}
+
+// The points of up to 32 pairs laid end to end and taken 32 at a time: which pair a lane's point belongs to. start, n: this
+// lane's pair's first point and number; nz: the non-empty pairs' lanes in order, filled here. (One reduction and one read
+// a round; a binary search in the pairs' offsets was five dependent reads.)
+struct PointWalk {
+    int start, n, before;  // before: non-empty pairs that begin before this round
+};
+__device__ __forceinline__ PointWalk point_walk(int start, int n, int lane, unsigned char* nz) {
+    const unsigned ne = __ballot_sync(0xffffffffu, n > 0);
+    if (n > 0) nz[__popc(ne & ((1u << lane) - 1u))] = (unsigned char)lane;
+    return {start, n, 0};
+}
+// the pair of point i0 + lane (below the total); called by the whole warp, i0 ascending by 32
+__device__ __forceinline__ int walk_point(PointWalk& w, int i0, int lane, const unsigned char* nz) {
+    const int d = w.start - i0;
+    const unsigned heads = __reduce_or_sync(0xffffffffu, w.n > 0 && d >= 0 && d < 32 ? 1u << d : 0u);
+    const int rank = w.before + __popc(heads & (0xffffffffu >> (31 - lane))) - 1;
+    w.before += __popc(heads);
+    return nz[max(rank, 0)];
+}
+
 // ------------------------------------------------------------------------------------------------------------------
 // host: tiles and colours
 
@@ -2266,6 +2311,7 @@ struct PairSetup {
     int* d_fil = nullptr;
     RulePt* d_rule[5] = {};
     float4* d_rulef[5] = {};
+    float4* d_leafpt = nullptr;
     std::vector<long long> nfptr, wfptr;
     long long *d_nfptr = nullptr, *d_wfptr = nullptr;
     int *d_nf = nullptr, *d_wf = nullptr;
@@ -2391,6 +2437,8 @@ int setup_pairs(vp_ctx* ctx, const PairInput& in, int ph_setup, int ph_classify,
                 f[i] = make_float4(float((*R[k])[i].l0), float((*R[k])[i].l1), float((*R[k])[i].l2), float((*R[k])[i].w));
             if ((r = dl.up(ctx, &ps.d_rule[k], *R[k])) || (r = dl.up(ctx, &ps.d_rulef[k], f))) return r;
         }
+        if ((r = dl.alloc(ctx, &ps.d_leafpt, LEAF_NODES * ps.rnear.size()))) return r;
+        leaf_points(ctx, int(ps.rnear.size()), ps.d_rulef[R_NEAR], ps.d_leafpt);
     }
     // touching pairs, both orders, sorted keys t * ntri + s
     for (int i = 0; i < in.ntouch; ++i) {
@@ -2530,6 +2578,7 @@ NearArgs near_args(const PairSetup& ps, const PairInput& in) {
     for (int k = 0; k < 5; ++k) {
         na.rule[k] = ps.d_rule[k];
         na.rulef[k] = ps.d_rulef[k];
+        na.leafpt = ps.d_leafpt;
         na.nrule[k] = nr[k];
     }
     na.lda = ps.ncols;

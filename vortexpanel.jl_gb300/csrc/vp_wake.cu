@@ -327,13 +327,8 @@ struct RhsSh {
 __device__ __forceinline__ bool near_eval32(const NearArgs& a, const NearPlanSh& pl, float areaT, int nr, int p, int k,
                                             v3<float>& w, float* ps) {
     const int leaf = k / nr, q = k - leaf * nr, code = pl.leaf[p][leaf];
-    float b[9];
-    leaf_corners32(code, b);
-    const float4 m = a.rulef[R_NEAR][q];
-    const float l0 = m.x * b[0] + m.y * b[3] + m.z * b[6];
-    const float l1 = m.x * b[1] + m.y * b[4] + m.z * b[7];
-    const float l2 = m.x * b[2] + m.y * b[5] + m.z * b[8];
-    const float W = m.w * (ldexpf(1.f, -2 * (code >> 6)) * areaT);
+    const float4 m = a.leafpt[leaf_node(code) * nr + q];
+    const float l0 = m.x, l1 = m.y, l2 = m.z, W = m.w * areaT;
     const float *E = pl.E32[p], *D = pl.D32[p], *Sf = pl.S32[p];
     SrcKern<float> K;
     for (int z = 0; z < 3; ++z) {
@@ -1668,6 +1663,7 @@ struct vp_freewake {
     int *pwte = nullptr, *pt = nullptr, *pf = nullptr;
     RulePt* rule[5] = {};
     float4* rulef[5] = {};
+    float4* leafpt = nullptr;
     int nrule[5] = {};
     // state
     double *rx = nullptr, *rmu = nullptr, *mul = nullptr;
@@ -1784,6 +1780,7 @@ NearArgs wake_near_args(const vp_freewake* fw, const vp_assembly_options& o) {
     for (int k = 0; k < 5; ++k) {
         na.rule[k] = fw->rule[k];
         na.rulef[k] = fw->rulef[k];
+        na.leafpt = fw->leafpt;
         na.nrule[k] = fw->nrule[k];
     }
     na.test_mode = o.test;
@@ -1975,6 +1972,8 @@ extern "C" int vp_freewake_create(vp_ctx* ctx, const vp_freewake_setup* s, vp_fr
             return fail(r);
         fw->nrule[k] = int(rl[k].size());
     }
+    if ((r = own_alloc(fw, &fw->leafpt, LEAF_NODES * size_t(fw->nrule[R_NEAR])))) return fail(r);
+    leaf_points(ctx, fw->nrule[R_NEAR], fw->rulef[R_NEAR], fw->leafpt);
     // state and work arrays at their capacities
     const int R = fw->R, nte = s->nte;
     fw->ns_cap = 2 * s->nstrip * (R - 1);
