@@ -302,7 +302,7 @@ def rooflines(per, points, adjoint_points, n, pk_src):
     touch = lambda p: sum(v for k, v in p.items() if k not in ("far", "near"))  # noqa: E731  self/edge/vertex/contact
     kern = {  # phase: (kernels, bound, flops, points)
         "far": ("far_kernel<float,TT> (TT the autotuner's tile)", "fp32", pts["far"] * FLOP_FWD_POINT, pts["far"]),
-        "near": ("near_kernel_lanes (+ near_kernel_rest)", "fp32", pts["near"] * FLOP_FWD_POINT, pts["near"]),
+        "near": ("near_kernel_lanes (+ near_kernel_filaments, near_kernel_gather)", "fp32", pts["near"] * FLOP_FWD_POINT, pts["near"]),
         "near_pairs": ("near_kernel_pairs", "fp32", touch(pts) * FLOP_FWD_POINT, touch(pts)),
         "adj_far": ("adj_far_kernel<float,8,2>", "fp32", apts["far"] * (FLOP_ADJ_EVAL + 2 * FLOP_ADJ_SUMS), apts["far"]),
         "adj_near": ("adj_lanes_kernel, both vectors (+ adj_near_kernel)", "fp32",

@@ -6,7 +6,8 @@
 //  - LU with partial pivoting (the reference calls LAPACK dgetrf): recursive (left half, swap, TRSM, GEMM, right
 //    half). Its leaf panels (m x 16 columns) are factored by one thread-block cluster (1 to 16 CTAs) that holds the panel in
 //    registers: per column, every CTA sends its pivot candidate's row to all, every thread picks the pivot, swaps and
-//    updates its rows. The trailing updates run on the tensor cores (vp_tcgemm.cu): VP_MIXED by
+//    updates its rows; panels of 64 columns are factored leaf by leaf with swap and update kernels of their own. The
+//    trailing updates run on the tensor cores (vp_tcgemm.cu): VP_MIXED by
 //    three-piece bf16 splits (FP32-class), VP_FP64 by exact products of 7-bit digits (FP64-class), for updates of at
 //    least a tile of the kernels, cuBLAS for the smaller ones; TRSM is cuBLAS, in FP64 on 64 x 64 diagonal blocks only;
 //  - VP_MIXED keeps the FP64 bordered matrix and refines every solve with FP64 residuals (iterative refinement) to

@@ -10,10 +10,10 @@
 // One step, in the reference's order (step.jl:113-146), all on the context's stream:
 //   1. vortex_elements (state.jl:241-253): the free rows' sheets (two per strip and panel row), the rows' tip sides,
 //      the interface filament along R0 and the far end filament, with their blobs (free_wake_blobs, state.jl:275-295);
-//   2. explicit_rhs (src/assembly/explicit.jl:31-85): one warp per body triangle over the sheets (the assembly's
-//      wake_pair_rule tiers: far points by lanes, contact and near pieces by the warp), the filaments (segment_rule:
-//      far, vertex or near) and the particles (far rule or near quadtree); the rows are summed per slot in a fixed
-//      order, then the bordered solve with the factors (no allocation) gives q, mu = C q and mu_w = K q;
+//   2. explicit_rhs (src/assembly/explicit.jl:31-85): a warp per body triangle and chunk of the sheets (the
+//      assembly's wake_pair_rule tiers: a far sheet by its lane, near ones by their points, one a lane, contact pieces
+//      by the warp), of the filaments (segment_rule: far, vertex or near) and of the particles (far rule or near
+//      quadtree); the chunks' rows are added in order and the rows summed per slot in a fixed order, then the bordered solve with the factors (no allocation) gives q, mu = C q and mu_w = K q;
 //   3. the loads (step_loads, step.jl:149-163): the gradient route's Cp with the backward difference of mu, the
 //      pressure force and moment, Kutta-Joukowski, and the total vorticity and impulse of every element's blobs;
 //   4. the velocities at the free nodes and particles: V + the body's exact kernels + every wake element as blobs
@@ -2055,7 +2055,7 @@ extern "C" int vp_freewake_step(vp_freewake* fw, vp_freewake_record* rec) {
     {
         RhsArgs ra{};
         ra.na = wake_near_args(fw, o);
-        // mixed: the particles go to the FP32 N-body kernel below; FP64: they stay in the warp kernel
+        // mixed: the particles go to the FP32 N-body kernel below; FP64: to particle_rhs64_kernel
         ra.sheet_G = fw->sheet_G, ra.sheet_ok = fw->sheet_ok, ra.nsh = nsh, ra.nsg = nsg, ra.npart = mixed ? 0 : fw->np;
         ra.seg = fw->seg, ra.part = fw->part;
         ra.pr.rfar = fw->rule[R_FAR], ra.pr.nfar = fw->nrule[R_FAR], ra.pr.rnear = fw->rule[R_NEAR];
