@@ -606,11 +606,10 @@ __device__ __forceinline__ void fwd_point64(const PairCtx& pc, FwdAcc& acc, doub
 
 // the records of a pair (walk_pair by one lane) evaluated by the warp. The buffer of leaves fills across the pair's pieces
 // and is evaluated when full, a rule piece at once, as when the walkers give the pieces to emit_leaf and emit_rule.
-// MIXED: a point is evaluated in FP32 under the guard; those it refuses are queued and evaluated 32 at a time. FP64: the
-// warp takes every nsplit-th round of 32 points, from `split` on.
+// MIXED: a point is evaluated in FP32 under the guard; those it refuses are queued and evaluated 32 at a time.
 template <bool MIXED>
 __device__ __forceinline__ void eval_records(PairCtx& pc, FwdAcc& acc, const PieceRec* rec, int nrec,
-                                             const unsigned* leaf, int split, int nsplit) {
+                                             const unsigned* leaf) {
     WarpSh& sh = *pc.sh;
     const int lane = pc.lane;
     const double areaT = pc.T->area;
@@ -665,7 +664,7 @@ __device__ __forceinline__ void eval_records(PairCtx& pc, FwdAcc& acc, const Pie
         const RulePt* R = pc.a->rule[rid];
         const float4* Rf = pc.a->rulef[rid];
         int nq = 0;
-        for (int i0 = MIXED ? 0 : 32 * split; i0 < tot; i0 += MIXED ? 32 : 32 * nsplit) {
+        for (int i0 = 0; i0 < tot; i0 += 32) {
             const int i = i0 + lane, k = nslot > 1 ? i / n : 0, q = i - k * n, lf = slot0 + k;
             if constexpr (MIXED) {
                 bool need = false;
@@ -749,25 +748,12 @@ __device__ __noinline__ int pair_direct(const NearArgs& a, WarpSh& sh, int t, in
 // walks one pair into records (in the warp's part of recs and leaves), then the warp evaluates the pairs one by one;
 // each block goes to its pair's place in blk. Mixed, 25k wing (1.1M pairs, 1.97G points): 189 ms, 358 ms when the warp
 // walked and evaluated piece by piece.
-//
-// FP64, one system: while there are few pairs for the warps, a pair's rounds of points go to pair_splits warps, each of
-// which writes its part of the block to `parts`; sum_splits_kernel adds them (a self pair's 4,544 points in one warp held
-// an 80-triangle sphere at 1.97 ms, 0.89 so). Mixed sums in FP32, whose order stays.
-constexpr int SPLIT_MAX = 8;
-__host__ __device__ __forceinline__ int pair_splits(long long pairs, long long warps) {
-    const long long n = SPLIT_MAX * warps / (pairs > 0 ? pairs : 1);
-    return int(n < 1 ? 1 : (n > SPLIT_MAX ? SPLIT_MAX : n));
-}
-
 template <bool BATCH, bool MIXED>
 __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs a1, const NearArgs* __restrict__ sys,
-                                                                     PieceRec* recs, unsigned* leaves, int gmax,
-                                                                     double* parts) {
+                                                                     PieceRec* recs, unsigned* leaves, int gmax) {
     __shared__ WarpSh shm[NEAR_WARPS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr bool SPLIT = !BATCH && !MIXED;
-    const int nsplit = SPLIT ? pair_splits((long long)*a1.rest_n, (long long)gridDim.x * NEAR_WARPS) : 1;
-    const long long total = (long long)*a1.rest_n * nsplit;
+    const long long total = (long long)*a1.rest_n;
     const int warp = blockIdx.x * NEAR_WARPS + w;
     recs += size_t(warp) * gmax * REC_MAX;
     leaves += size_t(warp) * gmax * REC_LEAVES;
@@ -798,7 +784,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
         ra.n = ra.nleaf = 0;
         ra.over = false;
         if (lane < cnt) {
-            item = a1.rest_item[SPLIT ? (idx0 + lane) / nsplit : idx0 + lane];
+            item = a1.rest_item[idx0 + lane];
             if (BATCH) sy = a1.rest_sys[idx0 + lane];
             const NearArgs& a = BATCH ? sys[sy] : a1;
             const int g = int(item >> REST_SHIFT), t = g >> 1;
@@ -825,13 +811,9 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
             const long long p = (long long)(it & ((1ull << REST_SHIFT) - 1));
             const TriGeo& S = wake ? a.wtri[sq] : a.tri[sq];
             double* out = a.blk[wake ? 1 : 0] + size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B);
-            const int split = SPLIT ? int((idx0 + q) % nsplit) : 0;
-            if (SPLIT && nsplit > 1) out = parts + size_t(idx0 + q) * BLK_B;
             pc.npts = 0;
             pc.n64 = 0;
-            if (over && split > 0) {
-                if (lane < (wake ? BLK_W : BLK_B)) out[lane] = 0.0;
-            } else if (over) {
+            if (over) {
                 long long np, n64;
                 tq = pair_direct(a, shm[w], t, sq, wake, out, &np, &n64);
                 pc.npts = np;
@@ -842,37 +824,17 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
                 setup_tri_source(pc, S);
                 pc.side = (!wake && sq == t) ? 1 : 0;
                 FwdAcc acc = {};
-                eval_records<MIXED>(pc, acc, recs + q * REC_MAX, nrec, leaves + q * REC_LEAVES, split, nsplit);
+                eval_records<MIXED>(pc, acc, recs + q * REC_MAX, nrec, leaves + q * REC_LEAVES);
                 pair_block_out(pc, acc, S, out, !wake);
             }
-            if (split == 0) {
-                P[tq] += 1;
-                Q[tq] += pc.npts;
-                Q64 += pc.n64;
-            }
+            P[tq] += 1;
+            Q[tq] += pc.npts;
+            Q64 += pc.n64;
             if (BATCH) flush(a);
         }
         __syncwarp();
     }
     if (!BATCH) flush(a1);
-}
-
-// the blocks of split pairs: the parts added in order (warps: near_kernel_pairs')
-__global__ void sum_splits_kernel(NearArgs a, long long warps, const double* __restrict__ parts) {
-    const long long np = (long long)*a.rest_n;
-    const int nsplit = pair_splits(np, warps);
-    if (nsplit == 1) return;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < np * BLK_B; i += (long long)gridDim.x * blockDim.x) {
-        const long long e = i / BLK_B;
-        const int k = int(i - e * BLK_B);
-        const unsigned long long item = a.rest_item[e];
-        const bool wake = (int(item >> REST_SHIFT) & 1) != 0;
-        const long long p = (long long)(item & ((1ull << REST_SHIFT) - 1));
-        if (wake && k >= BLK_W) continue;
-        double v = 0.0;
-        for (int c = 0; c < nsplit; ++c) v += parts[size_t(e * nsplit + c) * BLK_B + k];
-        a.blk[wake ? 1 : 0][size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B) + k] = v;
-    }
 }
 
 // one far tip filament of test triangle T, summed by one lane: segment_block (assemble.jl:312-321) with the far rule
@@ -1413,8 +1375,6 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
     if ((r = dl.alloc(ctx, &d_recs, size_t(npb) * NEAR_WARPS * gmax * REC_MAX)) ||
         (r = dl.alloc(ctx, &d_leaves, size_t(npb) * NEAR_WARPS * gmax * REC_LEAVES)))
         return r;
-    double* d_parts = nullptr;
-    if (!BATCH && !jobs[0]->ps.mixed && (r = dl.alloc(ctx, &d_parts, size_t(SPLIT_MAX) * npb * NEAR_WARPS * BLK_B))) return r;
     for (auto& pass : passes) {
         // the systems' places in the workspace, the work lists: all test triangles, then all rows
         std::vector<NearArgs> args(nsys);
@@ -1463,12 +1423,8 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         }
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR_PAIRS);
-        pairs<<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, d_recs, d_leaves, gmax, d_parts);
+        pairs<<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, d_recs, d_leaves, gmax);
         ctx->launches++;
-        if (d_parts) {
-            sum_splits_kernel<<<ctx->nsm, 256, 0, ctx->stream>>>(a1, (long long)npb * NEAR_WARPS, d_parts);
-            ctx->launches++;
-        }
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR);
         near_kernel_gather<BATCH><<<nrows, GATHER_NT, 0, ctx->stream>>>(a1, d_args, d_work + ntests);
