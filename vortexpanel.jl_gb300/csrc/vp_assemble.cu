@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
             ra.rec = recs + lane * REC_MAX;
             ra.leaf = leaves + lane * REC_LEAVES;
             ra.dep = ra.moves = false;
-            tier = walk_pair(wc, ra, t, s, wake ? a.wtri[s] : a.tri[s], wake);
+            if (MIXED || wake || s != t) tier = walk_pair(wc, ra, t, s, wake ? a.wtri[s] : a.tri[s], wake);
         }
         __syncwarp();
         for (int q = 0; q < cnt; ++q) {
@@ -809,6 +809,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
             const int g = int(it >> REST_SHIFT), t = g >> 1;
             const bool wake = (g & 1) != 0;
             const long long p = (long long)(it & ((1ull << REST_SHIFT) - 1));
+            if (!MIXED && !wake && sq == t) continue;  // near_kernel_self64's
             const TriGeo& S = wake ? a.wtri[sq] : a.tri[sq];
             double* out = a.blk[wake ? 1 : 0] + size_t(p - a.blk0[wake ? 1 : 0]) * (wake ? BLK_W : BLK_B);
             pc.npts = 0;
@@ -835,6 +836,65 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
         __syncwarp();
     }
     if (!BATCH) flush(a1);
+}
+
+// The self pairs in FP64, a CTA a test triangle: the rule's points over its warps, whose sums are added in warp order (one
+// warp took the 4,500 points in 142 rounds, which held an 80-triangle sphere at 1.97 ms: 1.19 so, 9.1 -> 8.4 ms on a 1,280-triangle one). Every
+// system and batch takes them so, as their sums' order shows in the last bits. Mixed sums in FP32, whose order stays.
+constexpr int SELF_WARPS = 8;
+template <bool BATCH>
+__global__ void __launch_bounds__(32 * SELF_WARPS) near_kernel_self64(NearArgs a1, const NearArgs* __restrict__ sys,
+                                                                    const int2* __restrict__ work) {
+    __shared__ WarpSh shm;
+    __shared__ double s_P[SELF_WARPS][9];
+    const int2 wk = work[blockIdx.x];
+    const NearArgs& a = BATCH ? sys[wk.x] : a1;
+    const int t = wk.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const TriGeo& T = a.tri[t];
+    PairCtx pc;
+    pc.a = &a;
+    pc.T = &T;
+    pc.sh = &shm;
+    pc.lane = lane;
+    pc.kind = 0;
+    pc.side = 1;
+    pc.fp32 = 0;
+    if (w == 0) setup_tri_source(pc, T);
+    __syncthreads();
+    const int n = a.nrule[R_SELF];
+    FwdAcc acc = {};
+    for (int i = threadIdx.x; i < n; i += 32 * SELF_WARPS) {
+        const RulePt m = a.rule[R_SELF][i];
+        fwd_point64<false>(pc, acc, m.l0, m.l1, m.l2, m.w * T.area);
+    }
+    for (int k = 0; k < 3; ++k) {
+        const v3<double> P = mk3(warp_sum(acc.P[k].x), warp_sum(acc.P[k].y), warp_sum(acc.P[k].z));
+        if (lane == 0) {
+            s_P[w][3 * k] = P.x;
+            s_P[w][3 * k + 1] = P.y;
+            s_P[w][3 * k + 2] = P.z;
+        }
+    }
+    __syncthreads();
+    if (w > 0) return;
+    // the pair's place: the test triangle among its own sources, which are in order
+    long long lo = a.nf_ptr[t], hi = a.nf_ptr[t + 1];
+    while (hi - lo > 1) {
+        const long long mid = (lo + hi) >> 1;
+        if (a.nf_src[mid] <= t) lo = mid;
+        else hi = mid;
+    }
+    acc = {};
+    if (lane == 0)
+        for (int k = 0; k < 3; ++k)
+            for (int c = 0; c < SELF_WARPS; ++c) acc.P[k] += mk3(s_P[c][3 * k], s_P[c][3 * k + 1], s_P[c][3 * k + 2]);
+    __syncwarp();
+    pair_block_out(pc, acc, T, a.blk[0] + size_t(lo - a.blk0[0]) * BLK_B, true);
+    if (lane == 0) {
+        atomicAdd(a.stats + TIER_SELF, 1ull);
+        atomicAdd(a.stats + 6 + TIER_SELF, (unsigned long long)n);
+        atomicAdd(a.stats + 12, (unsigned long long)n);
+    }
 }
 
 // one far tip filament of test triangle T, summed by one lane: segment_block (assemble.jl:312-321) with the far rule
@@ -1423,6 +1483,10 @@ int near_launch(vp_ctx* ctx, const std::vector<AsmJob*>& jobs, DevList& dl) {
         }
         vp_phase_end(ctx);
         vp_phase_begin(ctx, PH_NEAR_PAIRS);
+        if (!jobs[0]->ps.mixed) {
+            near_kernel_self64<BATCH><<<ntests, 32 * SELF_WARPS, 0, ctx->stream>>>(a1, d_args, d_work);
+            ctx->launches++;
+        }
         pairs<<<npb, 32 * NEAR_WARPS, 0, ctx->stream>>>(a1, d_args, d_recs, d_leaves, gmax);
         ctx->launches++;
         vp_phase_end(ctx);
