@@ -839,7 +839,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
 }
 
 // The self pairs in FP64, a CTA a test triangle: the rule's points over its warps, whose sums are added in warp order (one
-// warp took the 4,500 points in 142 rounds, which held an 80-triangle sphere at 1.97 ms: 1.19 so, 9.1 -> 8.4 ms on a 1,280-triangle one). Every
+// warp took the 4,500 points in 142 rounds, which held an 80-triangle sphere at 1.97 ms: 1.19
+// so, 9.1 -> 8.4 ms on a 1,280-triangle one). Every
 // system and batch takes them so, as their sums' order shows in the last bits. Mixed sums in FP32, whose order stays.
 constexpr int SELF_WARPS = 8;
 template <bool BATCH>

@@ -134,8 +134,8 @@ constexpr long long LEAF_WAIT_LIMIT = 1LL << 20;  // tries of a bounded wait
 // that chain: each warp finds its candidate and writes that row to shared memory, one warp picks the CTA's and sends it
 // to every CTA's shared memory, where an mbarrier counts the bytes; all threads wait for the candidates on their own
 // mbarrier, pick the pivot, swap and eliminate. (With the panel in shared memory, reads from the other CTAs after a
-// cluster barrier and three more block barriers a column took 7 us; with the candidates pushed and a cluster barrier
-// 2.3 us.) A panel that one CTA holds needs block barriers only. FP64 multiplies by the pivot's reciprocal, computed once
+// cluster barrier and three more block barriers a column took 7 us; now 2.9 us at 8 CTAs and 4.0 at 16, in a launch list of
+// the 12.8k mixed system.) A panel that one CTA holds needs block barriers only. FP64 multiplies by the pivot's reciprocal, computed once
 // by the CTA that sends it: a division per row is ten FP64 instructions of each warp.
 template <class T, int W, int RPT, int CL, int NT>
 __global__ void __launch_bounds__(NT)
