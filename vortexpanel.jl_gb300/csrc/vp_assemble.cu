@@ -852,6 +852,15 @@ __global__ void __launch_bounds__(32 * SELF_WARPS) near_kernel_self64(NearArgs a
     const NearArgs& a = BATCH ? sys[wk.x] : a1;
     const int t = wk.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const TriGeo& T = a.tri[t];
+    // the pair's place: the test triangle among its own sources, which are in order; none in an assembly of wake columns only
+    const long long e = a.nf_ptr[t + 1];
+    long long lo = a.nf_ptr[t], hi = e;
+    while (hi - lo > 1) {
+        const long long mid = (lo + hi) >> 1;
+        if (a.nf_src[mid] <= t) lo = mid;
+        else hi = mid;
+    }
+    if (lo >= e || a.nf_src[lo] != t) return;
     PairCtx pc;
     pc.a = &a;
     pc.T = &T;
@@ -878,13 +887,6 @@ __global__ void __launch_bounds__(32 * SELF_WARPS) near_kernel_self64(NearArgs a
     }
     __syncthreads();
     if (w > 0) return;
-    // the pair's place: the test triangle among its own sources, which are in order
-    long long lo = a.nf_ptr[t], hi = a.nf_ptr[t + 1];
-    while (hi - lo > 1) {
-        const long long mid = (lo + hi) >> 1;
-        if (a.nf_src[mid] <= t) lo = mid;
-        else hi = mid;
-    }
     acc = {};
     if (lane == 0)
         for (int k = 0; k < 3; ++k)
