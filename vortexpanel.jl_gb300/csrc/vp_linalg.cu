@@ -1146,8 +1146,22 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
     const cublasOperation_t op = trans ? CUBLAS_OP_T : CUBLAS_OP_N;
     std::vector<double> mx(2 * size_t(nrhs));
     int it = 0;
-    bool conv = false;
+    bool conv = false, lost = false;
     double prev = INFINITY;
+    // columns whose right hand side holds an infinity or NaN: their solutions do too, as in VP_FP64, and the others go on
+    // without them. Looked for once, when a column's numbers are not finite.
+    std::vector<char> skip;
+    auto not_finite = [&](int k) { return !std::isfinite(mx[2 * size_t(k)]) || !std::isfinite(mx[2 * size_t(k) + 1]); };
+    auto find_skipped = [&]() -> int {
+        std::vector<double> m(2 * size_t(nrhs));
+        col_max_kernel<<<nrhs, 512, 0, ctx->stream>>>(n, rhs, rhs, norms);
+        ctx->launches++;
+        VP_CUDA(ctx, vp_d2h(ctx, m.data(), norms, sizeof(double) * 2 * nrhs));
+        VP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        skip.assign(nrhs, 0);
+        for (int k = 0; k < nrhs; ++k) skip[k] = !std::isfinite(m[2 * size_t(k)]);
+        return VP_OK;
+    };
     for (it = 1; it <= 30; ++it) {
         VP_CUDA(ctx, cudaMemcpyAsync(res, rhs, sizeof(double) * tot, cudaMemcpyDeviceToDevice, ctx->stream));
         // one product on the tensor cores (nine-digit FP64) from RES_TC columns on, below and for M' a matrix-vector product
@@ -1167,10 +1181,16 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
         bool ok = true;
         double worst = 0;
         for (int k = 0; k < nrhs; ++k) {
+            if (not_finite(k)) {
+                if (skip.empty() && (r = find_skipped())) { cleanup(); return r; }
+                if (skip[k]) continue;
+                lost = true;  // an overflow of the FP32 factors or solves: more steps do not bring it back
+            }
             const double ratio = mx[2 * size_t(k)] / (norm1 * mx[2 * size_t(k) + 1] + 1e-300);
             worst = std::max(worst, ratio);
-            if (ratio > 4 * std::sqrt(double(n)) * 1.1102230246251565e-16) ok = false;
+            if (!(ratio <= 4 * std::sqrt(double(n)) * 1.1102230246251565e-16)) ok = false;
         }
+        if (lost) break;
         if (ok) {
             conv = true;
             break;
@@ -1185,6 +1205,7 @@ static int solve_core(vp_ctx* ctx, const vp_factor* F, int nrhs, double* x, bool
     }
     cleanup();
     if (iters) *iters = it;
+    if (lost) return vp_fail(ctx, VP_ERR_NOCONV, "iterative refinement: a solution overflowed FP32");
     if (!conv) {
         // stagnated at a level the FP32 factors cannot improve: accept when already tiny, else report
         return vp_fail(ctx, VP_ERR_NOCONV, "iterative refinement did not converge");
