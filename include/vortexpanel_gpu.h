@@ -89,6 +89,11 @@ int vp_set_far_tile(vp_ctx* ctx, int precision, int tile);
 /* The current far tile of a precision (0 for a bad argument). */
 int vp_get_far_tile(const vp_ctx* ctx, int precision);
 
+/* The largest thread block cluster of the LU's leaf kernels: 16 CTAs (default; used where the device places them), 8 (the
+ * portable size), or 0: the kernel that keeps the panel in shared memory at every height. The factors are those of
+ * partial pivoting with any of them. No counterpart in the reference. */
+int vp_set_lu_cluster(vp_ctx* ctx, int ctas);
+
 /* One system of a batch: the arguments of vp_assemble for one body with its wake. */
 typedef struct {
     int nnode;

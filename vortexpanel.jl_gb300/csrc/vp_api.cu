@@ -161,6 +161,13 @@ int vp_get_far_tile(const vp_ctx* ctx, int precision) {
     return ctx->far_tile[precision];
 }
 
+int vp_set_lu_cluster(vp_ctx* ctx, int ctas) {
+    if (!ctx) return VP_ERR_ARG;
+    if (ctas != 0 && ctas != 8 && ctas != 16) return vp_fail(ctx, VP_ERR_ARG, "LU leaf cluster: 0, 8 or 16 CTAs");
+    ctx->lu_cluster = ctas;
+    return VP_OK;
+}
+
 int vp_assemble_batch(vp_ctx* ctx, const vp_assembly_options* opts, int nsys, const vp_assembly_input* in,
                       vp_system** out, vp_assembly_stats* stats) {
     if (!ctx) return VP_ERR_ARG;

@@ -56,6 +56,10 @@ struct vp_ctx {
     TcWork tc;
     // test triangles per far-tier tile, per precision (vp_precision): set by vp_set_far_tile (the autotuner's choice)
     int far_tile[2] = {4, 8};
+    // the largest cluster of the LU's leaf kernels (vp_set_lu_cluster), and whether the device places clusters of 16 CTAs,
+    // per precision (FP64, FP32) and leaf of 16, 8, 4 columns: -1 not asked yet
+    int lu_cluster = 16;
+    signed char leaf16[2][3] = {{-1, -1, -1}, {-1, -1, -1}};
 };
 
 // record the start/end of a phase on the context's stream; vp_phase_flush() accumulates the elapsed times

@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(NT)
     if (CL > 1) cl.sync();  // no CTA leaves while another may still write its shared memory
 }
 
-// The LU leaf for panels too tall for the cluster's registers (over 16,384 rows): the panel in shared memory.
+// The LU leaf for panels too tall for the cluster's registers (over 16,384 rows, or where only clusters of 8 CTAs are to be
+// had): the panel in shared memory.
 template <class T, int W>
 __global__ void __cluster_dims__(LU_CL, 1, 1) __launch_bounds__(LU_THREADS)
     lu_leaf_tall_kernel(T* __restrict__ A, long long lda, int c0, int m, int w, int R, int* __restrict__ ipiv,
@@ -624,13 +625,39 @@ int launch_leaf_cl(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, 
     return VP_OK;
 }
 
+// whether the device places clusters of 16 CTAs (above the portable 8: 16 free SMs of one GPC) of this leaf kernel
+template <class T, int W>
+bool leaf16_fits(vp_ctx* ctx) {
+    signed char& fits = ctx->leaf16[sizeof(T) == 4][W == 16 ? 0 : (W == 8 ? 1 : 2)];
+    if (fits < 0) {
+        auto kern = lu_leaf_kernel<T, W, leaf_rpt_max<T, W>, 16, LU_THREADS>;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(LU_THREADS);
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 16;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
+        if (!ok) cudaGetLastError();  // the device does not take the size: not an error of the factorization
+        fits = ok && n > 0;
+    }
+    return fits != 0;
+}
+
 // The smallest cluster that holds the panel, as fewer CTAs exchange faster: FP32, one CTA up to 1,024 rows, 8 CTAs up to
 // 8,192, 16 (the largest) up to 16,384; FP64, whose elimination is bound by each SM's two FP64 operations a clock, one CTA
-// up to 256 rows, 8 up to 2,048, then 16; the tall kernel beyond.
+// up to 256 rows, 8 up to 2,048, then 16; the tall kernel beyond, and where clusters of 16 do not fit the device or are not
+// allowed: 131 KB of shared memory a CTA at the most rows that 16 CTAs take, for every width.
 template <class T, int W>
 int launch_leaf(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int* info) {
     if (w < 1 || w > W || w > m) return vp_fail(ctx, VP_ERR_ARG, "LU leaf width out of range");
     constexpr int RM = leaf_rpt_max<T, W>;
+    if (ctx->lu_cluster < LU_CL) return launch_leaf_tall<T, W>(ctx, A, lda, c0, m, w, ipiv, info);
     if constexpr (sizeof(T) == 4) {
         if (m <= 1024) return launch_leaf_cl<T, W, 1, 1, 1024>(ctx, A, lda, c0, m, w, ipiv, info);
         if (m <= 8 * RM * LU_THREADS) return launch_leaf_cl<T, W, RM, 8, LU_THREADS>(ctx, A, lda, c0, m, w, ipiv, info);
@@ -638,7 +665,8 @@ int launch_leaf(vp_ctx* ctx, T* A, int lda, int c0, int m, int w, int* ipiv, int
         if (m <= 256) return launch_leaf_cl<T, W, 1, 1, 256>(ctx, A, lda, c0, m, w, ipiv, info);
         if (m <= 2048) return launch_leaf_cl<T, W, 1, 8, 256>(ctx, A, lda, c0, m, w, ipiv, info);
     }
-    if (m <= 16 * RM * LU_THREADS) return launch_leaf_cl<T, W, RM, 16, LU_THREADS>(ctx, A, lda, c0, m, w, ipiv, info);
+    if (m <= 16 * RM * LU_THREADS && ctx->lu_cluster >= 16 && leaf16_fits<T, W>(ctx))
+        return launch_leaf_cl<T, W, RM, 16, LU_THREADS>(ctx, A, lda, c0, m, w, ipiv, info);
     return launch_leaf_tall<T, W>(ctx, A, lda, c0, m, w, ipiv, info);
 }
 

@@ -211,6 +211,10 @@ set_far_tile(ctx::Context, precision::Symbol, tile::Integer) = check(ctx.h, ccal
 far_tile(ctx::Context, precision::Symbol) = ccall((:vp_get_far_tile, LIB), Cint, (Ptr{Cvoid}, Cint), ctx.h,
     precision == :mixed ? 1 : 0)
 
+# the largest cluster of the LU's leaf kernels: 16 (default), 8, or 0 (the panel in shared memory)
+set_lu_cluster(ctx::Context, ctas::Integer) = check(ctx.h, ccall((:vp_set_lu_cluster, LIB), Cint, (Ptr{Cvoid}, Cint),
+    ctx.h, ctas))
+
 # ---- the bordered solve -----------------------------------------------------------------------------------------------
 
 mutable struct GalerkinFactorization

@@ -77,6 +77,7 @@ SIGNATURES = [
       ctypes.POINTER(vp_assembly_stats)]),
     ("vp_set_far_tile", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int]),
     ("vp_get_far_tile", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
+    ("vp_set_lu_cluster", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     ("vp_assemble_batch", ctypes.c_int,
      [ctypes.c_void_p, ctypes.POINTER(vp_assembly_options), ctypes.c_int, ctypes.POINTER(vp_assembly_input),
       ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(vp_assembly_stats)]),
