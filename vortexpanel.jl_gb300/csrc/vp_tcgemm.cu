@@ -280,7 +280,7 @@ constexpr int TD_STAGE_BYTES = TD_PAIRS * (TD_A_BYTES + TD_B_BYTES);  // 110 KB
 constexpr int TD_SMEM = TD_STAGES * TD_STAGE_BYTES + 1024;
 constexpr int TD_KMAX = 448;       // exact integer sums in FP32
 constexpr int TD_TMEM_COLS = 512;  // nine accumulators of 48 columns
-constexpr int TD_EMIN = -900;      // exponents below are taken as this (the values' digits vanish)
+constexpr int TD_EMID = 400;       // scales within 2^+-this combine in one factor
 
 // the largest exponent field of every row of A (m x k, column-major), or (rows = 0) of every column: into ex (zeroed).
 // Exponent fields order as the numbers; 2047 marks an infinity or NaN.
@@ -309,11 +309,20 @@ __global__ void col_exp_kernel(int k, int n, const double* __restrict__ B, int l
 
 // 2^e for the exponents of normal numbers
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-__device__ __forceinline__ int scale_exp(int field) { return max(field - 1022, TD_EMIN); }  // |x| < 2^this
+// |x| < 2^this for every x of the field (-1021 to 1024; 1025 for an infinity or NaN)
+__device__ __forceinline__ int scale_exp(int field) { return max(field, 1) - 1022; }
+// the scale 2^e of a row or column, or NaN (nan: it holds an infinity or NaN); 1 outside 2^+-TD_EMID, where the epilogue takes
+// the exponents: as factors cut at 2^-900, they lost the digits of smaller entries
+__device__ __forceinline__ double scale_of(int e, bool nan) {
+    return nan ? __longlong_as_double(0x7ff8000000000000LL) : (abs(e) <= TD_EMID ? pow2(e) : 1.0);
+}
+
+// x 2^(62 - e) where the factor is no normal number (out of line: the digit kernels are bound by their instructions)
+__device__ __noinline__ double digits_tiny(double x, int e) { return (x * pow2(1000)) * pow2(62 - 1000 - e); }
 
 // the digits of x, |x| < 2^e, to dst[q * plane + par * 32], digit 2 q + par
 __device__ __forceinline__ void put_digits(double x, int e, __nv_bfloat16* dst, size_t plane) {
-    long long u = __double2ll_rn(x * pow2(62 - e));
+    long long u = __double2ll_rn(e < 62 - 1000 ? digits_tiny(x, e) : x * pow2(62 - e));
 #pragma unroll
     for (int p = TD_DIGITS - 1; p >= 0; --p) {
         const int d = p ? (int(u + 64) & 127) - 64 : int(u);
@@ -380,6 +389,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __shared__ uint32_t tmem_holder;
     __shared__ int s_fail;
     __shared__ double s_scale[TD_BN];
+    __shared__ int s_exp[TD_BN];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TD_BN;
@@ -395,10 +405,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // the columns' scales: 2^(e - 68), so that a row's 2^e makes C's; NaN for a column with an infinity or NaN
+    // the columns' scales 2^(e - 68), which a row's 2^e makes C's
+    bool cfar = false;
     for (int j = threadIdx.x; j < TD_BN; j += TC_THREADS) {
-        const int f = n0 + j < n ? exB[n0 + j] : 0;
-        s_scale[j] = f == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : pow2(scale_exp(f) - 68);
+        const int f = n0 + j < n ? exB[n0 + j] : 1022, e = scale_exp(f) - 68;
+        s_exp[j] = e;
+        s_scale[j] = scale_of(e, f == 2047);
+        cfar |= f < 2047 && abs(e) > TD_EMID;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
@@ -407,7 +420,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    cfar = __syncthreads_or(cfar) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_holder;
 
@@ -452,32 +465,48 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __syncthreads();
     if (done && !s_fail) {
         const int row = m0 + warp * 32 + lane;
-        const int f = row < m ? exA[row] : 0;
-        const double sr = f == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : pow2(scale_exp(f));
+        const int f = row < m ? exA[row] : 1022, er = scale_exp(f);
+        const double sr = scale_of(er, f == 2047);
+        const bool far = cfar || (f < 2047 && abs(er) > TD_EMID);
         for (int c0 = 0; c0 < TD_BN; c0 += 8) {
             uint32_t v[TD_DIGITS][8];
             const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16) + uint32_t(c0);
 #pragma unroll
             for (int g = 0; g < TD_DIGITS; ++g) tmem_ld8(taddr + uint32_t(g * TD_BN), v[g]);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < m)
+            auto value = [&](int j) {
+                int t[4];  // groups 2 h and 2 h + 1: below 2^31 (group g is at most (g + 1) 448 2^12)
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    t[h] = __float2int_rn(__uint_as_float(v[2 * h][j])) * 128 + __float2int_rn(__uint_as_float(v[2 * h + 1][j]));
+                double x = double(t[0]);
+                x = fma(x, 16384.0, double(t[1]));
+                x = fma(x, 16384.0, double(t[2]));
+                x = fma(x, 16384.0, double(t[3]));
+                return fma(x, 128.0, double(__uint_as_float(v[8][j])));
+            };
+            if (row < m && !far) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int col = n0 + c0 + j;
-                    int t[4];  // groups 2 h and 2 h + 1: below 2^31 (group g is at most (g + 1) 448 2^12)
-#pragma unroll
-                    for (int h = 0; h < 4; ++h)
-                        t[h] = __float2int_rn(__uint_as_float(v[2 * h][j])) * 128 + __float2int_rn(__uint_as_float(v[2 * h + 1][j]));
-                    double x = double(t[0]);
-                    x = fma(x, 16384.0, double(t[1]));
-                    x = fma(x, 16384.0, double(t[2]));
-                    x = fma(x, 16384.0, double(t[3]));
-                    x = fma(x, 128.0, double(__uint_as_float(v[8][j])));
+                    const double x = value(j);
                     if (col < n) {
                         double* c = C + size_t(col) * ldc + row;
                         *c = fma(-x, sr * s_scale[c0 + j], *c);
                     }
                 }
+            } else if (row < m) {  // 2^(row + column) in two factors
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int col = n0 + c0 + j, e = er + s_exp[c0 + j], h = max(e / 2, -1022);
+                    const double x = value(j), s = sr * s_scale[c0 + j];
+                    if (col < n) {
+                        double* c = C + size_t(col) * ldc + row;
+                        *c = isnan(s) ? s : fma(-(x * pow2(h)), pow2(max(e - h, -1022)), *c);
+                    }
+                }
+            }
+            __syncwarp();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
