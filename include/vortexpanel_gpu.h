@@ -144,7 +144,8 @@ int vp_factorize(vp_ctx* ctx, const vp_system* sys, int precision, int nq, const
 
 /* solve_galerkin(F, b) (src/assembly/solve.jl:95-99) for nrhs right hand sides over the slots:
  *   b (nslot x nrhs, column-major), q (nq x nrhs, column-major), lambda (nbody x nrhs, column-major; may be NULL).
- * With VP_MIXED factors the solution is refined to FP64 accuracy with FP64 residuals of the bordered matrix. */
+ * With VP_MIXED factors the solution is refined to FP64 accuracy with FP64 residuals of the bordered matrix; a finite
+ * right hand side whose solution overflows FP32 is VP_ERR_NOCONV, one that is not finite gives a column that is not. */
 int vp_solve(vp_ctx* ctx, const vp_factor* F, int nrhs, const double* b, double* q, double* lambda);
 
 /* solve_galerkin(dm, A, b; W) (src/assembly/solve.jl:51-59) for the system's own b: q (nq), lambda (nbody),

@@ -207,17 +207,6 @@ __device__ inline void normal_area_grad(const v3<T>* v, v3<T> nbar, T Abar, v3<T
     g[0] -= ubar + w2bar;
 }
 
-// derivative of (V · area vector) with weight c of triangle v: the area vector is nA / 2
-template <class T>
-__device__ inline void area_vector_grad(const v3<T>* v, v3<T> V, T c, v3<T>* g) {
-    v3<T> u = v[1] - v[0], w2 = v[2] - v[0];
-    v3<T> nAbar = (T(0.5) * c) * V;
-    v3<T> ubar = cross(w2, nAbar), w2bar = cross(nAbar, u);
-    g[1] += ubar;
-    g[2] += w2bar;
-    g[0] -= ubar + w2bar;
-}
-
 // The derivative of a source's sums a with respect to its corners v, added to gout: through the offsets to the
 // corners and the centroid, the edge normals, edge lengths, unit normal and area (the shape, as SourceTriangle builds
 // it: src/kernels/source_triangle.jl:8-26), through Gamma_S = -sum_b mu_b e_b / 2A (e_b the edge opposite corner b)
@@ -320,16 +309,4 @@ __device__ inline void test_adj_grad(const v3<T>* xT, const v3<T>* Xg, v3<T> U, 
     T AT = vnorm(nA) / T(2);
     for (int k = 0; k < 3; ++k) gT[k] += Xg[k];
     normal_area_grad(xT, U, f / AT, gT);
-}
-
-// One pair's derivatives from its sums a: the test triangle's corners (gT), the source's (gS) and d/dalpha (dal),
-// for a source sheet with corner values mu and Gamma_S = gam, source strength sig (body sources: with_sigma).
-template <class T>
-__device__ inline void adj_pair_grad(const v3<T>* xT, const v3<T>* xS, const AdjSums<T>& a, v3<T> m, v3<T> gam, T sig,
-                                     const T* mu, bool with_sigma, v3<T> V, v3<T> dV, v3<T>* gT, v3<T>* gS, T* dal) {
-    v3<T> nT = cross(xT[1] - xT[0], xT[2] - xT[0]);
-    nT = nT / vnorm(nT);
-    test_adj_grad(xT, a.Xg, cross(gam, a.Q) + sig * a.Q, dot(a.Q, m), gT);
-    SrcAdj<T> s = src_of_pair(xS, a, m, nT);
-    src_adj_grad(xS, s, mu, with_sigma, V, dV, gS, dal);
 }

@@ -533,9 +533,10 @@ __device__ __forceinline__ void near_lanes_body(const NearArgs& a, const int t, 
 }
 
 // the kernels of the non-far tiers take one system's arguments by value, or (BATCH) those of system work[i].x from sys.
-// MIXED or FP64 by template: with both paths in one kernel the mixed one ran at 216 registers instead of 158 (near
-// phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles). Ten CTAs an SM: 106 ms on a 25k wing, 110 with
-// twelve (spills), 127 with eight, 135 with sixteen.
+// MIXED or FP64 by template: with both paths in one kernel the mixed one ran at 216 registers instead of 168 (near
+// phase 64 ms instead of 50 on five wings of 900 to 4,000 triangles, before the leaf table). Ten CTAs an SM (168 registers,
+// at most 96 bytes of them spilled in mixed precision): near phase 91 ms on a 25k wing; before the leaf table 106, 110 with
+// twelve, 127 with eight, 135 with sixteen.
 template <bool BATCH, bool MIXED>
 __global__ void __launch_bounds__(32, 10) near_kernel_lanes(NearArgs a, const NearArgs* __restrict__ sys,
                                                                   const int2* __restrict__ work) {
@@ -746,7 +747,7 @@ __device__ __noinline__ int pair_direct(const NearArgs& a, WarpSh& sh, int t, in
 // The self, touching and contact pairs: a persistent grid whose warps take the next pairs of the list from a counter, so
 // that test triangles with many contact pairs (thin panels at a sharp trailing edge) do not hold a launch. Each lane
 // walks one pair into records (in the warp's part of recs and leaves), then the warp evaluates the pairs one by one;
-// each block goes to its pair's place in blk. Mixed, 25k wing (1.1M pairs, 1.97G points): 189 ms, 358 ms when the warp
+// each block goes to its pair's place in blk. Mixed, 25k wing (1.1M pairs, 1.97G points): 150 ms, 358 ms when the warp
 // walked and evaluated piece by piece.
 template <bool BATCH, bool MIXED>
 __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs a1, const NearArgs* __restrict__ sys,
@@ -839,9 +840,9 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS, 3) near_kernel_pairs(NearArgs
 }
 
 // The self pairs in FP64, a CTA a test triangle: the rule's points over its warps, whose sums are added in warp order (one
-// warp took the 4,500 points in 142 rounds, which held an 80-triangle sphere at 1.97 ms: 1.19
-// so, 9.1 -> 8.4 ms on a 1,280-triangle one). Every
-// system and batch takes them so, as their sums' order shows in the last bits. Mixed sums in FP32, whose order stays.
+// warp took the 4,500 points in 142 rounds, which held an 80-triangle sphere at 1.97 ms: 1.19 so, 9.1 -> 8.4 ms on a
+// 1,280-triangle one). Every system and batch takes them so, as their sums' order shows in the last bits. Mixed sums in
+// FP32, whose order stays.
 constexpr int SELF_WARPS = 8;
 template <bool BATCH>
 __global__ void __launch_bounds__(32 * SELF_WARPS) near_kernel_self64(NearArgs a1, const NearArgs* __restrict__ sys,

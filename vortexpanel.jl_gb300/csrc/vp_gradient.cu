@@ -341,7 +341,7 @@ struct AdjMulti {
 
 struct AdjChunkSh {
     NearPlanSh pl;
-    float accf[ADJ_MAX][32][NSUM];  // per adjoint vector and pair: the sums of the pair's points
+    float accf[ADJ_MAX][32][NSUM];  // per adjoint vector and pair: the sums of the pair's points, FP32 in both precisions
     double m64[32][3];              // the pair's direction m
     int off[33];                    // points before each pair
     int qp[64], qk[64];             // queued FP64 points: pair, point within the pair

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(NT)
         const T* piv = s_cand[buf][pr].row;
         // 4. swap rows j and p, eliminate below the pivot (l = 0 leaves a row alone)
         const T pj = piv[j], rj = s_cand[buf][pr].rcp;
-        const bool mul = sizeof(T) == 8 && fabs(pj) > T(1e-300);
+        const bool mul = sizeof(T) == 8 && fabs(double(pj)) > 1e-300;
         T l[RPT];
 #pragma unroll
         for (int r = 0; r < RPT; ++r) {

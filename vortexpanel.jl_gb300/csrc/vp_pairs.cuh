@@ -382,7 +382,6 @@ struct Bary9 {
 
 struct WarpSh {
     double E[27];          // E[9k+3a+z]: x_T,k - v_S,a (filament: x_T,k - a, x_T,k - b)
-    double D[9];           // x_T,k - c_S
     double Sd[9], Sn[3], Snu[9], Slen[3], Sarea, Sdiam;
     float E32[27];         // E in FP32
     float D32[9];          // D in FP32
@@ -1779,9 +1778,8 @@ __device__ void setup_tri_source(PairCtx& pc, const TriGeo& S) {
         sh.E32[i] = float(e);
     }
     if (i < 9) {
-        const double d = T.x[i] - S.c[i % 3], sd = S.x[i] - S.c[i % 3];
-        sh.D[i] = d;
-        sh.D32[i] = float(d);
+        const double sd = S.x[i] - S.c[i % 3];
+        sh.D32[i] = float(T.x[i] - S.c[i % 3]);
         sh.Sd[i] = sd;
         sh.Sdf[i] = float(sd);
         sh.Snu[i] = S.nu[i];

@@ -594,7 +594,7 @@ int tc_reserve(vp_ctx* ctx, size_t elems, size_t nexp) {
 
 }  // namespace
 
-// k >= 64, and enough work: below about 8M multiply-adds the five launches (58 us) take longer than cuBLAS's DGEMM
+// k >= 64, and enough work: below about 16M multiply-adds the five launches (58 us) take longer than cuBLAS's DGEMM
 // (1000 x 64 x 64: 58 against 25 us; 6000 x 64 x 64: 63 against 81; 6000 x 128 x 128: 70 against 226)
 bool vp_tc_gemm64_fits(int m, int n, int k) {
     return m >= TC_BM && n >= TD_BN && k >= 64 && double(m) * n * k >= 1.6e7;
